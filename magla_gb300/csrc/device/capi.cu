@@ -402,7 +402,7 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
                 // mixed path: diagonal block, then its rows below as a GEMM with the block's inverse
                 if constexpr (sizeof(T) == 4) {
                     if (L.kind == Launch::DiagBlock)
-                        k_diag_block<<<L.count, 256, kDiagSmemBytes, st>>>(D.pivot_tasks.as<PanelTask>() + L.begin, sn,
+                        k_diag_block<<<L.count, kDiagThreads, kDiagSmemBytes, st>>>(D.pivot_tasks.as<PanelTask>() + L.begin, sn,
                                                                            panel, diag, F->minv.as<float>(), ctl, stats);
                     else if (F->precision == UCHOL_PRECISION_BF16)
                         k_panel_solve<__nv_bfloat16><<<L.count, 256, kPanelSmemBytes, st>>>(

@@ -184,7 +184,7 @@ int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, 
         stats.upload(pv, st, "check");
         CK(cudaFuncSetAttribute(k_diag_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmemBytes));
         CK(cudaFuncSetAttribute(k_panel_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemBytes));
-        k_diag_block<<<1, 256, kDiagSmemBytes, st>>>(ptask.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<float>(),
+        k_diag_block<<<1, kDiagThreads, kDiagSmemBytes, st>>>(ptask.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<float>(),
                                                       diag.as<double>(), minv.as<float>(), ctl.as<FactorCtl>(),
                                                       stats.as<PivotStats>());
         counted();

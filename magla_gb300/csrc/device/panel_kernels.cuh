@@ -42,7 +42,7 @@ constexpr int kSolveRows = 128;
 // float part: S and X (kDiagMax x kDiagLd each), Wt (kDiagMax x 33), D and D^{-1} in FP32;
 // then the FP64 part: the running diagonal and D (kDiagMax doubles each)
 constexpr size_t kDiagSmemFloats = 2 * kDiagMax * kDiagLd + kDiagMax * 33 + 2 * kDiagMax;
-constexpr size_t kDiagSmemBytes = sizeof(float) * kDiagSmemFloats + sizeof(double) * 2 * kDiagMax;
+constexpr size_t kDiagExactBytes = sizeof(float) * kDiagSmemFloats + sizeof(double) * 2 * kDiagMax;
 static_assert(sizeof(float) * kDiagSmemFloats % sizeof(double) == 0, "the FP64 part is aligned");
 
 // Pivot acceptance of the reference, !(d > tol*scale) -> regularise or reject,
@@ -150,11 +150,12 @@ __device__ __forceinline__ void warp_ldlt32(float* S, float* X, int b0, int bn, 
     }
 }
 
-__global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restrict__ tasks, const SnDev* __restrict__ sn,
-                                                    float* __restrict__ panel, double* __restrict__ diag,
-                                                    float* __restrict__ minv, const FactorCtl* __restrict__ ctlp,
-                                                    PivotStats* st) {
-    extern __shared__ float smem[];
+// The outer block with every elimination step's pivot taken on the FP64 diagonal as it is reached:
+// the form that k_diag_block falls back to.  Threads 0..255 of the CTA; `sync` is their barrier.
+__device__ __forceinline__ void diag_sync256() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __noinline__ void diag_block_exact(const PanelTask& tk, const SnDev& d, float* smem, float* __restrict__ panel,
+                                              double* __restrict__ diag, float* __restrict__ M, float* __restrict__ Md,
+                                              const FactorCtl& ctl, PivotStats* st) {
     float* S = smem;                         // block, row-major (S[r * kDiagLd + c]); L11 after the factorisation
     float* X = S + kDiagMax * kDiagLd;       // L11^{-1}, row-major
     float* Wt = X + kDiagMax * kDiagLd;      // W = L D of the current sub-block's rows below it
@@ -162,9 +163,6 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
     float* sdi = sd + kDiagMax;              // D^{-1}
     double* dg = reinterpret_cast<double*>(smem + kDiagSmemFloats);   // running diagonal, FP64
     double* sd64 = dg + kDiagMax;            // D, FP64
-    const PanelTask tk = tasks[blockIdx.x];
-    const SnDev d = sn[tk.s];
-    const FactorCtl ctl = *ctlp;
     const double thr = ctl.threshold, reg = ctl.regularization;
     const int nb = tk.nb, k0 = tk.j0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -186,7 +184,7 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
         }
     }
     if (tid < kDiagMax) dg[tid] = tid < nb ? (double)P[tid + (long long)tid * d.ldp] : 0.0;
-    __syncthreads();
+    diag_sync256();
 
     PivotAccD acc;
     for (int b0 = 0; b0 < nb; b0 += 32) {
@@ -195,7 +193,7 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
         if (warp == 0)   // Wt is free until step (3): its first 64 floats are the warp's scratch
             warp_ldlt32(S, X, b0, bn, lane, d.first_col + k0 + b0, thr, reg, ctl.allow_regularization, sd, sdi, dg,
                         sd64, acc, Wt);
-        __syncthreads();
+        diag_sync256();
         // (3) rows below the sub-block: w[r][j] = sum_{k<=j} A[r][b0+k] X_bb[j][k], l = w / d_j;
         //     lane j, rows r0 + 8 q (four independent sums per lane)
         const int rb0 = b0 + bn;
@@ -224,7 +222,7 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
                 }
             }
         }
-        __syncthreads();
+        diag_sync256();
         // (3b) the diagonal entries of the rows below, in FP64: d_r -= sum_k d_k L_rk^2, two threads per
         //      row (16 of the sub-block's columns each, four independent sums); reads only the
         //      sub-block's columns of S, which step (4) does not write
@@ -278,7 +276,7 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
                     if (r < nb && c <= r) S[r * kDiagLd + c] -= accu[p][q];
                 }
         }
-        __syncthreads();
+        diag_sync256();
     }
 
     // (5) off-diagonal blocks of X = L11^{-1}: X_ij = -X_ii sum_{j<=k<i} L_ik X_kj, by block diagonals;
@@ -312,7 +310,7 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
 #pragma unroll
                 for (int p = 0; p < 4; ++p) T[pr * 32 * 33 + (rr + 8 * q) * 33 + cc + 8 * p] = t[q][p];
         }
-        __syncthreads();
+        diag_sync256();
         if (active) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -340,21 +338,20 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
                 }
             }
         }
-        __syncthreads();
+        diag_sync256();
     }
 
     // (6) write L11 (unit diagonal), D, and the workspace slot
     for (int c = warp; c < nb; c += 8)
         for (int r = c + lane; r < nb; r += 32) P[r + (long long)c * d.ldp] = r == c ? 1.f : S[r * kDiagLd + c];
     if (tid < nb) diag[d.first_col + k0 + tid] = sd64[tid];
-    float* M = minv + (size_t)tk.slot * kMinvStride;
     for (int idx = tid; idx < kDiagMax * kDiagMax; idx += 256) {
         const int k = idx >> 7, j = idx & (kDiagMax - 1);
         M[idx] = (j < nb && k <= j) ? X[j * kDiagLd + k] : 0.f;
     }
     if (tid < kDiagMax) {
-        M[kDiagMax * kDiagMax + tid] = tid < nb ? sd[tid] : 0.f;
-        M[kDiagMax * kDiagMax + kDiagMax + tid] = tid < nb ? sdi[tid] : 0.f;
+        Md[tid] = tid < nb ? sd[tid] : 0.f;
+        Md[kDiagMax + tid] = tid < nb ? sdi[tid] : 0.f;
     }
     if (tid == 0) acc.flush(st);
     // smallest and largest |d| of the block, by the first warp
@@ -374,6 +371,474 @@ __global__ void __launch_bounds__(256, 1) k_diag_block(const PanelTask* __restri
             atomicMax(&st->max_bits, (unsigned long long)__double_as_longlong(hi));
         }
     }
+}
+
+// ---- k_diag_block: the outer block by one CTA of kDiagThreads threads with a role per warp.
+//
+// What bounds it: a chain of nb pivots on one SM, each needing the one before it.  FP64 instructions take 64
+// cycles each here (issue and latency, however few lanes are active), so a pivot taken wholly in FP64 costs six
+// of them; the chain therefore carries each row's diagonal as an unevaluated sum of two floats (df_sub: about
+// 48 bits, 12 dependent FP32 operations), and the FP64 diagonal D itself is accumulated beside it by three other
+// warps from the same FP32 L (the same sums d_r -= d_k l_rk^2).  The eliminations of the rows below the
+// sub-block and of the identity (which become X^T) follow the chain eight pivots behind in four warps, and the
+// rank-32 updates of the columns beyond the next sub-block run beside the next sub-block's chain.
+//   chain   (1 warp)   LDL^T of the 32 x 32 diagonal sub-block, lane = row
+//   rows    (4 warps)  lane = row: W = A L^-T of the rows below the sub-block, L = W / D, and the same
+//                      elimination of the identity's rows up to the sub-block, which gives X^T (128 rows in all)
+//   fp64    (3 warps)  D: the sub-block's own recursion, then its part of the later rows' diagonals
+//   update  (4 warps)  W L^T of later columns (of the next sub-block's columns together with the rows warps)
+// The chain shares its scheduler (warp number mod 4) with two FP64 warps only, which issue little.
+//
+// A pivot whose two-float value is not clearly above the rejection threshold, or that lost more than 20 bits of
+// its diagonal entry, or that leaves the range in which the low words are normal floats, is not decided here:
+// the whole block is factorised again by diag_block_exact (nothing has been written to the factor by then).
+constexpr int kDiagThreads = 384;
+constexpr int kDiagRowLd = 132;             // S[c * kDiagRowLd + r]: 16-byte aligned columns, conflict-free rows
+constexpr float kDiagKeep = 0x1p-20f;       // smallest pivot / diagonal entry taken by the fast chain
+// floats: S (128 x 132), W (2 x 32 x 132), per-pivot {D hi, D lo, 1/D, -} (128 x 4), pivot column (2 x 64),
+// running diagonal of every row and its limit (3 x 128); then FP64: running diagonal, D (128 each), partial sums (32)
+constexpr size_t kDiagFastFloats = (size_t)kDiagMax * kDiagRowLd + 2 * 32 * kDiagRowLd + 4 * kDiagMax + 128 + 3 * kDiagMax;
+constexpr size_t kDiagFastBytes = sizeof(float) * kDiagFastFloats + sizeof(double) * (2 * kDiagMax + 32);
+static_assert(sizeof(float) * kDiagFastFloats % 16 == 0, "the FP64 part is aligned");
+constexpr size_t kDiagSmemBytes = kDiagFastBytes > kDiagExactBytes ? kDiagFastBytes : kDiagExactBytes;
+
+// (h, l) -= (d, dl) x^2 on unevaluated two-float sums; x^2 and d x^2 are formed exactly (product and remainder).
+__device__ __forceinline__ void df_sub(float& h, float& l, float d, float dl, float x) {
+    const float p = __fmul_rn(x, x), pl = __fmaf_rn(x, x, -p);
+    const float q = __fmul_rn(d, p);
+    const float ql = __fmaf_rn(dl, p, __fmaf_rn(d, pl, __fmaf_rn(d, p, -q)));
+    const float s = __fsub_rn(h, q), bb = __fsub_rn(s, h);
+    const float err = __fsub_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fadd_rn(q, bb));
+    const float lo = __fsub_rn(__fadd_rn(l, err), ql);
+    h = __fadd_rn(s, lo);
+    l = __fsub_rn(lo, __fsub_rn(h, s));
+}
+
+// x^2 as a double, exactly, without FP64 instructions: the 48-bit product of the significands under the
+// doubled exponent (subnormal x counts as zero).
+__device__ __forceinline__ double exact_square(float x) {
+    const unsigned u = __float_as_uint(x), e = (u >> 23) & 255u;
+    const unsigned m = (u & 0x7fffffu) | 0x800000u;
+    const unsigned long long mm = (unsigned long long)m * m;   // [2^46, 2^48)
+    const unsigned top = (unsigned)(mm >> 47);
+    const unsigned long long bits = (mm << (6 - top)) + ((unsigned long long)(2 * e + 768 + top) << 52);
+    return e == 0 ? 0.0 : __longlong_as_double((long long)bits);
+}
+
+// Two FP32 multiply-adds in one instruction (the FP32 pipe's rate is the same; the issue slots saved go to the
+// shared-memory loads beside them).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+template <int kId, int kCount>
+__device__ __forceinline__ void diag_bar_sync() { asm volatile("bar.sync %0, %1;" ::"n"(kId), "n"(kCount) : "memory"); }
+__device__ __forceinline__ void diag_bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+__device__ __forceinline__ void diag_bar_arrive(int id, int count) {
+    __threadfence_block();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+// S[c][r] -= sum_k W[k][r] L[k][c] (L[k][c] = S[b0 + k][c]) for the NR x NC block at (r0, c0) by one warp:
+// lane tile of NR / 4 rows (groups of four, 16 apart) by NC / 8 columns.  Shared-memory bandwidth bounds it (a
+// 16-byte load occupies the SM's load path for four cycles), so the 32 x 32 block's lane tile is 8 x 4.
+template <int NR, int NC>
+__device__ __forceinline__ void diag_update_block(float* S, const float* W, int b0, int r0, int c0, int lane) {
+    constexpr int G = NR / 16, CL = NC / 8;
+    const int r = r0 + 4 * (lane & 3), c = c0 + CL * (lane >> 2);
+    f32x2 acc[CL][2 * G];
+#pragma unroll
+    for (int q = 0; q < CL; ++q)
+#pragma unroll
+        for (int p = 0; p < 2 * G; ++p) acc[q][p] = 0ull;
+    const float* wp = W + r;
+    const float* lp = S + b0 * kDiagRowLd + c;
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+        f32x2 w[2 * G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(wp + k * kDiagRowLd + 16 * g);
+            w[2 * g] = v.x;
+            w[2 * g + 1] = v.y;
+        }
+        float l[CL];
+        if constexpr (CL == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(lp + k * kDiagRowLd);
+            l[0] = v.x;
+            l[1] = v.y;
+            l[2] = v.z;
+            l[3] = v.w;
+        } else {
+            const float2 v = *reinterpret_cast<const float2*>(lp + k * kDiagRowLd);
+            l[0] = v.x;
+            l[1] = v.y;
+        }
+#pragma unroll
+        for (int q = 0; q < CL; ++q)
+#pragma unroll
+            for (int p = 0; p < 2 * G; ++p) acc[q][p] = fma2(w[p], pack2(l[q], l[q]), acc[q][p]);
+    }
+#pragma unroll
+    for (int q = 0; q < CL; ++q)
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            float4* o = reinterpret_cast<float4*>(S + (c + q) * kDiagRowLd + r + 16 * g);
+            float4 v = *o;
+            float x[4];
+            unpack2(acc[q][2 * g], x[0], x[1]);
+            unpack2(acc[q][2 * g + 1], x[2], x[3]);
+            v.x -= x[0];
+            v.y -= x[1];
+            v.z -= x[2];
+            v.w -= x[3];
+            *o = v;
+        }
+}
+
+__device__ __forceinline__ float diag_entry(const f32x2 (&a)[16], int j) {   // j: compile-time
+    float x, y;
+    unpack2(a[j >> 1], x, y);
+    return (j & 1) ? y : x;
+}
+
+struct DiagShared {
+    float *S, *W, *scr, *rh, *rl, *lim;
+    float4* piv;
+    double *dg, *sd64, *part;
+};
+
+// The chain's state (lane = row of the sub-block).
+struct DiagChain {
+    f32x2 a[16];      // this row's entries of columns 4 g + j, two a register pair (shifted down after each quad)
+    float h, l;       // the row's running diagonal
+    float least;
+    bool good;
+};
+// Pivots 4 g .. 4 g + 3 of the chain, NP register pairs of columns (those past the sub-block's end carry nothing).
+// Only the next pivot's column is updated at once; the other columns' updates wait until the next pivot, in the
+// shadow of its reciprocal.  Short loops over quads: unrolled further, instruction fetches bound the chain.
+// a[p] += m * v[p] for the register pairs p in [P0, P1).
+template <int P0, int P1>
+__device__ __forceinline__ void diag_axpy(f32x2 (&a)[16], f32x2 m, const ulonglong2 (&v)[8]) {
+#pragma unroll
+    for (int p = P0; p < P1; ++p) a[p] = fma2(m, (p & 1) ? v[p >> 1].y : v[p >> 1].x, a[p]);
+}
+template <int NP, int KK>
+__device__ __forceinline__ void diag_pivot(const DiagShared& X, DiagChain& C, ulonglong2 (&v)[8], f32x2& m, int b0, int g,
+                                           int lane) {
+    constexpr int kNext = (KK + 1) / 2;        // pair that holds column KK + 1
+    const int k = 4 * g + KK;
+    float* sc = X.scr + 64 * (KK & 1);         // two buffers: one warp barrier per pivot
+    const float ph = __shfl_sync(0xffffffffu, C.h, k), pl = __shfl_sync(0xffffffffu, C.l, k);
+    const float ak = diag_entry(C.a, KK);
+    sc[lane] = ak;
+    const float inv = rcp_approx(ph);
+    if constexpr (KK > 0) diag_axpy<KK / 2 + 1, NP>(C.a, m, v);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NP / 2; ++q) v[q] = reinterpret_cast<const ulonglong2*>(sc + 4 * g)[q];
+    const float lk = lane > k ? ak * inv : 0.f;
+    m = pack2(-lk, -lk);
+    diag_axpy<kNext, (KK == 3 ? NP : kNext + 1)>(C.a, m, v);
+    df_sub(C.h, C.l, ph, pl, lk);
+    X.S[(b0 + k) * kDiagRowLd + b0 + lane] = lk;
+    if (lane == k) X.piv[b0 + k] = make_float4(ph, pl, inv, 0.f);
+    C.good = lane == k ? ph > C.least && ph < 1e30f : C.good;
+}
+template <int NP>
+__device__ __forceinline__ void diag_quad(const DiagShared& X, DiagChain& C, int b0, int g, int lane) {
+    ulonglong2 v[8];   // the pivot's column (W)
+    f32x2 m = 0ull;    // -L of this row
+    diag_pivot<NP, 0>(X, C, v, m, b0, g, lane);
+    diag_pivot<NP, 1>(X, C, v, m, b0, g, lane);
+    diag_pivot<NP, 2>(X, C, v, m, b0, g, lane);
+    diag_pivot<NP, 3>(X, C, v, m, b0, g, lane);
+    __syncwarp();
+    if (g & 1) diag_bar_arrive(2 + (g >> 1), 192);   // eight more columns of L are in S
+#pragma unroll
+    for (int j = 0; j < NP - 2; ++j) C.a[j] = C.a[j + 2];
+}
+
+// The chain over sub-block b0: L into S, pivots into piv; columns are published to the rows and FP64 warps in eights
+// (barriers 2 .. 5).  Returns whether every pivot could be decided.
+__device__ __forceinline__ bool diag_chain(const DiagShared& X, int b0, int lane) {
+    DiagChain C;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {   // entries from the diagonal on are not the chain's
+        const float x = X.S[(b0 + 2 * j) * kDiagRowLd + b0 + lane], y = X.S[(b0 + 2 * j + 1) * kDiagRowLd + b0 + lane];
+        C.a[j] = pack2(2 * j < lane ? x : 0.f, 2 * j + 1 < lane ? y : 0.f);
+    }
+    C.h = X.rh[b0 + lane];
+    C.l = X.rl[b0 + lane];
+    C.least = X.lim[b0 + lane];
+    C.good = true;
+#pragma unroll 1
+    for (int g = 0; g < 4; ++g) diag_quad<16>(X, C, b0, g, lane);
+#pragma unroll 1
+    for (int g = 4; g < 8; ++g) diag_quad<8>(X, C, b0, g, lane);
+    return C.good;
+}
+
+// Row r = 32 rw + lane against sub-block b0: see k_diag_block.
+struct DiagRows {
+    f32x2 a[16];
+    float h, l;
+    int r;
+    bool below;   // the same in a warp
+};
+template <int NP, int KK>
+__device__ __forceinline__ void diag_rows_pivot(const DiagShared& X, DiagRows& R, float* W, int b0, int g) {
+    const int k = 4 * g + KK;
+    const float4 pv = X.piv[b0 + k];
+    ulonglong2 v[8];   // L of this pivot, zero up to its row
+#pragma unroll
+    for (int q = 0; q < NP / 2; ++q)
+        v[q] = reinterpret_cast<const ulonglong2*>(X.S + (b0 + k) * kDiagRowLd + b0 + 4 * g)[q];
+    const float w = diag_entry(R.a, KK);
+    diag_axpy<(KK + 1) / 2, NP>(R.a, pack2(-w, -w), v);
+    W[k * kDiagRowLd + R.r] = w;
+    const float lr = w * pv.z;
+    if (R.below) X.S[(b0 + k) * kDiagRowLd + R.r] = lr;
+    df_sub(R.h, R.l, pv.x, pv.y, lr);   // (of no use for the identity's rows)
+}
+template <int NP>
+__device__ __forceinline__ void diag_rows_quad(const DiagShared& X, DiagRows& R, float* W, float* M, int b0, int g, int nb) {
+    if (!(g & 1)) diag_bar_sync(2 + (g >> 1), 192);
+    diag_rows_pivot<NP, 0>(X, R, W, b0, g);
+    diag_rows_pivot<NP, 1>(X, R, W, b0, g);
+    diag_rows_pivot<NP, 2>(X, R, W, b0, g);
+    diag_rows_pivot<NP, 3>(X, R, W, b0, g);
+    // X^T of these columns: zero for the rows below, and past the block
+    float y[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) y[q] = !R.below && R.r < nb && b0 + 4 * g + q < nb ? diag_entry(R.a, q) : 0.f;
+    *reinterpret_cast<float4*>(M + R.r * kDiagMax + b0 + 4 * g) = make_float4(y[0], y[1], y[2], y[3]);
+#pragma unroll
+    for (int j = 0; j < NP - 2; ++j) R.a[j] = R.a[j + 2];
+}
+__device__ __forceinline__ void diag_rows(const DiagShared& X, float* W, float* M, int b0, int rw, int lane, int nb) {
+    DiagRows R;
+    const int r = 32 * rw + lane;
+    const bool own = 32 * rw == b0;
+    R.r = r;
+    R.below = 32 * rw > b0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const float x = X.S[(b0 + 2 * j) * kDiagRowLd + r], y = X.S[(b0 + 2 * j + 1) * kDiagRowLd + r];
+        R.a[j] = pack2(own ? (2 * j == lane ? 1.f : 0.f) : x, own ? (2 * j + 1 == lane ? 1.f : 0.f) : y);
+    }
+    R.h = X.rh[r];
+    R.l = X.rl[r];
+#pragma unroll 1
+    for (int g = 0; g < 4; ++g) diag_rows_quad<16>(X, R, W, M, b0, g, nb);
+#pragma unroll 1
+    for (int g = 4; g < 8; ++g) diag_rows_quad<8>(X, R, W, M, b0, g, nb);
+    if (R.below) {
+        X.rh[r] = R.h;
+        X.rl[r] = R.l;
+    }
+}
+
+// Sum of d_k l_rk^2 over pivots k0 .. k0 + n - 1 taken off dd (row r).
+__device__ __forceinline__ double diag_fp64_part(const DiagShared& X, int k0, int n, int r, double dd) {
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) dd = fma(-X.sd64[k0 + k], exact_square(X.S[(k0 + k) * kDiagRowLd + r]), dd);
+    return dd;
+}
+
+// D in FP64 beside the chain: warp q = 0 follows it with the sub-block's recursion, then shares the next sub-block's
+// rows with warp 1 (half of the pivots each); warps 2 and 1 take the rows after those.
+__device__ __forceinline__ void diag_fp64(const DiagShared& X, int nblk, int q, int lane) {
+    double next = q == 0 ? X.dg[lane] : 0.0;
+    for (int b = 0; b < nblk; ++b) {
+        const int b0 = 32 * b, r1 = b0 + 32 + lane;
+        if (q == 0) {
+            double dd = next;
+#pragma unroll 1
+            for (int g = 0; g < 8; ++g) {
+                if (!(g & 1)) diag_bar_sync(2 + (g >> 1), 192);
+                double sq[4];
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) sq[kk] = exact_square(X.S[(b0 + 4 * g + kk) * kDiagRowLd + b0 + lane]);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {   // zero squares up to the pivot's row
+                    const double dk = __shfl_sync(0xffffffffu, dd, 4 * g + kk);
+                    dd = fma(-dk, sq[kk], dd);
+                }
+            }
+            X.sd64[b0 + lane] = dd;
+        }
+        diag_bar_sync(12 + b, kDiagThreads);   // the sub-block's L is complete, and its D
+        if (b + 1 >= nblk) break;
+        if (q == 0) {
+            next = diag_fp64_part(X, b0, 16, r1, X.dg[r1]);
+            diag_bar_sync<10, 64>();
+            next += X.part[lane];
+        } else if (q == 1) {
+            X.part[lane] = diag_fp64_part(X, b0 + 16, 16, r1, 0.0);
+            diag_bar_sync<10, 64>();
+        }
+        const int rb = q == 2 ? b + 2 : q == 1 ? b + 3 : nblk;
+        if (rb < nblk) X.dg[32 * rb + lane] = diag_fp64_part(X, b0, 32, 32 * rb + lane, X.dg[32 * rb + lane]);
+    }
+}
+
+__global__ void __launch_bounds__(kDiagThreads, 1) k_diag_block(const PanelTask* __restrict__ tasks, const SnDev* __restrict__ sn,
+                                                             float* __restrict__ panel, double* __restrict__ diag,
+                                                             float* __restrict__ minv, const FactorCtl* __restrict__ ctlp,
+                                                             PivotStats* st) {
+    extern __shared__ __align__(16) float smem[];
+    DiagShared X;
+    X.S = smem;                                     // column c, row r at S[c * kDiagRowLd + r]; L as the columns finish
+    X.W = X.S + kDiagMax * kDiagRowLd;              // W of two sub-blocks, [k][row]
+    X.piv = reinterpret_cast<float4*>(X.W + 2 * 32 * kDiagRowLd);   // per pivot: D (two floats), 1/D
+    X.scr = reinterpret_cast<float*>(X.piv + kDiagMax);             // the chain's pivot column, two buffers
+    X.rh = X.scr + 128;                             // running diagonal of every row, two floats
+    X.rl = X.rh + kDiagMax;
+    X.lim = X.rl + kDiagMax;                        // smallest pivot the chain decides, per row
+    X.dg = reinterpret_cast<double*>(smem + kDiagFastFloats);       // running diagonal, FP64
+    X.sd64 = X.dg + kDiagMax;                       // D, FP64
+    X.part = X.sd64 + kDiagMax;
+    __shared__ int bad;
+    const PanelTask tk = tasks[blockIdx.x];
+    const SnDev d = sn[tk.s];
+    const FactorCtl ctl = *ctlp;
+    const int nb = tk.nb, k0 = tk.j0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* S = X.S;
+    float* P = panel + d.panel_off + k0 + (long long)k0 * d.ldp;   // A11 origin, column-major, ld = ldp
+    float* M = minv + (size_t)tk.slot * kMinvStride;
+    float* Md = M + kDiagMax * kDiagMax;
+
+    // lower triangle into S, 16 bytes at a time (zero above the diagonal's group of four and past nb rows)
+    for (int q = tid; q < kDiagMax * (kDiagMax / 4); q += kDiagThreads) {
+        const int c = q >> 5, r = (q & 31) * 4;
+        const int left = r + 3 < c || c >= nb ? 0 : min(4, max(0, nb - r));
+        const float* src = left > 0 ? P + r + (long long)c * d.ldp : P;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(S + c * kDiagRowLd + r)),
+                     "l"(src), "r"(4 * left)
+                     : "memory");
+    }
+    if (tid == 0) bad = 0;
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (tid < kDiagMax) {
+        if (tid >= nb) S[tid * kDiagRowLd + tid] = 1.f;   // rows past the block: identity, of no effect
+        const float a = S[tid * kDiagRowLd + tid];
+        X.rh[tid] = a;
+        X.rl[tid] = 0.f;
+        X.lim[tid] = tid < nb ? fmaxf(fmaxf(4.f * (float)ctl.threshold, 1e-25f), kDiagKeep * a) : 0.f;
+        X.dg[tid] = (double)a;
+    }
+    __syncthreads();
+
+    const int nblk = (nb + 31) >> 5;
+    // warp -> role: 0 chain; 1, 2, 3, 5 rows; 9, 8, 4 FP64; 6, 7, 10, 11 update
+    const int fp64 = warp == 9 ? 0 : warp == 8 ? 1 : warp == 4 ? 2 : -1;
+    const int rows = warp < 4 ? warp - 1 : warp == 5 ? 3 : -1;
+    // Each role runs its own loop over the sub-blocks (short jumps: a trip through shared code costs instruction
+    // fetches).  Barrier 1 ends a sub-block; barrier 11: the next diagonal sub-block is up to date.
+    if (fp64 >= 0) {
+        diag_fp64(X, nblk, fp64, lane);
+    } else if (warp == 0) {
+        bool good = true;
+#pragma unroll 1
+        for (int b = 0;; ++b) {
+            good &= diag_chain(X, 32 * b, lane);
+            if (!good) bad = 1;
+            diag_bar_sync<1, 288>();
+            diag_bar_arrive(12 + b, kDiagThreads);
+            if (b + 1 == nblk) break;
+            diag_bar_sync<11, 160>();
+        }
+    } else if (rows >= 0) {
+#pragma unroll 1
+        for (int b = 0;; ++b) {
+            float* W = X.W + (b & 1) * 32 * kDiagRowLd;
+            diag_rows(X, W, M, 32 * b, rows, lane, nb);
+            diag_bar_sync<1, 288>();
+            diag_bar_arrive(12 + b, kDiagThreads);
+            if (b + 1 == nblk) break;
+            // this warp's rows of the next sub-block's columns
+            if (rows != b + 1 && rows < nblk) diag_update_block<32, 32>(S, W, 32 * b, 32 * rows, 32 * b + 32, lane);
+            __syncwarp();
+        }
+    } else {
+        const int upd = warp < 8 ? warp - 6 : warp - 8;
+#pragma unroll 1
+        for (int b = 0;; ++b) {
+            diag_bar_sync<1, 288>();
+            diag_bar_arrive(12 + b, kDiagThreads);
+            if (b + 1 == nblk) break;
+            const float* W = X.W + (b & 1) * 32 * kDiagRowLd;
+            diag_update_block<16, 16>(S, W, 32 * b, 32 * b + 32 + 16 * (upd & 1), 32 * b + 32 + 16 * (upd >> 1), lane);
+            diag_bar_sync<11, 160>();
+            // the columns past the next sub-block, beside its chain
+            int unit = 0;
+            for (int c = b + 2; c < nblk; ++c)
+                for (int r = 0; r < nblk; ++r)
+                    if ((r <= b || r >= c) && (unit++ & 3) == upd)
+                        diag_update_block<32, 32>(S, W, 32 * b, 32 * r, 32 * c, lane);
+        }
+    }
+    __syncthreads();
+    if (bad) {
+        if (tid < 256) diag_block_exact(tk, d, smem, panel, diag, M, Md, ctl, st);
+        return;
+    }
+    // L11 to the factor: a thread per column, one bulk copy of whole groups of four rows below the diagonal's group
+    if (tid < nb) {
+        const int c = tid, r0 = min(nb, (c + 4) & ~3), r1 = max(r0, nb & ~3);
+        float* o = P + (long long)c * d.ldp;
+        const float* x = S + c * kDiagRowLd;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (r1 > r0)
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\ncp.async.bulk.commit_group;" ::"l"(o + r0),
+                         "r"((unsigned)__cvta_generic_to_shared(x + r0)), "r"(4 * (r1 - r0))
+                         : "memory");
+        o[c] = 1.f;
+        for (int r = c + 1; r < r0; ++r) o[r] = x[r];
+        for (int r = r1; r < nb; ++r) o[r] = x[r];
+    }
+    // D, the rest of the workspace slot (X^T past the last sub-block), the smallest and largest pivot
+    if (tid < nb) diag[d.first_col + k0 + tid] = X.sd64[tid];
+    if (tid < kDiagMax) {
+        const float4 pv = tid < nb ? X.piv[tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+        Md[tid] = pv.x;
+        Md[kDiagMax + tid] = pv.z;
+    }
+    for (int q = tid; q < kDiagMax * (kDiagMax - 32 * nblk); q += kDiagThreads) {
+        const int wc = kDiagMax - 32 * nblk;
+        M[q / wc * kDiagMax + 32 * nblk + q % wc] = 0.f;
+    }
+    if (warp == 11 && nb > 0) {
+        unsigned long long lo = ~0ull, hi = 0;   // every pivot is positive: ordered as its bits
+        for (int k = lane; k < nb; k += 32) {
+            const unsigned long long v = (unsigned long long)__double_as_longlong(X.sd64[k]);
+            lo = min(lo, v);
+            hi = max(hi, v);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (lane == 0) {
+            atomicMin(&st->min_bits, lo);
+            atomicMax(&st->max_bits, hi);
+        }
+    }
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the copies have read S
 }
 
 // 4-byte asynchronous copy global -> shared (zero fill when !valid: nothing is read then).

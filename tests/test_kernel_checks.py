@@ -207,3 +207,39 @@ def test_pivot_rule_counts_regularised_and_negative(gpu_lib):
     assert Dg[5] == Dg[17] == Dg[33] == 1e-10 * scale
     _, _, _, _, strict = diag_panel(A, threshold=1e-13 * scale, regularization=1e-10 * scale, allow=0)
     assert strict[2] == 5   # the first rejected column
+
+
+@pytest.mark.parametrize("nb", [1, 4, 31, 32, 33, 63, 64, 65, 97, 127, 128])
+def test_outer_block_sub_block_edges(gpu_lib, nb):
+    """The role-per-warp block at the edges of its 32-column sub-blocks: L and D against FP64, and D equal to
+    the FP64 recursion on the kernel's own L."""
+    A, Lg, Dg, _, counts = diag_panel(spd_front(nb + 5, nb, seed=300 + nb))
+    assert counts == [0, 0, -1]
+    A64 = A.astype(np.float64)
+    Lr, Dr = ldlt64(A64[:nb])
+    assert np.max(np.abs(Dg - Dr) / np.abs(Dr)) < 1e-4
+    L = np.tril(Lg[:nb].astype(np.float64))
+    assert np.array_equal(np.diag(L), np.ones(nb))
+    assert np.max(np.abs(L - np.tril(Lr))) < 1e-4
+    L21 = np.linalg.solve(Lr, A64[nb:].T).T / Dr
+    assert np.max(np.abs(Lg[nb:] - L21)) < 1e-4 * max(1.0, np.max(np.abs(L21)))
+    for r in range(nb):
+        d = A64[r, r] - np.sum(Dg[:r] * L[r, :r] ** 2)
+        assert abs(d - Dg[r]) <= 1e-13 * A64[r, r], r
+
+
+@pytest.mark.parametrize("nb,row", [(128, 127), (70, 40), (33, 32), (20, 3)])
+def test_outer_block_with_a_cancelling_pivot(gpu_lib, nb, row):
+    """A row that loses all but 2^-26 of its diagonal entry is left to the exact form of the block: up to that row
+    D is the FP64 one of the kernel's own L, to FP64 rounding of the entry (the rows after it take updates divided
+    by the tiny pivot, so nothing is said of them)."""
+    A = spd_front(nb, nb, seed=11 + nb)[:, :nb].astype(np.float32).astype(np.float64)
+    L, D = ldlt64(A)
+    A[row, row] += 2.0 ** -26 * A[row, row] - D[row]
+    _, Lg, Dg, _, _ = diag_panel(A)
+    Lf = np.tril(Lg[:nb].astype(np.float64))
+    A32 = A.astype(np.float32).astype(np.float64)
+    for r in range(row + 1):
+        d = A32[r, r] - np.sum(Dg[:r] * Lf[r, :r] ** 2)
+        if d > 1e-10:
+            assert abs(d - Dg[r]) <= 1e-13 * A32[r, r], r
