@@ -116,9 +116,18 @@ struct DevPlan {
     Plan plan;
     DBuf sn, rel, asm_pos, ea_items, ea_entries, small, pivot_tasks, panel_tasks, simt_jobs, tc_jobs,
         stage;
-    DBuf fvec_off, solve_fronts, solve_tasks, inv_blocks, inv_tasks;
+    DBuf fvec_off, solve_fronts, solve_tasks, inv_warp, inv_cta, inv_tasks;
     DBuf rows, child_ptr, children;   // structure of the device fronts
 };
+
+// Mixed path: the outer blocks' inverses are not the solves' blocks and live in the workspace slots.
+bool own_inverses(const PlanConfig& c) { return c.outer_block != c.solve_block; }
+
+// Scratch of the inverse fronts' inversion beyond the contribution arena, which is free by then.
+long long inv_scratch_elems(const Plan& P) {
+    const long long need = P.inv_scratch_blocks * P.cfg.solve_block * P.cfg.solve_block;
+    return need <= P.contrib_elems ? 0 : need;
+}
 
 // Device memory a factor of this plan reserves when it is created (the solve workspace,
 // which depends on the number of right-hand sides, comes on top).
@@ -128,9 +137,10 @@ int64_t planned_bytes(const Plan& P, int precision, long long nnz, long long ful
     const int64_t sb = P.cfg.solve_block;
     int64_t b = (P.factor_elems + P.contrib_elems) * elem;
     if (P.cfg.tensor_core)
-        b += 2 * P.stage_elems * op + (int64_t)std::max(1, P.diag_slots) * kMinvStride * 4 +
+        b += 2 * P.stage_elems * op + (int64_t)minv_floats(std::max(1, P.diag_slots), own_inverses(P.cfg)) * 4 +
              (int64_t)tc_ws_floats(152) * 4 + (int64_t)tc_counter_count(152) * 4;
     b += ((int64_t)P.inv_blocks.size() + P.inv_off_blocks) * sb * sb * elem;
+    b += inv_scratch_elems(P) * elem;
     b += (nnz + full_nnz) * 8 + (int64_t)n * 8;
     return b;
 }
@@ -201,7 +211,8 @@ struct uchol_symbolic_s {
         dp->fvec_off.upload(P.fvec_off, stream, "plan");
         dp->solve_fronts.upload(P.solve_fronts, stream, "plan");
         dp->solve_tasks.upload(P.solve_tasks, stream, "plan");
-        dp->inv_blocks.upload(P.inv_blocks, stream, "plan");
+        dp->inv_warp.upload(P.inv_warp, stream, "plan");
+        dp->inv_cta.upload(P.inv_cta, stream, "plan");
         dp->inv_tasks.upload(P.inv_tasks, stream, "plan");
         dp->rows.upload(P.front_rows, stream, "front rows");
         dp->child_ptr.upload(P.child_ptr, stream, "children");
@@ -223,6 +234,7 @@ struct uchol_factor_s {
     DBuf work, fv, fv2, vec[6], scal;   // solve workspace
     DBuf bwd_partial;                   // backward column dots split in row chunks: partial sums
     DBuf linv;                          // inverses of the diagonal blocks (solves)
+    DBuf inv_scratch;                   // inversion scratch, where the contribution arena is too small for it
     DBuf linv_off;                      // inverse fronts: off-diagonal blocks of the diagonal block's inverse
     DBuf inv_partial;                   // inverse fronts: backward partial sums (solve workspace)
     DBuf inv_diag_partial, inv_diag_cnt;   // inverse fronts: chunk partial sums of the diagonal products, counters
@@ -403,14 +415,14 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
                 if constexpr (sizeof(T) == 4) {
                     if (L.kind == Launch::DiagBlock)
                         k_diag_block<<<L.count, kDiagThreads, kDiagSmemBytes, st>>>(D.pivot_tasks.as<PanelTask>() + L.begin, sn,
-                                                                           panel, diag, F->minv.as<float>(), ctl, stats);
+                                                                           panel, diag, F->minv.as<float>(), F->linv.as<float>(), ctl, stats);
                     else if (F->precision == UCHOL_PRECISION_BF16)
                         k_panel_solve<__nv_bfloat16><<<L.count, 256, kPanelSmemBytes, st>>>(
-                            D.panel_tasks.as<PanelTask>() + L.begin, sn, panel, F->minv.as<float>(),
+                            D.panel_tasks.as<PanelTask>() + L.begin, sn, panel, F->minv.as<float>(), F->linv.as<float>(),
                             F->stage_a.as<__nv_bfloat16>(), F->stage_b.as<__nv_bfloat16>(), D.stage.as<StageInfo>());
                     else
                         k_panel_solve<float><<<L.count, 256, kPanelSmemBytes, st>>>(
-                            D.panel_tasks.as<PanelTask>() + L.begin, sn, panel, F->minv.as<float>(),
+                            D.panel_tasks.as<PanelTask>() + L.begin, sn, panel, F->minv.as<float>(), F->linv.as<float>(),
                             F->stage_a.as<float>(), F->stage_b.as<float>(), D.stage.as<StageInfo>());
                 } else {
                     throw Error(UCHOL_INTERNAL, "mixed-precision panel launch in an FP64 plan");
@@ -478,6 +490,17 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
     }
 }
 
+template <class T, int SB>
+void prepare_inversion() {
+    auto limit = [](auto* kernel, size_t bytes) {
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    };
+    limit(k_invert_cta<T, T, SB>, invert_cta_smem<T, SB>());
+    limit(k_inv_product<T, SB, SB>, InvTile<T, SB, SB>::bytes);
+    limit(k_inv_product<T, SB, SB / 4>, InvTile<T, SB, SB / 4>::bytes);
+    limit(k_inv_product<T, SB, SB / 8>, InvTile<T, SB, SB / 8>::bytes);
+}
+
 // Raises the dynamic shared-memory limits of every kernel a factorisation of
 // this configuration launches (done once, before any stream capture).  The
 // small-front kernel gets the limit of its largest bucket: the attribute is a
@@ -486,16 +509,10 @@ void prepare_factor_kernels(uchol_factor_s* F) {
     const int small = (int)((size_t)kSmallFrontLimit * kSmallFrontLimit * sizeof(double));
     if (F->elem == 8) {
         CK(cudaFuncSetAttribute(k_small_fronts<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(small, 1)));
-        CK(cudaFuncSetAttribute(k_invert_blocks<double, double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(2 * 64 * 64 * sizeof(double))));
-        CK(cudaFuncSetAttribute(k_inv_offdiag<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_offdiag_smem<double, 64>()));
+        prepare_inversion<double, 64>();
     } else {
         CK(cudaFuncSetAttribute(k_small_fronts<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(small, 1)));
-        CK(cudaFuncSetAttribute(k_invert_blocks<float, float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(2 * 128 * 128 * sizeof(float))));
-        CK(cudaFuncSetAttribute(k_inv_offdiag<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_offdiag_smem<float, 128>()));
+        prepare_inversion<float, 128>();
         CK(cudaFuncSetAttribute(k_diag_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmemBytes));
         CK(cudaFuncSetAttribute(k_panel_solve<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kPanelSmemBytes));
@@ -506,37 +523,30 @@ void prepare_factor_kernels(uchol_factor_s* F) {
 }
 
 // Inverses of the diagonal blocks used by the solves (FP64 factor: FP64,
-// 64-wide blocks; FP32 factor: FP32, 128-wide blocks).
+// 64-wide blocks; FP32 factor: FP32, 128-wide blocks): those the factorisation
+// kernels have not left in the arena, then the whole inverses of the inverse fronts.
+template <class T, int SB>
 void invert_diagonal_blocks(uchol_factor_s* F, cudaStream_t st) {
     DevPlan& D = *F->dp;
     const Plan& P = D.plan;
-    const int nb = (int)P.inv_blocks.size();
-    if (nb == 0) return;
-    if (F->elem == 8) {
-        constexpr int SB = 64;
-        const size_t smem = 2 * SB * SB * sizeof(double);
-        k_invert_blocks<double, double, SB><<<nb, SB, smem, st>>>(D.inv_blocks.as<SolveBlockTask>(), D.sn.as<SnDev>(),
-                                                                  F->panel.as<double>(), F->linv.as<double>());
-        // inverse fronts: off-diagonal blocks of the inverse, one launch per block diagonal
-        for (const InvLaunch& L : P.inv_launches) {
-            k_inv_offdiag<double, SB><<<L.count, 256, inv_offdiag_smem<double, SB>(), st>>>(
-                D.inv_tasks.as<SolveBlockTask>() + L.begin, D.sn.as<SnDev>(), F->panel.as<double>(),
-                F->linv.as<double>(), F->linv_off.as<double>());
-            counted();
-        }
-    } else {
-        constexpr int SB = 128;
-        const size_t smem = 2 * SB * SB * sizeof(float);
-        k_invert_blocks<float, float, SB><<<nb, SB, smem, st>>>(D.inv_blocks.as<SolveBlockTask>(), D.sn.as<SnDev>(),
-                                                                F->panel.as<float>(), F->linv.as<float>());
-        for (const InvLaunch& L : P.inv_launches) {
-            k_inv_offdiag<float, SB><<<L.count, 256, inv_offdiag_smem<float, SB>(), st>>>(
-                D.inv_tasks.as<SolveBlockTask>() + L.begin, D.sn.as<SnDev>(), F->panel.as<float>(),
-                F->linv.as<float>(), F->linv_off.as<float>());
-            counted();
-        }
+    const SnDev* sn = D.sn.as<SnDev>();
+    const T* panel = F->panel.as<T>();
+    T* linv = F->linv.as<T>();
+    if (const int n = (int)P.inv_warp.size()) {
+        k_invert_warp<T, T, SB><<<(n + kInvWarps - 1) / kInvWarps, 32 * kInvWarps, 0, st>>>(
+            D.inv_warp.as<SolveBlockTask>(), n, sn, panel, linv);
+        counted();
     }
-    counted();
+    if (const int n = (int)P.inv_cta.size()) {
+        k_invert_cta<T, T, SB><<<n, 256, invert_cta_smem<T, SB>(), st>>>(D.inv_cta.as<SolveBlockTask>(), sn, panel, linv);
+        counted();
+    }
+    T* scratch = F->inv_scratch.p ? F->inv_scratch.as<T>() : F->contrib.as<T>();
+    for (const InvLaunch& L : P.inv_launches) {
+        launch_inv_product<T, SB>(D.inv_tasks.as<SolveBlockTask>() + L.begin, L.count, L.second, F->sms, sn, panel, linv,
+                                  F->linv_off.as<T>(), scratch, st);
+        counted();
+    }
     CK(cudaGetLastError());
 }
 
@@ -598,9 +608,13 @@ void enqueue_factorization(uchol_factor_s* F, cudaStream_t st) {
             k_assemble<float><<<grid_for(S->nnz, 256), 256, 0, st>>>(F->values.as<double>(), F->dp->asm_pos.as<long long>(),
                                                                      S->nnz, F->panel.as<float>());
         counted();
-        if (F->elem == 8) run_factor_launches<double>(F, st);
-        else run_factor_launches<float>(F, st);
-        invert_diagonal_blocks(F, st);
+        if (F->elem == 8) {
+            run_factor_launches<double>(F, st);
+            invert_diagonal_blocks<double, 64>(F, st);
+        } else {
+            run_factor_launches<float>(F, st);
+            invert_diagonal_blocks<float, 128>(F, st);
+        }
     }
 }
 
@@ -777,10 +791,12 @@ uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_o
         CK(cudaStreamSynchronize(st));
     }
     if (cfg.tensor_core)
-        F->minv.alloc((size_t)std::max(1, P.diag_slots) * kMinvStride * sizeof(float), "diagonal-block inverses");
+        F->minv.alloc(minv_floats(std::max(1, P.diag_slots), own_inverses(cfg)) * sizeof(float), "diagonal-block inverses");
     F->diag.alloc((size_t)std::max(1, S->n) * sizeof(double), "pivots");
     F->linv.alloc((size_t)std::max<size_t>(1, P.inv_blocks.size()) * cfg.solve_block * cfg.solve_block * F->elem,
                   "inverse diagonal blocks");
+    CK(cudaMemsetAsync(F->linv.p, 0, F->linv.bytes, st));   // only lower triangles are written
+    if (inv_scratch_elems(P) > 0) F->inv_scratch.alloc((size_t)inv_scratch_elems(P) * F->elem, "inversion scratch");
     F->linv_off.alloc((size_t)std::max<long long>(1, P.inv_off_blocks) * cfg.solve_block * cfg.solve_block * F->elem,
                       "inverse blocks of the inverse fronts");
     F->values.alloc((size_t)std::max(1, S->nnz) * sizeof(double), "matrix values");
@@ -1484,7 +1500,7 @@ int uchol_estimate_device_bytes(const uchol_symbolic_desc* d, const uchol_option
         if (factor_bytes) *factor_bytes = P.factor_elems * elem;
         if (contribution_bytes) *contribution_bytes = P.contrib_elems * elem;
         if (staging_bytes)
-            *staging_bytes = cfg.tensor_core ? 2 * P.stage_elems * op + (int64_t)P.diag_slots * kMinvStride * 4 +
+            *staging_bytes = cfg.tensor_core ? 2 * P.stage_elems * op + (int64_t)minv_floats(P.diag_slots, own_inverses(cfg)) * 4 +
                                                    (int64_t)tc_ws_floats(152) * 4 + (int64_t)tc_counter_count(152) * 4
                                              : 0;
         if (levels) *levels = P.levels;

@@ -69,6 +69,7 @@ struct PanelTask {     // pivot block [j0, j0+nb) of front s, or its solve for r
     int stage;         // 1: also write the K-major staging copies W = L D and L (tensor-core path)
     int slot;          // mixed path: workspace slot of the block's inverse (index within its launch)
     int stage_zero_to; // > 0: also clear staging columns [j0 + nb, stage_zero_to) of these rows
+    int inv = -1;      // mixed path: block of the diagonal-inverse arena that holds the block's inverse (-1: the slot does)
 };
 
 // Staging region of a large front on the tensor-core path: m rows (front

@@ -11,10 +11,10 @@
 // (CAESolvers/UCHOL/UtduNumericFactorization.cs:139-207) with the triangular solve of
 // the diagonal block written as a product with its inverse; the result differs only
 // in rounding.  The inverse is built once per factorisation from the inverses of the
-// SB x SB diagonal blocks (k_invert_blocks): block (i, j), i > j, is
-// -Linv(i, i) sum_{j <= k < i} L(i, k) Linv(k, j), by increasing i - j (k_inv_offdiag).
+// SB x SB diagonal blocks, by doubling halves: X_21 = -X_22 (L_21 X_11) (k_inv_product).
 #pragma once
 
+#include "panel_kernels.cuh"
 #include "solve_kernels.cuh"
 
 namespace uchol_dev {
@@ -27,83 +27,146 @@ __device__ __forceinline__ const Cv* inv_block(const Cv* linv, const Cv* linv_of
                   : linv_off + ((long long)ob + (long long)i * (i - 1) / 2 + j) * SB * SB;
 }
 
-// C (SB x SB, in registers: thread (tx, ty) holds rows tx TM .. +TM, columns ty TN .. +TN)
-// += A B for column-major SB x SB A and B in shared memory.
-template <class T, int SB>
-struct BlockGemm {
-    static constexpr int TM = SB / 16, TN = SB / 16;
-    T c[TM][TN];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int a = 0; a < TM; ++a)
-#pragma unroll
-            for (int b = 0; b < TN; ++b) c[a][b] = T(0);
-    }
-    __device__ __forceinline__ void mma(const T* A, const T* B, int tx, int ty) {
-#pragma unroll 4
-        for (int kk = 0; kk < SB; ++kk) {
-            T a[TM], b[TN];
-#pragma unroll
-            for (int u = 0; u < TM; ++u) a[u] = A[tx * TM + u + kk * SB];
-#pragma unroll
-            for (int v = 0; v < TN; ++v) b[v] = B[kk + (ty * TN + v) * SB];
-#pragma unroll
-            for (int u = 0; u < TM; ++u)
-#pragma unroll
-                for (int v = 0; v < TN; ++v) c[u][v] += a[u] * b[v];
-        }
-    }
+// ---- inversion by halves: one SB x CG strip of a block product sum per CTA ----
+//
+// What bounds it: few products run at once (a front of nb blocks has at most nb^2 / 4 in a round) and each is long on
+// one SM (a 64^3 product takes 66 us on an SM's two FP64 lanes), so a block's columns are dealt out in strips of CG as
+// long as that fills the device (launch_inv_product), and the rounds double: 2 log2(nb) launches whose longest sums
+// add up to 2 (nb - 1) block products, where building the blocks by diagonals took nb - 1 launches and nb^2 / 2.
+// Columns of both operands arrive in chunks of KC rows of B by asynchronous 16-byte copies, the next chunk's under
+// the current one's products.
+template <class T, int SB, int CG>
+struct InvTile {
+    static constexpr int V = 16 / (int)sizeof(T);          // elements of a 16-byte load
+    static constexpr int OUT = SB * CG / 256;              // outputs of a thread
+    static constexpr int TR = OUT >= 64 ? 8 : OUT >= 8 ? 4 : V < OUT ? V : OUT;   // rows of a thread: groups of V, V NX apart
+    static constexpr int TC = OUT / TR;
+    static constexpr int NX = SB / TR, NY = CG / TC, G = TR / V;
+    static constexpr int KC = 128 / (int)sizeof(T);        // rows of B per chunk
+    static constexpr int LDB = KC + V;
+    static constexpr int kStage = KC * SB + CG * LDB;      // elements of a stage (A chunk, B chunk)
+    static constexpr size_t bytes = (size_t)2 * kStage * sizeof(T);
+    static_assert(TR % V == 0 && NX * NY == 256, "thread tiles must cover the strip");
 };
-
-// Off-diagonal inverse block (i, j) of an inverse front (task {s, i, j, ob, -, -, blk}).
-template <class T, int SB>
-__global__ void __launch_bounds__(256) k_inv_offdiag(const SolveBlockTask* __restrict__ tasks, const SnDev* __restrict__ sn,
-                                                     const T* __restrict__ panel, const T* __restrict__ linv,
-                                                     T* __restrict__ linv_off) {
-    extern __shared__ __align__(16) unsigned char inv_smem[];
-    T* A = reinterpret_cast<T*>(inv_smem);
-    T* B = A + SB * SB;
-    const SolveBlockTask tk = tasks[blockIdx.x];
-    const SnDev d = sn[tk.s];
-    const int i = tk.k0, j = tk.kn, ob = tk.r0, blk = tk.blk;
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    const T* P = panel + d.panel_off;
-    BlockGemm<T, SB> g;
-    g.zero();
-    for (int k = j; k < i; ++k) {
-        __syncthreads();
-        // A = L(i, k), rows past the front's columns (its trailing rows) read as zero
-        for (int e = tid; e < SB * SB; e += blockDim.x) {
-            const int r = e % SB, c = e / SB, gr = i * SB + r;
-            A[e] = gr < d.w ? P[gr + (long long)(k * SB + c) * d.ldp] : T(0);
-        }
-        const T* Bk = inv_block<T, SB>(linv, linv_off, blk, ob, k, j);
-        for (int e = tid; e < SB * SB; e += blockDim.x) B[e] = Bk[e];
-        __syncthreads();
-        g.mma(A, B, tx, ty);
-    }
-    // X = the sum, into B; then -Linv(i, i) X
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < BlockGemm<T, SB>::TM; ++u)
-#pragma unroll
-        for (int v = 0; v < BlockGemm<T, SB>::TN; ++v)
-            B[tx * BlockGemm<T, SB>::TM + u + (ty * BlockGemm<T, SB>::TN + v) * SB] = g.c[u][v];
-    const T* Di = linv + (long long)(blk + i) * SB * SB;
-    for (int e = tid; e < SB * SB; e += blockDim.x) A[e] = Di[e];
-    __syncthreads();
-    g.zero();
-    g.mma(A, B, tx, ty);
-    T* out = linv_off + ((long long)ob + (long long)i * (i - 1) / 2 + j) * SB * SB;
-#pragma unroll
-    for (int u = 0; u < BlockGemm<T, SB>::TM; ++u)
-#pragma unroll
-        for (int v = 0; v < BlockGemm<T, SB>::TN; ++v)
-            out[tx * BlockGemm<T, SB>::TM + u + (ty * BlockGemm<T, SB>::TN + v) * SB] = -g.c[u][v];
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(bytes)
+                 : "memory");
 }
 
+template <class T, int SB, int CG>
+__global__ void __launch_bounds__(256) k_inv_product(const SolveBlockTask* __restrict__ tasks, const SnDev* __restrict__ sn,
+                                                     const T* __restrict__ panel, const T* linv, T* linv_off, T* scratch,
+                                                     int second) {
+    using K = InvTile<T, SB, CG>;
+    constexpr int V = K::V, TR = K::TR, TC = K::TC, G = K::G, KC = K::KC;
+    extern __shared__ __align__(16) unsigned char inv_smem[];
+    T* const sm = reinterpret_cast<T*>(inv_smem);
+    const SolveBlockTask tk = tasks[blockIdx.x];
+    const SnDev d = sn[tk.s];
+    const int i = tk.k0, j = tk.kn, kb = tk.r1, ke = tk.flags, col0 = blockIdx.y * CG;
+    const int tid = threadIdx.x, tx = tid % K::NX, ty = tid / K::NX;
+    const T* P = panel + d.panel_off + (long long)i * SB;
+    const int rows = min(SB, d.w - i * SB);   // rows of block row i (zero past the front's columns)
+    // chunk c: rows [KC c, KC c + KC) of the sum's index, block k = kb + c / (SB / KC)
+    auto issue = [&](int c) {
+        T* As = sm + (c & 1) * K::kStage;
+        T* Bs = As + KC * SB;
+        const int k = kb + c / (SB / KC), o = c % (SB / KC) * KC;
+        const T* A = second ? inv_block<T, SB>(linv, linv_off, tk.blk, tk.r0, i, k) + o * SB
+                            : P + (long long)(k * SB + o) * d.ldp;
+        const long long lda = second ? SB : d.ldp;
+        const T* B = (second ? scratch + (long long)(tk.c0 - (i - k) * tk.c1) * SB * SB
+                             : inv_block<T, SB>(linv, linv_off, tk.blk, tk.r0, k, j)) + (long long)col0 * SB + o;
+        for (int e = tid; e < KC * SB / V; e += 256) {
+            const int r = e % (SB / V) * V, kk = e / (SB / V);
+            const int n = second ? V : min(V, max(0, rows - r));
+            cp_async16(As + kk * SB + r, n > 0 ? A + r + kk * lda : A, n * (int)sizeof(T));
+        }
+        for (int e = tid; e < CG * KC / V; e += 256) {
+            const int kk = e % (KC / V) * V, c2 = e / (KC / V);
+            cp_async16(Bs + c2 * K::LDB + kk, B + (long long)c2 * SB + kk, 16);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    T acc[TC][TR];
+#pragma unroll
+    for (int q = 0; q < TC; ++q)
+#pragma unroll
+        for (int u = 0; u < TR; ++u) acc[q][u] = T(0);
+    const int nc = (ke - kb) * (SB / KC);
+    issue(0);
+    for (int c = 0; c < nc; ++c) {
+        if (c + 1 < nc) {
+            issue(c + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const T* As = sm + (c & 1) * K::kStage + V * tx;
+        const T* Bs = sm + (c & 1) * K::kStage + KC * SB + ty * TC * K::LDB;
+#pragma unroll 2
+        for (int kk = 0; kk < KC; kk += V) {
+            T b[TC][V];
+#pragma unroll
+            for (int q = 0; q < TC; ++q) *reinterpret_cast<uint4*>(b[q]) = *reinterpret_cast<const uint4*>(Bs + q * K::LDB + kk);
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                T a[TR];
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    *reinterpret_cast<uint4*>(a + g * V) = *reinterpret_cast<const uint4*>(As + (kk + v) * SB + g * V * K::NX);
+                if constexpr (sizeof(T) == 4) {
+#pragma unroll
+                    for (int q = 0; q < TC; ++q) {
+                        const f32x2 bb = pack2(b[q][v], b[q][v]);
+#pragma unroll
+                        for (int u = 0; u < TR; u += 2) {
+                            const f32x2 r = fma2(pack2(a[u], a[u + 1]), bb, pack2(acc[q][u], acc[q][u + 1]));
+                            unpack2(r, acc[q][u], acc[q][u + 1]);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < TC; ++q)
+#pragma unroll
+                        for (int u = 0; u < TR; ++u) acc[q][u] += a[u] * b[q][v];
+                }
+            }
+        }
+        __syncthreads();   // this stage is refilled by the chunk after next
+    }
+    T* out = second ? linv_off + ((long long)tk.r0 + (long long)i * (i - 1) / 2 + j) * SB * SB
+                    : scratch + (long long)tk.c0 * SB * SB;
+#pragma unroll
+    for (int q = 0; q < TC; ++q)
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            T v[V];
+#pragma unroll
+            for (int u = 0; u < V; ++u) v[u] = second ? -acc[q][g * V + u] : acc[q][g * V + u];
+            *reinterpret_cast<uint4*>(out + (long long)(col0 + ty * TC + q) * SB + V * tx + g * V * K::NX) =
+                *reinterpret_cast<const uint4*>(v);
+        }
+}
+
+template <class T, int SB, int CG>
+inline void launch_inv_product_cg(const SolveBlockTask* tasks, int count, int second, const SnDev* sn, const T* panel,
+                                  const T* linv, T* linv_off, T* scratch, cudaStream_t st) {
+    k_inv_product<T, SB, CG><<<dim3(count, SB / CG), 256, InvTile<T, SB, CG>::bytes, st>>>(tasks, sn, panel, linv, linv_off,
+                                                                                      scratch, second);
+}
+// Strip width: whole blocks (the fewest operand reads per product) once they make two CTAs per SM, else the widest
+// strips that do, else the narrowest.
 template <class T, int SB>
-constexpr size_t inv_offdiag_smem() { return (size_t)2 * SB * SB * sizeof(T); }
+inline void launch_inv_product(const SolveBlockTask* tasks, int count, int second, int sms, const SnDev* sn, const T* panel,
+                               const T* linv, T* linv_off, T* scratch, cudaStream_t st) {
+    if (count >= 2 * sms) launch_inv_product_cg<T, SB, SB>(tasks, count, second, sn, panel, linv, linv_off, scratch, st);
+    else if (4LL * count >= 2 * sms)
+        launch_inv_product_cg<T, SB, SB / 4>(tasks, count, second, sn, panel, linv, linv_off, scratch, st);
+    else launch_inv_product_cg<T, SB, SB / 8>(tasks, count, second, sn, panel, linv, linv_off, scratch, st);
+}
 
 // Shared memory of the inverse-front solve kernels: two SB x SB tile stages, two
 // right-hand blocks (SB rows x RG, stride RS) and the partial sums.

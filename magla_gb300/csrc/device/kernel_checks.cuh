@@ -162,7 +162,7 @@ int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, 
         const int ld = round_up_int(nb, 64);
         DBuf diag, minv, sa, sb, info, ptask, ttask, ctl, stats;
         diag.alloc(sizeof(double) * nb, "check");
-        minv.alloc(sizeof(float) * kMinvStride, "check");
+        minv.alloc(sizeof(float) * minv_floats(1, true), "check");
         sa.alloc((size_t)m * ld * sizeof(float), "check");
         sb.alloc((size_t)m * ld * sizeof(float), "check");
         CK(cudaMemsetAsync(sa.p, 0, sa.bytes, st));
@@ -185,12 +185,12 @@ int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, 
         CK(cudaFuncSetAttribute(k_diag_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmemBytes));
         CK(cudaFuncSetAttribute(k_panel_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemBytes));
         k_diag_block<<<1, kDiagThreads, kDiagSmemBytes, st>>>(ptask.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<float>(),
-                                                      diag.as<double>(), minv.as<float>(), ctl.as<FactorCtl>(),
+                                                      diag.as<double>(), minv.as<float>(), nullptr, ctl.as<FactorCtl>(),
                                                       stats.as<PivotStats>());
         counted();
         if (!tt.empty()) {
             k_panel_solve<float><<<(unsigned)tt.size(), 256, kPanelSmemBytes, st>>>(
-                ttask.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<float>(), minv.as<float>(), sa.as<float>(),
+                ttask.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<float>(), minv.as<float>(), nullptr, sa.as<float>(),
                 sb.as<float>(), info.as<StageInfo>());
             counted();
         }

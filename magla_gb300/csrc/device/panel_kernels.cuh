@@ -35,9 +35,20 @@ namespace uchol_dev {
 
 constexpr int kDiagMax = 128;
 constexpr int kDiagLd = kDiagMax + 1;
-// workspace slot: X^T as kDiagMax x kDiagMax (row k, column j: X[j][k], zero for k > j
-// and beyond nb), then D and D^{-1} (kDiagMax floats each)
-constexpr int kMinvStride = kDiagMax * kDiagMax + 2 * kDiagMax;
+// A block's inverse: X^T as kDiagMax x kDiagMax (row k, column j: X[j][k], zero for k > j and beyond nb), which is
+// X column-major: the solves' inverse of the same block (PanelTask::inv), where there is one.  Workspace: a slot of D
+// and D^{-1} (kDiagMax floats each) per block of the launch, then, where the solves have no such block, the inverses.
+constexpr int kDiagSlotD = 2 * kDiagMax;
+__host__ __device__ constexpr size_t minv_floats(size_t slots, bool with_inverses) {
+    return slots * (kDiagSlotD + (with_inverses ? (size_t)kDiagMax * kDiagMax : 0));
+}
+__device__ __forceinline__ float* diag_slot_d(float* minv, const PanelTask& tk) {
+    return minv + (size_t)tk.slot * (kDiagSlotD + (tk.inv < 0 ? kDiagMax * kDiagMax : 0));
+}
+template <class F>   // float or const float
+__device__ __forceinline__ F* diag_slot_inverse(float* minv, F* linv, const PanelTask& tk) {
+    return tk.inv < 0 ? diag_slot_d(minv, tk) + kDiagSlotD : linv + (size_t)tk.inv * kDiagMax * kDiagMax;
+}
 constexpr int kSolveRows = 128;
 // float part: S and X (kDiagMax x kDiagLd each), Wt (kDiagMax x 33), D and D^{-1} in FP32;
 // then the FP64 part: the running diagonal and D (kDiagMax doubles each)
@@ -695,8 +706,8 @@ __device__ __forceinline__ void diag_fp64(const DiagShared& X, int nblk, int q, 
 
 __global__ void __launch_bounds__(kDiagThreads, 1) k_diag_block(const PanelTask* __restrict__ tasks, const SnDev* __restrict__ sn,
                                                              float* __restrict__ panel, double* __restrict__ diag,
-                                                             float* __restrict__ minv, const FactorCtl* __restrict__ ctlp,
-                                                             PivotStats* st) {
+                                                             float* __restrict__ minv, float* __restrict__ linv,
+                                                             const FactorCtl* __restrict__ ctlp, PivotStats* st) {
     extern __shared__ __align__(16) float smem[];
     DiagShared X;
     X.S = smem;                                     // column c, row r at S[c * kDiagRowLd + r]; L as the columns finish
@@ -717,8 +728,8 @@ __global__ void __launch_bounds__(kDiagThreads, 1) k_diag_block(const PanelTask*
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* S = X.S;
     float* P = panel + d.panel_off + k0 + (long long)k0 * d.ldp;   // A11 origin, column-major, ld = ldp
-    float* M = minv + (size_t)tk.slot * kMinvStride;
-    float* Md = M + kDiagMax * kDiagMax;
+    float* Md = diag_slot_d(minv, tk);
+    float* M = diag_slot_inverse(minv, linv, tk);
 
     // lower triangle into S, 16 bytes at a time (zero above the diagonal's group of four and past nb rows)
     for (int q = tid; q < kDiagMax * (kDiagMax / 4); q += kDiagThreads) {
@@ -885,8 +896,8 @@ __device__ __forceinline__ void store_op1(float* p, float a) { *p = a; }
 template <class Op>
 __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restrict__ tasks,
                                                      const SnDev* __restrict__ sn, float* __restrict__ panel,
-                                                     const float* __restrict__ minv, Op* __restrict__ stage_a,
-                                                     Op* __restrict__ stage_b,
+                                                     float* __restrict__ minv, const float* __restrict__ linv,
+                                                     Op* __restrict__ stage_a, Op* __restrict__ stage_b,
                                                      const StageInfo* __restrict__ stage_info) {
     constexpr int KC = kPanelKc, LDS = kPanelLds;
     extern __shared__ __align__(16) float psm[];   // stage s: As = psm + 2 s KC LDS, Ms = As + KC LDS
@@ -894,7 +905,7 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
     const SnDev d = sn[tk.s];
     const int nb = tk.nb, k0 = tk.j0, row0 = tk.row0, rows = tk.rows;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const float* M = minv + (size_t)tk.slot * kMinvStride;
+    const float* M = diag_slot_inverse<const float>(minv, linv, tk);
     float* A = panel + d.panel_off + row0 + (long long)k0 * d.ldp;   // A21 rows of this task, column-major
     float acc[8][8];
 #pragma unroll
@@ -950,7 +961,7 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
         __syncthreads();   // this stage is refilled two chunks later
     }
     // epilogue: L21 = W21 D^{-1} to the factor (column-major), W21 and L21 to the staging rows (K-major)
-    const float* dinv = M + kDiagMax * kDiagMax + kDiagMax;
+    const float* dinv = diag_slot_d(minv, tk) + kDiagMax;
     const bool vec_rows = ((d.panel_off + row0) & 3) == 0;
 #pragma unroll
     for (int jg = 0; jg < 2; ++jg) {

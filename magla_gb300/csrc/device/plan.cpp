@@ -234,6 +234,22 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
             if (P.assemble_pos[k] < 0) fail("a matrix value is not referenced by the symbolic pattern");
     }
 
+    // ---- diagonal blocks of the solves (inverted once per factorisation).  The mixed path's outer blocks are those
+    // blocks when both are as wide, and k_diag_block leaves each one's inverse in the arena itself ----
+    const int SB = cfg.solve_block;
+    std::vector<int>& first_blk = P.front_blk;
+    first_blk.assign(count, 0);
+    const bool outer_inverts = cfg.tensor_core && cfg.outer_block == SB;
+    for (int s = 0; s < count; ++s) {
+        first_blk[s] = (int)P.inv_blocks.size();
+        for (int k0 = 0; k0 < P.sn[s].w; k0 += SB) {
+            const SolveBlockTask t{s, k0, std::min(SB, P.sn[s].w - k0), 0, 0, 1, (int)P.inv_blocks.size()};
+            P.inv_blocks.push_back(t);
+            if (outer_inverts && !small_front(cfg, P.sn[s].m)) continue;
+            (t.kn <= kInvWarpCols ? P.inv_warp : P.inv_cta).push_back(t);
+        }
+    }
+
     // ---- factorisation launches, level by level ----
     P.stage.assign(count, StageInfo{0, 0, -1});
     const int PB = cfg.pivot_block;
@@ -364,11 +380,12 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                     const SnDev& d = P.sn[s];
                     if (d.w <= k0) continue;
                     int nbo = std::min(NB, d.w - k0);
-                    P.pivot_tasks.push_back({s, k0, nbo, k0 + nbo, 0, -1, slot, 0});
+                    const int inv = outer_inverts ? first_blk[s] + k0 / NB : -1;
+                    P.pivot_tasks.push_back({s, k0, nbo, k0 + nbo, 0, -1, slot, 0, inv});
                     int zero_to = (k0 + nbo == d.w && P.stage[s].ld > d.w) ? P.stage[s].ld : 0;
                     for (int r = k0 + nbo; r < d.m; r += kSolveRowsPlan) {
                         int rows = std::min(kSolveRowsPlan, d.m - r);
-                        P.panel_tasks.push_back({s, k0, nbo, r, rows, 1, slot, zero_to});
+                        P.panel_tasks.push_back({s, k0, nbo, r, rows, 1, slot, zero_to, inv});
                         P.panel_flops += 2.0 * rows * nbo * nbo;
                     }
                     ++slot;
@@ -464,14 +481,6 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         fo += round_up(P.sn[s].m, 8);
     }
     P.fvec_elems = std::max<long long>(fo, 8);
-    const int SB = cfg.solve_block;
-    // diagonal blocks of every supernode (inverted once per factorisation)
-    std::vector<int> first_blk(count, 0);
-    for (int s = 0; s < count; ++s) {
-        first_blk[s] = (int)P.inv_blocks.size();
-        for (int k0 = 0; k0 < P.sn[s].w; k0 += SB)
-            P.inv_blocks.push_back({s, k0, std::min(SB, P.sn[s].w - k0), 0, 0, 1, (int)P.inv_blocks.size()});
-    }
     // inverse fronts: SB < w <= inv_cols; their off-diagonal inverse blocks, by diagonal i - j
     std::vector<int> inv_ob(count, -1);
     {
@@ -485,14 +494,38 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
             P.inv_off_blocks += (long long)nb * (nb - 1) / 2;
             max_nb = std::max(max_nb, nb);
         }
-        for (int dg = 1; dg < max_nb; ++dg) {
-            const int b0 = (int)P.inv_tasks.size();
+        // by halves: z = 1, 2, 4, ... blocks; each round needs the one before it for every group
+        for (int z = 1; z < max_nb; z *= 2) {
+            long long scratch = 0;
+            std::vector<SolveBlockTask> first, second;
             for (int s = 0; s < count; ++s) {
                 if (inv_ob[s] < 0) continue;
                 const int nb = (P.sn[s].w + SB - 1) / SB;
-                for (int i = dg; i < nb; ++i) P.inv_tasks.push_back({s, i, i - dg, inv_ob[s], 0, 0, first_blk[s]});
+                for (int J = 0; J + z < nb; J += 2 * z) {
+                    const int I = J + z, rows = std::min(z, nb - I);
+                    if (scratch + (long long)rows * z > INT32_MAX) fail("too many inverse blocks");
+                    for (int i = I; i < I + rows; ++i)
+                        for (int j = J; j < I; ++j) {
+                            SolveBlockTask t{s, i, j, inv_ob[s], j, I, first_blk[s]};
+                            t.c0 = (int)scratch + (i - I) * z + (j - J);
+                            t.c1 = z;
+                            first.push_back(t);
+                            t.r1 = I;
+                            t.flags = i + 1;
+                            second.push_back(t);
+                        }
+                    scratch += (long long)rows * z;
+                }
             }
-            if ((int)P.inv_tasks.size() > b0) P.inv_launches.push_back({b0, (int)P.inv_tasks.size() - b0});
+            // the longest sums first
+            auto longer = [](const SolveBlockTask& x, const SolveBlockTask& y) { return x.flags - x.r1 > y.flags - y.r1; };
+            std::stable_sort(first.begin(), first.end(), longer);
+            std::stable_sort(second.begin(), second.end(), longer);
+            P.inv_scratch_blocks = std::max(P.inv_scratch_blocks, scratch);
+            P.inv_launches.push_back({(int)P.inv_tasks.size(), (int)first.size(), 0});
+            P.inv_tasks.insert(P.inv_tasks.end(), first.begin(), first.end());
+            P.inv_launches.push_back({(int)P.inv_tasks.size(), (int)second.size(), 1});
+            P.inv_tasks.insert(P.inv_tasks.end(), second.begin(), second.end());
         }
     }
     constexpr int kGatherChunk = 512;   // rows per gather CTA (one CTA per chunk and right-hand side)

@@ -19,6 +19,7 @@ constexpr int kInvColRowsPlan = 1024;   // trailing rows per backward partial-su
 constexpr int kDefaultInvCols = 2048;   // widest front whose diagonal block is kept inverted for the solves
 constexpr int kSuperBlocks = 4;       // tensor-core path: outer blocks per super-block of the own-column updates
 constexpr int kDefaultMergeCols = 2048;   // widest device front made of a chain of supernodes (merge_chains)
+constexpr int kInvWarpCols = 32;         // widest diagonal block inverted by one warp
 constexpr int kInvDiagChunk = 2;         // inverse blocks per task of the inverse-front diagonal products
 
 struct PlanConfig {
@@ -85,8 +86,10 @@ struct SolveLaunch {
 // Inverse fronts (cfg.inv_cols): the off-diagonal blocks (i, j), i > j, of the
 // inverse of the unit-lower diagonal block, SB x SB column-major each, front s's
 // at block index ob_s + i (i - 1) / 2 + j of the off-diagonal arena.  Tasks:
-//   inversion            {s, i, j, ob_s, -, -, blk}: block (i, j) from the blocks
-//                        (k, j), j <= k < i (launched by diagonal i - j);
+//   inversion            {s, i, j, ob_s, k0, k1, blk, t, z}: by halves.  A group of 2 z blocks whose two halves
+//                        are inverted gets its off-diagonal half X_IJ = -X_II (L_IJ X_JJ): first
+//                        T(i, j) = sum_{k0 <= k < k1} L(i, k) X(k, j), T's block at index t of the scratch arena
+//                        (T(k, j) at t - (i - k) z), then X(i, j) = -sum_{k0 <= k < k1} X(i, k) T(k, j);
 //   FwdInvDiag           {s, i, nb, ob_s, slot0, nc, blk, j0, j1}: the part j0 <= j <= j1 of
 //                        y_i = sum_{j <= i} Linv(i, j) f_j; block row i is split in nc chunks of
 //                        kInvDiagChunk blocks (partial slots slot0 .. slot0+nc-1; nc = 1: no split);
@@ -98,7 +101,8 @@ struct SolveLaunch {
 //                        x_j = sum_{i >= j} Linv(i, j)^T g_i, in chunks as FwdInvDiag.
 // blk is the diagonal-inverse index of the front's block 0.
 struct InvLaunch {
-    int begin, count;   // inversion tasks of one diagonal i - j
+    int begin, count;   // inversion tasks
+    int second;         // 0: T = L X, 1: X = -X T
 };
 
 // Solve task of supernode s.  Gathers: rows [r0, r1) of the front vector.
@@ -169,9 +173,13 @@ struct Plan {
     std::vector<SolveBlockTask> solve_tasks;
     std::vector<SolveBlockTask> inv_blocks;    // every diagonal block, for the inversion after a factorisation
     std::vector<SolveLaunch> fwd_launches, bwd_launches;
-    std::vector<SolveBlockTask> inv_tasks;     // inverse fronts: off-diagonal inverse blocks, by diagonal
+    std::vector<SolveBlockTask> inv_warp, inv_cta;   // those the factorisation kernels do not invert themselves: up to
+                                               // kInvWarpCols columns (a warp each), wider (a CTA each)
+    std::vector<int> front_blk;                // per front: index of its first diagonal block
+    std::vector<SolveBlockTask> inv_tasks;     // inverse fronts: off-diagonal inverse blocks, by doubling halves
     std::vector<InvLaunch> inv_launches;
     long long inv_off_blocks = 0;              // blocks of the off-diagonal inverse arena
+    long long inv_scratch_blocks = 0;          // blocks of the inversion's scratch (T of one round)
     int inv_partial_slots = 0;                 // most BwdInvCols partial slots of one launch (SB x nrhs each)
     int inv_diag_slots = 0;                    // most inverse-diagonal partial slots of one launch (SB x nrhs each)
     int progress_count = 0;                    // progress counters of all level launches

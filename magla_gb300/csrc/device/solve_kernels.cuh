@@ -112,37 +112,99 @@ __global__ void k_fwd_gather(const SolveBlockTask* __restrict__ tasks, SolveArgs
     }
 }
 
-// Inverse of every unit-lower diagonal block (SB x SB, column-major), one
-// CTA per block, thread c computing column c by forward substitution.
+// ---- inverses of unit-lower diagonal blocks (SB x SB, column-major; the arena starts as zeros, and only the lower
+// triangle of the block's kn columns is written) ----
+//
+// A column's forward substitution is a chain of kn^2 / 2 multiply-adds: 2016 of them, 64 cycles each in FP64, took
+// 130 us for one 64-column block.  So chains are kept to 16 columns and the rest are products spread over the CTA.
+
+// Blocks of at most 32 columns: a warp each, lane = column of the inverse, its column in shared memory.
+constexpr int kInvWarps = 4;   // warps per CTA
 template <class T, class Cv, int SB>
-__global__ void __launch_bounds__(SB) k_invert_blocks(const SolveBlockTask* __restrict__ blocks, const SnDev* __restrict__ sn,
-                                                      const T* __restrict__ panel, Cv* __restrict__ linv) {
-    extern __shared__ unsigned char inv_smem[];
-    Cv* Lb = reinterpret_cast<Cv*>(inv_smem);
-    Cv* X = Lb + SB * SB;
+__global__ void __launch_bounds__(32 * kInvWarps) k_invert_warp(const SolveBlockTask* __restrict__ blocks, int count,
+                                                               const SnDev* __restrict__ sn, const T* __restrict__ panel,
+                                                               Cv* __restrict__ linv) {
+    constexpr int N = kInvWarpCols, LD = N + 1;
+    __shared__ Cv Ls[kInvWarps][N * LD];   // row-major L (strictly lower); X over the rows already used
+    __shared__ Cv Xs[kInvWarps][N * LD];   // X[k * LD + column]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * kInvWarps + warp;
+    if (q >= count) return;
+    const SolveBlockTask tk = blocks[q];
+    const SnDev d = sn[tk.s];
+    const int kn = tk.kn;
+    const T* P = panel + d.panel_off + tk.k0 + (long long)tk.k0 * d.ldp;
+    Cv* L = Ls[warp];
+    Cv* X = Xs[warp];
+    if (lane < kn)
+        for (int c = 0; c < lane; ++c) L[lane * LD + c] = (Cv)P[lane + (long long)c * d.ldp];
+    __syncwarp();
+    for (int r = 0; r < kn; ++r) {
+        Cv v = r == lane ? Cv(1) : Cv(0);
+        for (int k = 0; k < r; ++k) v -= L[r * LD + k] * X[k * LD + lane];   // X is zero above its diagonal
+        X[r * LD + lane] = v;
+    }
+    __syncwarp();
+    Cv* out = linv + (long long)tk.blk * SB * SB;
+    if (lane < kn)   // lane = row: consecutive rows of each column
+        for (int c = 0; c <= lane; ++c) out[lane + c * SB] = X[lane * LD + c];
+}
+
+// Wider blocks: a CTA each.  The 16-column diagonal sub-blocks by chains, then doubling halves:
+// X_21 = -X_22 (L_21 X_11), each product's entries dealt over the CTA.
+template <class Cv, int SB>
+constexpr size_t invert_cta_smem() { return ((size_t)2 * SB * (SB + 1) + (size_t)SB / 2 * (SB / 2 + 1)) * sizeof(Cv); }
+template <class T, class Cv, int SB>
+__global__ void __launch_bounds__(256) k_invert_cta(const SolveBlockTask* __restrict__ blocks, const SnDev* __restrict__ sn,
+                                                    const T* __restrict__ panel, Cv* __restrict__ linv) {
+    extern __shared__ __align__(16) unsigned char inv_smem[];
+    constexpr int LD = SB + 1, LT = SB / 2 + 1, B = 16;
+    Cv* L = reinterpret_cast<Cv*>(inv_smem);   // L[r * LD + c]
+    Cv* X = L + SB * LD;                       // X[r * LD + c]
+    Cv* W = X + SB * LD;                       // L_21 X_11 of every pair of a round, [r][c]
     const SolveBlockTask tk = blocks[blockIdx.x];
     const SnDev d = sn[tk.s];
-    const T* P = panel + d.panel_off;
-    const int kn = tk.kn;
-    for (int idx = threadIdx.x; idx < kn * kn; idx += blockDim.x) {
-        int r = idx % kn, c = idx / kn;
-        Lb[r + c * SB] = r > c ? (Cv)P[(tk.k0 + r) + (long long)(tk.k0 + c) * d.ldp] : Cv(0);
+    const T* P = panel + d.panel_off + tk.k0 + (long long)tk.k0 * d.ldp;
+    const int kn = tk.kn, tid = threadIdx.x;
+    for (int e = tid; e < SB * SB; e += 256) {
+        const int r = e % SB, c = e / SB;
+        L[r * LD + c] = r > c && r < kn ? (Cv)P[r + (long long)c * d.ldp] : Cv(0);
+        X[r * LD + c] = Cv(0);
     }
     __syncthreads();
-    const int c = threadIdx.x;
-    if (c < kn) {
-        for (int r = 0; r < kn; ++r) {
-            Cv v = r == c ? Cv(1) : Cv(0);
-            if (r > c)
-                for (int k = c; k < r; ++k) v -= Lb[r + k * SB] * X[k + c * SB];
-            X[r + c * SB] = v;
+    if (tid < kn) {   // column tid of its diagonal sub-block's inverse
+        const int b = tid / B * B;
+        X[tid * LD + tid] = Cv(1);
+        for (int r = tid + 1; r < min(kn, b + B); ++r) {
+            Cv v = Cv(0);
+            for (int k = tid; k < r; ++k) v -= L[r * LD + k] * X[k * LD + tid];
+            X[r * LD + tid] = v;
+        }
+    }
+    for (int z = B; z < kn; z *= 2) {
+        // groups of 2 z columns from 2 z q: rows [2 z q + z, .. + z), columns [2 z q, .. + z)
+        const int per = z * z, all = (kn + 2 * z - 1) / (2 * z) * per;
+        __syncthreads();
+        for (int e = tid; e < all; e += 256) {
+            const int q = e / per, r = e % per / z, c = e % z, b = 2 * z * q;
+            if (b + z + r >= kn) continue;
+            Cv v = Cv(0);
+            for (int k = c; k < z; ++k) v += L[(b + z + r) * LD + b + k] * X[(b + k) * LD + b + c];
+            W[(q * z + r) * LT + c] = v;
+        }
+        __syncthreads();
+        for (int e = tid; e < all; e += 256) {
+            const int q = e / per, r = e % per / z, c = e % z, b = 2 * z * q;
+            if (b + z + r >= kn) continue;
+            Cv v = Cv(0);
+            for (int k = 0; k <= r; ++k) v -= X[(b + z + r) * LD + b + z + k] * W[(q * z + k) * LT + c];
+            X[(b + z + r) * LD + b + c] = v;
         }
     }
     __syncthreads();
     Cv* out = linv + (long long)tk.blk * SB * SB;
-    for (int idx = threadIdx.x; idx < SB * SB; idx += blockDim.x) {
-        int r = idx % SB, cc = idx / SB;
-        out[idx] = (r < kn && cc < kn) ? X[r + cc * SB] : Cv(0);
+    for (int e = tid; e < SB * SB; e += 256) {
+        const int r = e % SB, c = e / SB;
+        if (r >= c && r < kn) out[e] = X[r * LD + c];
     }
 }
 
