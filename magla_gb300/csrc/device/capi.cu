@@ -344,7 +344,7 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
     const bool timing = phase_timing();
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev;
     std::vector<int> ev_kind;
-    const size_t small_smem = (size_t)P.max_small_m * P.max_small_m * sizeof(double);
+    const size_t small_smem = small_front_smem(P.max_small_m);
     // side-stream launches fork from the main stream and are joined before the launch that
     // needs them (plan.hpp, Launch::stream); under per-launch timing everything runs in order
     const bool overlap = !timing && F->side_stream;
@@ -386,8 +386,18 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
                 break;
             }
             case Launch::SmallFronts:
-                k_small_fronts<T><<<L.count, 256, small_smem, st>>>(D.small.as<int>() + L.begin, sn, panel, contrib,
-                                                                    diag, ctl, stats);
+                if (L.variant == 0) {
+                    k_small_fronts<T><<<L.count, kSmallFrontThreads, small_smem, st>>>(D.small.as<int>() + L.begin, sn, panel,
+                                                                                      contrib, diag, ctl, stats);
+                } else {
+                    auto lanes = [&](auto* kernel) {
+                        const int per = kLaneFrontThreads / L.variant;
+                        kernel<<<(L.count + per - 1) / per, kLaneFrontThreads, 0, st>>>(
+                            D.small.as<int>() + L.begin, L.count, sn, panel, contrib, diag, ctl, stats);
+                    };
+                    lanes(L.variant == 8 ? k_small_fronts_lanes<T, 8> : L.variant == 16 ? k_small_fronts_lanes<T, 16>
+                                                                                       : k_small_fronts_lanes<T, 32>);
+                }
                 break;
             case Launch::PivotBlock:
             case Launch::Trsm:
@@ -398,13 +408,16 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
                     const PanelTask* tk = D.panel_tasks.as<PanelTask>() + L.begin;
                     if (L.kind == Launch::PivotBlock)
                         k_pivot_block<T><<<L.count, 128, 0, st>>>(pt, sn, panel, diag, ctl, stats);
+                    else if (L.kind == Launch::SimtUpdate && L.variant == 32)
+                        k_simt_update<T, 32><<<(unsigned)L.tiles, simt_threads<32>(), 0, st>>>(
+                            D.simt_jobs.as<UpdJob>() + L.begin, L.count, sn, panel, contrib, diag);
                     else if (L.kind == Launch::SimtUpdate)
-                        k_simt_update<T, double><<<(unsigned)L.tiles, 256, 0, st>>>(
+                        k_simt_update<T, 16><<<(unsigned)L.tiles, simt_threads<16>(), 0, st>>>(
                             D.simt_jobs.as<UpdJob>() + L.begin, L.count, sn, panel, contrib, diag);
                     else if (P.cfg.pivot_block <= 32)
-                        k_trsm<T, double, 32><<<L.count, 128, 0, st>>>(tk, sn, panel, diag);
+                        k_trsm<T, 32><<<L.count * kTrsmSplit, 128, 0, st>>>(tk, sn, panel, diag);
                     else
-                        k_trsm<T, double, 64><<<L.count, 128, 0, st>>>(tk, sn, panel, diag);
+                        k_trsm<T, 64><<<L.count * kTrsmSplit, 128, 0, st>>>(tk, sn, panel, diag);
                 } else {
                     throw Error(UCHOL_INTERNAL, "FP64 panel launch in a mixed-precision plan");
                 }
@@ -506,7 +519,7 @@ void prepare_inversion() {
 // small-front kernel gets the limit of its largest bucket: the attribute is a
 // per-function maximum shared by every factor, so it never goes down.
 void prepare_factor_kernels(uchol_factor_s* F) {
-    const int small = (int)((size_t)kSmallFrontLimit * kSmallFrontLimit * sizeof(double));
+    const int small = (int)small_front_smem(kSmallFrontLimit);
     if (F->elem == 8) {
         CK(cudaFuncSetAttribute(k_small_fronts<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(small, 1)));
         prepare_inversion<double, 64>();

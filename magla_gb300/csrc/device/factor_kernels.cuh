@@ -148,52 +148,148 @@ __global__ void k_extend_add(const EaItem* __restrict__ items, int count, const 
     }
 }
 
-// Whole small front in shared memory (FP64), unblocked right-looking LDL^T
-// of its w pivots; writes the unit factor block and the contribution.
+// ---- FP64 pivots, panels and updates ----
+//
+// What bounds them: the FP64 pipe.  A scheduler issues one FP64 warp instruction per 64 cycles, however few of its
+// lanes are active, so an SM does two multiply-adds per clock: a 64 x 64 x 32 update tile alone takes one SM 32 us,
+// a 128-row panel solve 16 us, a division about ten instructions.  So work is cut fine enough to reach every SM
+// (16- and 32-row tiles), operands take one multiply-add per entry (the unscaled column times L, no separate
+// product with the pivot), and the chain of pivots has a warp, and as far as possible a scheduler, to itself.
+
+// Small fronts (m <= LW): LW lanes a front, lane = row, the front's rows in registers.  The row is a shift register
+// (a[j] is column k + j at pivot k), so every register index is a constant while the pivots' loop stays rolled.
+constexpr int kLaneFrontThreads = 128;
+template <class T, int LW>
+__global__ void __launch_bounds__(kLaneFrontThreads) k_small_fronts_lanes(const int* __restrict__ fronts, int count,
+                                                                         const SnDev* __restrict__ sn, T* __restrict__ panel,
+                                                                         T* __restrict__ contrib, double* __restrict__ diag,
+                                                                         const FactorCtl* __restrict__ ctlp, PivotStats* st) {
+    const int r = threadIdx.x & (LW - 1), q = (blockIdx.x * kLaneFrontThreads + threadIdx.x) / LW;
+    const FactorCtl ctl = *ctlp;
+    SnDev d{};   // m = w = 0 past the last front
+    if (q < count) d = sn[fronts[q]];
+    const int m = d.m, w = d.w;
+    T* P = panel + d.panel_off;
+    T* C = contrib + d.contrib_off;
+    double a[LW];
+#pragma unroll
+    for (int j = 0; j < LW; ++j)
+        a[j] = r < m && j <= r ? (j < w ? (double)P[r + (long long)j * d.ldp] : (double)C[(r - w) + (long long)(j - w) * d.ldc]) : 0.0;
+    int wmax = w, mmax = m;
+    for (int o = 16; o >= LW && o > 0; o >>= 1) {
+        wmax = max(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
+        mmax = max(mmax, __shfl_xor_sync(0xffffffffu, mmax, o));
+    }
+    PivotAcc acc;
+    for (int k = 0; k < wmax; ++k) {
+        const bool live = k < w;   // the same in the front's lanes
+        const double raw = __shfl_sync(0xffffffffu, a[0], k, LW);
+        const double piv = live ? acc.accept(raw, d.first_col + k, ctl) : 1.0;
+        const double inv = 1.0 / piv;
+        const double wk = a[0];
+        const double l = live && r > k && r < m ? wk * inv : 0.0;
+        if (live && r >= k && r < m) P[r + (long long)k * d.ldp] = r == k ? (T)1 : (T)l;
+        if (live && r == k) diag[d.first_col + k] = piv;
+        const int rem = mmax - 1 - k;
+#pragma unroll
+        for (int j = 1; j < LW; ++j) {
+            if (j > rem) break;
+            const double wj = __shfl_sync(0xffffffffu, wk, (k + j) & (LW - 1), LW);
+            const double v = fma(-l, wj, a[j]);
+            if (live) a[j - 1] = v;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < LW; ++j)   // column w + j of the contribution
+        if (w + j <= r && r < m) C[(r - w) + (long long)j * d.ldc] = (T)a[j];
+    // statistics: one set of atomics a warp
+    if (r != 0) acc = PivotAcc();
+    for (int o = 16; o > 0; o >>= 1) {
+        acc.regularized += __shfl_xor_sync(0xffffffffu, acc.regularized, o);
+        acc.negative += __shfl_xor_sync(0xffffffffu, acc.negative, o);
+        acc.failed = min(acc.failed, __shfl_xor_sync(0xffffffffu, acc.failed, o));
+        acc.min_bits = min(acc.min_bits, __shfl_xor_sync(0xffffffffu, acc.min_bits, o));
+        acc.max_bits = max(acc.max_bits, __shfl_xor_sync(0xffffffffu, acc.max_bits, o));
+    }
+    if ((threadIdx.x & 31) == 0) acc.flush(st);
+}
+
+// LDL^T of the first w columns of the m x m matrix at S (column-major, leading dimension ld, lower triangle) in
+// shared memory, by kWarps warps: warp 0 is the chain (pivot, division, the scaled column, the next column's update),
+// the others update the columns after that; one barrier a pivot.  Wc: two buffers of wstride entries for the
+// unscaled column.
+template <int kWarps, class Pivot>
+__device__ __forceinline__ void smem_ldlt(double* S, int ld, int m, int w, double* Wc, int wstride, Pivot&& pivot) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int k = 0; k < w; ++k) {
+        double* W = Wc + (k & 1) * wstride;
+        double* Lk = S + (long long)k * ld;
+        if (warp == 0) {
+            const double piv = pivot(k, Lk[k]);
+            const double inv = 1.0 / piv;
+            __syncwarp();
+            for (int i = k + 1 + lane; i < m; i += 32) {
+                const double v = Lk[i];
+                W[i] = v;
+                Lk[i] = v * inv;
+            }
+            if (lane == 0) Lk[k] = 1.0;
+        }
+        __syncthreads();
+        const bool next = k + 1 < w;   // the next column is the chain's
+        if (warp == 0) {
+            if (next) {
+                double* c = S + (long long)(k + 1) * ld;
+                const double wj = W[k + 1];
+                for (int i = k + 1 + lane; i < m; i += 32) c[i] = fma(-Lk[i], wj, c[i]);
+                __syncwarp();
+            }
+        } else {
+            for (int j = k + 1 + (next ? 1 : 0) + warp - 1; j < m; j += kWarps - 1) {
+                double* c = S + (long long)j * ld;
+                const double wj = W[j];
+                for (int i = j + lane; i < m; i += 32) c[i] = fma(-Lk[i], wj, c[i]);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Whole front of 32 < m <= kSmallFrontLimit rows in shared memory (FP64); writes the unit factor block and the
+// contribution.
+constexpr int kSmallFrontThreads = 256;
+__host__ __device__ constexpr size_t small_front_smem(int m) { return ((size_t)m * m + 2 * (size_t)m) * sizeof(double); }
 template <class T>
-__global__ void __launch_bounds__(256) k_small_fronts(const int* __restrict__ fronts, const SnDev* __restrict__ sn,
-                                                      T* __restrict__ panel, T* __restrict__ contrib,
-                                                      double* __restrict__ diag, const FactorCtl* __restrict__ ctlp,
-                                                      PivotStats* st) {
+__global__ void __launch_bounds__(kSmallFrontThreads) k_small_fronts(const int* __restrict__ fronts, const SnDev* __restrict__ sn,
+                                                                     T* __restrict__ panel, T* __restrict__ contrib,
+                                                                     double* __restrict__ diag, const FactorCtl* __restrict__ ctlp,
+                                                                     PivotStats* st) {
     extern __shared__ double S[];
     const SnDev d = sn[fronts[blockIdx.x]];
     const FactorCtl ctl = *ctlp;
     const int m = d.m, w = d.w, ld = m;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int idx = tid; idx < m * m; idx += nt) {
-        int i = idx % m, j = idx / m;
-        if (i < j) continue;
-        S[i + j * ld] = j < w ? (double)panel[d.panel_off + i + (long long)j * d.ldp]
-                              : (double)contrib[d.contrib_off + (i - w) + (long long)(j - w) * d.ldc];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kWarps = kSmallFrontThreads / 32;
+    T* P = panel + d.panel_off;
+    T* C = contrib + d.contrib_off;
+    for (int j = warp; j < m; j += kWarps) {
+        const T* src = j < w ? P + (long long)j * d.ldp : C + (long long)(j - w) * d.ldc - w;
+#pragma unroll 4
+        for (int i = j + lane; i < m; i += 32) S[i + j * ld] = (double)src[i];
     }
     PivotAcc acc;
     __syncthreads();
-    for (int k = 0; k < w; ++k) {
-        double piv = acc.accept(S[k + k * ld], d.first_col + k, ctl);  // identical in every thread
-        const double inv = 1.0 / piv;
-        __syncthreads();
-        for (int i = k + 1 + tid; i < m; i += nt) S[i + k * ld] *= inv;
-        if (tid == 0) {
-            diag[d.first_col + k] = piv;
-            S[k + k * ld] = 1.0;
-        }
-        __syncthreads();
-        const int r = m - k - 1;
-        for (int idx = tid; idx < r * r; idx += nt) {
-            int ii = idx % r, jj = idx / r;
-            if (ii < jj) continue;
-            int i = k + 1 + ii, j = k + 1 + jj;
-            S[i + j * ld] -= S[i + k * ld] * (piv * S[j + k * ld]);
-        }
-        __syncthreads();
+    smem_ldlt<kWarps>(S, ld, m, w, S + (size_t)m * m, m, [&](int k, double raw) {
+        const double piv = acc.accept(raw, d.first_col + k, ctl);
+        if (lane == 0) diag[d.first_col + k] = piv;
+        return piv;
+    });
+    for (int j = warp; j < m; j += kWarps) {
+        T* dst = j < w ? P + (long long)j * d.ldp : C + (long long)(j - w) * d.ldc - w;
+#pragma unroll 4
+        for (int i = j + lane; i < m; i += 32) dst[i] = (T)S[i + j * ld];
     }
-    for (int idx = tid; idx < m * m; idx += nt) {
-        int i = idx % m, j = idx / m;
-        if (i < j) continue;
-        if (j < w) panel[d.panel_off + i + (long long)j * d.ldp] = (T)S[i + j * ld];
-        else contrib[d.contrib_off + (i - w) + (long long)(j - w) * d.ldc] = (T)S[i + j * ld];
-    }
-    if (tid == 0) acc.flush(st);
+    if (threadIdx.x == 0) acc.flush(st);
 }
 
 // Pivot block [j0, j0+nb) of a large front: FP64 LDL^T of the nb x nb
@@ -207,154 +303,145 @@ __global__ void __launch_bounds__(128) k_pivot_block(const PanelTask* __restrict
                                                      T* __restrict__ panel, double* __restrict__ diag,
                                                      const FactorCtl* __restrict__ ctlp, PivotStats* st) {
     __shared__ double Dg[kMaxPivotBlock * (kMaxPivotBlock + 1)];
+    __shared__ double Wc[2 * kMaxPivotBlock];
     const PanelTask tk = tasks[blockIdx.x];
     const SnDev d = sn[tk.s];
     const FactorCtl ctl = *ctlp;
     const int nb = tk.nb, j0 = tk.j0, ld = kMaxPivotBlock + 1;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    T* P = panel + d.panel_off;
-    for (int idx = tid; idx < nb * nb; idx += nt) {
-        int r = idx % nb, c = idx / nb;
-        if (r >= c) Dg[r + c * ld] = (double)P[(j0 + r) + (long long)(j0 + c) * d.ldp];
+    const int tid = threadIdx.x, lane = tid & 31;
+    T* P = panel + d.panel_off + j0 + (long long)j0 * d.ldp;
+#pragma unroll 4
+    for (int e = tid; e < kMaxPivotBlock * nb; e += 128) {
+        const int r = e % kMaxPivotBlock, c = e / kMaxPivotBlock;
+        if (r >= c && r < nb) Dg[r + c * ld] = (double)P[r + (long long)c * d.ldp];
     }
     PivotAcc acc;
     __syncthreads();
-    for (int k = 0; k < nb; ++k) {
-        const double piv = acc.accept(Dg[k + k * ld], d.first_col + j0 + k, ctl);
-        const double inv = 1.0 / piv;
-        __syncthreads();
-        for (int r = k + 1 + tid; r < nb; r += nt) Dg[r + k * ld] *= inv;
-        if (tid == 0) {
-            diag[d.first_col + j0 + k] = piv;
-            Dg[k + k * ld] = 1.0;
-        }
-        __syncthreads();
-        const int q = nb - k - 1;
-        for (int idx = tid; idx < q * q; idx += nt) {
-            int rr = idx % q, cc = idx / q;
-            if (rr < cc) continue;
-            int r = k + 1 + rr, c = k + 1 + cc;
-            Dg[r + c * ld] -= Dg[r + k * ld] * (piv * Dg[c + k * ld]);
-        }
-        __syncthreads();
-    }
-    for (int idx = tid; idx < nb * nb; idx += nt) {
-        int r = idx % nb, c = idx / nb;
-        if (r >= c) P[(j0 + r) + (long long)(j0 + c) * d.ldp] = (T)Dg[r + c * ld];
+    smem_ldlt<4>(Dg, ld, nb, nb, Wc, kMaxPivotBlock, [&](int k, double raw) {
+        const double piv = acc.accept(raw, d.first_col + j0 + k, ctl);
+        if (lane == 0) diag[d.first_col + j0 + k] = piv;
+        return piv;
+    });
+#pragma unroll 4
+    for (int e = tid; e < kMaxPivotBlock * nb; e += 128) {
+        const int r = e % kMaxPivotBlock, c = e / kMaxPivotBlock;
+        if (r >= c && r < nb) P[r + (long long)c * d.ldp] = (T)Dg[r + c * ld];
     }
     if (tid == 0) acc.flush(st);
 }
 
-// Rows [row0, row0+rows) under the pivot block (FP64 path): Y = F21 L11^-T
-// (forward substitution per row), L21 = Y / D.
-template <class T, class Cc, int NBMAX>
+// Rows under the pivot block (FP64 path): Y = F21 L11^-T (forward substitution
+// per row), L21 = Y / D.  Eight lanes a row, lane q holding columns q, q + 8, ...
+// (at pivot column k each lane has at most NBMAX / 8 - k / 8 entries to update:
+// 80 multiply-adds a lane for 32 columns where a thread per row takes 496 one
+// after another, 16 us); kTrsmRows rows a CTA, kTrsmSplit CTAs a task.
+constexpr int kTrsmRows = 16, kTrsmSplit = 128 / kTrsmRows;
+template <class T, int NBMAX>
 __global__ void __launch_bounds__(128) k_trsm(const PanelTask* __restrict__ tasks, const SnDev* __restrict__ sn,
                                               T* __restrict__ panel, const double* __restrict__ diag) {
-    __shared__ Cc L11[NBMAX * (NBMAX + 1)];
+    constexpr int NC = NBMAX / 8;
+    __shared__ double L11[NBMAX * (NBMAX + 1)];   // L11[k * (NBMAX + 1) + c], zero for c <= k
     __shared__ double dinv[NBMAX];
-    const PanelTask tk = tasks[blockIdx.x];
+    const PanelTask tk = tasks[blockIdx.x / kTrsmSplit];
+    const int sub = blockIdx.x % kTrsmSplit * kTrsmRows;
+    if (sub >= tk.rows) return;
     const SnDev d = sn[tk.s];
     const int nb = tk.nb, j0 = tk.j0, ld = NBMAX + 1;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    T* P = panel + d.panel_off;
-    for (int idx = tid; idx < nb * nb; idx += nt) {
-        int r = idx % nb, c = idx / nb;
-        L11[r + c * ld] = r > c ? (Cc)P[(j0 + r) + (long long)(j0 + c) * d.ldp] : Cc(0);
+    const int tid = threadIdx.x, lane = tid & 31, q = lane >> 2;
+    const int row = sub + 4 * (tid >> 5) + (lane & 3), i = tk.row0 + row;
+    T* P = panel + d.panel_off + (long long)j0 * d.ldp;
+    const bool live = row < tk.rows;
+    double a[NC];
+#pragma unroll
+    for (int t = 0; t < NC; ++t) a[t] = live && q + 8 * t < nb ? (double)P[i + (long long)(q + 8 * t) * d.ldp] : 0.0;
+#pragma unroll 8
+    for (int e = tid; e < NBMAX * NBMAX; e += 128) {
+        const int r = e % NBMAX, c = e / NBMAX;   // L(r, c)
+        L11[c * ld + r] = r > c && r < nb ? (double)P[j0 + r + (long long)c * d.ldp] : 0.0;
     }
-    if (tid < nb) dinv[tid] = 1.0 / diag[d.first_col + j0 + tid];
+    if (tid < NBMAX) dinv[tid] = tid < nb ? 1.0 / diag[d.first_col + j0 + tid] : 0.0;
     __syncthreads();
-    if (tid < tk.rows) {
-        const int i = tk.row0 + tid;
-        Cc y[NBMAX];
 #pragma unroll
-        for (int k = 0; k < NBMAX; ++k) {
-            if (k < nb) {
-                Cc v = (Cc)P[i + (long long)(j0 + k) * d.ldp];
+    for (int k = 0; k < NBMAX; ++k) {
+        if (k >= nb) break;
+        const double y = __shfl_sync(0xffffffffu, a[k / 8], (lane & 3) + 4 * (k & 7));
 #pragma unroll
-                for (int j = 0; j < k; ++j) v -= y[j] * L11[k + j * ld];
-                y[k] = v;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < NBMAX; ++k)
-            if (k < nb) P[i + (long long)(j0 + k) * d.ldp] = (T)((double)y[k] * dinv[k]);
+        for (int t = k / 8; t < NC; ++t) a[t] = fma(-y, L11[k * ld + q + 8 * t], a[t]);
     }
+#pragma unroll
+    for (int t = 0; t < NC; ++t)
+        if (live && q + 8 * t < nb) P[i + (long long)(q + 8 * t) * d.ldp] = (T)(a[t] * dinv[q + 8 * t]);
 }
 
-// SIMT tile update C[i, j] -= sum_k L[i,k] d_k L[j,k] over a 64 x 64 tile,
-// lower triangle only (i >= j).  Compute type C: double on the FP64 path,
-// float for the inner updates of the mixed path.
-template <class T, class C>
-__global__ void __launch_bounds__(256) k_simt_update(const UpdJob* __restrict__ jobs, int njobs,
-                                                     const SnDev* __restrict__ sn, T* __restrict__ panel,
-                                                     T* __restrict__ contrib, const double* __restrict__ diag) {
-    constexpr int TS = 64, KC = 32;
-    __shared__ C As[KC][TS + 1];
-    __shared__ C Bs[KC][TS + 1];
+// Update C[i, j] -= sum_k L[i,k] d_k L[j,k] of one TS x TS tile (lower triangle, i >= j), TS = 16 or 32: 2 or 8 us of
+// the SM's FP64 pipe at 32 columns (Launch::tile: 32 once that still makes two CTAs per SM).  Consecutive threads
+// hold consecutive rows of C.
+template <int TS>
+__host__ __device__ constexpr int simt_threads() { return TS == 32 ? 128 : 64; }
+template <class T, int TS>
+__global__ void __launch_bounds__(simt_threads<TS>()) k_simt_update(const UpdJob* __restrict__ jobs, int njobs,
+                                                                   const SnDev* __restrict__ sn, T* __restrict__ panel,
+                                                                   T* __restrict__ contrib, const double* __restrict__ diag) {
+    constexpr int KC = 32, NT = simt_threads<TS>(), NY = NT / 16, PI = TS / 16, QJ = TS / NY;
+    __shared__ double As[KC][TS];
+    __shared__ double Bs[KC][TS];
     const UpdJob J = jobs[find_job(jobs, njobs, blockIdx.x)];
     const SnDev d = sn[J.s];
-    TileTask tk;
-    tk.s = J.s;
-    tk.k0 = J.k0;
-    tk.kn = J.kn;
-    decode_tile(J, d, TS, (long long)blockIdx.x - J.tile_begin, tk.i0, tk.j0, tk.jend);
+    int i0, j0, jend;
+    decode_tile(J, d, TS, (long long)blockIdx.x - J.tile_begin, i0, j0, jend);
     const T* Pn = panel + d.panel_off;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    C acc[4][4];
+    // the tile's entries of C, in flight during the products
+    const bool in_panel = j0 < d.w;
+    T* base = in_panel ? panel : contrib;
+    long long off[PI][QJ];
+    double old[PI][QJ], acc[PI][QJ];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int q = 0; q < QJ; ++q)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = C(0);
-    for (int kc = 0; kc < tk.kn; kc += KC) {
-        const int kl = min(KC, tk.kn - kc);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < KC * TS; idx += 256) {
-            int r = idx % TS, k = idx / TS;
-            int kk = tk.k0 + kc + k;
-            C av = C(0), bv = C(0);
+        for (int p = 0; p < PI; ++p) {
+            const int j = j0 + ty + NY * q, i = i0 + tx + 16 * p;
+            const bool ok = j < jend && i < d.m && i >= j;
+            off[p][q] = !ok ? -1
+                            : in_panel ? d.panel_off + i + (long long)j * d.ldp
+                                       : d.contrib_off + (i - d.w) + (long long)(j - d.w) * d.ldc;
+            old[p][q] = ok ? (double)base[off[p][q]] : 0.0;
+            acc[p][q] = 0.0;
+        }
+    for (int kc = 0; kc < J.kn; kc += KC) {
+        const int kl = min(KC, J.kn - kc);
+        if (kc > 0) __syncthreads();
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < KC * TS; idx += NT) {
+            const int r = idx % TS, k = idx / TS, kk = J.k0 + kc + k;
+            double av = 0.0, bv = 0.0;
             if (k < kl) {
-                int i = tk.i0 + r, j = tk.j0 + r;
-                if (i < d.m) av = (C)Pn[i + (long long)kk * d.ldp];
-                if (j < d.m) bv = (C)((double)Pn[j + (long long)kk * d.ldp] * diag[d.first_col + kk]);
+                const int i = i0 + r, j = j0 + r;
+                if (i < d.m) av = (double)Pn[i + (long long)kk * d.ldp];
+                if (j < d.m) bv = (double)Pn[j + (long long)kk * d.ldp] * diag[d.first_col + kk];
             }
             As[k][r] = av;
             Bs[k][r] = bv;
         }
         __syncthreads();
+#pragma unroll 4
         for (int k = 0; k < kl; ++k) {
-            C a[4], b[4];
+            double a[PI], b[QJ];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                a[q] = As[k][ty + 16 * q];
-                b[q] = Bs[k][tx + 16 * q];
-            }
+            for (int p = 0; p < PI; ++p) a[p] = As[k][tx + 16 * p];
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
+            for (int q = 0; q < QJ; ++q) b[q] = Bs[k][ty + NY * q];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) acc[p][q] += a[p] * b[q];
+            for (int p = 0; p < PI; ++p)
+#pragma unroll
+                for (int q = 0; q < QJ; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
         }
     }
-    const bool in_panel = tk.j0 < d.w;
-    T* base = in_panel ? panel : contrib;
-    long long off[4][4];
-    T old[4][4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < QJ; ++q)
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const int j = tk.j0 + tx + 16 * q;
-            const int i = tk.i0 + ty + 16 * p;
-            const bool ok = j < tk.jend && i < d.m && i >= j;
-            off[p][q] = !ok ? -1
-                            : in_panel ? d.panel_off + i + (long long)j * d.ldp
-                                       : d.contrib_off + (i - d.w) + (long long)(j - d.w) * d.ldc;
-            old[p][q] = ok ? base[off[p][q]] : T(0);   // loads first, then stores: no serialised round trips
-        }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-            if (off[p][q] >= 0) base[off[p][q]] = (T)((C)old[p][q] - acc[p][q]);
+        for (int p = 0; p < PI; ++p)
+            if (off[p][q] >= 0) base[off[p][q]] = (T)(old[p][q] - acc[p][q]);
 }
 
 }  // namespace uchol_dev

@@ -254,7 +254,6 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
     P.stage.assign(count, StageInfo{0, 0, -1});
     const int PB = cfg.pivot_block;
     const int NB = cfg.tensor_core ? cfg.outer_block : cfg.pivot_block;
-    const int TS = cfg.tile;
     for (int L = 0; L < P.levels; ++L) {
         const auto& fronts = at_level[L];
         // extend-add: one item per receiving parent column.  With side_extend_add the items of
@@ -315,18 +314,23 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         }
         if (main_items > 0) P.launches.push_back({Launch::ExtendAdd, ib, main_items, 0});
 
-        // small fronts: one CTA each
-        int sb = (int)P.small_fronts.size();
+        // small fronts: up to 32 rows by 8, 16 or 32 lanes each, the others by a CTA each
         std::vector<int> large;
+        std::vector<int> small_by[4];
         for (int s : fronts) {
-            if (small_front(cfg, P.sn[s].m)) {
-                P.small_fronts.push_back(s);
-                P.max_small_m = std::max(P.max_small_m, P.sn[s].m);
-            } else {
-                large.push_back(s);
-            }
+            const int m = P.sn[s].m;
+            if (!small_front(cfg, m)) large.push_back(s);
+            else small_by[m <= 8 ? 0 : m <= 16 ? 1 : m <= 32 ? 2 : 3].push_back(s);
         }
-        if ((int)P.small_fronts.size() > sb) P.launches.push_back({Launch::SmallFronts, sb, (int)P.small_fronts.size() - sb, 0});
+        for (int c = 0; c < 4; ++c) {
+            if (small_by[c].empty()) continue;
+            Launch Ls{Launch::SmallFronts, (int)P.small_fronts.size(), (int)small_by[c].size(), 0};
+            Ls.variant = c == 3 ? 0 : 8 << c;
+            P.launches.push_back(Ls);
+            P.small_fronts.insert(P.small_fronts.end(), small_by[c].begin(), small_by[c].end());
+            if (c == 3)
+                for (int s : small_by[c]) P.max_small_m = std::max(P.max_small_m, P.sn[s].m);
+        }
 
         // large fronts: blocked right-looking factorisation in lockstep
         int max_w = 0;
@@ -398,8 +402,6 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
             for (int j0r = 0; j0r < NB; j0r += PB) {
                 int qb = (int)P.pivot_tasks.size();
                 int pb = (int)P.panel_tasks.size();
-                int ub = (int)P.simt_jobs.size();
-                long long utiles = 0;
                 for (int s : large) {
                     const SnDev& d = P.sn[s];
                     if (d.w <= k0) continue;
@@ -407,7 +409,6 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                     int j0 = k0 + j0r;
                     if (j0r >= nbo) continue;
                     int nbi = std::min(PB, k0 + nbo - j0);
-                    int outer_end = k0 + nbo;
                     P.pivot_tasks.push_back({s, j0, nbi, j0 + nbi, 0, -1, 0, 0});
                     // TRSM tasks over rows [j0+nbi, m)
                     int r = j0 + nbi;
@@ -418,37 +419,37 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                         P.panel_tasks.push_back({s, j0, nbi, r, rows, stage, 0, zero_to});
                         r += rows;
                     }
-                    // inner update of the rest of the outer block (tensor-core configuration only)
-                    if (NB != PB && j0 + nbi < outer_end) {
-                        UpdJob J{utiles, s, j0 + nbi, outer_end, j0, nbi, -1};
-                        utiles += job_tiles(J, d, TS);
-                        P.simt_flops += job_flops(J, d);
-                        P.simt_jobs.push_back(J);
-                    }
                 }
                 if ((int)P.pivot_tasks.size() > qb) P.launches.push_back({Launch::PivotBlock, qb, (int)P.pivot_tasks.size() - qb, 0});
                 if ((int)P.panel_tasks.size() > pb) P.launches.push_back({Launch::Trsm, pb, (int)P.panel_tasks.size() - pb, 0});
-                if ((int)P.simt_jobs.size() > ub)
-                    P.launches.push_back({Launch::SimtUpdate, ub, (int)P.simt_jobs.size() - ub, utiles});
                 if (!cfg.tensor_core) break;  // FP64 path: one pivot block per outer step
             }
-            // FP64 path: right-looking update of the whole trailing triangle per step
+            // FP64 path: right-looking update of the whole trailing triangle per step, in 32 x 32 tiles once they
+            // make two CTAs per SM, else 16 x 16 (an SM takes 8 or 2 us of FP64 pipe for one)
             if (!cfg.tensor_core) {
                 int jb = (int)P.simt_jobs.size();
-                long long tiles = 0;
+                long long tiles32 = 0;
                 for (int s : large) {
                     const SnDev& d = P.sn[s];
                     if (d.w <= k0) continue;
-                    int nbo = std::min(NB, d.w - k0);
-                    int c0 = k0 + nbo;
+                    const int nbo = std::min(NB, d.w - k0), c0 = k0 + nbo;
                     if (c0 >= d.m) continue;
-                    UpdJob J{tiles, s, c0, d.m, k0, nbo, -1};
-                    tiles += job_tiles(J, d, TS);
+                    UpdJob J{0, s, c0, d.m, k0, nbo, -1};
+                    tiles32 += job_tiles(J, d, 32);
                     P.simt_flops += job_flops(J, d);
                     P.simt_jobs.push_back(J);
                 }
-                if ((int)P.simt_jobs.size() > jb)
-                    P.launches.push_back({Launch::SimtUpdate, jb, (int)P.simt_jobs.size() - jb, tiles});
+                if ((int)P.simt_jobs.size() > jb) {
+                    const int TS = tiles32 >= 2LL * (cfg.sms > 0 ? cfg.sms : 152) ? 32 : 16;
+                    long long tiles = 0;
+                    for (int j = jb; j < (int)P.simt_jobs.size(); ++j) {
+                        P.simt_jobs[j].tile_begin = tiles;
+                        tiles += job_tiles(P.simt_jobs[j], P.sn[P.simt_jobs[j].s], TS);
+                    }
+                    Launch Lu{Launch::SimtUpdate, jb, (int)P.simt_jobs.size() - jb, tiles};
+                    Lu.variant = TS;
+                    P.launches.push_back(Lu);
+                }
             }
         }
         // tensor-core path: contribution block of every large front, K = its whole width

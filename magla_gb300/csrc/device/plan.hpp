@@ -26,7 +26,6 @@ struct PlanConfig {
     int pivot_block = 32;     // FP64 pivot block (the reference's PanelWidth)
     int outer_block = 32;     // Schur-update block (== pivot_block on the FP64 path)
     int small_mask = 0x7;     // bit b: fronts with 32b < m <= 32(b+1) are factorised by one CTA in shared memory
-    int tile = 64;            // SIMT tile edge (update kernels)
     bool tensor_core = false; // outer updates on tcgen05 from staged operands
     int solve_block = 64;     // column block of the triangular solves
     int inv_cols = 0;         // > 0: fronts of solve_block < w <= inv_cols columns keep the whole inverse of their
@@ -64,6 +63,7 @@ struct Launch {
     } kind;
     int begin, count;   // task range
     long long tiles;    // update launches: total tiles (= grid size)
+    int variant = 0;    // SmallFronts: lanes per front (8, 16, 32) or 0 (a CTA each); SimtUpdate: tile edge (16 or 32)
     int stream = 0;     // 0: main stream; 1: side stream, forked from the main stream at this point;
                         // 2: main stream after joining the side stream
 };
@@ -163,7 +163,7 @@ struct Plan {
     std::vector<StageInfo> stage;              // per supernode (tensor-core path)
     std::vector<int> map_front;                // front of each tensor-map pair
     std::vector<Launch> launches;
-    int max_small_m = 0;
+    int max_small_m = 0;                  // of the fronts taken by a CTA each
     long long stage_elems = 0;                 // elements of each operand staging arena (tensor-core path)
     double tc_flops = 0.0;                     // algorithmic flops of the tensor-core updates (lower triangle)
     double simt_flops = 0.0;                   // algorithmic flops of the SIMT updates
