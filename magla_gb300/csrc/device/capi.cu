@@ -918,7 +918,9 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
     int* status = F->solve_status.as<int>();
     CK(cudaMemsetAsync(fwd_flags, 0, sizeof(int) * ((size_t)2 * nblocks + P.progress_count), st));
     const size_t smem = level_smem_bytes<T, Cv, SB, RG>();
-    constexpr int RGD = RG == 1 ? 1 : 8;   // right-hand sides per CTA of the inverse-front diagonal kernels
+    constexpr int RGD = RG == 1 ? 1 : diag_rhs_group<T>();
+    // right-hand sides (groups of them) over the grid's second dimension
+    auto grid = [&](int count, int per) { return dim3((unsigned)count, (unsigned)std::min((nrhs + per - 1) / per, 65535)); };
     auto level_args = [&](const SolveLaunch& L, int* flags, int grid) {
         LevelArgs la;
         la.chains = tasks + L.begin;
@@ -954,24 +956,24 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
         if (L.count == 0) continue;
         if (timer) timer->begin((int)L.kind, st);
         if (L.kind == SolveLaunch::FwdGather) {
-            k_fwd_gather<Cv><<<dim3(L.count, std::min(nrhs, 65535)), 256, 0, st>>>(tasks + L.begin, A, work, fv);
+            k_fwd_gather<Cv><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, work, fv);
         } else if (L.kind == SolveLaunch::FwdSolo) {
-            k_fwd_solo<T, Cv, SB><<<L.count, 256, 0, st>>>(tasks + L.begin, A, panel, linv, fv, fv2, diag, work);
+            k_fwd_solo<T, Cv, SB><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, linv, fv, fv2, diag, work);
         } else if (L.kind == SolveLaunch::FwdInvDiag) {
-            k_fwd_inv_diag<T, Cv, SB, RGD><<<dim3(L.count, (nrhs + RGD - 1) / RGD), 256, inv_solve_smem<T, Cv, SB, RGD>(), st>>>(
+            k_fwd_inv_diag<T, Cv, SB, RGD><<<grid(L.count, RGD), 256, inv_solve_smem<T, Cv, SB, RGD>(), st>>>(
                 tasks + L.begin, A, linv, F->linv_off.as<Cv>(), fv, fv2, diag, work, F->inv_diag_partial.as<Cv>(),
                 F->inv_diag_cnt.as<unsigned>(), status);
         } else if (L.kind == SolveLaunch::FwdInvTail) {
-            k_fwd_inv_tail<T, Cv, SB, RG><<<L.count, 256, inv_tail_smem<T, Cv, SB, RG, false>(), st>>>(
+            k_fwd_inv_tail<T, Cv, SB, RG><<<grid(L.count, RG), 256, inv_tail_smem<T, Cv, SB, RG, false>(), st>>>(
                 tasks + L.begin, A, F->solve_maps.as<CUtensorMap>() + P.count, fv2, fv, status);
         } else if (L.kind == SolveLaunch::FwdTail) {
             if (nrhs == 1)
-                k_fwd_tail<T, Cv, SB, 1><<<L.count, kTailRows / 4, 0, st>>>(tasks + L.begin, A, panel, fv2, fv);
+                k_fwd_tail<T, Cv, SB, 1><<<L.count, tail_threads<T>(), 0, st>>>(tasks + L.begin, A, panel, fv2, fv);
             else
-                k_fwd_tail<T, Cv, SB, 4><<<L.count, kTailRows / 4, 0, st>>>(tasks + L.begin, A, panel, fv2, fv);
+                k_fwd_tail<T, Cv, SB, 4><<<grid(L.count, 4), tail_threads<T>(), 0, st>>>(tasks + L.begin, A, panel, fv2, fv);
         } else {
-            const int grid = F->coop_fwd;
-            launch_cooperative(k_fwd_level<T, Cv, SB, RG>, grid, 256, smem, st, level_args(L, fwd_flags, grid), A, panel,
+            const int ctas = F->coop_fwd;
+            launch_cooperative(k_fwd_level<T, Cv, SB, RG>, ctas, 256, smem, st, level_args(L, fwd_flags, ctas), A, panel,
                                linv, fv, fv2, diag, work);
         }
         if (timer) timer->end(st);
@@ -980,34 +982,32 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
         if (L.count == 0) continue;
         if (timer) timer->begin((int)L.kind, st);
         if (L.kind == SolveLaunch::BwdGather) {
-            k_bwd_gather<Cv><<<dim3(L.count, std::min(nrhs, 65535)), 256, 0, st>>>(tasks + L.begin, A, work, fv);
+            k_bwd_gather<Cv><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, work, fv);
         } else if (L.kind == SolveLaunch::BwdTail) {
-            k_bwd_cols<T, Cv, RG><<<L.count, 256, 0, st>>>(tasks + L.begin, A, panel, fv, F->bwd_partial.as<Cv>());
+            k_bwd_cols<T, Cv, RG><<<grid(L.count, RG), 256, 0, st>>>(tasks + L.begin, A, panel, fv, F->bwd_partial.as<Cv>());
         } else if (L.kind == SolveLaunch::BwdTailReduce) {
             k_bwd_cols_reduce<Cv><<<L.count, 128, 0, st>>>(tasks + L.begin, A, F->bwd_partial.as<Cv>(), fv);
         } else if (L.kind == SolveLaunch::BwdInvCols) {
-            k_bwd_inv_cols<T, Cv, SB, RG><<<L.count, 256, inv_tail_smem<T, Cv, SB, RG, true>(), st>>>(
+            k_bwd_inv_cols<T, Cv, SB, RG><<<grid(L.count, RG), 256, inv_tail_smem<T, Cv, SB, RG, true>(), st>>>(
                 tasks + L.begin, A, F->solve_maps.as<CUtensorMap>() + 2 * P.count, fv, F->inv_partial.as<Cv>(), status);
         } else if (L.kind == SolveLaunch::BwdInvReduce) {
-            k_bwd_inv_reduce<Cv, SB><<<dim3(L.count, std::min(nrhs, 65535)), SB, 0, st>>>(tasks + L.begin, A, fv,
+            k_bwd_inv_reduce<Cv, SB><<<grid(L.count, 1), SB, 0, st>>>(tasks + L.begin, A, fv,
                                                                                         F->inv_partial.as<Cv>());
         } else if (L.kind == SolveLaunch::BwdInvDiag) {
-            k_bwd_inv_diag<T, Cv, SB, RGD><<<dim3(L.count, (nrhs + RGD - 1) / RGD), 256, inv_solve_smem<T, Cv, SB, RGD>(), st>>>(
+            k_bwd_inv_diag<T, Cv, SB, RGD><<<grid(L.count, RGD), 256, inv_solve_smem<T, Cv, SB, RGD>(), st>>>(
                 tasks + L.begin, A, linv, F->linv_off.as<Cv>(), fv, work, F->inv_diag_partial.as<Cv>(),
                 F->inv_diag_cnt.as<unsigned>(), status);
         } else if (L.kind == SolveLaunch::BwdSolo) {
-            k_bwd_solo<Cv, SB><<<L.count, 256, 0, st>>>(tasks + L.begin, A, linv, fv, fv2, work);
+            k_bwd_solo<Cv, SB><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, linv, fv, fv2, work);
         } else {
-            const int grid = F->coop_bwd;
-            launch_cooperative(k_bwd_level<T, Cv, SB, RG>, grid, 256, smem, st, level_args(L, bwd_flags, grid), A, panel,
+            const int ctas = F->coop_bwd;
+            launch_cooperative(k_bwd_level<T, Cv, SB, RG>, ctas, 256, smem, st, level_args(L, bwd_flags, ctas), A, panel,
                                linv, fv, fv2, work);
         }
         if (timer) timer->end(st);
     }
     CK(cudaGetLastError());
 }
-
-static_assert(kTailRows == kTailRowsPlan, "forward tail chunk of the plan and the kernel");
 
 int solve_launch_count(const Plan& P) {
     int c = 0;
@@ -1020,6 +1020,7 @@ int solve_launch_count(const Plan& P) {
 // CUDA graph over the factor's fixed work buffers and replayed on each call.
 template <class T, class Cv, int SB>
 void launch_solve_graph(uchol_factor_s* F, int nrhs, Cv* work, cudaStream_t st) {
+    constexpr int RGM = solve_rhs_group<T>(), RGD = diag_rhs_group<T>();
     if (!F->solve_graph || F->solve_graph_nrhs != nrhs) {
         if (F->solve_graph) {
             CK(cudaGraphExecDestroy(F->solve_graph));
@@ -1039,25 +1040,20 @@ void launch_solve_graph(uchol_factor_s* F, int nrhs, Cv* work, cudaStream_t st) 
         if (nrhs == 1)
             level_kernels(k_fwd_level<T, Cv, SB, 1>, k_bwd_level<T, Cv, SB, 1>, (int)level_smem_bytes<T, Cv, SB, 1>());
         else
-            level_kernels(k_fwd_level<T, Cv, SB, kSolveRhsGroup>, k_bwd_level<T, Cv, SB, kSolveRhsGroup>,
-                          (int)level_smem_bytes<T, Cv, SB, kSolveRhsGroup>());
+            level_kernels(k_fwd_level<T, Cv, SB, RGM>, k_bwd_level<T, Cv, SB, RGM>,
+                          (int)level_smem_bytes<T, Cv, SB, RGM>());
         // inverse-front kernels of both groupings
-        CK(cudaFuncSetAttribute(k_fwd_inv_diag<T, Cv, SB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_solve_smem<T, Cv, SB, 1>()));
-        CK(cudaFuncSetAttribute(k_fwd_inv_diag<T, Cv, SB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_solve_smem<T, Cv, SB, 8>()));
-        CK(cudaFuncSetAttribute(k_bwd_inv_diag<T, Cv, SB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_solve_smem<T, Cv, SB, 1>()));
-        CK(cudaFuncSetAttribute(k_bwd_inv_diag<T, Cv, SB, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_solve_smem<T, Cv, SB, 8>()));
-        CK(cudaFuncSetAttribute(k_fwd_inv_tail<T, Cv, SB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_tail_smem<T, Cv, SB, 1, false>()));
-        CK(cudaFuncSetAttribute(k_fwd_inv_tail<T, Cv, SB, kSolveRhsGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_tail_smem<T, Cv, SB, kSolveRhsGroup, false>()));
-        CK(cudaFuncSetAttribute(k_bwd_inv_cols<T, Cv, SB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_tail_smem<T, Cv, SB, 1, true>()));
-        CK(cudaFuncSetAttribute(k_bwd_inv_cols<T, Cv, SB, kSolveRhsGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)inv_tail_smem<T, Cv, SB, kSolveRhsGroup, true>()));
+        auto limit = [&](auto* kernel, size_t bytes) {
+            CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        };
+        limit(k_fwd_inv_diag<T, Cv, SB, 1>, inv_solve_smem<T, Cv, SB, 1>());
+        limit(k_fwd_inv_diag<T, Cv, SB, RGD>, inv_solve_smem<T, Cv, SB, RGD>());
+        limit(k_bwd_inv_diag<T, Cv, SB, 1>, inv_solve_smem<T, Cv, SB, 1>());
+        limit(k_bwd_inv_diag<T, Cv, SB, RGD>, inv_solve_smem<T, Cv, SB, RGD>());
+        limit(k_fwd_inv_tail<T, Cv, SB, 1>, inv_tail_smem<T, Cv, SB, 1, false>());
+        limit(k_fwd_inv_tail<T, Cv, SB, RGM>, inv_tail_smem<T, Cv, SB, RGM, false>());
+        limit(k_bwd_inv_cols<T, Cv, SB, 1>, inv_tail_smem<T, Cv, SB, 1, true>());
+        limit(k_bwd_inv_cols<T, Cv, SB, RGM>, inv_tail_smem<T, Cv, SB, RGM, true>());
         if (F->coop_fwd < 2 || F->coop_bwd < 2) throw Error(UCHOL_CUDA_ERROR, "the level solve kernels do not fit");
         if (!F->solve_maps.p) {
             // tile copies of the solves: each front's panel (m x w), in boxes of SB x SB (level
@@ -1101,7 +1097,7 @@ void launch_solve_graph(uchol_factor_s* F, int nrhs, Cv* work, cudaStream_t st) 
             if (nrhs == 1)
                 run_solve<T, Cv, SB, 1>(F, nrhs, work, F->fv.as<Cv>(), F->fv2.as<Cv>(), F->capture_stream);
             else
-                run_solve<T, Cv, SB, kSolveRhsGroup>(F, nrhs, work, F->fv.as<Cv>(), F->fv2.as<Cv>(), F->capture_stream);
+                run_solve<T, Cv, SB, RGM>(F, nrhs, work, F->fv.as<Cv>(), F->fv2.as<Cv>(), F->capture_stream);
         } catch (...) {
             cudaStreamEndCapture(F->capture_stream, &g);
             if (g) cudaGraphDestroy(g);
@@ -1120,7 +1116,7 @@ void launch_solve_graph(uchol_factor_s* F, int nrhs, Cv* work, cudaStream_t st) 
         if (nrhs == 1)
             run_solve<T, Cv, SB, 1>(F, nrhs, work, F->fv.as<Cv>(), F->fv2.as<Cv>(), st, &timer);
         else
-            run_solve<T, Cv, SB, kSolveRhsGroup>(F, nrhs, work, F->fv.as<Cv>(), F->fv2.as<Cv>(), st, &timer);
+            run_solve<T, Cv, SB, RGM>(F, nrhs, work, F->fv.as<Cv>(), F->fv2.as<Cv>(), st, &timer);
         CK(cudaStreamSynchronize(st));
         timer.collect(F->phases);
         counted(F->solve_graph_nodes);

@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "plan.hpp"
 
 namespace uchol_dev {
 
@@ -52,13 +53,36 @@ __global__ void k_finish_scale(PivotStats* st, FactorCtl* ctl, double pivot_tole
     ctl->allow_regularization = allow;
 }
 
+// 1 / p for p > 0 without a division's FP64 instructions (64 cycles each): the FP32 reciprocal of p's leading bits as
+// x0, then one third-order Newton step, x = x0 + x0 (e + e^2) with e = 1 - p x0.  |e| < 2^-21, so the step's own error
+// is below 2^-63 and x is 1 / p rounded once (0.5003 ulp at most).  p outside 2^+-120 is divided.
+__device__ __forceinline__ double reciprocal(double p) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(p);
+    const unsigned e = (unsigned)(b >> 52);
+    if (e - (1023u - 120u) > 240u) return 1.0 / p;
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(((e - 1023u + 127u) << 23) | ((unsigned)(b >> 29) & 0x7fffffu))));
+    const unsigned rb = __float_as_uint(r);
+    const double x0 = __longlong_as_double((long long)(((unsigned long long)((rb >> 23) + (1023u - 127u)) << 52) |
+                                                       ((unsigned long long)(rb & 0x7fffffu) << 29)));
+    const double err = fma(-p, x0, 1.0);
+    return fma(x0, fma(err, err, err), x0);
+}
+
 // Pivot acceptance exactly as the reference: !(d > tol*scale) (which also
 // catches NaN) is regularised or rejected (UtduNumericFactorization.cs:557-575).
+// The comparison is on the bits, which order like the numbers here: the threshold is
+// not negative, a negative d has the sign bit, a NaN lies past infinity.
 struct PivotAcc {
     int regularized = 0, negative = 0, failed = INT_MAX;
     unsigned long long min_bits = 0x7fefffffffffffffull, max_bits = 0;
+    static __device__ __forceinline__ bool above(double piv, double threshold) {
+        constexpr long long kInf = 0x7ff0000000000000ll;
+        const long long t = __double_as_longlong(threshold), b = __double_as_longlong(piv);
+        return b > t && b <= kInf && (unsigned long long)t <= (unsigned long long)kInf;   // a NaN threshold rejects
+    }
     __device__ __forceinline__ double accept(double piv, int column, const FactorCtl& ctl) {
-        if (!(piv > ctl.threshold)) {
+        if (!above(piv, ctl.threshold)) {
             if (!ctl.allow_regularization) failed = min(failed, column);
             if (piv < 0.0) ++negative;
             ++regularized;
@@ -185,7 +209,7 @@ __global__ void __launch_bounds__(kLaneFrontThreads) k_small_fronts_lanes(const 
         const bool live = k < w;   // the same in the front's lanes
         const double raw = __shfl_sync(0xffffffffu, a[0], k, LW);
         const double piv = live ? acc.accept(raw, d.first_col + k, ctl) : 1.0;
-        const double inv = 1.0 / piv;
+        const double inv = reciprocal(piv);
         const double wk = a[0];
         const double l = live && r > k && r < m ? wk * inv : 0.0;
         if (live && r >= k && r < m) P[r + (long long)k * d.ldp] = r == k ? (T)1 : (T)l;
@@ -214,41 +238,82 @@ __global__ void __launch_bounds__(kLaneFrontThreads) k_small_fronts_lanes(const 
     if ((threadIdx.x & 31) == 0) acc.flush(st);
 }
 
-// LDL^T of the first w columns of the m x m matrix at S (column-major, leading dimension ld, lower triangle) in
-// shared memory, by kWarps warps: warp 0 is the chain (pivot, division, the scaled column, the next column's update),
-// the others update the columns after that; one barrier a pivot.  Wc: two buffers of wstride entries for the
-// unscaled column.
-template <int kWarps, class Pivot>
+// LDL^T of the first w columns of the m x m matrix at S (column-major, leading dimension ld, lower triangle,
+// m <= 32 NQ) in shared memory, by kWarps warps: warp 0 is the chain (its current column in registers: pivot,
+// reciprocal, the scaled column, the next column's update), the others update the columns after that, four at a time
+// (loads of all four, then the products, then the stores: one at a time, the latencies of one column after another
+// made the others the chain's bottleneck); one barrier a pivot.  Wc: two buffers of wstride entries for the unscaled
+// column.
+template <int kWarps, int NQ, class Pivot>
 __device__ __forceinline__ void smem_ldlt(double* S, int ld, int m, int w, double* Wc, int wstride, Pivot&& pivot) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = 0; k < w; ++k) {
-        double* W = Wc + (k & 1) * wstride;
-        double* Lk = S + (long long)k * ld;
-        if (warp == 0) {
-            const double piv = pivot(k, Lk[k]);
-            const double inv = 1.0 / piv;
-            __syncwarp();
-            for (int i = k + 1 + lane; i < m; i += 32) {
-                const double v = Lk[i];
-                W[i] = v;
-                Lk[i] = v * inv;
+    if (warp == 0) {
+        double c[NQ];   // rows lane + 32 q of the current column
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) c[q] = lane + 32 * q < m ? S[lane + 32 * q] : 0.0;
+        for (int k = 0; k < w; ++k) {
+            double* W = Wc + (k & 1) * wstride;
+            double* Lk = S + (long long)k * ld;
+            double mine = 0.0, after = 0.0;   // rows k and k + 1 of the column, in their lanes
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                if (q == k >> 5) mine = c[q];
+                if (q == (k + 1) >> 5) after = c[q];
             }
-            if (lane == 0) Lk[k] = 1.0;
+            const double piv = pivot(k, __shfl_sync(0xffffffffu, mine, k & 31));
+            const double wj = __shfl_sync(0xffffffffu, after, (k + 1) & 31);
+            const double inv = reciprocal(piv);
+            double l[NQ];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const int i = lane + 32 * q;
+                if (32 * q + 31 <= k || 32 * q >= m) continue;
+                l[q] = i == k ? 1.0 : c[q] * inv;
+                if (i >= k && i < m) {
+                    W[i] = c[q];
+                    Lk[i] = l[q];
+                }
+            }
+            if (k % 32 == 31 && lane == 31) Lk[k] = 1.0;   // row k is the last of a group that the loop left out
+            __syncthreads();
+            if (k + 1 < w) {
+                const double* n = S + (long long)(k + 1) * ld;
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    const int i = lane + 32 * q;
+                    if (32 * q + 31 <= k || 32 * q >= m) continue;
+                    c[q] = fma(-l[q], wj, i < m ? n[i] : 0.0);
+                }
+            }
         }
-        __syncthreads();
-        const bool next = k + 1 < w;   // the next column is the chain's
-        if (warp == 0) {
-            if (next) {
-                double* c = S + (long long)(k + 1) * ld;
-                const double wj = W[k + 1];
-                for (int i = k + 1 + lane; i < m; i += 32) c[i] = fma(-Lk[i], wj, c[i]);
-                __syncwarp();
-            }
-        } else {
-            for (int j = k + 1 + (next ? 1 : 0) + warp - 1; j < m; j += kWarps - 1) {
-                double* c = S + (long long)j * ld;
-                const double wj = W[j];
-                for (int i = j + lane; i < m; i += 32) c[i] = fma(-Lk[i], wj, c[i]);
+    } else {
+        for (int k = 0; k < w; ++k) {
+            __syncthreads();
+            const double* W = Wc + (k & 1) * wstride;
+            const double* Lk = S + (long long)k * ld;
+            const int first = k + 1 + (k + 1 < w ? 1 : 0) + warp - 1;   // the next column is the chain's
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const int i = lane + 32 * q, last = min(m - 1, 32 * q + 31);   // columns up to this group's last row
+                if (32 * q >= m || first > last) continue;
+                const double li = i > k && i < m ? Lk[i] : 0.0;
+                for (int j = first; j <= last; j += 4 * (kWarps - 1)) {
+                    double v[4], x[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int jj = j + u * (kWarps - 1);
+                        const bool on = jj <= last;
+                        x[u] = on ? W[jj] : 0.0;
+                        v[u] = on && i >= jj && i < m ? S[i + (long long)jj * ld] : 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int jj = j + u * (kWarps - 1);
+                        if (jj > last) break;
+                        v[u] = fma(-li, x[u], v[u]);
+                        if (i >= jj && i < m) S[i + (long long)jj * ld] = v[u];
+                    }
+                }
             }
         }
     }
@@ -279,7 +344,7 @@ __global__ void __launch_bounds__(kSmallFrontThreads) k_small_fronts(const int* 
     }
     PivotAcc acc;
     __syncthreads();
-    smem_ldlt<kWarps>(S, ld, m, w, S + (size_t)m * m, m, [&](int k, double raw) {
+    smem_ldlt<kWarps, kSmallFrontLimit / 32>(S, ld, m, w, S + (size_t)m * m, m, [&](int k, double raw) {
         const double piv = acc.accept(raw, d.first_col + k, ctl);
         if (lane == 0) diag[d.first_col + k] = piv;
         return piv;
@@ -317,7 +382,7 @@ __global__ void __launch_bounds__(128) k_pivot_block(const PanelTask* __restrict
     }
     PivotAcc acc;
     __syncthreads();
-    smem_ldlt<4>(Dg, ld, nb, nb, Wc, kMaxPivotBlock, [&](int k, double raw) {
+    smem_ldlt<4, kMaxPivotBlock / 32>(Dg, ld, nb, nb, Wc, kMaxPivotBlock, [&](int k, double raw) {
         const double piv = acc.accept(raw, d.first_col + j0 + k, ctl);
         if (lane == 0) diag[d.first_col + j0 + k] = piv;
         return piv;
@@ -359,7 +424,7 @@ __global__ void __launch_bounds__(128) k_trsm(const PanelTask* __restrict__ task
         const int r = e % NBMAX, c = e / NBMAX;   // L(r, c)
         L11[c * ld + r] = r > c && r < nb ? (double)P[j0 + r + (long long)c * d.ldp] : 0.0;
     }
-    if (tid < NBMAX) dinv[tid] = tid < nb ? 1.0 / diag[d.first_col + j0 + tid] : 0.0;
+    if (tid < NBMAX) dinv[tid] = tid < nb ? reciprocal(diag[d.first_col + j0 + tid]) : 0.0;
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NBMAX; ++k) {
@@ -377,12 +442,12 @@ __global__ void __launch_bounds__(128) k_trsm(const PanelTask* __restrict__ task
 // the SM's FP64 pipe at 32 columns (Launch::tile: 32 once that still makes two CTAs per SM).  Consecutive threads
 // hold consecutive rows of C.
 template <int TS>
-__host__ __device__ constexpr int simt_threads() { return TS == 32 ? 128 : 64; }
+__host__ __device__ constexpr int simt_threads() { return 128; }   // a warp per scheduler
 template <class T, int TS>
 __global__ void __launch_bounds__(simt_threads<TS>()) k_simt_update(const UpdJob* __restrict__ jobs, int njobs,
                                                                    const SnDev* __restrict__ sn, T* __restrict__ panel,
                                                                    T* __restrict__ contrib, const double* __restrict__ diag) {
-    constexpr int KC = 32, NT = simt_threads<TS>(), NY = NT / 16, PI = TS / 16, QJ = TS / NY;
+    constexpr int KC = 32, NT = simt_threads<TS>(), NY = NT / 16, PI = TS / 16, QJ = TS / NY;   // rows, columns of a thread
     __shared__ double As[KC][TS];
     __shared__ double Bs[KC][TS];
     const UpdJob J = jobs[find_job(jobs, njobs, blockIdx.x)];

@@ -343,6 +343,10 @@ __global__ void __launch_bounds__(256, 1) k_fwd_inv_diag(const SolveBlockTask* _
     }
 }
 
+// Right-hand sides per CTA of the inverse-front diagonal kernels.
+template <class T>
+__host__ __device__ constexpr int diag_rhs_group() { return sizeof(T) == 8 ? 4 : 8; }
+
 // Register tiles of the trailing-row kernels.  A thread accumulates RT rows (forward) or
 // RT columns (backward) by GT right-hand sides; RT elements are 16 bytes, so the forward
 // kernel reads them as one vector.  NG groups of RT rows (columns) cover SB, NH groups of
@@ -370,7 +374,7 @@ constexpr size_t inv_tail_smem() {
 }
 static_assert((size_t)TailTiles<float, 128, 16>::NS * 128 * 16 * sizeof(float) <= (size_t)128 * 128 * sizeof(float),
               "the partial sums fit in the tile stages");
-static_assert((size_t)TailTiles<double, 64, 16>::NS * 64 * 16 * sizeof(double) <= (size_t)64 * 64 * sizeof(double),
+static_assert((size_t)TailTiles<double, 64, 4>::NS * 64 * 4 * sizeof(double) <= (size_t)64 * 64 * sizeof(double),
               "the partial sums fit in the tile stages");
 
 // Starts a tensor-map tile copy of `bytes` bytes at (x, y) into dst, completing on bar (one thread).
@@ -449,7 +453,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_inv_tail(const SolveBlockTask* _
     __syncthreads();
     unsigned phase = 0;
     RhsPrefetch<Cv, HC, RG> pf;
-    for (int rg = 0; rg < A.nrhs; rg += RG) {
+    for (int rg = blockIdx.y * RG; rg < A.nrhs; rg += gridDim.y * RG) {
         const int ng = min(RG, A.nrhs - rg);
         auto fetch = [&](int h) {
             const int kn = min(HC, d.w - h * HC);
@@ -547,7 +551,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* _
     __syncthreads();
     unsigned phase = 0;
     RhsPrefetch<Cv, HR, RG> pf;
-    for (int rg = 0; rg < A.nrhs; rg += RG) {
+    for (int rg = blockIdx.y * RG; rg < A.nrhs; rg += gridDim.y * RG) {
         const int ng = min(RG, A.nrhs - rg);
         auto fetch = [&](int t) {
             const int tr = ra + t * HR;

@@ -619,8 +619,9 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         for (int s : fronts) {
             const SnDev& d = P.sn[s];
             if (d.w > SB || d.m == d.w) continue;
-            for (int r = d.w & ~3; r < d.m; r += kTailRowsPlan)
-                P.solve_tasks.push_back({s, 0, d.w, r, std::min(d.m, r + kTailRowsPlan), 0, 0});
+            const int height = cfg.tensor_core ? kTailRowsPlan : kTailRowsPlan64;
+            for (int r = d.w & ~3; r < d.m; r += height)
+                P.solve_tasks.push_back({s, 0, d.w, r, std::min(d.m, r + height), 0, 0});
         }
         if ((int)P.solve_tasks.size() > tb)
             P.fwd_launches.push_back({SolveLaunch::FwdTail, tb, (int)P.solve_tasks.size() - tb, 0, 0, 0, 0, 0, 0, 0, 0, 0});
@@ -667,7 +668,8 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         for (int s : fronts) {
             const SnDev& d = P.sn[s];
             if (d.m == d.w || inv_ob[s] >= 0) continue;
-            const int nch = (d.m - d.w + kColRowsPlan - 1) / kColRowsPlan;
+            const int height = cfg.tensor_core ? kColRowsPlan : kColRowsPlan64;
+            const int nch = (d.m - d.w + height - 1) / height;
             for (int c = 0; c < d.w; c += 8) {
                 const int kn = std::min(8, d.w - c);
                 if (nch == 1) {
@@ -676,8 +678,8 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 }
                 reduce.push_back({s, c, kn, slot, nch, 0, 0});
                 for (int q = 0; q < nch; ++q) {
-                    const int r0 = d.w + q * kColRowsPlan;
-                    P.solve_tasks.push_back({s, c, kn, r0, std::min(d.m, r0 + kColRowsPlan), 1, slot++});
+                    const int r0 = d.w + q * height;
+                    P.solve_tasks.push_back({s, c, kn, r0, std::min(d.m, r0 + height), 1, slot++});
                 }
             }
         }

@@ -13,8 +13,10 @@
 namespace uchol_dev {
 
 constexpr int kSolveRowsPlan = 128;   // rows per panel-solve task (kSolveRows of the kernel)
-constexpr int kTailRowsPlan = 1024;  // trailing rows per forward tail task (kTailRows of the kernel)
+constexpr int kTailRowsPlan = 1024;  // trailing rows per forward tail task, mixed path
+constexpr int kTailRowsPlan64 = 128; // and FP64 (its products hold the SM's FP64 pipe: 2 us at 64 columns)
 constexpr int kColRowsPlan = 2048;   // trailing rows per backward column-dot task (longer columns: partial sums)
+constexpr int kColRowsPlan64 = 1024; // and FP64
 constexpr int kInvColRowsPlan = 1024;   // trailing rows per backward partial-sum task of an inverse front
 constexpr int kDefaultInvCols = 2048;   // widest front whose diagonal block is kept inverted for the solves
 constexpr int kSuperBlocks = 4;       // tensor-core path: outer blocks per super-block of the own-column updates

@@ -227,7 +227,10 @@ __global__ void __launch_bounds__(256) k_invert_cta(const SolveBlockTask* __rest
 // or counter of step b-1, so no CTA can block its own producer.
 
 constexpr size_t kLevelSmemSlack = 1024;                      // alignment slack of the level kernels' dynamic smem
-constexpr int kSolveRhsGroup = 16;                            // right-hand sides per group of the multi-column solves
+// Right-hand sides per group of the multi-column solves: 16 share each FP32 tile; in FP64 the pipe bounds the products
+// (two multiply-adds a clock and SM), so groups of four make more CTAs of the same work.
+template <class T>
+__host__ __device__ constexpr int solve_rhs_group() { return sizeof(T) == 8 ? 4 : 16; }
 constexpr int kSolveStatusTimeout = 2;
 
 __device__ __forceinline__ unsigned long long solve_ns() {
@@ -1015,38 +1018,44 @@ __global__ void __launch_bounds__(256, 1) k_bwd_level(LevelArgs L, SolveArgs A, 
 // Fronts of one diagonal block (most fronts low in the tree) need no chain:
 // one CTA per front solves its block and, forward, updates its trailing rows.
 
-// Forward: y = L_0^-1 f_0 (thread per row), y / D to the work vector, then
-// f[i] -= L[i, 0:w] y for the trailing rows (thread per row, coalesced columns).
+// Forward: y = L_0^-1 f_0, y / D to the work vector.  Thread (row, part): the row's sum over its part of the columns
+// (the inverse is zero above its diagonal), eight loads in flight; right-hand sides blockIdx.y, + gridDim.y, ...
 template <class T, class Cv, int SB>
 __global__ void __launch_bounds__(256) k_fwd_solo(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
-                                                  const T* __restrict__ panel, const Cv* __restrict__ linv,
-                                                  Cv* __restrict__ fv, Cv* __restrict__ yv,
-                                                  const double* __restrict__ diag, Cv* __restrict__ work) {
+                                                  const Cv* __restrict__ linv, const Cv* __restrict__ fv,
+                                                  Cv* __restrict__ yv, const double* __restrict__ diag,
+                                                  Cv* __restrict__ work) {
+    constexpr int NP = 256 / SB;
     __shared__ Cv f0[SB];
-    __shared__ Cv y[SB];
+    __shared__ Cv part[NP][SB];
     const SolveBlockTask tk = tasks[blockIdx.x];
     const SnDev d = A.sn[tk.s];
-    const int w = d.w, tid = threadIdx.x;
-    const Cv* Li = linv + (long long)tk.blk * SB * SB;
-    const T* P = panel + d.panel_off;
-    for (int r = 0; r < A.nrhs; ++r) {
+    const int w = d.w, tid = threadIdx.x, row = tid % SB, p = tid / SB;
+    const int per = (w + NP - 1) / NP, k0 = p * per, k1 = min(w, k0 + per);
+    const Cv* Li = linv + (long long)tk.blk * SB * SB + row;
+    for (int r = blockIdx.y; r < A.nrhs; r += gridDim.y) {
         const long long base = A.fvec_off[tk.s] + r * A.fv_stride;
-        Cv* f = fv + base;
         __syncthreads();
-        for (int t = tid; t < w; t += blockDim.x) f0[t] = f[t];
+        if (tid < w) f0[tid] = fv[base + tid];
         __syncthreads();
-        for (int t = tid; t < w; t += blockDim.x) {
-            Cv a0 = Cv(0), a1 = Cv(0);
-            int k = 0;
-            for (; k + 1 <= t; k += 2) {
-                a0 += Li[t + k * SB] * f0[k];
-                a1 += Li[t + (k + 1) * SB] * f0[k + 1];
+        Cv a = Cv(0);
+        if (row < w)
+            for (int k = k0; k < k1; k += 8) {
+                Cv v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = k + u < k1 ? Li[(k + u) * SB] : Cv(0);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (k + u < k1) a += v[u] * f0[k + u];
             }
-            for (; k <= t; ++k) a0 += Li[t + k * SB] * f0[k];
-            const Cv v = a0 + a1;
-            y[t] = v;
-            yv[base + t] = v;
-            work[d.first_col + t + (long long)r * A.ldw] = (Cv)((double)v / diag[d.first_col + t]);
+        part[p][row] = a;
+        __syncthreads();
+        if (tid < w) {
+            Cv v = part[0][tid];
+#pragma unroll
+            for (int q = 1; q < NP; ++q) v += part[q][tid];
+            yv[base + tid] = v;
+            work[d.first_col + tid + (long long)r * A.ldw] = (Cv)((double)v / diag[d.first_col + tid]);
         }
     }
 }
@@ -1068,22 +1077,30 @@ __device__ __forceinline__ void load4(const double* p, double* v) {
 }
 
 // Forward, trailing rows of single-block fronts (after k_fwd_solo): f[i] -= sum_k L[i, k] y[k]
-// for rows [r0, r1) of the task's front (r0 a multiple of 4; rows below w are skipped).
-// Four consecutive rows per thread, one aligned group per column, eight columns in flight,
-// so a front's trailing block streams at HBM speed over many CTAs instead of one.  The
-// right-hand sides go in groups of G: each factor entry is read once per group.
-constexpr int kTailRows = 1024;
+// for rows [r0, r1) of the task's front (r0 a multiple of 4; rows below w are skipped).  RT consecutive rows per
+// thread: four in FP32 (16-byte loads); one in FP64, where a CTA of 1024 rows would hold its SM's FP64 pipe for
+// 16 us.  Eight columns are in flight, and the right-hand sides go in groups of G (blockIdx.y, + gridDim.y, ...):
+// each factor entry is read once per group.
+template <class T>
+__host__ __device__ constexpr int tail_rows() { return sizeof(T) == 8 ? kTailRowsPlan64 : kTailRowsPlan; }
+template <class T>
+__host__ __device__ constexpr int tail_threads() { return sizeof(T) == 8 ? kTailRowsPlan64 : kTailRowsPlan / 4; }
 template <class T, class Cv, int SB, int G>
-__global__ void __launch_bounds__(kTailRows / 4) k_fwd_tail(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
-                                                            const T* __restrict__ panel, const Cv* __restrict__ yv,
-                                                            Cv* __restrict__ fv) {
+__global__ void __launch_bounds__(tail_threads<T>()) k_fwd_tail(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
+                                                                const T* __restrict__ panel, const Cv* __restrict__ yv,
+                                                                Cv* __restrict__ fv) {
+    constexpr int RT = tail_rows<T>() / tail_threads<T>();
     __shared__ Cv y[G][SB];
     const SolveBlockTask tk = tasks[blockIdx.x];
     const SnDev d = A.sn[tk.s];
     const int w = d.w;
-    const int i = tk.r0 + 4 * (int)threadIdx.x;
+    const int i = tk.r0 + RT * (int)threadIdx.x;
     const T* p = panel + d.panel_off + i;
-    for (int r0 = 0; r0 < A.nrhs; r0 += G) {
+    auto load = [&](const T* q, T* v) {
+        if constexpr (RT == 4) load4(q, v);
+        else v[0] = *q;
+    };
+    for (int r0 = blockIdx.y * G; r0 < A.nrhs; r0 += gridDim.y * G) {
         const int ng = min(G, A.nrhs - r0);
         __syncthreads();
         for (int t = threadIdx.x; t < G * SB; t += blockDim.x) {
@@ -1092,33 +1109,33 @@ __global__ void __launch_bounds__(kTailRows / 4) k_fwd_tail(const SolveBlockTask
         }
         __syncthreads();
         if (i >= tk.r1) continue;
-        Cv a[G][4];
+        Cv a[G][RT];
 #pragma unroll
         for (int g = 0; g < G; ++g)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) a[g][e] = Cv(0);
+            for (int e = 0; e < RT; ++e) a[g][e] = Cv(0);
         int k = 0;
         for (; k + 8 <= w; k += 8) {
-            T v[8][4];
+            T v[8][RT];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) load4(p + (long long)(k + u) * d.ldp, v[u]);
+            for (int u = 0; u < 8; ++u) load(p + (long long)(k + u) * d.ldp, v[u]);
 #pragma unroll
             for (int u = 0; u < 8; ++u)
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
                     const Cv yk = y[g][k + u];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) a[g][e] += (Cv)v[u][e] * yk;
+                    for (int e = 0; e < RT; ++e) a[g][e] += (Cv)v[u][e] * yk;
                 }
         }
         for (; k < w; ++k) {
-            T v[4];
-            load4(p + (long long)k * d.ldp, v);
+            T v[RT];
+            load(p + (long long)k * d.ldp, v);
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 const Cv yk = y[g][k];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) a[g][e] += (Cv)v[e] * yk;
+                for (int e = 0; e < RT; ++e) a[g][e] += (Cv)v[e] * yk;
             }
         }
 #pragma unroll
@@ -1126,33 +1143,45 @@ __global__ void __launch_bounds__(kTailRows / 4) k_fwd_tail(const SolveBlockTask
             if (g >= ng) break;
             Cv* f = fv + A.fvec_off[tk.s] + (r0 + g) * A.fv_stride;
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
+            for (int e = 0; e < RT; ++e)
                 if (i + e >= w && i + e < tk.r1) f[i + e] -= a[g][e];
         }
     }
 }
 
-// Backward: x = L_0^-T g (warp per output, lanes over the inverse's column),
-// after the trailing rows' contribution; x to the work vector.
+// Backward: x = L_0^-T g after the trailing rows' contribution; x to the work vector.  Eight lanes per output, each
+// reading 16 bytes of the inverse's column at a time (zero above its diagonal).
 template <class Cv, int SB>
 __global__ void __launch_bounds__(256) k_bwd_solo(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
-                                                  const Cv* __restrict__ linv, Cv* __restrict__ fv,
+                                                  const Cv* __restrict__ linv, const Cv* __restrict__ fv,
                                                   Cv* __restrict__ xv, Cv* __restrict__ work) {
-    __shared__ Cv g0[SB];
+    constexpr int V = 16 / (int)sizeof(Cv);
+    __shared__ __align__(16) Cv g0[SB];
     const SolveBlockTask tk = tasks[blockIdx.x];
     const SnDev d = A.sn[tk.s];
-    const int w = d.w, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+    const int w = d.w, tid = threadIdx.x, q = tid & 7;
     const Cv* Li = linv + (long long)tk.blk * SB * SB;
-    for (int r = 0; r < A.nrhs; ++r) {
+    for (int r = blockIdx.y; r < A.nrhs; r += gridDim.y) {
         const long long base = A.fvec_off[tk.s] + r * A.fv_stride;
         __syncthreads();
-        for (int t = tid; t < w; t += blockDim.x) g0[t] = fv[base + t];
+        if (tid < SB) g0[tid] = tid < w ? fv[base + tid] : Cv(0);
         __syncthreads();
-        for (int t = warp; t < w; t += nwarps) {
+        for (int t0 = 0; t0 < w; t0 += 32) {
+            const int t = t0 + (tid >> 3);
             Cv acc = Cv(0);
-            for (int k = t + lane; k < w; k += 32) acc += Li[k + t * SB] * g0[k];
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) {
+            if (t < w)
+#pragma unroll
+                for (int b = 0; b < SB; b += 8 * V) {
+                    const int k = b + q * V;
+                    if (k >= w || k + V <= t) continue;
+                    Cv v[V];
+                    *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(Li + (long long)t * SB + k);
+#pragma unroll
+                    for (int e = 0; e < V; ++e) acc += v[e] * g0[k + e];
+                }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (t < w && q == 0) {
                 xv[base + t] = acc;
                 work[d.first_col + t + (long long)r * A.ldw] = acc;
             }
@@ -1174,7 +1203,7 @@ __global__ void k_bwd_gather(const SolveBlockTask* __restrict__ tasks, SolveArgs
 }
 
 // g[k] -= sum_{i in [r0, r1)} L[i,k] g[i] for columns k in [k0, k0+kn), one warp per column,
-// RG right-hand sides at a time (each column entry is loaded once per group).
+// RG right-hand sides at a time (each column entry is loaded once per group), groups over blockIdx.y.
 // Rows are read 16 bytes at a time between a scalar head and tail: a panel
 // column and the front vector start on 16-byte boundaries (panel offsets are
 // multiples of 64 elements, ldp, front-vector offsets and their stride of 8),
@@ -1197,7 +1226,7 @@ __global__ void k_bwd_cols(const SolveBlockTask* __restrict__ tasks, SolveArgs A
         if constexpr (V == 4) return (Cv)a.x * b.x + (Cv)a.y * b.y + (Cv)a.z * b.z + (Cv)a.w * b.w;
         else return (Cv)a.x * b.x + (Cv)a.y * b.y;
     };
-    for (int rg = 0; rg < A.nrhs; rg += RG) {
+    for (int rg = blockIdx.y * RG; rg < A.nrhs; rg += gridDim.y * RG) {
         const int ng = min(RG, A.nrhs - rg);
         Cv* g = fv + A.fvec_off[tk.s] + (long long)rg * A.fv_stride;
         Cv acc[RG];
