@@ -1223,8 +1223,8 @@ void apply_factor(uchol_factor_s* F, int nrhs, const double* b, int ldb, double*
 void residual(uchol_factor_s* F, int nrhs, const double* x, int ldx, const double* b, int ldb, double* r, int ldr) {
     uchol_symbolic_s* S = F->sym;
     if (S->n == 0) return;
-    k_spmv_residual<<<(S->n + 7) / 8, 256, 0, S->stream>>>(S->d_full_ptr.as<int>(), S->d_full_col.as<int>(),
-                                                          F->full_val.as<double>(), S->n, nrhs, x, ldx, b, ldb, r, ldr);
+    launch_spmv_residual(S->d_full_ptr.as<int>(), S->d_full_col.as<int>(), F->full_val.as<double>(), S->n, nrhs, x, ldx, b,
+                         ldb, r, ldr, S->stream);
     counted();
 }
 

@@ -160,20 +160,25 @@ __global__ void __launch_bounds__(256) k_cg_start(const double* __restrict__ inv
     }
 }
 
-// q = A p for the active columns (one warp per row of the both-triangle structure).
+// q = A p for the active columns (eight lanes per row of the both-triangle structure, as k_spmv_residual).
 __global__ void k_cg_spmv(const int* __restrict__ ptr, const int* __restrict__ col, const double* __restrict__ val,
                           int n, int nrhs, const double* __restrict__ p, int ld, double* __restrict__ q,
                           const CgCol* __restrict__ cols) {
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const int p0 = ptr[row], p1 = ptr[row + 1];
+    const int lane = threadIdx.x & 31, sub = lane & 7, row = blockIdx.x * kCsrRowsPerCta + (threadIdx.x >> 3);
+    const int p0 = row < n ? ptr[row] : 0, p1 = row < n ? ptr[row + 1] : 0;
+    const bool is_long = p1 - p0 > kCsrLongRow;
+    const unsigned longs = __ballot_sync(0xffffffffu, is_long && sub == 0);
     for (int c = 0; c < nrhs; ++c) {
         if (!cols[c].active) continue;
-        const double* pc = p + (long long)c * ld;
-        double acc = 0.0;
-        for (int k = p0 + lane; k < p1; k += 32) acc += val[k] * pc[col[k]];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) q[row + (long long)c * ld] = acc;
+        double acc[1], whole[1];
+        csr_row_sums<8, 1>(p0, is_long ? p0 : p1, sub, col, val, p + (long long)c * ld, ld, 1, acc);
+        for (unsigned m = longs; m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            csr_row_sums<32, 1>(__shfl_sync(0xffffffffu, p0, src), __shfl_sync(0xffffffffu, p1, src), lane, col, val,
+                                p + (long long)c * ld, ld, 1, whole);
+            if (lane == src) acc[0] = whole[0];
+        }
+        if (row < n && sub == 0) q[row + (long long)c * ld] = acc[0];
     }
 }
 
@@ -403,8 +408,8 @@ void jacobi_pcg(uchol_dmatrix_s* m, int nrhs, const double* b, int ldb, double* 
     dmatrix_full_values(m);
     // b norms, first residual r = b - A x0 and its norm
     dm_dots(m, nrhs, db, ldbd, db, ldbd, w.partial, w.bn2);
-    k_spmv_residual<<<(n + 7) / 8, 256, 0, st>>>(m->full_ptr.as<int>(), m->full_col.as<int>(), m->full_val.as<double>(),
-                                                 n, nrhs, dx, ldxd, db, ldbd, w.r, n);
+    launch_spmv_residual(m->full_ptr.as<int>(), m->full_col.as<int>(), m->full_val.as<double>(),
+                                                 n, nrhs, dx, ldxd, db, ldbd, w.r, n, st);
     counted();
     dm_dots(m, nrhs, w.r, n, w.r, n, w.partial, w.rn2);
     k_cg_init<<<1, 32 * ((nrhs + 31) / 32), 0, st>>>(w.bn2, w.rn2, o.relative_tolerance, nrhs, w.cols);
@@ -434,7 +439,7 @@ void jacobi_pcg(uchol_dmatrix_s* m, int nrhs, const double* b, int ldb, double* 
     while (any) {
         const int chunk = std::min(kCgPoll, max_it - steps);
         for (int k = 0; k < chunk; ++k) {
-            k_cg_spmv<<<(n + 7) / 8, 256, 0, st>>>(m->full_ptr.as<int>(), m->full_col.as<int>(), m->full_val.as<double>(),
+            k_cg_spmv<<<(n + kCsrRowsPerCta - 1) / kCsrRowsPerCta, 256, 0, st>>>(m->full_ptr.as<int>(), m->full_col.as<int>(), m->full_val.as<double>(),
                                                    n, nrhs, w.p, n, w.q, w.cols);
             k_cg_alpha<<<gv, 256, 0, st>>>(w.p, w.q, n, n, w.cols, w.partial, w.counters);
             k_cg_update<<<gv, 256, 0, st>>>(dx, ldxd, w.r, w.z, w.p, w.q, w.inv, n, n, max_it, w.cols, w.partial,
@@ -827,15 +832,15 @@ int uchol_dmatrix_multiply(uchol_dmatrix m, int nrhs, const double* x, int ldx, 
         cudaStream_t st = m->stream;
         dmatrix_full_values(m);
         if (on_device) {
-            k_spmv_residual<<<(n + 7) / 8, 256, 0, st>>>(m->full_ptr.as<int>(), m->full_col.as<int>(),
-                                                         m->full_val.as<double>(), n, nrhs, x, ldx, nullptr, 0, y, ldy);
+            launch_spmv_residual(m->full_ptr.as<int>(), m->full_col.as<int>(),
+                                                         m->full_val.as<double>(), n, nrhs, x, ldx, nullptr, 0, y, ldy, st);
             counted();
         } else {
             CgWs w = dmatrix_ws(m, nrhs);
             CK(cudaMemcpy2DAsync(w.xd, (size_t)n * 8, x, (size_t)ldx * 8, (size_t)n * 8, nrhs, cudaMemcpyHostToDevice,
                                  st));
-            k_spmv_residual<<<(n + 7) / 8, 256, 0, st>>>(m->full_ptr.as<int>(), m->full_col.as<int>(),
-                                                         m->full_val.as<double>(), n, nrhs, w.xd, n, nullptr, 0, w.bd, n);
+            launch_spmv_residual(m->full_ptr.as<int>(), m->full_col.as<int>(),
+                                                         m->full_val.as<double>(), n, nrhs, w.xd, n, nullptr, 0, w.bd, n, st);
             counted();
             CK(cudaMemcpy2DAsync(y, (size_t)ldy * 8, w.bd, (size_t)n * 8, (size_t)n * 8, nrhs, cudaMemcpyDeviceToHost,
                                  st));
