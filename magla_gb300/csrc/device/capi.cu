@@ -25,6 +25,7 @@
 #include "plan.hpp"
 #include "solve_kernels.cuh"
 #include "tc_gemm.cuh"
+#include "oz_gemm.cuh"
 #include "inv_solve.cuh"
 
 using namespace uchol_dev;
@@ -139,6 +140,7 @@ int64_t planned_bytes(const Plan& P, int precision, long long nnz, long long ful
     if (P.cfg.tensor_core)
         b += 2 * P.stage_elems * op + (int64_t)minv_floats(std::max(1, P.diag_slots), own_inverses(P.cfg)) * 4 +
              (int64_t)tc_ws_floats(152) * 4 + (int64_t)tc_counter_count(152) * 4;
+    else b += 2 * (P.stage_elems * 2 + P.oz_exps * 4);
     b += ((int64_t)P.inv_blocks.size() + P.inv_off_blocks) * sb * sb * elem;
     b += inv_scratch_elems(P) * elem;
     b += (nnz + full_nnz) * 8 + (int64_t)n * 8;
@@ -181,7 +183,7 @@ struct uchol_symbolic_s {
                           std::to_string(c.small_mask) + "/" + std::to_string(c.tensor_core) + "/" +
                           std::to_string(c.solve_block) + "/" + std::to_string(c.merge_cols) + "/" +
                           std::to_string(c.merge_fill) + "/" + std::to_string(c.inv_cols) + "/" +
-                          std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
+                          std::to_string(c.oz_rows) + "/" + std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
         auto it = plans.find(key);
         if (it != plans.end()) {
             check_budget(budget, planned_bytes(it->second->plan, precision, nnz, full_nnz, n));
@@ -230,6 +232,7 @@ struct uchol_factor_s {
     uchol_options opts{};
     int precision = UCHOL_PRECISION_FP64;
     size_t elem = 8;              // bytes per front element
+    DBuf oz_exps;                       // FP64 tensor-core updates: row exponents of the digits
     DBuf panel, contrib, stage_a, stage_b, diag, values, full_val, stats, ctl;
     DBuf work, fv, fv2, vec[6], scal;   // solve workspace
     DBuf bwd_partial;                   // backward column dots split in row chunks: partial sums
@@ -317,6 +320,7 @@ PlanConfig config_for(const uchol_options& o) {
     if (o.precision == UCHOL_PRECISION_FP64) {
         c.tensor_core = false;
         c.outer_block = c.pivot_block;
+        if (kOzBlock % c.pivot_block == 0) c.oz_rows = kOzMinRows;
         c.solve_block = 64;
     } else {
         c.solve_block = 128;
@@ -441,9 +445,21 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
                     throw Error(UCHOL_INTERNAL, "mixed-precision panel launch in an FP64 plan");
                 }
                 break;
+            case Launch::OzSlice:
+                if constexpr (sizeof(T) == 8)
+                    k_oz_slice<<<L.count * kOzSplit, 256, 0, st>>>(D.panel_tasks.as<PanelTask>() + L.begin, sn, panel, diag,
+                                                                   F->stage_a.as<__nv_bfloat16>(), F->stage_b.as<__nv_bfloat16>(),
+                                                                   F->oz_exps.as<int>(), P.oz_exps, D.stage.as<StageInfo>());
+                break;
             case Launch::KindCount:
                 throw Error(UCHOL_INTERNAL, "invalid launch kind");
             case Launch::TcUpdate: {
+                if constexpr (sizeof(T) == 8) {
+                    k_oz_gemm<<<(unsigned)L.tiles, kOzThreads, oz_smem_bytes(), st>>>(
+                        D.tc_jobs.as<TcJob>() + L.begin, L.count, sn, panel, contrib, F->maps.as<CUtensorMap>(),
+                        F->oz_exps.as<int>(), P.oz_exps, D.stage.as<StageInfo>(), &stats->status);
+                    break;
+                }
                 // K blocks of every job when all share one K (the launch may then be split in K)
                 const bool bf16 = F->precision == UCHOL_PRECISION_BF16;
                 const int kbe = bf16 ? 64 : 32;
@@ -496,7 +512,7 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
         if (log) fclose(log);
         F->phases.extend_add_ms = sum[Launch::ExtendAdd];
         F->phases.small_fronts_ms = sum[Launch::SmallFronts];
-        F->phases.panel_ms = sum[Launch::PivotBlock] + sum[Launch::Trsm] + sum[Launch::DiagBlock] + sum[Launch::PanelSolve];
+        F->phases.panel_ms = sum[Launch::PivotBlock] + sum[Launch::Trsm] + sum[Launch::DiagBlock] + sum[Launch::PanelSolve] + sum[Launch::OzSlice];
         F->phases.schur_ms = sum[Launch::SimtUpdate] + sum[Launch::TcUpdate];
         F->phases.pivot_block_ms = sum[Launch::PivotBlock] + sum[Launch::DiagBlock];
         F->phases.schur_tensor_ms = sum[Launch::TcUpdate];
@@ -523,6 +539,7 @@ void prepare_factor_kernels(uchol_factor_s* F) {
     if (F->elem == 8) {
         CK(cudaFuncSetAttribute(k_small_fronts<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(small, 1)));
         prepare_inversion<double, 64>();
+        CK(cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz_smem_bytes()));
     } else {
         CK(cudaFuncSetAttribute(k_small_fronts<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(small, 1)));
         prepare_inversion<float, 128>();
@@ -767,7 +784,14 @@ uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_o
     PlanConfig cfg = config_for(F->opts);
     CK(cudaDeviceGetAttribute(&F->sms, cudaDevAttrMultiProcessorCount, S->device));
     cfg.sms = F->sms;
-    F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
+    try {
+        F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
+    } catch (const Error& e) {
+        // a budget too small for the digits of the FP64 tensor-core updates: without them
+        if (e.code != UCHOL_OOM || cfg.oz_rows == 0) throw;
+        cfg.oz_rows = 0;
+        F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
+    }
     const Plan& P = F->dp->plan;
     cudaStream_t st = S->stream;
     F->panel.alloc((size_t)P.factor_elems * F->elem, "factor panels");
@@ -801,6 +825,22 @@ uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_o
         F->tc_ws.alloc(tc_ws_floats(F->sms) * sizeof(float), "K-split workspace");
         F->tc_counters.alloc(tc_counter_count(F->sms) * sizeof(int), "K-split workspace");
         CK(cudaMemsetAsync(F->tc_counters.p, 0, F->tc_counters.bytes, st));
+        CK(cudaStreamSynchronize(st));
+    }
+    if (!cfg.tensor_core && P.stage_elems > 0) {
+        F->stage_a.alloc((size_t)P.stage_elems * 2, "digit staging");
+        F->stage_b.alloc((size_t)P.stage_elems * 2, "digit staging");
+        F->oz_exps.alloc((size_t)P.oz_exps * 2 * sizeof(int), "digit staging");
+        std::vector<CUtensorMap> maps(2 * P.map_front.size());
+        for (size_t k = 0; k < P.map_front.size(); ++k) {
+            const int s = P.map_front[k];
+            try {
+                make_oz_maps((char*)F->stage_a.p + P.stage[s].off * 2, (char*)F->stage_b.p + P.stage[s].off * 2, P.sn[s].m, P.stage[s].ld, &maps[2 * k]);
+            } catch (const std::runtime_error& e) {
+                throw Error(UCHOL_CUDA_ERROR, e.what());
+            }
+        }
+        F->maps.upload(maps, st, "tensor maps");
         CK(cudaStreamSynchronize(st));
     }
     if (cfg.tensor_core)
@@ -1496,13 +1536,21 @@ int uchol_estimate_device_bytes(const uchol_symbolic_desc* d, const uchol_option
         PlanConfig cfg = config_for(o);
         const int n = d->n, count = d->supernode_count;
         if (n < 0 || count < 0) throw Error(UCHOL_BAD_ARG, "negative size");
+        const long long nnz = d->nnz;
         Plan P;
-        try {
-            P = build_plan(n, count, d->first_column, d->parent, d->child_ptr, d->children, d->front_ptr, d->front_rows,
-                           d->diag_value_index, d->pattern_ptr, d->pattern_rows, d->lower_start, d->lower_value_ptr,
-                           d->lower_value_index, d->nnz, cfg);
-        } catch (const std::runtime_error& e) {
-            throw Error(UCHOL_BAD_ARG, std::string("inconsistent symbolic factorization: ") + e.what());
+        for (;;) {
+            try {
+                P = build_plan(n, count, d->first_column, d->parent, d->child_ptr, d->children, d->front_ptr, d->front_rows,
+                               d->diag_value_index, d->pattern_ptr, d->pattern_rows, d->lower_start, d->lower_value_ptr,
+                               d->lower_value_index, d->nnz, cfg);
+            } catch (const std::runtime_error& e) {
+                throw Error(UCHOL_BAD_ARG, std::string("inconsistent symbolic factorization: ") + e.what());
+            }
+            // as create_factor: a budget too small for the digits goes without them
+            if (cfg.oz_rows == 0 || o.device_memory_budget <= 0 ||
+                planned_bytes(P, o.precision, nnz, 2 * nnz - n, n) <= o.device_memory_budget)
+                break;
+            cfg.oz_rows = 0;
         }
         const int64_t elem = o.precision == UCHOL_PRECISION_FP64 ? 8 : 4;
         const int64_t op = o.precision == UCHOL_PRECISION_BF16 ? 2 : 4;
@@ -1511,10 +1559,9 @@ int uchol_estimate_device_bytes(const uchol_symbolic_desc* d, const uchol_option
         if (staging_bytes)
             *staging_bytes = cfg.tensor_core ? 2 * P.stage_elems * op + (int64_t)minv_floats(P.diag_slots, own_inverses(cfg)) * 4 +
                                                    (int64_t)tc_ws_floats(152) * 4 + (int64_t)tc_counter_count(152) * 4
-                                             : 0;
+                                             : 2 * (P.stage_elems * 2 + P.oz_exps * 4);
         if (levels) *levels = P.levels;
         if (launches) *launches = (int)P.launches.size();
-        const long long nnz = d->nnz;
         check_budget(o.device_memory_budget, planned_bytes(P, o.precision, nnz, 2 * nnz - n, n));
     });
 }

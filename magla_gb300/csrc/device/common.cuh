@@ -79,6 +79,7 @@ struct StageInfo {
     long long off;     // element offset of the front's region in each staging arena
     int ld;
     int map;           // index of the front's tensor-map pair
+    long long eoff = 0;   // FP64 path: offset of the front's row exponents
 };
 
 struct TileTask {      // C[i0:i0+TM, j0:j0+TN] -= sum_k A[i,k] B[j,k], k in [k0, k0+kn)
@@ -117,22 +118,24 @@ __host__ __device__ __forceinline__ long long tc_half_sum(long long X) {
     const long long P = X >> 1;
     return P * (P - 1) + ((X & 1) ? P : 0);
 }
-// R_0 and delta of a job with columns from c0 in a front of m rows.
+// R_0 and delta of a job with columns from c0 in a front of m rows.  (Tiles of TC columns x 2 TC rows.)
+template <int TC = kTcCols>
 __host__ __device__ __forceinline__ void tc_col_shape(int c0, int m, int& R0, int& delta) {
     const int h = m - c0;
-    R0 = (h + kTcRows - 1) / kTcRows;
-    delta = (h > kTcCols && (h - kTcCols + kTcRows - 1) / kTcRows < R0) ? 1 : 0;
+    R0 = (h + 2 * TC - 1) / (2 * TC);
+    delta = (h > TC && (h - TC + 2 * TC - 1) / (2 * TC) < R0) ? 1 : 0;
 }
 // Tiles of the first Q column tiles.
 __host__ __device__ __forceinline__ long long tc_col_prefix(long long Q, int R0, int delta) {
     return Q * R0 - tc_half_sum(Q + delta);
 }
 // Tiles of a whole update job: result columns [c0, cend) of a front with m rows.
+template <int TC = kTcCols>
 __host__ __device__ __forceinline__ long long tc_job_tiles(int c0, int cend, int m) {
     if (cend <= c0) return 0;
     int R0, delta;
-    tc_col_shape(c0, m, R0, delta);
-    return tc_col_prefix((cend - c0 + kTcCols - 1) / kTcCols, R0, delta);
+    tc_col_shape<TC>(c0, m, R0, delta);
+    return tc_col_prefix((cend - c0 + TC - 1) / TC, R0, delta);
 }
 
 // Tile t (0 <= t < tc_job_tiles) of the job with columns [c0, cend) of a front of m rows:
@@ -142,11 +145,12 @@ __host__ __device__ __forceinline__ long long tc_job_tiles(int c0, int cend, int
 // R_g is the first column's row-tile count is held by 2 (R_g - r) - delta of its columns
 // (all g of them for the first F rows), a prefix since R_q does not grow with q.
 constexpr int kTcGroup = 8;
+template <int TC = kTcCols>
 __host__ __device__ __forceinline__ void tc_decode_tile(int c0, int cend, int m, long long t, int& i0, int& j0,
                                                         int& jend) {
-    const int nc = (cend - c0 + kTcCols - 1) / kTcCols;
+    const int nc = (cend - c0 + TC - 1) / TC;
     int R0, delta;
-    tc_col_shape(c0, m, R0, delta);
+    tc_col_shape<TC>(c0, m, R0, delta);
     int lo = 0, hi = (nc - 1) / kTcGroup;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -175,9 +179,9 @@ __host__ __device__ __forceinline__ void tc_decode_tile(int c0, int cend, int m,
             t -= c;
         }
     }
-    j0 = c0 + (lo * kTcGroup + q) * kTcCols;
-    i0 = j0 + r * kTcRows;
-    jend = j0 + kTcCols < cend ? j0 + kTcCols : cend;
+    j0 = c0 + (lo * kTcGroup + q) * TC;
+    i0 = j0 + r * (2 * TC);
+    jend = j0 + TC < cend ? j0 + TC : cend;
 }
 
 #ifdef __CUDACC__

@@ -349,6 +349,38 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
             }
             P.stage_elems = std::max(P.stage_elems, top);
         }
+        // FP64 tensor-core fronts: digit staging of the level, and an update of the columns [c0, cend) with K columns
+        // [kbeg, kbeg + kn) of every front that `job` names
+        auto oz_front = [&](int s) { return cfg.oz_rows > 0 && P.sn[s].m >= cfg.oz_rows; };
+        if (!cfg.tensor_core) {
+            long long top = 0, etop = 0;
+            for (int s : large) {
+                if (!oz_front(s)) continue;
+                const SnDev& d = P.sn[s];
+                StageInfo& g = P.stage[s];
+                g.ld = (d.w + 31) / 32 * 256;   // 512 bytes per 32 columns
+                g.off = top;
+                g.eoff = etop;
+                g.map = (int)P.map_front.size();
+                P.map_front.push_back(s);
+                top += round_up((long long)d.m * g.ld, 512);
+                etop += (long long)((d.w + kOzBlock - 1) / kOzBlock) * d.ldp;
+            }
+            P.stage_elems = std::max(P.stage_elems, top);
+            P.oz_exps = std::max(P.oz_exps, etop);
+        }
+        auto oz_update = [&](auto&& job) {
+            const int jb = (int)P.tc_jobs.size();
+            long long tiles = 0;
+            for (int s : large) {
+                int c0, cend, kbeg, kn;
+                if (!oz_front(s) || !job(s, c0, cend, kbeg, kn)) continue;
+                P.tc_jobs.push_back({tiles, s, c0, cend, kbeg, kn, P.stage[s].map});
+                tiles += tc_job_tiles<64>(c0, cend, P.sn[s].m);
+                P.simt_flops += job_flops(UpdJob{0, s, c0, cend, kbeg, kn, -1}, P.sn[s]);
+            }
+            if ((int)P.tc_jobs.size() > jb) P.launches.push_back({Launch::TcUpdate, jb, (int)P.tc_jobs.size() - jb, tiles});
+        };
         // tensor-core path, left-looking in two levels.  At the start of each super-block of
         // kSuperBlocks outer blocks, one update brings all of its columns up to date with every
         // earlier column of the supernode (K = sb0); each later outer block of the super-block
@@ -399,42 +431,49 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 if ((int)P.panel_tasks.size() > pb) P.launches.push_back({Launch::PanelSolve, pb, (int)P.panel_tasks.size() - pb, 0});
                 continue;
             }
-            for (int j0r = 0; j0r < NB; j0r += PB) {
+            // FP64 path, one pivot block per step.  Plain fronts are right-looking: every step updates the whole
+            // trailing triangle.  Tensor-core fronts are left-looking by outer blocks of kOzBlock columns, as the mixed
+            // path: a step updates the rest of its outer block only, an outer block that is complete is split into
+            // digits, and the next one starts by taking the earlier ones' updates from them.
+            if (k0 > 0 && k0 % kOzBlock == 0) {
+                const int blk0 = k0 / (kSuperBlocks * kOzBlock) * (kSuperBlocks * kOzBlock);
+                oz_update([&](int s, int& c0, int& cend, int& kbeg, int& kn) {
+                    const int w = P.sn[s].w;
+                    if (w <= k0) return false;
+                    const bool super = k0 == blk0;
+                    c0 = k0;
+                    cend = std::min(w, k0 + (super ? kSuperBlocks * kOzBlock : kOzBlock));
+                    kbeg = super ? 0 : blk0;
+                    kn = super ? k0 : k0 - blk0;
+                    return true;
+                });
+            }
+            {
                 int qb = (int)P.pivot_tasks.size();
                 int pb = (int)P.panel_tasks.size();
                 for (int s : large) {
                     const SnDev& d = P.sn[s];
                     if (d.w <= k0) continue;
-                    int nbo = std::min(NB, d.w - k0);
-                    int j0 = k0 + j0r;
-                    if (j0r >= nbo) continue;
-                    int nbi = std::min(PB, k0 + nbo - j0);
-                    P.pivot_tasks.push_back({s, j0, nbi, j0 + nbi, 0, -1, 0, 0});
-                    // TRSM tasks over rows [j0+nbi, m)
-                    int r = j0 + nbi;
-                    while (r < d.m) {
-                        int rows = std::min(128, d.m - r);
-                        int stage = cfg.tensor_core ? 1 : 0, zero_to = 0;
-                        if (cfg.tensor_core && j0 + nbi == d.w && P.stage[s].ld > d.w) zero_to = P.stage[s].ld;
-                        P.panel_tasks.push_back({s, j0, nbi, r, rows, stage, 0, zero_to});
-                        r += rows;
-                    }
+                    const int nbi = std::min(PB, d.w - k0);
+                    P.pivot_tasks.push_back({s, k0, nbi, k0 + nbi, 0, -1, 0, 0});
+                    for (int r = k0 + nbi; r < d.m; r += 128)
+                        P.panel_tasks.push_back({s, k0, nbi, r, std::min(128, d.m - r), 0, 0, 0});
                 }
                 if ((int)P.pivot_tasks.size() > qb) P.launches.push_back({Launch::PivotBlock, qb, (int)P.pivot_tasks.size() - qb, 0});
                 if ((int)P.panel_tasks.size() > pb) P.launches.push_back({Launch::Trsm, pb, (int)P.panel_tasks.size() - pb, 0});
-                if (!cfg.tensor_core) break;  // FP64 path: one pivot block per outer step
             }
-            // FP64 path: right-looking update of the whole trailing triangle per step, in 32 x 32 tiles once they
-            // make two CTAs per SM, else 16 x 16 (an SM takes 8 or 2 us of FP64 pipe for one)
-            if (!cfg.tensor_core) {
+            {
+                // updates in 32 x 32 tiles once they make two CTAs per SM, else 16 x 16 (an SM takes 8 or 2 us of FP64
+                // pipe for one)
                 int jb = (int)P.simt_jobs.size();
                 long long tiles32 = 0;
                 for (int s : large) {
                     const SnDev& d = P.sn[s];
                     if (d.w <= k0) continue;
                     const int nbo = std::min(NB, d.w - k0), c0 = k0 + nbo;
-                    if (c0 >= d.m) continue;
-                    UpdJob J{0, s, c0, d.m, k0, nbo, -1};
+                    const int cend = oz_front(s) ? std::min(d.w, (k0 / kOzBlock + 1) * kOzBlock) : d.m;
+                    if (c0 >= cend) continue;
+                    UpdJob J{0, s, c0, cend, k0, nbo, -1};
                     tiles32 += job_tiles(J, d, 32);
                     P.simt_flops += job_flops(J, d);
                     P.simt_jobs.push_back(J);
@@ -451,7 +490,28 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                     P.launches.push_back(Lu);
                 }
             }
+            {
+                // digits of the outer blocks completed by this step
+                int pb = (int)P.panel_tasks.size();
+                for (int s : large) {
+                    const SnDev& d = P.sn[s];
+                    if (!oz_front(s) || d.w <= k0) continue;
+                    const int b0 = k0 / kOzBlock * kOzBlock, be = std::min(d.w, b0 + kOzBlock);
+                    if (std::min(d.w, k0 + PB) != be) continue;
+                    for (int r = be; r < d.m; r += 128)
+                        P.panel_tasks.push_back({s, b0, be - b0, r, std::min(128, d.m - r), 0, 0, 0});
+                }
+                if ((int)P.panel_tasks.size() > pb) P.launches.push_back({Launch::OzSlice, pb, (int)P.panel_tasks.size() - pb, 0});
+            }
         }
+        if (!cfg.tensor_core)
+            oz_update([&](int s, int& c0, int& cend, int& kbeg, int& kn) {
+                c0 = P.sn[s].w;
+                cend = P.sn[s].m;
+                kbeg = 0;
+                kn = P.sn[s].w;
+                return c0 < cend;
+            });
         // tensor-core path: contribution block of every large front, K = its whole width
         if (cfg.tensor_core) {
             int jb = (int)P.tc_jobs.size();

@@ -19,6 +19,11 @@ constexpr int kColRowsPlan = 2048;   // trailing rows per backward column-dot ta
 constexpr int kColRowsPlan64 = 1024; // and FP64
 constexpr int kInvColRowsPlan = 1024;   // trailing rows per backward partial-sum task of an inverse front
 constexpr int kDefaultInvCols = 2048;   // widest front whose diagonal block is kept inverted for the solves
+constexpr int kOzBlock = 128;         // FP64 tensor-core updates: columns of an outer block (one chunk of digits)
+// Fewest rows of a front that takes them.  Refactorisation plus solve, fronts from this size / the FP64 pipe for all:
+// elasticity 30^3 84 / 539 ms, 20^3 20.1 / 53.9, 14^3 7.3 / 10.2, one modulus 12^3 5.4 / 6.8; from 1024 rows 3 to 7%
+// slower than from 384, and below 384 the difference is within 2%.
+constexpr int kOzMinRows = 384;
 constexpr int kSuperBlocks = 4;       // tensor-core path: outer blocks per super-block of the own-column updates
 constexpr int kDefaultMergeCols = 2048;   // widest device front made of a chain of supernodes (merge_chains)
 constexpr int kInvWarpCols = 32;         // widest diagonal block inverted by one warp
@@ -37,6 +42,8 @@ struct PlanConfig {
     double merge_fill = 0.05; // largest growth of the stored entries a grouping may cost
     bool side_extend_add = false;   // tensor-core path: the extend-add into the contribution columns of
                                     // large fronts runs on a second stream, beside the level's outer blocks
+    int oz_rows = 0;                // FP64 path, > 0: fronts of at least this many rows take their updates on the tensor
+                                    // cores, from digit slices (oz_gemm.cuh)
     int sms = 0;                    // > 0: the device's SM count (sizes the backward inverse-front chunks)
 };
 
@@ -60,7 +67,7 @@ FrontStructure merge_chains(int n, int count, const int* first_column, const int
 // One kernel launch: a contiguous range of tasks in one of the task arrays.
 struct Launch {
     enum Kind : int {
-        ExtendAdd, SmallFronts, PivotBlock, Trsm, SimtUpdate, TcUpdate, DiagBlock, PanelSolve,
+        ExtendAdd, SmallFronts, PivotBlock, Trsm, SimtUpdate, TcUpdate, DiagBlock, PanelSolve, OzSlice,
         KindCount
     } kind;
     int begin, count;   // task range
@@ -166,7 +173,8 @@ struct Plan {
     std::vector<int> map_front;                // front of each tensor-map pair
     std::vector<Launch> launches;
     int max_small_m = 0;                  // of the fronts taken by a CTA each
-    long long stage_elems = 0;                 // elements of each operand staging arena (tensor-core path)
+    long long stage_elems = 0;                 // elements of each operand staging arena (tensor-core path; FP64: digits)
+    long long oz_exps = 0;                     // row exponents of a level (FP64 tensor-core updates)
     double tc_flops = 0.0;                     // algorithmic flops of the tensor-core updates (lower triangle)
     double simt_flops = 0.0;                   // algorithmic flops of the SIMT updates
 
