@@ -104,7 +104,7 @@ typedef struct {
                                            FP64) and at most this many columns keep the inverse of their
                                            diagonal block's unit-lower triangle (built after each
                                            factorisation), so that their triangular solves are products
-                                           instead of a chain of block solves.  0 = 2048, < 0 = off. */
+                                           instead of a chain of block solves.  0 = 8192 on the mixed paths and 2048 in FP64, < 0 = off. */
     int64_t device_memory_budget;       /* > 0: a factorisation whose factor, contribution arena, staging,
                                            inverses and value copies (uchol_estimate_device_bytes) exceed
                                            this many bytes fails with UCHOL_OOM before any of it is

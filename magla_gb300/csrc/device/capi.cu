@@ -314,7 +314,8 @@ PlanConfig config_for(const uchol_options& o) {
     c.small_mask = o.small_front_buckets ? o.small_front_buckets : 0x7;
     c.pivot_block = std::min(kMaxPivotBlock, std::max(4, std::min(128, o.panel_width)));
     c.merge_cols = o.chain_merge_width == 0 ? kDefaultMergeCols : std::max(0, o.chain_merge_width);
-    c.inv_cols = o.inverse_block_width == 0 ? kDefaultInvCols : std::max(0, o.inverse_block_width);
+    c.inv_cols = o.inverse_block_width != 0 ? std::max(0, o.inverse_block_width)
+                 : o.precision == UCHOL_PRECISION_FP64 ? kDefaultInvCols64 : kDefaultInvCols;
     c.side_extend_add = o.extend_add_overlap >= 0;
     if (o.chain_merge_fill > 0.0) c.merge_fill = o.chain_merge_fill;
     if (o.precision == UCHOL_PRECISION_FP64) {
@@ -331,6 +332,15 @@ PlanConfig config_for(const uchol_options& o) {
         c.outer_block = std::max(64, std::min(kDiagMax, nb / 64 * 64));
     }
     return c;
+}
+
+// The next smaller configuration for a memory budget that this one's plan exceeds: default choices that cost memory only
+// for speed are given up, the wider inverse fronts and the digits of the FP64 tensor-core updates; false: none is left.
+bool relax_for_budget(PlanConfig& c, const uchol_options& o) {
+    if (o.inverse_block_width == 0 && c.inv_cols > kDefaultInvCols64) c.inv_cols = kDefaultInvCols64;
+    else if (c.oz_rows > 0) c.oz_rows = 0;
+    else return false;
+    return true;
 }
 
 template <class T>
@@ -784,13 +794,12 @@ uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_o
     PlanConfig cfg = config_for(F->opts);
     CK(cudaDeviceGetAttribute(&F->sms, cudaDevAttrMultiProcessorCount, S->device));
     cfg.sms = F->sms;
-    try {
-        F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
-    } catch (const Error& e) {
-        // a budget too small for the digits of the FP64 tensor-core updates: without them
-        if (e.code != UCHOL_OOM || cfg.oz_rows == 0) throw;
-        cfg.oz_rows = 0;
-        F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
+    while (!F->dp) {
+        try {
+            F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
+        } catch (const Error& e) {
+            if (e.code != UCHOL_OOM || !relax_for_budget(cfg, F->opts)) throw;
+        }
     }
     const Plan& P = F->dp->plan;
     cudaStream_t st = S->stream;
@@ -1546,11 +1555,10 @@ int uchol_estimate_device_bytes(const uchol_symbolic_desc* d, const uchol_option
             } catch (const std::runtime_error& e) {
                 throw Error(UCHOL_BAD_ARG, std::string("inconsistent symbolic factorization: ") + e.what());
             }
-            // as create_factor: a budget too small for the digits goes without them
-            if (cfg.oz_rows == 0 || o.device_memory_budget <= 0 ||
-                planned_bytes(P, o.precision, nnz, 2 * nnz - n, n) <= o.device_memory_budget)
+            // as create_factor
+            if (o.device_memory_budget <= 0 || planned_bytes(P, o.precision, nnz, 2 * nnz - n, n) <= o.device_memory_budget ||
+                !relax_for_budget(cfg, o))
                 break;
-            cfg.oz_rows = 0;
         }
         const int64_t elem = o.precision == UCHOL_PRECISION_FP64 ? 8 : 4;
         const int64_t op = o.precision == UCHOL_PRECISION_BF16 ? 2 : 4;

@@ -18,7 +18,13 @@ constexpr int kTailRowsPlan64 = 128; // and FP64 (its products hold the SM's FP6
 constexpr int kColRowsPlan = 2048;   // trailing rows per backward column-dot task (longer columns: partial sums)
 constexpr int kColRowsPlan64 = 1024; // and FP64
 constexpr int kInvColRowsPlan = 1024;   // trailing rows per backward partial-sum task of an inverse front
-constexpr int kDefaultInvCols = 2048;   // widest front whose diagonal block is kept inverted for the solves
+// Widest front whose diagonal block is kept inverted for the solves.  The inverse costs w^3 / 3 operations per
+// factorisation and saves a chain of w / SB block solves (about 9 us each in the mixed path) per solve and direction.
+// FP32 at 8192 columns: 3.4 ms against 1.1 ms per application of the factor, of which a refined solve makes two at least
+// (40^3 contrast, eight steps: 62.5 -> 58.0 ms; 30^3 BF16 78.1 -> 76.2).  FP64, where the pipe does 1.2 TFLOP/s and one
+// application is usual: 4096 columns cost 20 ms more on 30^3 elasticity (84 -> 105 ms).
+constexpr int kDefaultInvCols = 8192;     // mixed path
+constexpr int kDefaultInvCols64 = 2048;   // FP64
 constexpr int kOzBlock = 128;         // FP64 tensor-core updates: columns of an outer block (one chunk of digits)
 // Fewest rows of a front that takes them.  Refactorisation plus solve, fronts from this size / the FP64 pipe for all:
 // elasticity 30^3 84 / 539 ms, 20^3 20.1 / 53.9, 14^3 7.3 / 10.2, one modulus 12^3 5.4 / 6.8; from 1024 rows 3 to 7%
