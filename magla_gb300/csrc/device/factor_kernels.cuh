@@ -112,22 +112,31 @@ __global__ void k_assemble(const double* __restrict__ values, const long long* _
 // Extend-add: one warp per receiving parent column; the children's columns
 // that land in it are added in child order (deterministic, no atomics).
 // UtduNumericFactorization.cs:471-509.  A column of the parent's contribution
-// block is first cleared from its diagonal down (the reference zeroes the
-// whole front, :441-447; only the lower triangle is ever read), so the
-// clearing costs no pass of its own and the adds find the lines in L2.
+// block starts from zero (the reference zeroes the whole front, :441-447; only
+// the lower triangle is ever read): its first child's column is written out
+// together with the zeros between its entries, window by window of kEaWindow
+// rows through shared memory, so that every row is written once.  (Clearing the
+// column first and adding to it afterwards let 6,000 warps' columns leave L2 in
+// between: the traffic of a 10,000-row front was twice the bytes.)  Later
+// children, and columns of the panel, which hold the assembled values, are
+// added to what is there.  HBM bounds it.
 // Side = true: the instance launched on the side stream (its graph nodes run at
 // the lowest priority, so that the main stream's CTAs are scheduled first).
+constexpr int kEaWindow = 256, kEaThreads = 256;
 template <class T, bool Side = false>
-__global__ void k_extend_add(const EaItem* __restrict__ items, int count, const EaEntry* __restrict__ entries,
-                             const SnDev* __restrict__ sn, const int* __restrict__ rel, T* __restrict__ panel,
-                             T* __restrict__ contrib) {
+__global__ void __launch_bounds__(kEaThreads) k_extend_add(const EaItem* __restrict__ items, int count,
+                                                           const EaEntry* __restrict__ entries, const SnDev* __restrict__ sn,
+                                                           const int* __restrict__ rel, T* __restrict__ panel,
+                                                           T* __restrict__ contrib) {
+    __shared__ __align__(16) T windows[kEaThreads / 32][kEaWindow];
     const int lane = threadIdx.x & 31;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < count; warp += warps) {
+    const int warps = gridDim.x * (kEaThreads >> 5);
+    constexpr int D = kEaWindow / 32;   // loads of a batch in flight per lane
+    for (int warp = (blockIdx.x * kEaThreads + threadIdx.x) >> 5; warp < count; warp += warps) {
         const EaItem it = items[warp];
         const SnDev P = sn[it.parent];
         T* dst;
-        int shift;
+        int shift, first = it.begin;
         if (it.pcol < P.w) {
             dst = panel + P.panel_off + (long long)it.pcol * P.ldp;
             shift = 0;
@@ -135,23 +144,64 @@ __global__ void k_extend_add(const EaItem* __restrict__ items, int count, const 
             const int c = it.pcol - P.w, t = P.m - P.w;
             dst = contrib + P.contrib_off + (long long)c * P.ldc;
             shift = P.w;
-            // rows [c, t): 16-byte stores between a scalar head and tail (the column starts on a
-            // 16-byte boundary: contribution offsets are multiples of 64 elements, ldc of 8)
-            constexpr int V = 16 / (int)sizeof(T);
-            const int head = min(t, (c + V - 1) / V * V), body = max(head, t / V * V);
-            for (int r = c + lane; r < head; r += 32) dst[r] = T(0);
-            for (int v = head / V + lane; v < body / V; v += 32) reinterpret_cast<uint4*>(dst)[v] = make_uint4(0u, 0u, 0u, 0u);
-            for (int r = body + lane; r < t; r += 32) dst[r] = T(0);
-            __syncwarp();
+            T* win = windows[threadIdx.x >> 5];
+            const int* r = rel;
+            const T* src = nullptr;
+            int b = 0, bt = 0;   // the first child's entries still to come
+            if (first < it.end) {
+                const EaEntry en = entries[first++];
+                const SnDev C = sn[en.child];
+                r += C.rel_off;
+                src = contrib + C.contrib_off + (long long)en.a * C.ldc;
+                b = en.a;
+                bt = C.m - C.w;
+            }
+            // rows [c, t) in windows that start on multiples of kEaWindow (the column starts on a 16-byte boundary:
+            // contribution offsets are multiples of 64 elements, ldc of 8)
+            for (int R = c / kEaWindow * kEaWindow; R < t; R += kEaWindow) {
+                constexpr int V = 16 / (int)sizeof(T);
+                for (int v = lane; v < kEaWindow / V; v += 32) reinterpret_cast<uint4*>(win)[v] = make_uint4(0u, 0u, 0u, 0u);
+                __syncwarp();
+                int taken = 0;
+                if (b < bt) {
+                    int idx[D];
+                    T sv[D];
+#pragma unroll
+                    for (int u = 0; u < D; ++u) {
+                        const int q = b + lane + 32 * u;
+                        idx[u] = q < bt ? r[q] - shift - R : kEaWindow;   // ascending, so at most kEaWindow of them here
+                        sv[u] = q < bt ? src[q] : T(0);
+                    }
+#pragma unroll
+                    for (int u = 0; u < D; ++u) {
+                        const bool in = idx[u] < kEaWindow;
+                        if (in) win[idx[u]] = sv[u];
+                        taken += __popc(__ballot_sync(0xffffffffu, in));
+                    }
+                    __syncwarp();
+                }
+                b += taken;
+                const int lo = max(c, R), hi = min(t, R + kEaWindow);
+                for (int v = R / V + lane; v < (R + kEaWindow) / V; v += 32) {
+                    const int e = v * V;
+                    if (e >= lo && e + V <= hi) {
+                        reinterpret_cast<uint4*>(dst)[v] = reinterpret_cast<const uint4*>(win)[v - R / V];
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < V; ++k)
+                            if (e + k >= lo && e + k < hi) dst[e + k] = win[e + k - R];
+                    }
+                }
+                __syncwarp();
+            }
         }
-        for (int e = it.begin; e < it.end; ++e) {
+        for (int e = first; e < it.end; ++e) {
             const EaEntry en = entries[e];
             const SnDev C = sn[en.child];
             const int t = C.m - C.w;
             const int* r = rel + C.rel_off;
             const T* src = contrib + C.contrib_off + (long long)en.a * C.ldc;
             // rows of one child column are distinct, so loads of a batch are issued before its stores
-            constexpr int D = 8;   // loads of a batch in flight per lane
             for (int b0 = en.a + lane; b0 < t; b0 += 32 * D) {
                 int idx[D];
                 T sv[D], dv[D];
