@@ -169,6 +169,7 @@ constexpr int kTcPartial = kTcCols * kTcRows;       // floats of one partial til
 constexpr int kTcEpiLd = 33;                        // epilogue transpose buffer: 32 x 33 floats per warp
 constexpr int kTcMinSplitKb = 8;           // K blocks of a tile below which it is never split
 constexpr int kTcMaxParts = 4;             // most CTAs sharing one split tile (bounds the fixup's reads)
+constexpr int kTcSplitCost = 20;           // what a split tile costs beyond its K blocks, in K blocks (about 0.31 us each)
 
 // One rank-kn update C[rows, cols] -= W[rows, kbeg:kbeg+kn] L[cols, kbeg:kbeg+kn]^T of front s,
 // operands in the front's staging region (tensor maps 2*map (W, 256-row box), 2*map+1 (L,
@@ -274,36 +275,6 @@ __device__ __forceinline__ bool tc_epi_any(bool pred) {
         : "r"((uint32_t)pred), "n"(32 * kTcEpiWarps)
         : "memory");
     return r != 0;
-}
-
-// C[i0 + cc*32 + r, j] -= v[r] for the lower-triangle entries of rows below m; whole
-// float4 groups are read and written back (entries outside the triangle unchanged).
-__device__ __forceinline__ void tc_update_chunk(float* __restrict__ col, int ib, int j, int m, const float* v) {
-    float4 o[8];
-#pragma unroll
-    for (int r4 = 0; r4 < 8; ++r4) {
-        const int i = ib + 4 * r4;
-        if (i < m && i + 3 >= j) o[r4] = *reinterpret_cast<const float4*>(col + i);
-    }
-#pragma unroll
-    for (int r4 = 0; r4 < 8; ++r4) {
-        const int i = ib + 4 * r4;
-        if (i < m && i + 3 >= j) {
-            float4 x = o[r4];
-            if (i >= j && i + 3 < m) {
-                x.x -= v[4 * r4];
-                x.y -= v[4 * r4 + 1];
-                x.z -= v[4 * r4 + 2];
-                x.w -= v[4 * r4 + 3];
-            } else {
-                if (i >= j && i < m) x.x -= v[4 * r4];
-                if (i + 1 >= j && i + 1 < m) x.y -= v[4 * r4 + 1];
-                if (i + 2 >= j && i + 2 < m) x.z -= v[4 * r4 + 2];
-                if (i + 3 >= j && i + 3 < m) x.w -= v[4 * r4 + 3];
-            }
-            *reinterpret_cast<float4*>(col + i) = x;
-        }
-    }
 }
 
 template <bool BF16>
@@ -417,7 +388,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // and 32-row chunks [4h, 4h + 4), h = (w - 2) / 4
         const int q = warp & 3;
         const int c_first = ((warp - 2) >> 2) * 4;
-        const int jl = q * 32 + lane;
         int acc = 0;
         uint32_t acc_phase = 0;
         TcSegIter it(S, blockIdx.x, gridDim.x);
@@ -433,47 +403,52 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase));   // warp-uniform
             if (!ok) fail();
             tc_fence_after();
-            const int j = j0 + jl;
-            float* col = tc_column(panel, contrib, d, j0, j);   // column j of C, indexed by front row
             const uint32_t ta = tmem + (uint32_t)(acc * kTcRows) + ((uint32_t)(q * 32) << 16);
+            // C -= v for this warp's 32 columns x the 32 rows of chunk cc (thread = column on entry): through a
+            // shared-memory transpose, so that every global access of the warp is 32 consecutive rows of one column.  Each
+            // entry of C takes exactly one update per launch, so a reduction in L2 (no load, nothing to wait for) gives the
+            // same sum as a read-modify-write.
+            float* tb = epi_buf + (warp - 2) * 32 * kTcEpiLd;
+            const int jw = j0 + q * 32;   // the warp's first column
+            const long long ld = jw < d.w ? d.ldp : d.ldc;
+            float* colw = tc_column(panel, contrib, d, j0, jw);
+            auto update = [&](int cc, const float (&v)[32]) {
+#pragma unroll
+                for (int r = 0; r < 32; ++r) tb[r * kTcEpiLd + lane] = v[r];
+                __syncwarp();
+                const int i = i0 + cc * 32 + lane;   // this thread's row from here on
+                if (i < d.m && i0 + cc * 32 + 31 >= jw) {
+#pragma unroll
+                    for (int c = 0; c < 32; ++c)
+                        if (jw + c < jend && i >= jw + c) atomicAdd(colw + (long long)c * ld + i, -tb[lane * kTcEpiLd + c]);
+                }
+                __syncwarp();
+            };
+            // partial tiles in the workspace: float4 r4 of (quadrant, chunk, lane) at ((quadrant * 8 + chunk) * 8 + r4) * 32 +
+            // lane, so that a warp's accesses are whole 512-byte segments
+            auto part_at = [&](long long slot, int cc) {
+                return reinterpret_cast<float4*>(S.ws + slot * kTcPartial) + (q * 8 + cc) * 256 + lane;
+            };
             if (g.parts == 1) {
                 if (ok) {
-                    // the warp's 32 columns x 32 rows go through a shared-memory transpose, so that
-                    // every global access of the warp is 32 consecutive rows of one column
-                    float* tb = epi_buf + (warp - 2) * 32 * kTcEpiLd;
-                    const int jw = j0 + q * 32;   // the warp's first column
-                    const long long ld = jw < d.w ? d.ldp : d.ldc;
-                    float* colw = tc_column(panel, contrib, d, j0, jw);
 #pragma unroll 1
                     for (int cc = c_first; cc < c_first + 4; ++cc) {
                         float v[32];
                         tmem_ld32(ta + (uint32_t)(cc * 32), v);
-#pragma unroll
-                        for (int r = 0; r < 32; ++r) tb[r * kTcEpiLd + lane] = v[r];
-                        __syncwarp();
-                        const int i = i0 + cc * 32 + lane;   // this thread's row from here on
-                        // each entry of C takes exactly one update per launch, so a reduction in L2
-                        // (no load, nothing to wait for) gives the same sum as a read-modify-write
-                        if (i < d.m && i0 + cc * 32 + 31 >= jw) {
-#pragma unroll
-                            for (int c = 0; c < 32; ++c)
-                                if (jw + c < jend && i >= jw + c) atomicAdd(colw + (long long)c * ld + i, -tb[lane * kTcEpiLd + c]);
-                        }
-                        __syncwarp();
+                        update(cc, v);
                     }
                 }
             } else {
                 // partial tile: to the workspace; the last CTA of the tile adds all of them
                 if (ok) {
-                    float* mine = S.ws + (long long)g.slot * kTcPartial + (long long)jl * kTcRows;
 #pragma unroll 1
                     for (int cc = c_first; cc < c_first + 4; ++cc) {
                         float v[32];
                         tmem_ld32(ta + (uint32_t)(cc * 32), v);
+                        float4* mine = part_at(g.slot, cc);
 #pragma unroll
                         for (int r4 = 0; r4 < 8; ++r4)
-                            __stcg(reinterpret_cast<float4*>(mine + cc * 32) + r4,
-                                   make_float4(v[4 * r4], v[4 * r4 + 1], v[4 * r4 + 2], v[4 * r4 + 3]));
+                            __stcg(mine + r4 * 32, make_float4(v[4 * r4], v[4 * r4 + 1], v[4 * r4 + 2], v[4 * r4 + 3]));
                     }
                 }
                 __threadfence();
@@ -501,16 +476,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         // two partial tiles in flight per step, added in CTA order
 #pragma unroll 1
                         for (long long c = c_lo; c <= c_hi; c += 2) {
-                            const float4* p0 = reinterpret_cast<const float4*>(
-                                S.ws + it.slot_of(c, tt) * kTcPartial + (long long)jl * kTcRows + cc * 32);
                             const bool two = c + 1 <= c_hi;
-                            const float4* p1 = reinterpret_cast<const float4*>(
-                                S.ws + it.slot_of(two ? c + 1 : c, tt) * kTcPartial + (long long)jl * kTcRows + cc * 32);
+                            const float4* p0 = part_at(it.slot_of(c, tt), cc);
+                            const float4* p1 = part_at(it.slot_of(two ? c + 1 : c, tt), cc);
                             float4 x0[8], x1[8];
 #pragma unroll
                             for (int r4 = 0; r4 < 8; ++r4) {
-                                x0[r4] = __ldcg(p0 + r4);
-                                if (two) x1[r4] = __ldcg(p1 + r4);
+                                x0[r4] = __ldcg(p0 + r4 * 32);
+                                if (two) x1[r4] = __ldcg(p1 + r4 * 32);
                             }
 #pragma unroll
                             for (int r4 = 0; r4 < 8; ++r4) {
@@ -529,7 +502,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                 }
                             }
                         }
-                        if (j < jend) tc_update_chunk(col, i0 + cc * 32, j, d.m, v);
+                        update(cc, v);
                     }
                 }
             }
@@ -601,7 +574,8 @@ inline size_t tc_counter_count(int sms) { return (size_t)2 * sms; }
 // Grid and split of one launch of `tiles` tiles.  nkb: K blocks of every tile when all
 // tiles have the same K (0 otherwise: never split).  A launch with fewer tiles than SMs is
 // split in K when that is estimated faster: time in K blocks per CTA, a split tile costing
-// about kTcMinSplitKb more (its partial tiles through L2).  Larger launches take whole
+// kTcSplitCost more (its partial tiles through L2: 45 tiles of K = 1024 take 28 us whole and 37 us in 152 parts; 100 us
+// when the parts were written 16 bytes a lane apart).  Larger launches take whole
 // tiles round robin: the CTAs working on the column tiles that share W rows then stay at
 // the same K offsets, which a split tail breaks (operands read from HBM several times).
 struct TcPlanned {
@@ -617,7 +591,7 @@ inline TcPlanned tc_schedule(long long tiles, int nkb, int sms, int min_kb = kTc
     const long long G = std::max<long long>(1, std::min<long long>({(long long)sms, W / std::max(1, min_kb),
                                                                      tiles * kTcMaxParts}));
     const double t_whole = nkb;   // one wave of whole tiles
-    const double t_split = (double)((W + G - 1) / G) + std::max(1, min_kb);
+    const double t_split = (double)((W + G - 1) / G) + std::max(kTcSplitCost, min_kb);
     if (t_split < 0.9 * t_whole) {
         p.grid = (unsigned)G;
         p.dp_tiles = 0;
