@@ -858,6 +858,12 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool val
                  "l"(src), "r"(valid ? 4 : 0)
                  : "memory");
 }
+// 16-byte asynchronous copy global -> shared of the first `bytes` bytes (zero fill after them).
+__device__ __forceinline__ void cp_async16z(float* dst, const float* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(bytes)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -865,6 +871,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // Shared memory of k_panel_solve: two stages of (A21 chunk, X^T chunk), 32 K columns each.
 constexpr int kPanelKc = 32, kPanelLds = kSolveRows + 4;
 constexpr size_t kPanelSmemBytes = sizeof(float) * 2 * 2 * kPanelKc * kPanelLds;
+static_assert(4 * kPanelKc >= kDiagMax, "the stages hold the tile of L21 on its way to the factor");
 
 __device__ __forceinline__ void store_op4(__nv_bfloat16* p, float a, float b, float c, float e) {
     __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, e);
@@ -891,8 +898,11 @@ __device__ __forceinline__ void store_op1(float* p, float a) { *p = a; }
 // W21 = A21 X^T and L21 = W21 D^{-1} for rows [row0, row0 + rows) of the
 // front, 256 threads: thread (ty, tx) owns rows {4ty..4ty+3, 64+4ty..} and
 // columns {4tx..4tx+3, 64+4tx..} of the 128 x 128 tile (conflict-free 128-bit
-// shared loads).  X^T is upper triangular, so columns below 64 take no
-// updates from K >= 64.
+// shared loads; two rows per FP32 instruction).  X^T is upper triangular, so
+// columns below 64 take no updates from K >= 64.  L21 goes to the factor through
+// shared memory, so that a column's rows are written together.  The SM's FP32 pipe
+// (6 us a tile) and the launch bound it: 11,000 rows, 25.9 us with 4-byte
+// copies and stores of 16 scattered bytes a thread, 22.5 us now (timed alone).
 template <class Op>
 __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restrict__ tasks,
                                                      const SnDev* __restrict__ sn, float* __restrict__ panel,
@@ -907,22 +917,36 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const float* M = diag_slot_inverse<const float>(minv, linv, tk);
     float* A = panel + d.panel_off + row0 + (long long)k0 * d.ldp;   // A21 rows of this task, column-major
-    float acc[8][8];
+    f32x2 acc2[2][2][8];   // [row group][pair of rows][column]
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < 8; ++j) acc2[i][0][j] = acc2[i][1][j] = 0ull;
     // K chunks of KC columns copied asynchronously into two stages: every copy of a chunk in
     // flight at once, and the next chunk's copies under the current chunk's products
+    const bool aligned = ((row0 | (int)(d.panel_off & 3)) & 3) == 0;   // rows on 16-byte boundaries
     auto issue_chunk = [&](int kc, int st) {
         float* As = psm + 2 * st * KC * LDS;
         float* Ms = As + KC * LDS;
+        if (aligned) {
 #pragma unroll
-        for (int q = 0; q < (KC * kSolveRows) / 256; ++q) {
-            const int idx = tid + 256 * q, r = idx & (kSolveRows - 1), k = idx >> 7;
-            const bool ok = r < rows && kc + k < nb;
-            cp_async4(&As[k * LDS + r], ok ? A + r + (long long)(kc + k) * d.ldp : A, ok);
-            cp_async4(&Ms[k * LDS + r], M + (kc + k) * kDiagMax + r, true);
+            for (int q = 0; q < (KC * kSolveRows) / 1024; ++q) {
+                const int idx = tid + 256 * q, r = (idx & 31) * 4, k = idx >> 5;
+                const int left = kc + k < nb ? min(4, max(0, rows - r)) : 0;
+                cp_async16z(&As[k * LDS + r], left > 0 ? A + r + (long long)(kc + k) * d.ldp : A, 4 * left);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < (KC * kSolveRows) / 256; ++q) {
+                const int idx = tid + 256 * q, r = idx & (kSolveRows - 1), k = idx >> 7;
+                const bool ok = r < rows && kc + k < nb;
+                cp_async4(&As[k * LDS + r], ok ? A + r + (long long)(kc + k) * d.ldp : A, ok);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < (KC * kDiagMax) / 1024; ++q) {
+            const int idx = tid + 256 * q, r = (idx & 31) * 4, k = idx >> 5;
+            cp_async16z(&Ms[k * LDS + r], M + (kc + k) * kDiagMax + r, 16);
         }
         cp_async_commit();
     };
@@ -940,50 +964,69 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
         const bool low_cols = kc < 64;   // X^T[k][j] = 0 for j < k: columns 0..63 see K < 64 only
 #pragma unroll 4
         for (int k = 0; k < KC; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[k * LDS + 4 * ty]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[k * LDS + 64 + 4 * ty]);
+            const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[k * LDS + 4 * ty]);
+            const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[k * LDS + 64 + 4 * ty]);
             const float4 b1 = *reinterpret_cast<const float4*>(&Ms[k * LDS + 64 + 4 * tx]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
             const float bh[4] = {b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][4 + j] = fmaf(av[i], bh[j], acc[i][4 + j]);
+            for (int j = 0; j < 4; ++j) {
+                const f32x2 bb = pack2(bh[j], bh[j]);
+                acc2[0][0][4 + j] = fma2(a0.x, bb, acc2[0][0][4 + j]);
+                acc2[0][1][4 + j] = fma2(a0.y, bb, acc2[0][1][4 + j]);
+                acc2[1][0][4 + j] = fma2(a1.x, bb, acc2[1][0][4 + j]);
+                acc2[1][1][4 + j] = fma2(a1.y, bb, acc2[1][1][4 + j]);
+            }
             if (low_cols) {
                 const float4 b0 = *reinterpret_cast<const float4*>(&Ms[k * LDS + 4 * tx]);
                 const float bl[4] = {b0.x, b0.y, b0.z, b0.w};
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bl[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) {
+                    const f32x2 bb = pack2(bl[j], bl[j]);
+                    acc2[0][0][j] = fma2(a0.x, bb, acc2[0][0][j]);
+                    acc2[0][1][j] = fma2(a0.y, bb, acc2[0][1][j]);
+                    acc2[1][0][j] = fma2(a1.x, bb, acc2[1][0][j]);
+                    acc2[1][1][j] = fma2(a1.y, bb, acc2[1][1][j]);
+                }
             }
         }
         __syncthreads();   // this stage is refilled two chunks later
     }
+    float acc[8][8];   // [row][column]
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            unpack2(acc2[i][0][j], acc[4 * i][j], acc[4 * i + 1][j]);
+            unpack2(acc2[i][1][j], acc[4 * i + 2][j], acc[4 * i + 3][j]);
+        }
     // epilogue: L21 = W21 D^{-1} to the factor (column-major), W21 and L21 to the staging rows (K-major)
     const float* dinv = diag_slot_d(minv, tk) + kDiagMax;
-    const bool vec_rows = ((d.panel_off + row0) & 3) == 0;
+    // column col of the tile at shared column (col % 4) * 32 + col / 4: a warp's 16-byte stores fall on distinct banks
 #pragma unroll
-    for (int jg = 0; jg < 2; ++jg) {
+    for (int jg = 0; jg < 2; ++jg)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int col = 64 * jg + 4 * tx + j;
-            if (col >= nb) continue;
             const float di = dinv[col];
 #pragma unroll
-            for (int ig = 0; ig < 2; ++ig) {
-                const int r = 64 * ig + 4 * ty;
-                float* dst = A + r + (long long)col * d.ldp;
-                const float l0 = acc[4 * ig + 0][4 * jg + j] * di, l1 = acc[4 * ig + 1][4 * jg + j] * di;
-                const float l2 = acc[4 * ig + 2][4 * jg + j] * di, l3 = acc[4 * ig + 3][4 * jg + j] * di;
-                if (vec_rows && r + 4 <= rows) {
-                    *reinterpret_cast<float4*>(dst) = make_float4(l0, l1, l2, l3);
-                } else {
-                    if (r + 0 < rows) dst[0] = l0;
-                    if (r + 1 < rows) dst[1] = l1;
-                    if (r + 2 < rows) dst[2] = l2;
-                    if (r + 3 < rows) dst[3] = l3;
-                }
+            for (int ig = 0; ig < 2; ++ig)
+                *reinterpret_cast<float4*>(&psm[(j * 32 + 16 * jg + tx) * LDS + 64 * ig + 4 * ty]) =
+                    make_float4(acc[4 * ig + 0][4 * jg + j] * di, acc[4 * ig + 1][4 * jg + j] * di,
+                                acc[4 * ig + 2][4 * jg + j] * di, acc[4 * ig + 3][4 * jg + j] * di);
+        }
+    __syncthreads();
+    {
+        const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll 4
+        for (int col = warp; col < nb; col += 8) {
+            const float* src = &psm[((col & 3) * 32 + (col >> 2)) * LDS];
+            float* dst = A + (long long)col * d.ldp;
+            if (aligned && 4 * lane + 4 <= rows) {
+                *reinterpret_cast<float4*>(dst + 4 * lane) = *reinterpret_cast<const float4*>(src + 4 * lane);
+            } else if (aligned) {
+                for (int r = 4 * lane; r < rows; ++r) dst[r] = src[r];
+            } else {
+                for (int r = lane; r < rows; r += 32) dst[r] = src[r];
             }
         }
     }
