@@ -453,8 +453,10 @@ class UtduNumericFactorization:
     def Refactorize(self, matrix: SymmetricCSRMatrix) -> None:
         """New values, same pattern, same device storage."""
         self._symbolic.EnsureCompatible(matrix)
+        self._refactorize_values(np.ascontiguousarray(matrix.Values, np.float64))
+
+    def _refactorize_values(self, vals) -> None:
         lib = _native.gpu()
-        vals = np.ascontiguousarray(matrix.Values, np.float64)
         st = lib.uchol_refactorize(self._h, vals.ctypes.data_as(C.c_void_p), 0, C.byref(self._stats))
         raise_for_status(st, lib.uchol_last_error())
         self._diag = None
@@ -724,7 +726,9 @@ class BatchedUtduSolver:
                                      C.byref(h))
         raise_for_status(st, lib.uchol_host_last_error())
         union = self.Union(mats)
-        return BatchedUtduSymbolic(UtduSymbolicFactorization._from_analysis(h, union), sizes)
+        symbolic = BatchedUtduSymbolic(UtduSymbolicFactorization._from_analysis(h, union), sizes)
+        symbolic._structure = BatchedUtduSymbolic._joined(rp, cl)
+        return symbolic
 
     def Factorize(self, matrices, symbolic: "BatchedUtduSymbolic | None" = None) -> "BatchedUtduFactorization":
         mats = list(matrices)
@@ -744,6 +748,23 @@ class BatchedUtduSymbolic:
         self.Union = union
         self.Sizes = np.asarray(sizes, np.int64)
         self.Offsets = np.concatenate([[0], np.cumsum(self.Sizes)]).astype(np.int64)
+        self._structure = None   # row pointers and columns of the analysed systems, one after the other
+
+    @staticmethod
+    def _joined(row_ptrs, cols):
+        return (np.concatenate(row_ptrs) if row_ptrs else np.zeros(0, np.int32),
+                np.concatenate(cols) if cols else np.zeros(0, np.int32))
+
+    def _union_values(self, matrices):
+        """The union's values (the systems' values one after the other) when the systems have exactly the analysed
+        structure, which the union matrix need then not be built for again; None otherwise."""
+        if self._structure is None or not matrices or any(m is None for m in matrices):
+            return None
+        rp, cl = self._joined([m.RowPointers for m in matrices], [m.ColumnIndices for m in matrices])
+        if not (np.array_equal(rp, self._structure[0]) and np.array_equal(cl, self._structure[1])):
+            return None
+        values = np.concatenate([np.asarray(m.Values, np.float64) for m in matrices])
+        return values if len(values) == len(cl) else None
 
     @property
     def Count(self) -> int:
@@ -806,7 +827,11 @@ class BatchedUtduFactorization:
         mats = list(matrices)
         if len(mats) != self.Symbolic.Count:
             raise ArgumentException("The systems do not match the batch analysis.")
-        self.Union.Refactorize(BatchedUtduSolver(self._options).Union(mats))
+        values = self.Symbolic._union_values(mats)
+        if values is None:
+            self.Union.Refactorize(BatchedUtduSolver(self._options).Union(mats))
+        else:
+            self.Union._refactorize_values(values)
 
 
 class ResidualCalculator:

@@ -122,3 +122,16 @@ def test_batch_refactorize_equals_fresh_factor(gpu_lib):
         assert np.array_equal(a, b)
     with pytest.raises(ArgumentException):
         f.Solve(bs[:-1])
+
+
+def test_union_values_follow_the_analysed_structure():
+    """The joined values equal the union matrix's; another structure, order or a missing system is left to the union."""
+    mats = small_batch(6)
+    solver = BatchedUtduSolver()
+    sym = solver.Analyze(mats)
+    assert np.array_equal(sym._union_values(mats), solver.Union(mats).Values)
+    assert sym._union_values(mats[::-1]) is None
+    assert sym._union_values(mats[:-1]) is None
+    assert sym._union_values(mats[:-1] + [None]) is None
+    other = small_batch(6, seed=4)
+    assert sym._union_values(other) is None
