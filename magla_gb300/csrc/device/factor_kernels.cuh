@@ -411,10 +411,10 @@ __global__ void __launch_bounds__(kSmallFrontThreads) k_small_fronts(const int* 
 // diagonal block in shared memory, one CTA per block; writes the unit L11,
 // the pivots D and the statistics (UtduNumericFactorization.cs:553-592
 // restricted to the diagonal block).
-constexpr int kMaxPivotBlock = 64;
+constexpr int kMaxPivotBlock = 64, kPivotThreads = 256;
 
 template <class T>
-__global__ void __launch_bounds__(128) k_pivot_block(const PanelTask* __restrict__ tasks, const SnDev* __restrict__ sn,
+__global__ void __launch_bounds__(kPivotThreads) k_pivot_block(const PanelTask* __restrict__ tasks, const SnDev* __restrict__ sn,
                                                      T* __restrict__ panel, double* __restrict__ diag,
                                                      const FactorCtl* __restrict__ ctlp, PivotStats* st) {
     __shared__ double Dg[kMaxPivotBlock * (kMaxPivotBlock + 1)];
@@ -426,19 +426,19 @@ __global__ void __launch_bounds__(128) k_pivot_block(const PanelTask* __restrict
     const int tid = threadIdx.x, lane = tid & 31;
     T* P = panel + d.panel_off + j0 + (long long)j0 * d.ldp;
 #pragma unroll 4
-    for (int e = tid; e < kMaxPivotBlock * nb; e += 128) {
+    for (int e = tid; e < kMaxPivotBlock * nb; e += kPivotThreads) {
         const int r = e % kMaxPivotBlock, c = e / kMaxPivotBlock;
         if (r >= c && r < nb) Dg[r + c * ld] = (double)P[r + (long long)c * d.ldp];
     }
     PivotAcc acc;
     __syncthreads();
-    smem_ldlt<4, kMaxPivotBlock / 32>(Dg, ld, nb, nb, Wc, kMaxPivotBlock, [&](int k, double raw) {
+    smem_ldlt<kPivotThreads / 32, kMaxPivotBlock / 32>(Dg, ld, nb, nb, Wc, kMaxPivotBlock, [&](int k, double raw) {
         const double piv = acc.accept(raw, d.first_col + j0 + k, ctl);
         if (lane == 0) diag[d.first_col + j0 + k] = piv;
         return piv;
     });
 #pragma unroll 4
-    for (int e = tid; e < kMaxPivotBlock * nb; e += 128) {
+    for (int e = tid; e < kMaxPivotBlock * nb; e += kPivotThreads) {
         const int r = e % kMaxPivotBlock, c = e / kMaxPivotBlock;
         if (r >= c && r < nb) P[r + (long long)c * d.ldp] = (T)Dg[r + c * ld];
     }
