@@ -309,16 +309,9 @@ struct StreamTimer {
 // K blocks of a tensor-core tile below which a launch is never split in K.
 int split_min_kb(const uchol_options& o) { return o.split_min_kblocks == 0 ? kTcMinSplitKb : o.split_min_kblocks; }
 
-// Front-size buckets (32 rows each) factorised whole.  Mixed: up to 96 rows by default.  FP64: up to 32, by lanes; the
-// blocked path spreads the wider ones over the device, where one SM does two multiply-adds a clock (up to 96 rows / up to
-// 32: 48 batched Laplacians 11.2 / 9.8 ms, 6^3 elasticity 1.13 / 1.07 ms, 20^3 Laplacian 3.10 / 3.00 ms).
-int small_front_mask(const uchol_options& o) {
-    return o.small_front_buckets ? o.small_front_buckets : o.precision == UCHOL_PRECISION_FP64 ? 0x1 : 0x7;
-}
-
 PlanConfig config_for(const uchol_options& o) {
     PlanConfig c;
-    c.small_mask = small_front_mask(o);
+    c.small_mask = o.small_front_buckets ? o.small_front_buckets : 0x7;
     c.pivot_block = std::min(kMaxPivotBlock, std::max(4, std::min(128, o.panel_width)));
     c.merge_cols = o.chain_merge_width == 0 ? kDefaultMergeCols : std::max(0, o.chain_merge_width);
     c.inv_cols = o.inverse_block_width != 0 ? std::max(0, o.inverse_block_width)
@@ -1675,7 +1668,7 @@ int uchol_autotune(uchol_symbolic s, int n, int nnz, const double* values, const
                 return std::numeric_limits<double>::infinity();
             }
         };
-        int mask = small_front_mask(o0);
+        int mask = o0.small_front_buckets ? o0.small_front_buckets : 0x7;
         int bw = mixed ? (o0.block_width > 0 ? o0.block_width : kDiagMax) : 0;
         int merge = o0.chain_merge_width, split = o0.split_min_kblocks;
         const double t_default = timed(mask, bw, merge, split);
