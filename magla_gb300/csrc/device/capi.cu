@@ -13,6 +13,7 @@
 #include <type_traits>
 #include <limits>
 #include <map>
+#include <set>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
@@ -117,7 +118,7 @@ struct DevPlan {
     Plan plan;
     DBuf sn, rel, asm_pos, ea_items, ea_entries, small, pivot_tasks, panel_tasks, simt_jobs, tc_jobs,
         stage;
-    DBuf fvec_off, solve_fronts, solve_tasks, inv_warp, inv_cta, inv_tasks;
+    DBuf fvec_off, gather_ptr, gather_src, solve_tasks, inv_warp, inv_cta, inv_tasks;
     DBuf rows, child_ptr, children;   // structure of the device fronts
 };
 
@@ -211,7 +212,8 @@ struct uchol_symbolic_s {
         dp->tc_jobs.upload(P.tc_jobs, stream, "plan");
         dp->stage.upload(P.stage, stream, "plan");
         dp->fvec_off.upload(P.fvec_off, stream, "plan");
-        dp->solve_fronts.upload(P.solve_fronts, stream, "plan");
+        dp->gather_ptr.upload(P.gather_ptr, stream, "plan");
+        dp->gather_src.upload(P.gather_src, stream, "plan");
         dp->solve_tasks.upload(P.solve_tasks, stream, "plan");
         dp->inv_warp.upload(P.inv_warp, stream, "plan");
         dp->inv_cta.upload(P.inv_cta, stream, "plan");
@@ -240,6 +242,7 @@ struct uchol_factor_s {
     DBuf inv_scratch;                   // inversion scratch, where the contribution arena is too small for it
     DBuf linv_off;                      // inverse fronts: off-diagonal blocks of the diagonal block's inverse
     DBuf inv_partial;                   // inverse fronts: backward partial sums (solve workspace)
+    DBuf inv_cols_cnt;                  // inverse fronts: chunks done per column block (backward)
     DBuf inv_diag_partial, inv_diag_cnt;   // inverse fronts: chunk partial sums of the diagonal products, counters
     DBuf minv;                          // mixed path: per outer block X^T, D, D^{-1} of each diagonal block
     DBuf solve_flags;                   // per diagonal block: forward and backward "solution published" flags
@@ -895,6 +898,9 @@ void check_solve_status(uchol_factor_s* F) {
     CK(cudaMemcpy(&h, F->solve_status.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (h != 0) {
         CK(cudaMemset(F->solve_status.p, 0, sizeof(int)));
+        // chunks that gave up have not counted in
+        if (F->inv_diag_cnt.p) CK(cudaMemset(F->inv_diag_cnt.p, 0, F->inv_diag_cnt.bytes));
+        if (F->inv_cols_cnt.p) CK(cudaMemset(F->inv_cols_cnt.p, 0, F->inv_cols_cnt.bytes));
         throw Error(UCHOL_TIMEOUT, "a bounded device wait expired during a triangular solve (status " +
                                        std::to_string(h) + ")");
     }
@@ -943,6 +949,8 @@ SolveArgs solve_args(uchol_factor_s* F, int nrhs) {
     A.child_ptr = D.child_ptr.as<int>();
     A.children = D.children.as<int>();
     A.fvec_off = D.fvec_off.as<long long>();
+    A.gather_ptr = D.gather_ptr.as<unsigned>();
+    A.gather_src = D.gather_src.as<unsigned>();
     A.fv_stride = D.plan.fvec_elems;
     A.n = F->sym->n;
     A.nrhs = nrhs;
@@ -1010,7 +1018,7 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
             k_fwd_solo<T, Cv, SB><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, linv, fv, fv2, diag, work);
         } else if (L.kind == SolveLaunch::FwdInvDiag) {
             k_fwd_inv_diag<T, Cv, SB, RGD><<<grid(L.count, RGD), 256, inv_solve_smem<T, Cv, SB, RGD>(), st>>>(
-                tasks + L.begin, A, linv, F->linv_off.as<Cv>(), fv, fv2, diag, work, F->inv_diag_partial.as<Cv>(),
+                tasks + L.begin, A, linv, F->linv_off.as<Cv>(), fv, fv2, work, F->inv_diag_partial.as<Cv>(),
                 F->inv_diag_cnt.as<unsigned>(), status);
         } else if (L.kind == SolveLaunch::FwdInvTail) {
             k_fwd_inv_tail<T, Cv, SB, RG><<<grid(L.count, RG), 256, inv_tail_smem<T, Cv, SB, RG, false>(), st>>>(
@@ -1038,13 +1046,14 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
             k_bwd_cols_reduce<Cv><<<L.count, 128, 0, st>>>(tasks + L.begin, A, F->bwd_partial.as<Cv>(), fv);
         } else if (L.kind == SolveLaunch::BwdInvCols) {
             k_bwd_inv_cols<T, Cv, SB, RG><<<grid(L.count, RG), 256, inv_tail_smem<T, Cv, SB, RG, true>(), st>>>(
-                tasks + L.begin, A, F->solve_maps.as<CUtensorMap>() + 2 * P.count, fv, F->inv_partial.as<Cv>(), status);
+                tasks + L.begin, A, F->solve_maps.as<CUtensorMap>() + 2 * P.count, fv, fv2, diag, work,
+                F->inv_partial.as<Cv>(), F->inv_cols_cnt.as<unsigned>(), status);
         } else if (L.kind == SolveLaunch::BwdInvReduce) {
-            k_bwd_inv_reduce<Cv, SB><<<grid(L.count, 1), SB, 0, st>>>(tasks + L.begin, A, fv,
-                                                                                        F->inv_partial.as<Cv>());
+            k_bwd_inv_reduce<Cv, SB><<<grid(L.count, 1), SB, 0, st>>>(tasks + L.begin, A, fv, fv2, diag,
+                                                                      F->inv_partial.as<Cv>());
         } else if (L.kind == SolveLaunch::BwdInvDiag) {
             k_bwd_inv_diag<T, Cv, SB, RGD><<<grid(L.count, RGD), 256, inv_solve_smem<T, Cv, SB, RGD>(), st>>>(
-                tasks + L.begin, A, linv, F->linv_off.as<Cv>(), fv, work, F->inv_diag_partial.as<Cv>(),
+                tasks + L.begin, A, linv, F->linv_off.as<Cv>(), fv, fv2, diag, work, F->inv_diag_partial.as<Cv>(),
                 F->inv_diag_cnt.as<unsigned>(), status);
         } else if (L.kind == SolveLaunch::BwdSolo) {
             k_bwd_solo<Cv, SB><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, linv, fv, fv2, work);
@@ -1236,7 +1245,9 @@ void ensure_workspace(uchol_factor_s* F, int nrhs) {
     F->inv_partial.alloc((size_t)std::max(1, P.inv_partial_slots) * P.cfg.solve_block * nrhs * cv, "solve workspace");
     F->inv_diag_partial.alloc((size_t)std::max(1, P.inv_diag_slots) * P.cfg.solve_block * nrhs * cv, "solve workspace");
     F->inv_diag_cnt.alloc((size_t)std::max(1, P.inv_diag_slots) * nrhs * sizeof(unsigned), "solve workspace");
+    F->inv_cols_cnt.alloc((size_t)std::max(1, P.inv_partial_slots) * nrhs * sizeof(unsigned), "solve workspace");
     CK(cudaMemsetAsync(F->inv_diag_cnt.p, 0, F->inv_diag_cnt.bytes, S->stream));   // the last chunk resets each
+    CK(cudaMemsetAsync(F->inv_cols_cnt.p, 0, F->inv_cols_cnt.bytes, S->stream));
     if (F->solve_graph) {
         CK(cudaGraphExecDestroy(F->solve_graph));
         F->solve_graph = nullptr;
@@ -1283,7 +1294,7 @@ void dots(uchol_factor_s* F, int nrhs, const double* u, int ldu, const double* v
     double* partial = F->scal.as<double>();
     dim3 g(kDotBlocks, nrhs);
     k_dot_partial<<<g, 256, 0, S->stream>>>(u, ldu, v, ldv, S->n, partial);
-    k_dot_finish<<<1, 32 * ((nrhs + 31) / 32), 0, S->stream>>>(partial, kDotBlocks, nrhs, out);
+    k_dot_finish<<<(nrhs + 7) / 8, 256, 0, S->stream>>>(partial, kDotBlocks, nrhs, out);
     counted(2);
 }
 

@@ -377,7 +377,7 @@ void dm_dots(uchol_dmatrix_s* m, int nrhs, const double* u, int ldu, const doubl
              double* out) {
     dim3 g(kDotBlocks, nrhs);
     k_dot_partial<<<g, 256, 0, m->stream>>>(u, ldu, v, ldv, m->n, partial);
-    k_dot_finish<<<1, 32 * ((nrhs + 31) / 32), 0, m->stream>>>(partial, kDotBlocks, nrhs, out);
+    k_dot_finish<<<(nrhs + 7) / 8, 256, 0, m->stream>>>(partial, kDotBlocks, nrhs, out);
     counted(2);
 }
 

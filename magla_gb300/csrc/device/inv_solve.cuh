@@ -4,12 +4,15 @@
 //   y_1 = Linv_11 f_1                  (k_fwd_inv_diag: one CTA per block row),
 //   f_2 -= L_21 y_1                    (k_fwd_inv_tail: one CTA per chunk of trailing rows);
 // backward:
-//   g_1 -= L_21^T g_2                  (k_bwd_inv_cols: partial sums per chunk of rows;
-//                                       k_bwd_inv_reduce adds them in chunk order),
+//   g_1 = D^-1 y_1 - L_21^T g_2        (k_bwd_inv_cols: partial sums per chunk of rows, added in
+//                                       chunk order by the last chunk of a column block or, of
+//                                       fronts of more than kGatherRows rows, by k_bwd_inv_reduce),
 //   x_1 = Linv_11^T g_1                (k_bwd_inv_diag: one CTA per block column).
 // The algebra is the reference's supernodal substitution
 // (CAESolvers/UCHOL/UtduNumericFactorization.cs:139-207) with the triangular solve of
-// the diagonal block written as a product with its inverse; the result differs only
+// the diagonal block written as a product with its inverse (fronts of up to kGatherRows rows gather f
+// from the children and g_2 from the ancestors where they are read: two launches a level and direction, which
+// are what a chain of small fronts waits for); the result differs only
 // in rounding.  The inverse is built once per factorisation from the inverses of the
 // SB x SB diagonal blocks, by doubling halves: X_21 = -X_22 (L_21 X_11) (k_inv_product).
 #pragma once
@@ -239,15 +242,14 @@ __device__ __forceinline__ bool inv_chunk_combine(Cv (&v)[FG], bool fin, int row
 }
 
 // Forward y_i = sum_{j <= i} Linv(i, j) f_j for right-hand sides [RG blockIdx.y, +RG);
-// writes y_i (front vector yv) and y_i / D (work).  Thread (row, pid) sums columns
-// [pid CPT, pid CPT + CPT) of each block.
+// writes y_i (front vector yv).  Thread (row, pid) sums columns [pid CPT, pid CPT + CPT)
+// of each block.
 template <class T, class Cv, int SB, int RG>
 __global__ void __launch_bounds__(256, 1) k_fwd_inv_diag(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
                                                          const Cv* __restrict__ linv, const Cv* __restrict__ linv_off,
                                                          const Cv* __restrict__ fv, Cv* __restrict__ yv,
-                                                         const double* __restrict__ diag, Cv* __restrict__ work,
-                                                         Cv* __restrict__ pbuf, unsigned* __restrict__ cnt,
-                                                         int* status) {
+                                                         const Cv* __restrict__ work, Cv* __restrict__ pbuf,
+                                                         unsigned* __restrict__ cnt, int* status) {
     using R = LevelRhs<Cv, SB, RG>;
     constexpr int TPR = R::TP, CPT = SB / TPR, RS = R::RS, FG = R::FG;
     extern __shared__ __align__(128) unsigned char blk_smem[];
@@ -284,7 +286,9 @@ __global__ void __launch_bounds__(256, 1) k_fwd_inv_diag(const SolveBlockTask* _
     auto fetch = [&](int j) {
         pf.fetch([&](int c, int g) {
             const int col = j * SB + c;
-            return (g < ng && col < d.w) ? fv[fo + (long long)(rg + g) * A.fv_stride + col] : Cv(0);
+            if (g >= ng || col >= d.w) return Cv(0);
+            if (d.m > kGatherRows) return fv[fo + col + (long long)(rg + g) * A.fv_stride];
+            return add_children<Cv>(A, fo + col, rg + g, fv, work[d.first_col + col + (long long)(rg + g) * A.ldw]);
         });
     };
     fetch(j0);
@@ -338,7 +342,6 @@ __global__ void __launch_bounds__(256, 1) k_fwd_inv_diag(const SolveBlockTask* _
             if (g >= ng || row >= kn) break;
             const int col = i * SB + row;
             yv[fo + (long long)(rg + g) * A.fv_stride + col] = y[q];
-            work[d.first_col + col + (long long)(rg + g) * A.ldw] = (Cv)((double)y[q] / diag[d.first_col + col]);
         }
     }
 }
@@ -360,6 +363,7 @@ struct TailTiles {
     static constexpr int NG = SB / RT;
     static constexpr int NS = 256 / (NG * NH);
     static constexpr int RS = LevelRhs<Cv, SB, RG>::RS;   // row stride of the right-hand blocks
+    static constexpr int FQ = (SB * RG + 255) / 256;      // results of a thread (forward)
     static_assert(NG * NH * NS == 256 && RG % GT == 0, "thread tiles must cover the CTA");
 };
 
@@ -419,7 +423,7 @@ __device__ __forceinline__ void lds_rhs(const Cv* p, Cv (&v)[GT]) {
     }
 }
 
-// Forward trailing rows [r0, r1) of an inverse front: f -= L[r0:r1, 0:w] y, by half tiles
+// Forward trailing rows [r0, r1) of an inverse front: f = the children's entries - L[r0:r1, 0:w] y, by half tiles
 // of SB rows x SB/2 columns (tensor map `maps`: box {SB, SB/2}); the tiles start at r0
 // rounded down to 16 bytes.  Thread (row group, right-hand group, column split) keeps an
 // RT x GT tile of sums.
@@ -466,6 +470,14 @@ __global__ void __launch_bounds__(256, 2) k_fwd_inv_tail(const SolveBlockTask* _
             start_box_tile(stage(0), maps + tk.s, ra, 0, kBytes, &bar[0]);
             if (nh > 1) start_box_tile(stage(1), maps + tk.s, ra, HC, kBytes, &bar[1]);
         }
+        Cv f0[W::FQ];   // the children's entries of this thread's results
+#pragma unroll
+        for (int q = 0; q < W::FQ; ++q) {
+            const int e = tid + 256 * q, g = e / SB, i = ra + e - g * SB;
+            f0[q] = !(e < SB * RG && g < ng && i >= r0 && i < r1) ? Cv(0)
+                    : d.m > kGatherRows ? fv[fo + i + (long long)(rg + g) * A.fv_stride]
+                                              : add_children<Cv>(A, fo + i, rg + g, fv, Cv(0));
+        }
         pf.commit(ybuf(0));
         if (nh > 1) fetch(1);
         Cv acc[RT][GT];
@@ -500,16 +512,53 @@ __global__ void __launch_bounds__(256, 2) k_fwd_inv_tail(const SolveBlockTask* _
 #pragma unroll
             for (int g = 0; g < GT; ++g) part[(cs * SB + rgp * RT + a) * RG + rh * GT + g] = acc[a][g];
         __syncthreads();
-        for (int e = tid; e < SB * RG; e += blockDim.x) {
-            const int g = e / SB, lr = e - g * SB, i = ra + lr;
-            if (g >= ng || i < r0 || i >= r1) continue;
+#pragma unroll
+        for (int q = 0; q < W::FQ; ++q) {
+            const int e = tid + 256 * q, g = e / SB, lr = e - g * SB, i = ra + lr;
+            if (e >= SB * RG || g >= ng || i < r0 || i >= r1) continue;
             Cv sum = part[lr * RG + g];
 #pragma unroll
             for (int p = 1; p < NS; ++p) sum += part[(p * SB + lr) * RG + g];
-            fv[fo + (long long)(rg + g) * A.fv_stride + i] -= sum;
+            fv[fo + (long long)(rg + g) * A.fv_stride + i] = f0[q] - sum;
         }
         __syncthreads();
     }
+}
+
+// g = y / D - the nq chunks' partial sums of one column block, in chunk order, for ng right-hand sides: N results a
+// thread, the loads of U chunks in flight: the latency of these loads is what the level waits for (23 x 17 x 11
+// elasticity, 5 right-hand sides: 28.9 ms with 6 chunks in flight, 29.7 with 2).
+template <class Cv, int SB, int N, int U>
+__device__ __forceinline__ void add_chunks(const Cv* __restrict__ slot, int nq, const SolveArgs& A, const SnDev& d, int c0,
+                                           int ng, long long fo, Cv* __restrict__ fv, const Cv* __restrict__ yv,
+                                           const double* __restrict__ diag) {
+    const long long step = (long long)A.nrhs * SB;
+    long long at[N];
+    bool on[N];
+    Cv v[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int e = threadIdx.x + 256 * k, g = e / SB, col = c0 + e - g * SB;
+        on[k] = g < ng && col < d.w;
+        at[k] = fo + (long long)g * A.fv_stride + col;
+        v[k] = on[k] ? (Cv)((double)yv[at[k]] / diag[d.first_col + col]) : Cv(0);
+    }
+    for (int q0 = 0; q0 < nq; q0 += U) {
+        Cv p[U][N];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                p[u][k] = on[k] && q0 + u < nq ? __ldcg(slot + (q0 + u) * step + threadIdx.x + 256 * k) : Cv(0);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                if (q0 + u < nq) v[k] -= p[u][k];
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+        if (on[k]) fv[at[k]] = v[k];
 }
 
 // Backward: column block kb of an inverse front against its trailing rows [r0, r1) (task
@@ -517,12 +566,15 @@ __global__ void __launch_bounds__(256, 2) k_fwd_inv_tail(const SolveBlockTask* _
 // box {SB/2, SB}), each transposed in shared memory so that a thread's RT columns are read
 // without bank conflicts and g is a broadcast.  Thread (column group, right-hand group, row
 // split) keeps an RT x GT tile of sums; column group q holds columns q + NG a.  The sums go
-// to partial slot `slot` ((slot nrhs + r) SB + c for right-hand side r, column c), which
-// k_bwd_inv_reduce adds to g of the block's columns.
+// to partial slot `slot` ((slot nrhs + r) SB + c for right-hand side r, column c); the CTA
+// that completes the block's chunks (a counter, no waiting) adds them in chunk order into g,
+// k_bwd_inv_reduce those of fronts of more than kGatherRows rows.
 template <class T, class Cv, int SB, int RG>
 __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
-                                                         const CUtensorMap* __restrict__ maps, const Cv* __restrict__ fv,
-                                                         Cv* __restrict__ partial, int* status) {
+                                                         const CUtensorMap* __restrict__ maps, Cv* __restrict__ fv,
+                                                         const Cv* __restrict__ yv, const double* __restrict__ diag,
+                                                         const Cv* __restrict__ work, Cv* __restrict__ partial,
+                                                         unsigned* __restrict__ cnt, int* status) {
     static_assert(sizeof(T) == sizeof(Cv), "factor and vector elements of one size");
     using W = TailTiles<Cv, SB, RG>;
     constexpr int HR = SB / 2, RT = W::RT, GT = W::GT, NG = W::NG, NH = W::NH, NS = W::NS, RS = W::RS;
@@ -539,7 +591,10 @@ __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* _
     auto xbuf = [&](int k) { return xb0 + k * HR * RS; };
     Cv* const part = reinterpret_cast<Cv*>(stage0);      // after the last tile: NS x SB x RG
     __shared__ unsigned long long bar[2];
+    __shared__ int last;
     const SolveBlockTask tk = tasks[blockIdx.x];
+    const SnDev d = A.sn[tk.s];
+    const int* rows = A.rows + d.rows_off;
     const int kb = tk.k0, r0 = tk.r0, r1 = tk.r1, ra = r0 & ~(kAlign - 1);
     const int ntile = (r1 - ra + HR - 1) / HR;
     const int tid = threadIdx.x, cgp = tid % NG, rh = (tid / NG) % NH, rsp = tid / (NG * NH);
@@ -557,7 +612,9 @@ __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* _
             const int tr = ra + t * HR;
             pf.fetch([&](int r, int g) {
                 const int gr = tr + r;
-                return (g < ng && gr >= r0 && gr < r1) ? fv[fo + (long long)(rg + g) * A.fv_stride + gr] : Cv(0);
+                if (g >= ng || gr < r0 || gr >= r1) return Cv(0);
+                return d.m > kGatherRows ? fv[fo + gr + (long long)(rg + g) * A.fv_stride]
+                                               : work[rows[gr] + (long long)(rg + g) * A.ldw];
             });
         };
         fetch(0);
@@ -619,23 +676,44 @@ __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* _
             for (int p = 1; p < NS; ++p) sum += part[(p * SB + c) * RG + g];
             partial[((long long)tk.blk * A.nrhs + rg + g) * SB + c] = sum;
         }
+        const int slot0 = tk.c0, nq = tk.c1;
+        if (nq == 0) {   // a wide front: k_bwd_inv_reduce adds the chunks
+            __syncthreads();
+            continue;
+        }
+        __threadfence();
         __syncthreads();
+        if (tid == 0) {
+            unsigned* n = cnt + (long long)slot0 * A.nrhs + rg;   // one counter per group of right-hand sides
+            last = atomicAdd(n, 1u) == (unsigned)(nq - 1);
+            if (last) *n = 0u;   // every chunk has counted in: ready for the next launch
+            __threadfence();
+        }
+        __syncthreads();
+        if (!last) continue;
+        const Cv* slot = partial + ((long long)slot0 * A.nrhs + rg) * SB;
+        const int na = (ng * SB + 255) / 256;   // sums of a thread; about 16 loads in flight
+        if (na <= 1) add_chunks<Cv, SB, 1, 16>(slot, nq, A, d, kb * SB, ng, fo + (long long)rg * A.fv_stride, fv, yv, diag);
+        else if (na <= 3) add_chunks<Cv, SB, 3, 6>(slot, nq, A, d, kb * SB, ng, fo + (long long)rg * A.fv_stride, fv, yv, diag);
+        else add_chunks<Cv, SB, W::FQ, 2>(slot, nq, A, d, kb * SB, ng, fo + (long long)rg * A.fv_stride, fv, yv, diag);
     }
 }
 
-// Backward: g of column block kb of an inverse front -= its nq partial sums, added in chunk
+// Backward, wide fronts: g of column block kb = y / D - its nq partial sums, subtracted in chunk
 // order (task {s, kb, nb, slot0, nq, -, -}: the block's chunks have slots slot0 .. slot0+nq-1),
 // one CTA per block and right-hand side (blockIdx.y), one thread per column.
 template <class Cv, int SB>
 __global__ void __launch_bounds__(SB) k_bwd_inv_reduce(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
-                                                       Cv* __restrict__ fv, const Cv* __restrict__ partial) {
+                                                       Cv* __restrict__ fv, const Cv* __restrict__ yv,
+                                                       const double* __restrict__ diag,
+                                                       const Cv* __restrict__ partial) {
     const SolveBlockTask tk = tasks[blockIdx.x];
     const SnDev d = A.sn[tk.s];
     const int kb = tk.k0, slot0 = tk.r0, nq = tk.r1, c = threadIdx.x;
     if (kb * SB + c >= d.w) return;
     for (int r = blockIdx.y; r < A.nrhs; r += gridDim.y) {
-        Cv* gp = fv + A.fvec_off[tk.s] + (long long)r * A.fv_stride + kb * SB + c;
-        Cv v = *gp;
+        const long long at = A.fvec_off[tk.s] + (long long)r * A.fv_stride + kb * SB + c;
+        Cv v = (Cv)((double)yv[at] / diag[d.first_col + kb * SB + c]);
         const Cv* pp = partial + ((long long)slot0 * A.nrhs + r) * SB + c;
         for (int q0 = 0; q0 < nq; q0 += 8) {   // eight loads in flight, subtracted in chunk order
             Cv p8[8];
@@ -645,16 +723,17 @@ __global__ void __launch_bounds__(SB) k_bwd_inv_reduce(const SolveBlockTask* __r
             for (int k = 0; k < 8; ++k)
                 if (q0 + k < nq) v -= p8[k];
         }
-        *gp = v;
+        fv[at] = v;
     }
 }
 
-// Backward x_j = sum_{i >= j} Linv(i, j)^T g_i (g_i already reduced by k_bwd_inv_cols),
-// right-hand sides [RG blockIdx.y, +RG); writes x_j to the work vector.
+// Backward x_j = sum_{i >= j} Linv(i, j)^T g_i (g_i left by k_bwd_inv_cols; y_i / D where the front has no trailing
+// rows), right-hand sides [RG blockIdx.y, +RG); writes x_j to the work vector.
 template <class T, class Cv, int SB, int RG>
 __global__ void __launch_bounds__(256, 1) k_bwd_inv_diag(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
                                                          const Cv* __restrict__ linv, const Cv* __restrict__ linv_off,
-                                                         const Cv* __restrict__ fv, Cv* __restrict__ work,
+                                                         const Cv* __restrict__ fv, const Cv* __restrict__ yv,
+                                                         const double* __restrict__ diag, Cv* __restrict__ work,
                                                          Cv* __restrict__ pbuf, unsigned* __restrict__ cnt,
                                                          int* status) {
     using R = LevelRhs<Cv, SB, RG>;
@@ -692,7 +771,9 @@ __global__ void __launch_bounds__(256, 1) k_bwd_inv_diag(const SolveBlockTask* _
     auto fetch = [&](int i) {
         pf.fetch([&](int c, int g) {
             const int col = i * SB + c;
-            return (g < ng && col < d.w) ? fv[fo + (long long)(rg + g) * A.fv_stride + col] : Cv(0);
+            if (g >= ng || col >= d.w) return Cv(0);
+            const long long at = fo + (long long)(rg + g) * A.fv_stride + col;
+            return d.m > d.w ? fv[at] : (Cv)((double)yv[at] / diag[d.first_col + col]);
         });
     };
     fetch(i0);

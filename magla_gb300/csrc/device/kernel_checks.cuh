@@ -339,15 +339,21 @@ int uchol_check_plan(const uchol_symbolic_desc* d, const uchol_options* opts, in
                     }
                     if (next != P.sn[kv.first.first].m) fail("backward chunks do not reach the front's end");
                 }
-                if (li + 1 >= P.bwd_launches.size() || P.bwd_launches[li + 1].kind != SolveLaunch::BwdInvReduce)
-                    fail("backward chunks without their reduction");
-                const SolveLaunch& R = P.bwd_launches[li + 1];
-                for (int q = R.begin; q < R.begin + R.count; ++q) {
-                    const SolveBlockTask& t = P.solve_tasks[q];
-                    auto it = cols.find({t.s, t.k0});
-                    if (it == cols.end() || t.r1 != (int)it->second.size() || t.r0 != it->second[0]->blk)
-                        fail("a reduction does not match its chunks");
+                std::set<std::pair<int, int>> reduced;
+                if (li + 1 < P.bwd_launches.size() && P.bwd_launches[li + 1].kind == SolveLaunch::BwdInvReduce) {
+                    const SolveLaunch& R = P.bwd_launches[li + 1];
+                    for (int q = R.begin; q < R.begin + R.count; ++q) {
+                        const SolveBlockTask& t = P.solve_tasks[q];
+                        auto it = cols.find({t.s, t.k0});
+                        if (it == cols.end() || t.r1 != (int)it->second.size() || t.r0 != it->second[0]->blk)
+                            fail("a reduction does not match its chunks");
+                        if (!reduced.insert(it->first).second) fail("a block is reduced twice");
+                    }
                 }
+                for (auto& kv : cols)
+                    for (const SolveBlockTask* t : kv.second)
+                        if (t->c0 != kv.second[0]->blk || t->c1 != (reduced.count(kv.first) ? 0 : (int)kv.second.size()))
+                            fail("a backward chunk does not name its block's chunks");
             }
         }
         if (counts) {

@@ -542,6 +542,26 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         fo += round_up(P.sn[s].m, 8);
     }
     P.fvec_elems = std::max<long long>(fo, 8);
+    if (P.fvec_elems > (long long)UINT32_MAX) fail("the front vectors exceed 32-bit positions");
+    // the children's entries of every front-vector position, child by child
+    P.gather_ptr.assign(P.fvec_elems + 1, 0);
+    for (int s = 0; s < count; ++s)
+        for (int c = child_ptr[s]; c < child_ptr[s + 1]; ++c) {
+            const SnDev& cd = P.sn[children[c]];
+            for (int a = 0; a < cd.m - cd.w; ++a) ++P.gather_ptr[P.fvec_off[s] + P.rel[cd.rel_off + a] + 1];
+        }
+    for (long long q = 0; q < P.fvec_elems; ++q) P.gather_ptr[q + 1] += P.gather_ptr[q];
+    P.gather_src.assign(P.gather_ptr[P.fvec_elems], 0);
+    {
+        std::vector<unsigned> fill(P.gather_ptr.begin(), P.gather_ptr.end() - 1);
+        for (int s = 0; s < count; ++s)
+            for (int c = child_ptr[s]; c < child_ptr[s + 1]; ++c) {
+                const int ch = children[c];
+                const SnDev& cd = P.sn[ch];
+                for (int a = 0; a < cd.m - cd.w; ++a)
+                    P.gather_src[fill[P.fvec_off[s] + P.rel[cd.rel_off + a]]++] = (unsigned)(P.fvec_off[ch] + cd.w + a);
+            }
+    }
     // inverse fronts: SB < w <= inv_cols; their off-diagonal inverse blocks, by diagonal i - j
     std::vector<int> inv_ob(count, -1);
     {
@@ -670,9 +690,16 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
     std::vector<int> multi, inv;
     for (int L = 0; L < P.levels; ++L) {
         const auto& fronts = at_level[L];
-        auto g = gather_tasks(fronts);
-        P.fwd_launches.push_back({SolveLaunch::FwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+        // the front vectors of the level kernels' fronts and of large inverse fronts are gathered first; the others' as
+        // they are read
         SolveLaunch solo = split(fronts, multi, inv);
+        std::vector<int> gathered = multi;
+        for (int s : fronts)
+            if (inv_ob[s] >= 0 && P.sn[s].m > kGatherRows) gathered.push_back(s);
+        if (!gathered.empty()) {
+            auto g = gather_tasks(gathered);
+            P.fwd_launches.push_back({SolveLaunch::FwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+        }
         if (solo.count > 0) P.fwd_launches.push_back(solo);
         // trailing rows of the single-block fronts, in chunks from w rounded down to 4
         int tb = (int)P.solve_tasks.size();
@@ -717,8 +744,14 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
     }
     for (int L = P.levels - 1; L >= 0; --L) {
         const auto& fronts = at_level[L];
-        auto g = gather_tasks(fronts);
-        P.bwd_launches.push_back({SolveLaunch::BwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+        // the smaller inverse fronts' kernels read the ancestors' values themselves
+        std::vector<int> gathered;
+        for (int s : fronts)
+            if (inv_ob[s] < 0 || P.sn[s].m > kGatherRows) gathered.push_back(s);
+        if (!gathered.empty()) {
+            auto g = gather_tasks(gathered);
+            P.bwd_launches.push_back({SolveLaunch::BwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+        }
         // column dots against the trailing rows, 8 columns per task; columns longer than
         // kColRowsPlan rows are split into row chunks (flags = 1, blk = partial slot) whose
         // partial sums a reduction task (k0, kn; r0 = first slot, r1 = slots) adds in order
@@ -756,8 +789,8 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         if (solo.count > 0) P.bwd_launches.push_back(solo);
         if (!multi.empty()) P.bwd_launches.push_back(level_launch(SolveLaunch::BwdLevel, multi, false));
         if (!inv.empty()) {
-            // partial sums per (column block, chunk of trailing rows), their sums per column block
-            // in chunk order, then x_1 per block column.  With the SM count known, the level's
+            // partial sums per (column block, chunk of trailing rows), added per column block in chunk order (by
+            // the last chunk done, or a launch of large fronts), then x_1 per block column.  With the SM count known, the level's
             // trailing rows are cut into as many chunks as make at most two tasks per SM (one
             // round of the two CTAs an SM holds); otherwise chunks of kInvColRowsPlan rows.
             int b = (int)P.solve_tasks.size(), slots = 0, dslots = 0;
@@ -768,6 +801,7 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 const SnDev& d = P.sn[s];
                 const int nb = (d.w + SB - 1) / SB;
                 const int t = d.m - d.w;
+                const bool wide = d.m > kGatherRows;
                 int nq = (t + kInvColRowsPlan - 1) / kInvColRowsPlan, height = kInvColRowsPlan;
                 if (cfg.sms > 0 && t > 0) {
                     nq = std::max(1, std::min((t + SB / 2 - 1) / (SB / 2), 2 * cfg.sms / std::max(1, level_blocks)));
@@ -777,9 +811,12 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 for (int kb = 0; kb < nb; ++kb)
                     for (int q = 0; q < nq; ++q) {
                         const int r0 = d.w + q * height;
-                        P.solve_tasks.push_back({s, kb, nb, r0, std::min(d.m, r0 + height), 0, slots + kb * nq + q});
+                        SolveBlockTask ct{s, kb, nb, r0, std::min(d.m, r0 + height), 0, slots + kb * nq + q};
+                        ct.c0 = slots + kb * nq;
+                        ct.c1 = wide ? 0 : nq;
+                        P.solve_tasks.push_back(ct);
                     }
-                if (nq > 0)
+                if (nq > 0 && wide)
                     for (int kb = 0; kb < nb; ++kb) reduce_tasks.push_back({s, kb, nb, slots + kb * nq, nq, 0, 0});
                 for (int j = 0; j < nb; ++j) {
                     const int nc = (nb - j + kInvDiagChunk - 1) / kInvDiagChunk;   // blocks j .. nb-1

@@ -106,15 +106,26 @@ struct SolveLaunch {
 //                        T(i, j) = sum_{k0 <= k < k1} L(i, k) X(k, j), T's block at index t of the scratch arena
 //                        (T(k, j) at t - (i - k) z), then X(i, j) = -sum_{k0 <= k < k1} X(i, k) T(k, j);
 //   FwdInvDiag           {s, i, nb, ob_s, slot0, nc, blk, j0, j1}: the part j0 <= j <= j1 of
-//                        y_i = sum_{j <= i} Linv(i, j) f_j; block row i is split in nc chunks of
-//                        kInvDiagChunk blocks (partial slots slot0 .. slot0+nc-1; nc = 1: no split);
-//   FwdInvTail           {s, -, nb, r0, r1, -, -}: f[r0, r1) -= L[r0:r1, 0:w] y;
-//   BwdInvCols           {s, kb, nb, r0, r1, -, slot}: partial sums of L[r0:r1, block kb]^T g
-//                        into partial slot `slot` (a block's nq chunks have consecutive slots);
-//   BwdInvReduce         {s, kb, nb, slot0, nq, -, -}: g of block kb -= its nq partial sums;
+//                        y_i = sum_{j <= i} Linv(i, j) f_j (f gathered from the children as it is read); block row i
+//                        is split in nc chunks of kInvDiagChunk blocks (partial slots slot0 .. slot0+nc-1; nc = 1: no
+//                        split);
+//   FwdInvTail           {s, -, nb, r0, r1, -, -}: f[r0, r1) = the children's entries - L[r0:r1, 0:w] y;
+//   BwdInvCols           {s, kb, nb, r0, r1, -, slot, slot0, nq}: partial sums of L[r0:r1, block kb]^T g
+//                        into partial slot `slot` (the block's nq chunks have slots slot0 .. slot0+nq-1); the last of
+//                        them to be done writes g = y / D - their sum of the block's columns, unless the front has
+//                        more than kGatherRows rows (nq = 0 in the task);
+//   BwdInvReduce         {s, kb, nb, slot0, nq, -, -}: that sum for these fronts;
 //   BwdInvDiag           {s, j, nb, ob_s, slot0, nc, blk, i0, i1}: the part i0 <= i <= i1 of
 //                        x_j = sum_{i >= j} Linv(i, j)^T g_i, in chunks as FwdInvDiag.
-// blk is the diagonal-inverse index of the front's block 0.
+// blk is the diagonal-inverse index of the front's block 0.  Fronts of more than kGatherRows rows have their vectors
+// gathered by launches of their own, and FwdInvTail subtracts from those.
+// Inverse fronts of up to kGatherRows rows read the children's and the ancestors' entries inside their kernels and the
+// last chunk of a column block adds its partial sums; a level then has four launches, not seven, which bounds chains of
+// small fronts (FP64: 20^3 elasticity 1.02 -> 0.97 ms a solve, 24^3 x 3 grid with 33 right-hand sides 7.53 -> 7.16 ms).  Every
+// block row and column of a front reads the entries again, and in larger fronts that costs more than the launches (60^3
+// elasticity, 16 right-hand sides: 401 ms with them, 423 ms without).
+constexpr int kGatherRows = 4096;
+
 struct InvLaunch {
     int begin, count;   // inversion tasks
     int second;         // 0: T = L X, 1: X = -X T
@@ -129,7 +140,7 @@ struct InvLaunch {
 struct SolveBlockTask {
     int s, k0, kn, r0, r1;
     int flags, blk;
-    int c0 = 0, c1 = 0;   // inverse-front diagonal tasks: the range of inverse blocks summed
+    int c0 = 0, c1 = 0;   // inverse-front diagonal tasks: the range of inverse blocks summed; BwdInvCols: slot0, nq
 };
 
 // Host mirror of the device TcJob (tc_gemm.cuh): one rank-kn update of a front.
@@ -185,7 +196,8 @@ struct Plan {
     double simt_flops = 0.0;                   // algorithmic flops of the SIMT updates
 
     // solve tasks
-    std::vector<int> solve_fronts;             // supernode lists for gather/finish launches
+    std::vector<unsigned> gather_ptr;              // per position of the front vectors: its entries of gather_src
+    std::vector<unsigned> gather_src;          // front-vector positions of the children's update entries, in child order
     std::vector<SolveBlockTask> solve_tasks;
     std::vector<SolveBlockTask> inv_blocks;    // every diagonal block, for the inversion after a factorisation
     std::vector<SolveLaunch> fwd_launches, bwd_launches;

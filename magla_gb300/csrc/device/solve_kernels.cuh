@@ -29,6 +29,8 @@ struct SolveArgs {
     const int* child_ptr;
     const int* children;
     const long long* fvec_off;
+    const unsigned* gather_ptr;  // per front-vector position: its entries of gather_src
+    const unsigned* gather_src;  // positions of the children's update entries, in child order
     long long fv_stride;    // elements between RHS columns in the front-vector workspace
     int n, nrhs, ldw;       // ldw: leading dimension of the work vector
 };
@@ -70,6 +72,15 @@ __device__ __forceinline__ int warp_lower_bound(const int* __restrict__ a, int n
     }
     const int pos = lo + lane;
     return lo + __popc(__ballot_sync(0xffffffffu, pos < hi && a[pos] < key));
+}
+
+// v plus the children's update entries that land on front-vector position `pos`, added in child order: what a gather
+// launch of the front would have left there, without the launch.
+template <class Cv>
+__device__ __forceinline__ Cv add_children(const SolveArgs& A, long long pos, int r, const Cv* fv, Cv v) {
+    const unsigned p1 = A.gather_ptr[pos + 1];
+    for (unsigned p = A.gather_ptr[pos]; p < p1; ++p) v += fv[A.gather_src[p] + (long long)r * A.fv_stride];
+    return v;
 }
 
 template <class Cv>
@@ -1018,7 +1029,7 @@ __global__ void __launch_bounds__(256, 1) k_bwd_level(LevelArgs L, SolveArgs A, 
 // Fronts of one diagonal block (most fronts low in the tree) need no chain:
 // one CTA per front solves its block and, forward, updates its trailing rows.
 
-// Forward: y = L_0^-1 f_0, y / D to the work vector.  Thread (row, part): the row's sum over its part of the columns
+// Forward: y = L_0^-1 f_0 (f_0 gathered as it is read), y / D to the work vector.  Thread (row, part): the row's sum over its part of the columns
 // (the inverse is zero above its diagonal), eight loads in flight; right-hand sides blockIdx.y, + gridDim.y, ...
 template <class T, class Cv, int SB>
 __global__ void __launch_bounds__(256) k_fwd_solo(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
@@ -1036,7 +1047,8 @@ __global__ void __launch_bounds__(256) k_fwd_solo(const SolveBlockTask* __restri
     for (int r = blockIdx.y; r < A.nrhs; r += gridDim.y) {
         const long long base = A.fvec_off[tk.s] + r * A.fv_stride;
         __syncthreads();
-        if (tid < w) f0[tid] = fv[base + tid];
+        if (tid < w)
+            f0[tid] = add_children<Cv>(A, A.fvec_off[tk.s] + tid, r, fv, work[d.first_col + tid + (long long)r * A.ldw]);
         __syncthreads();
         Cv a = Cv(0);
         if (row < w)
@@ -1076,7 +1088,7 @@ __device__ __forceinline__ void load4(const double* p, double* v) {
     v[3] = z.y;
 }
 
-// Forward, trailing rows of single-block fronts (after k_fwd_solo): f[i] -= sum_k L[i, k] y[k]
+// Forward, trailing rows of single-block fronts (after k_fwd_solo): f[i] = the children's entries - sum_k L[i, k] y[k]
 // for rows [r0, r1) of the task's front (r0 a multiple of 4; rows below w are skipped).  RT consecutive rows per
 // thread: four in FP32 (16-byte loads); one in FP64, where a CTA of 1024 rows would hold its SM's FP64 pipe for
 // 16 us.  Eight columns are in flight, and the right-hand sides go in groups of G (blockIdx.y, + gridDim.y, ...):
@@ -1109,6 +1121,13 @@ __global__ void __launch_bounds__(tail_threads<T>()) k_fwd_tail(const SolveBlock
         }
         __syncthreads();
         if (i >= tk.r1) continue;
+        Cv f0[G][RT];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int e = 0; e < RT; ++e)
+                f0[g][e] = g < ng && i + e >= w && i + e < tk.r1
+                               ? add_children<Cv>(A, A.fvec_off[tk.s] + i + e, r0 + g, fv, Cv(0)) : Cv(0);
         Cv a[G][RT];
 #pragma unroll
         for (int g = 0; g < G; ++g)
@@ -1144,7 +1163,7 @@ __global__ void __launch_bounds__(tail_threads<T>()) k_fwd_tail(const SolveBlock
             Cv* f = fv + A.fvec_off[tk.s] + (r0 + g) * A.fv_stride;
 #pragma unroll
             for (int e = 0; e < RT; ++e)
-                if (i + e >= w && i + e < tk.r1) f[i + e] -= a[g][e];
+                if (i + e >= w && i + e < tk.r1) f[i + e] = f0[g][e] - a[g][e];
         }
     }
 }
@@ -1378,12 +1397,14 @@ __global__ void k_dot_partial(const double* __restrict__ u, int ldu, const doubl
     }
     if (threadIdx.x == 0) partial[blockIdx.x + r * gridDim.x] = red[0];
 }
+// Stage 2: a warp per column (one thread adding 256 sums one after another took 15 us).
 __global__ void k_dot_finish(const double* __restrict__ partial, int blocks, int nrhs, double* __restrict__ out) {
-    const int r = threadIdx.x;
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (r >= nrhs) return;
     double s = 0.0;
-    for (int b = 0; b < blocks; ++b) s += partial[b + r * blocks];
-    out[r] = s;
+    for (int b = lane; b < blocks; b += 32) s += partial[b + (long long)r * blocks];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[r] = s;
 }
 
 // x += alpha_r * p (per column), with alpha read from device memory.
