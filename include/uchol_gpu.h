@@ -294,6 +294,10 @@ int uchol_check_solve_wait(uchol_factor f, double wait_ms);
 int uchol_check_schur_update(int bf16, int m, int w, int c0, int cend, int kbeg, int kn, const float* front,
                              const float* w_op, const float* l_op, int ld, int max_ctas, float* front_out,
                              int64_t* tiles_out, int* split_out);
+/* The same by tiles of tile_rows (64, 128 or 256) rows; uchol_check_schur_update takes 256. */
+int uchol_check_schur_update_rows(int tile_rows, int bf16, int m, int w, int c0, int cend, int kbeg, int kn,
+                                  const float* front, const float* w_op, const float* l_op, int ld, int max_ctas,
+                                  float* front_out, int64_t* tiles_out, int* split_out);
 /* uchol_check_diag_panel: the outer block of the mixed path (k_diag_block + k_panel_solve) on
  * the first nb <= 128 columns of an m-row front: front, l_out column-major m x nb (l_out: unit
  * L11 and L21), d_out the nb FP64 pivots, w_stage_out (optional) the staged W = L D rows,

@@ -481,7 +481,7 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
                     if (P.tc_jobs[j].kn != P.tc_jobs[L.begin].kn) nkb = 0;
                 const TcPlanned tp = tc_schedule(L.tiles, nkb, F->sms, split_min_kb(F->opts));
                 const TcSched S{L.tiles, tp.dp_tiles, tp.sk_nkb, F->tc_ws.as<float>(), F->tc_counters.as<int>()};
-                launch_tc_gemm(bf16, D.tc_jobs.as<TcJob>() + L.begin, L.count, S, tp.grid, sn, (float*)panel,
+                launch_tc_gemm(bf16, L.variant, D.tc_jobs.as<TcJob>() + L.begin, L.count, S, tp.grid, sn, (float*)panel,
                                (float*)contrib, F->maps.as<CUtensorMap>(), &stats->status, st);
                 break;
             }
@@ -560,8 +560,9 @@ void prepare_factor_kernels(uchol_factor_s* F) {
         CK(cudaFuncSetAttribute(k_panel_solve<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kPanelSmemBytes));
         CK(cudaFuncSetAttribute(k_panel_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemBytes));
-        CK(cudaFuncSetAttribute(k_tc_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
-        CK(cudaFuncSetAttribute(k_tc_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
+        tc_for_each([](auto k) {
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
+        });
     }
 }
 

@@ -70,7 +70,15 @@ extern "C" {
 int uchol_check_schur_update(int bf16, int m, int w, int c0, int cend, int kbeg, int kn, const float* front,
                              const float* w_op, const float* l_op, int ld, int max_ctas, float* front_out,
                              int64_t* tiles_out, int* split_out) {
+    return uchol_check_schur_update_rows(kTcRows, bf16, m, w, c0, cend, kbeg, kn, front, w_op, l_op, ld, max_ctas,
+                                         front_out, tiles_out, split_out);
+}
+
+int uchol_check_schur_update_rows(int tile_rows, int bf16, int m, int w, int c0, int cend, int kbeg, int kn,
+                                  const float* front, const float* w_op, const float* l_op, int ld, int max_ctas,
+                                  float* front_out, int64_t* tiles_out, int* split_out) {
     return guarded([&] {
+        if (tile_rows != 64 && tile_rows != 128 && tile_rows != 256) throw Error(UCHOL_BAD_ARG, "tiles have 64, 128 or 256 rows");
         if (!front || !w_op || !l_op || !front_out) throw Error(UCHOL_BAD_ARG, "null argument");
         if (m <= 0 || w <= 0 || w > m || c0 < 0 || cend <= c0 || cend > m || (c0 < w && cend > w))
             throw Error(UCHOL_BAD_ARG, "the columns must lie in [0, m), all in the panel or all in the contribution");
@@ -115,7 +123,8 @@ int uchol_check_schur_update(int bf16, int m, int w, int c0, int cend, int kbeg,
             throw Error(UCHOL_CUDA_ERROR, e.what());
         }
         maps.upload(mp, st, "check maps");
-        const long long tiles = tc_job_tiles(c0, cend, m);
+        long long tiles = tile_rows == kTcRows ? tc_job_tiles(c0, cend, m) : 0;
+        for (int c = c0; tile_rows < kTcRows && c < cend; c += kTcCols) tiles += (m - c + tile_rows - 1) / tile_rows;
         std::vector<TcJob> jv{TcJob{0, 0, c0, cend, kbeg, kn, 0}};
         jobs.upload(jv, st, "check job");
         ws.alloc(tc_ws_floats(sms) * sizeof(float), "check workspace");
@@ -123,11 +132,12 @@ int uchol_check_schur_update(int bf16, int m, int w, int c0, int cend, int kbeg,
         status.alloc(sizeof(int), "check workspace");
         CK(cudaMemsetAsync(counters.p, 0, counters.bytes, st));
         CK(cudaMemsetAsync(status.p, 0, sizeof(int), st));
-        CK(cudaFuncSetAttribute(k_tc_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
-        CK(cudaFuncSetAttribute(k_tc_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
+        tc_for_each([](auto k) {
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
+        });
         const TcPlanned tp = tc_schedule(tiles, (kn + kbe - 1) / kbe, sms);
         const TcSched S{tiles, tp.dp_tiles, tp.sk_nkb, ws.as<float>(), counters.as<int>()};
-        launch_tc_gemm(bf16 != 0, jobs.as<TcJob>(), 1, S, tp.grid, F.sn.as<SnDev>(), F.panel.as<float>(),
+        launch_tc_gemm(bf16 != 0, tile_rows, jobs.as<TcJob>(), 1, S, tp.grid, F.sn.as<SnDev>(), F.panel.as<float>(),
                        F.contrib.as<float>(), maps.as<CUtensorMap>(), status.as<int>(), st);
         counted();
         CK(cudaGetLastError());

@@ -77,6 +77,31 @@ double job_flops(const UpdJob& J, const SnDev& d) {
 }
 
 // Tile count of an update job (must match decode_tile).
+// Rows of the tiles of the tensor-core launch of jobs jb and after, whose tiles of kTcRows rows are counted in `tiles`:
+// the fewest that keep the launch within one tile an SM (its tiles are counted anew then).  A small tile's time is its
+// operands' way to the SM and its epilogue, both nearly proportional to its rows: an outer block's own update takes
+// 13 us in tiles of 256 rows and 6 us in tiles of 64 (23 x 17 x 11 elasticity).
+int narrow_tiles(Plan& P, int jb, long long& tiles, int sms) {
+    if (tiles >= sms) return kTcRows;
+    for (int rows = 64; rows < kTcRows; rows *= 2) {
+        long long n = 0;
+        auto count = [&](bool set) {
+            n = 0;
+            for (size_t j = jb; j < P.tc_jobs.size(); ++j) {
+                TcJobHost& J = P.tc_jobs[j];
+                if (set) J.tile_begin = n;
+                for (int c = J.c0; c < J.cend; c += kTcCols) n += (P.sn[J.s].m - c + rows - 1) / rows;
+            }
+        };
+        count(false);
+        if (n > sms) continue;
+        count(true);
+        tiles = n;
+        return rows;
+    }
+    return kTcRows;
+}
+
 long long job_tiles(const UpdJob& J, const SnDev& d, int T) {
     auto region = [&](int base, int lim) -> long long {
         if (lim <= base) return 0;
@@ -405,7 +430,10 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                     tiles += tc_job_tiles(k0, cend, d.m);
                     P.tc_flops += job_flops(U, d);
                 }
-                if ((int)P.tc_jobs.size() > jb) P.launches.push_back({Launch::TcUpdate, jb, (int)P.tc_jobs.size() - jb, tiles});
+                if ((int)P.tc_jobs.size() > jb) {
+                    const int rows = narrow_tiles(P, jb, tiles, cfg.sms > 0 ? cfg.sms : 152);
+                    P.launches.push_back({Launch::TcUpdate, jb, (int)P.tc_jobs.size() - jb, tiles, rows});
+                }
             }
             // mixed path: the whole outer block in two launches (diagonal block, then its rows below)
             if (cfg.tensor_core) {
@@ -525,7 +553,8 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 P.tc_flops += job_flops(U, d);
             }
             if ((int)P.tc_jobs.size() > jb) {
-                Launch Lc{Launch::TcUpdate, jb, (int)P.tc_jobs.size() - jb, tiles};
+                const int rows = narrow_tiles(P, jb, tiles, cfg.sms > 0 ? cfg.sms : 152);
+                Launch Lc{Launch::TcUpdate, jb, (int)P.tc_jobs.size() - jb, tiles, rows};
                 Lc.stream = side_pending ? 2 : 0;   // the contribution columns are complete first
                 P.launches.push_back(Lc);
                 side_pending = false;

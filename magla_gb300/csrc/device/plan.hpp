@@ -78,7 +78,8 @@ struct Launch {
     } kind;
     int begin, count;   // task range
     long long tiles;    // update launches: total tiles (= grid size)
-    int variant = 0;    // SmallFronts: lanes per front (8, 16, 32) or 0 (a CTA each); SimtUpdate: tile edge (16 or 32)
+    int variant = 0;    // SmallFronts: lanes per front (8, 16, 32) or 0 (a CTA each); SimtUpdate: tile edge (16 or 32);
+                        // TcUpdate: rows of a tile (64, 128, 256)
     int stream = 0;     // 0: main stream; 1: side stream, forked from the main stream at this point;
                         // 2: main stream after joining the side stream
 };

@@ -5,8 +5,11 @@
 // 48 KB of operands per 128-byte K block for 4.2 MFLOP (a 128 x 128 tile
 // moves 32 KB for half the flops), which is what bounds the kernel, since the
 // SM's operand bandwidth from L2 and HBM, not the tensor pipe, is the limit.
-// Operands arrive through TMA (128-byte swizzle) into a four-stage ring, the
-// accumulator lives in TMEM (two 256-column buffers), and eight epilogue warps
+// Launches that would leave SMs idle take tiles of 64 or 128 rows instead
+// (narrow_tiles in plan.cpp; N = 64 or 128): a small launch waits for one tile's
+// operands and its epilogue, 13 us at 256 rows and 6 us at 64.
+// Operands arrive through TMA (128-byte swizzle) into a ring of four to eight
+// stages, the accumulator lives in TMEM (two buffers of ROWS columns), and eight epilogue warps
 // subtract it from the FP32 front in place: each warp's 32 columns x 32 rows go
 // through a shared-memory transpose, so that every global access of the warp
 // covers 32 consecutive rows of one column, and C takes the update as an L2
@@ -161,9 +164,10 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 
 // ---------------------------------------------------------------- kernel
 constexpr int kTcABytes = kTcCols * 128;   // one 128-byte K block of the L operand (columns of C)
-constexpr int kTcBBytes = kTcRows * 128;   // one 128-byte K block of the W operand (rows of C)
-constexpr int kTcStages = 4;               // shared-memory ring of (A, B) K blocks: 192 KB
-constexpr int kTcEpiWarps = 8;             // two warps per TMEM lane quadrant, four 32-row chunks each
+constexpr int kTcBoxRows = 64;             // rows of the W operand's TMA box (a tile takes 1, 2 or 4)
+constexpr int kTcRingBytes = 4 * (kTcCols + kTcRows) * 128;   // shared-memory ring of (A, B) K blocks: 192 KB
+constexpr int kTcBarBytes = 256;           // barriers and flags
+constexpr int kTcEpiWarps = 8;             // two warps per TMEM lane quadrant, ROWS / 64 32-row chunks each
 constexpr int kTcThreads = 64 + 32 * kTcEpiWarps;   // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int kTcPartial = kTcCols * kTcRows;       // floats of one partial tile
 constexpr int kTcEpiLd = 33;                        // epilogue transpose buffer: 32 x 33 floats per warp
@@ -172,7 +176,7 @@ constexpr int kTcMaxParts = 4;             // most CTAs sharing one split tile (
 constexpr int kTcSplitCost = 20;           // what a split tile costs beyond its K blocks, in K blocks (about 0.31 us each)
 
 // One rank-kn update C[rows, cols] -= W[rows, kbeg:kbeg+kn] L[cols, kbeg:kbeg+kn]^T of front s,
-// operands in the front's staging region (tensor maps 2*map (W, 256-row box), 2*map+1 (L,
+// operands in the front's staging region (tensor maps 2*map (W, 64-row box), 2*map+1 (L,
 // 128-row box); staging row = front row).  Columns [c0, cend) lie all in the panel or all in
 // the contribution block.
 struct TcJob {
@@ -247,9 +251,21 @@ __device__ __forceinline__ int tc_find_job(const TcJob* __restrict__ jobs, int n
     return lo;
 }
 
-// Tile t of job J (front of m rows): first row i0, first column j0, column limit jend.
+// Tile t of job J (front of m rows): first row i0, first column j0, column limit jend.  Tiles of fewer than
+// kTcRows rows (launches of up to one tile an SM) go column tile by column tile.
+template <int ROWS>
 __device__ __forceinline__ void tc_tile(const TcJob& J, int m, long long t, int& i0, int& j0, int& jend) {
-    tc_decode_tile(J.c0, J.cend, m, t, i0, j0, jend);
+    if constexpr (ROWS == kTcRows) {
+        tc_decode_tile(J.c0, J.cend, m, t, i0, j0, jend);
+    } else {
+        for (j0 = J.c0;; j0 += kTcCols) {
+            const int n = (m - j0 + ROWS - 1) / ROWS;
+            if (t < n || j0 + kTcCols >= J.cend) break;
+            t -= n;
+        }
+        i0 = j0 + (int)t * ROWS;
+        jend = min(j0 + kTcCols, J.cend);
+    }
 }
 
 // Barriers of the epilogue warps only (named barrier 1).  Every epilogue warp walks the
@@ -277,12 +293,15 @@ __device__ __forceinline__ bool tc_epi_any(bool pred) {
     return r != 0;
 }
 
-template <bool BF16>
+template <bool BF16, int ROWS>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_tc_gemm(const TcJob* __restrict__ jobs, int njobs, TcSched S, const SnDev* __restrict__ sn,
               float* __restrict__ panel, float* __restrict__ contrib, const CUtensorMap* __restrict__ maps,
               int* status) {
     constexpr int KBE = BF16 ? 64 : 32;  // K elements per 128-byte block
+    constexpr int kTcBBytes = ROWS * 128;   // one 128-byte K block of the W operand (rows of C)
+    constexpr int kTcStages = kTcRingBytes / (kTcABytes + kTcBBytes);   // 4, 6 or 8
+    static_assert((2 * kTcStages + 4) * 8 + 12 <= kTcBarBytes, "barriers and flags fit before the epilogue buffers");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sA = smem;                              // L rows (C columns)
@@ -294,7 +313,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
-    float* epi_buf = reinterpret_cast<float*>(full + 16);   // after the barriers and flags (128 bytes)
+    float* epi_buf = reinterpret_cast<float*>(full + kTcBarBytes / 8);   // after the barriers and flags
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -311,7 +330,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         mbar_fence_init();
     }
     if (warp == 0) {
-        tmem_alloc(tmem_slot, 2 * kTcRows);
+        tmem_alloc(tmem_slot, 2 * ROWS);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -334,7 +353,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             while (!*abort_flag && it.next(g)) {
                 const TcJob J = jobs[tc_find_job(jobs, njobs, g.t)];
                 int i0, j0, jend;
-                tc_tile(J, sn[J.s].m, g.t - J.tile_begin, i0, j0, jend);
+                tc_tile<ROWS>(J, sn[J.s].m, g.t - J.tile_begin, i0, j0, jend);
                 const CUtensorMap* mw = maps + 2 * J.map;
                 const CUtensorMap* ml = mw + 1;
                 const int kb1 = g.kb1 < 0 ? (J.kn + KBE - 1) / KBE : g.kb1;
@@ -344,7 +363,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     mbar_arrive_expect_tx(&full[stage], kTcABytes + kTcBBytes);
                     const int kx = J.kbeg + kb * KBE;
                     tma_load_2d(sA + stage * kTcABytes, ml, &full[stage], kx, j0);
-                    tma_load_2d(sB + stage * kTcBBytes, mw, &full[stage], kx, i0);
+#pragma unroll
+                    for (int r = 0; r < ROWS; r += kTcBoxRows)
+                        tma_load_2d(sB + stage * kTcBBytes + r * 128, mw, &full[stage], kx, i0 + r);
                     if (++stage == kTcStages) { stage = 0; phase ^= 1; }
                 }
                 if (!ok) break;
@@ -357,14 +378,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             uint32_t phase = 0;
             int acc = 0;
             uint32_t acc_phase = 0;
-            constexpr uint32_t idesc = mma_idesc(BF16 ? 1u : 2u, kTcCols, kTcRows);
+            constexpr uint32_t idesc = mma_idesc(BF16 ? 1u : 2u, kTcCols, ROWS);
             TcSegIter it(S, blockIdx.x, gridDim.x);
             TcSeg g;
             while (!*abort_flag && it.next(g)) {
                 const int kb1 = g.kb1 < 0 ? (jobs[tc_find_job(jobs, njobs, g.t)].kn + KBE - 1) / KBE : g.kb1;
                 if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1)) { fail(); break; }
                 tc_fence_after();
-                const uint32_t dt = tmem + (uint32_t)(acc * kTcRows);
+                const uint32_t dt = tmem + (uint32_t)(acc * ROWS);
                 bool ok = true;
                 for (int kb = g.kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(&full[stage], phase)) { fail(); ok = false; break; }
@@ -385,9 +406,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
     } else {
         // ---------------- epilogue: warp w reads TMEM lanes 32*(w%4) .. +31 (columns of C)
-        // and 32-row chunks [4h, 4h + 4), h = (w - 2) / 4
+        // and 32-row chunks [CH h, CH h + CH), h = (w - 2) / 4
         const int q = warp & 3;
-        const int c_first = ((warp - 2) >> 2) * 4;
+        constexpr int CH = ROWS / 64;
+        const int c_first = ((warp - 2) >> 2) * CH;
         int acc = 0;
         uint32_t acc_phase = 0;
         TcSegIter it(S, blockIdx.x, gridDim.x);
@@ -398,12 +420,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const TcJob J = jobs[tc_find_job(jobs, njobs, g.t)];
             const SnDev d = sn[J.s];
             int i0, j0, jend;
-            tc_tile(J, d.m, g.t - J.tile_begin, i0, j0, jend);
+            tc_tile<ROWS>(J, d.m, g.t - J.tile_begin, i0, j0, jend);
             // on an expired wait this thread skips its work but still meets the barriers below
             const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase));   // warp-uniform
             if (!ok) fail();
             tc_fence_after();
-            const uint32_t ta = tmem + (uint32_t)(acc * kTcRows) + ((uint32_t)(q * 32) << 16);
+            const uint32_t ta = tmem + (uint32_t)(acc * ROWS) + ((uint32_t)(q * 32) << 16);
             // C -= v for this warp's 32 columns x the 32 rows of chunk cc (thread = column on entry): through a
             // shared-memory transpose, so that every global access of the warp is 32 consecutive rows of one column.  Each
             // entry of C takes exactly one update per launch, so a reduction in L2 (no load, nothing to wait for) gives the
@@ -424,15 +446,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 }
                 __syncwarp();
             };
-            // partial tiles in the workspace: float4 r4 of (quadrant, chunk, lane) at ((quadrant * 8 + chunk) * 8 + r4) * 32 +
+            // partial tiles in the workspace: float4 r4 of (quadrant, chunk, lane) at ((quadrant * chunks + chunk) * 8 + r4) * 32 +
             // lane, so that a warp's accesses are whole 512-byte segments
             auto part_at = [&](long long slot, int cc) {
-                return reinterpret_cast<float4*>(S.ws + slot * kTcPartial) + (q * 8 + cc) * 256 + lane;
+                return reinterpret_cast<float4*>(S.ws + slot * kTcPartial) + (q * (ROWS / 32) + cc) * 256 + lane;
             };
             if (g.parts == 1) {
                 if (ok) {
 #pragma unroll 1
-                    for (int cc = c_first; cc < c_first + 4; ++cc) {
+                    for (int cc = c_first; cc < c_first + CH; ++cc) {
                         float v[32];
                         tmem_ld32(ta + (uint32_t)(cc * 32), v);
                         update(cc, v);
@@ -442,7 +464,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 // partial tile: to the workspace; the last CTA of the tile adds all of them
                 if (ok) {
 #pragma unroll 1
-                    for (int cc = c_first; cc < c_first + 4; ++cc) {
+                    for (int cc = c_first; cc < c_first + CH; ++cc) {
                         float v[32];
                         tmem_ld32(ta + (uint32_t)(cc * 32), v);
                         float4* mine = part_at(g.slot, cc);
@@ -469,7 +491,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     __threadfence();
                     const long long c_lo = it.first_cta(tt), c_hi = it.last_cta(tt);
 #pragma unroll 1
-                    for (int cc = c_first; cc < c_first + 4; ++cc) {
+                    for (int cc = c_first; cc < c_first + CH; ++cc) {
                         float v[32];
 #pragma unroll
                         for (int r = 0; r < 32; ++r) v[r] = 0.f;
@@ -521,7 +543,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
     }
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, 2 * kTcRows);
+    if (warp == 0) tmem_dealloc(tmem, 2 * ROWS);
 }
 
 // ---------------------------------------------------------------- host side
@@ -555,16 +577,14 @@ inline CUtensorMap make_region_map(bool bf16, void* base, long long rows, int ld
     return m;
 }
 
-// The tensor-map pair of one front's staging regions: W rows (256-row box), L rows (128-row box).
+// The tensor-map pair of one front's staging regions: W rows (64-row box), L rows (128-row box).
 inline void make_stage_maps(bool bf16, void* w_base, void* l_base, long long rows, int ld, CUtensorMap* out) {
-    out[0] = make_region_map(bf16, w_base, rows, ld, kTcRows);
+    out[0] = make_region_map(bf16, w_base, rows, ld, kTcBoxRows);
     out[1] = make_region_map(bf16, l_base, rows, ld, kTcCols);
 }
 
 inline size_t tc_smem_bytes() {
-    static_assert((2 * kTcStages + 4) * 8 + 12 <= 128, "barriers and flags fit before the epilogue buffers");
-    return 1024 + (size_t)kTcStages * (kTcABytes + kTcBBytes) + 128 +
-           (size_t)kTcEpiWarps * 32 * kTcEpiLd * sizeof(float);
+    return 1024 + (size_t)kTcRingBytes + kTcBarBytes + (size_t)kTcEpiWarps * 32 * kTcEpiLd * sizeof(float);
 }
 
 // Workspace of the K-split tiles: two partial tiles per CTA, one counter per split tile.
@@ -600,14 +620,23 @@ inline TcPlanned tc_schedule(long long tiles, int nkb, int sms, int min_kb = kTc
     return p;
 }
 
-inline void launch_tc_gemm(bool bf16, const TcJob* jobs, int njobs, const TcSched& S, unsigned grid, const SnDev* sn,
-                           float* panel, float* contrib, const CUtensorMap* maps, int* status, cudaStream_t st) {
-    const size_t smem = tc_smem_bytes();
-    if (bf16) {
-        k_tc_gemm<true><<<grid, kTcThreads, smem, st>>>(jobs, njobs, S, sn, panel, contrib, maps, status);
-    } else {
-        k_tc_gemm<false><<<grid, kTcThreads, smem, st>>>(jobs, njobs, S, sn, panel, contrib, maps, status);
-    }
+template <class F>
+inline void tc_for_each(F f) {   // f(kernel) for every instantiation
+    f(k_tc_gemm<false, 256>);
+    f(k_tc_gemm<false, 128>);
+    f(k_tc_gemm<false, 64>);
+    f(k_tc_gemm<true, 256>);
+    f(k_tc_gemm<true, 128>);
+    f(k_tc_gemm<true, 64>);
+}
+
+inline void launch_tc_gemm(bool bf16, int rows, const TcJob* jobs, int njobs, const TcSched& S, unsigned grid,
+                           const SnDev* sn, float* panel, float* contrib, const CUtensorMap* maps, int* status,
+                           cudaStream_t st) {
+    auto k = rows == 64 ? (bf16 ? k_tc_gemm<true, 64> : k_tc_gemm<false, 64>)
+             : rows == 128 ? (bf16 ? k_tc_gemm<true, 128> : k_tc_gemm<false, 128>)
+                           : (bf16 ? k_tc_gemm<true, 256> : k_tc_gemm<false, 256>);
+    k<<<grid, kTcThreads, tc_smem_bytes(), st>>>(jobs, njobs, S, sn, panel, contrib, maps, status);
 }
 
 }  // namespace uchol_dev
