@@ -306,6 +306,10 @@ int uchol_check_schur_update_rows(int tile_rows, int bf16, int m, int w, int c0,
 int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, double regularization,
                            int allow_regularization, float* l_out, double* d_out, float* w_stage_out,
                            int* counts_out);
+/* The same with the rows below by tiles of tile_rows (64 or 128); uchol_check_diag_panel takes 128. */
+int uchol_check_diag_panel_rows(int tile_rows, int m, int nb, const float* front, double threshold, double regularization,
+                           int allow_regularization, float* l_out, double* d_out, float* w_stage_out,
+                           int* counts_out);
 
 /* ---- Device-resident matrix values ------------------------------------
  * A uchol_dmatrix holds a SymmetricCSRMatrix on the device: its upper-triangle

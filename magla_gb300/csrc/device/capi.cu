@@ -447,13 +447,13 @@ void run_factor_launches(uchol_factor_s* F, cudaStream_t st) {
                         k_diag_block<<<L.count, kDiagThreads, kDiagSmemBytes, st>>>(D.pivot_tasks.as<PanelTask>() + L.begin, sn,
                                                                            panel, diag, F->minv.as<float>(), F->linv.as<float>(), ctl, stats);
                     else if (F->precision == UCHOL_PRECISION_BF16)
-                        k_panel_solve<__nv_bfloat16><<<L.count, 256, kPanelSmemBytes, st>>>(
-                            D.panel_tasks.as<PanelTask>() + L.begin, sn, panel, F->minv.as<float>(), F->linv.as<float>(),
-                            F->stage_a.as<__nv_bfloat16>(), F->stage_b.as<__nv_bfloat16>(), D.stage.as<StageInfo>());
+                        launch_panel_solve(L.variant, D.panel_tasks.as<PanelTask>() + L.begin, L.count, sn, panel,
+                                           F->minv.as<float>(), F->linv.as<float>(), F->stage_a.as<__nv_bfloat16>(),
+                                           F->stage_b.as<__nv_bfloat16>(), D.stage.as<StageInfo>(), st);
                     else
-                        k_panel_solve<float><<<L.count, 256, kPanelSmemBytes, st>>>(
-                            D.panel_tasks.as<PanelTask>() + L.begin, sn, panel, F->minv.as<float>(), F->linv.as<float>(),
-                            F->stage_a.as<float>(), F->stage_b.as<float>(), D.stage.as<StageInfo>());
+                        launch_panel_solve(L.variant, D.panel_tasks.as<PanelTask>() + L.begin, L.count, sn, panel,
+                                           F->minv.as<float>(), F->linv.as<float>(), F->stage_a.as<float>(),
+                                           F->stage_b.as<float>(), D.stage.as<StageInfo>(), st);
                 } else {
                     throw Error(UCHOL_INTERNAL, "mixed-precision panel launch in an FP64 plan");
                 }
@@ -557,9 +557,9 @@ void prepare_factor_kernels(uchol_factor_s* F) {
         CK(cudaFuncSetAttribute(k_small_fronts<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(small, 1)));
         prepare_inversion<float, 128>();
         CK(cudaFuncSetAttribute(k_diag_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmemBytes));
-        CK(cudaFuncSetAttribute(k_panel_solve<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kPanelSmemBytes));
-        CK(cudaFuncSetAttribute(k_panel_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemBytes));
+        panel_for_each([](auto k, size_t smem) {
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        });
         tc_for_each([](auto k) {
             CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
         });

@@ -153,7 +153,14 @@ int uchol_check_schur_update_rows(int tile_rows, int bf16, int m, int w, int c0,
 int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, double regularization,
                            int allow_regularization, float* l_out, double* d_out, float* w_stage_out,
                            int* counts_out) {
+    return uchol_check_diag_panel_rows(kSolveRows, m, nb, front, threshold, regularization, allow_regularization, l_out, d_out, w_stage_out, counts_out);
+}
+
+int uchol_check_diag_panel_rows(int tile_rows, int m, int nb, const float* front, double threshold, double regularization,
+                           int allow_regularization, float* l_out, double* d_out, float* w_stage_out,
+                           int* counts_out) {
     return guarded([&] {
+        if (tile_rows != 64 && tile_rows != 128) throw Error(UCHOL_BAD_ARG, "tiles have 64 or 128 rows");
         if (!front || !l_out || !d_out) throw Error(UCHOL_BAD_ARG, "null argument");
         if (nb <= 0 || nb > kDiagMax || m < nb) throw Error(UCHOL_BAD_ARG, "need 0 < nb <= 128 and m >= nb");
         cudaStream_t st = nullptr;
@@ -182,8 +189,8 @@ int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, 
         std::vector<PanelTask> pt{PanelTask{0, 0, nb, nb, 0, -1, 0, 0}};
         ptask.upload(pt, st, "check");
         std::vector<PanelTask> tt;
-        for (int r = nb; r < m; r += kSolveRows)
-            tt.push_back(PanelTask{0, 0, nb, r, std::min(kSolveRows, m - r), 1, 0, 0});
+        for (int r = nb; r < m; r += tile_rows)
+            tt.push_back(PanelTask{0, 0, nb, r, std::min(tile_rows, m - r), 1, 0, 0});
         if (!tt.empty()) ttask.upload(tt, st, "check");
         std::vector<FactorCtl> cv{FactorCtl{threshold, regularization, allow_regularization}};
         ctl.upload(cv, st, "check");
@@ -193,15 +200,16 @@ int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, 
         std::vector<PivotStats> pv{ps0};
         stats.upload(pv, st, "check");
         CK(cudaFuncSetAttribute(k_diag_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmemBytes));
-        CK(cudaFuncSetAttribute(k_panel_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemBytes));
+        panel_for_each([](auto k, size_t smem) {
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        });
         k_diag_block<<<1, kDiagThreads, kDiagSmemBytes, st>>>(ptask.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<float>(),
                                                       diag.as<double>(), minv.as<float>(), nullptr, ctl.as<FactorCtl>(),
                                                       stats.as<PivotStats>());
         counted();
         if (!tt.empty()) {
-            k_panel_solve<float><<<(unsigned)tt.size(), 256, kPanelSmemBytes, st>>>(
-                ttask.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<float>(), minv.as<float>(), nullptr, sa.as<float>(),
-                sb.as<float>(), info.as<StageInfo>());
+            launch_panel_solve(tile_rows, ttask.as<PanelTask>(), (int)tt.size(), F.sn.as<SnDev>(), F.panel.as<float>(),
+                               minv.as<float>(), nullptr, sa.as<float>(), sb.as<float>(), info.as<StageInfo>(), st);
             counted();
         }
         CK(cudaGetLastError());

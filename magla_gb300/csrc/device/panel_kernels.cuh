@@ -8,7 +8,7 @@
 //                  by a small product with that inverse, a rank-32 trailing
 //                  update), then X = L11^{-1}.  Writes L11
 //                  and D to the factor, X^T, D and D^{-1} to a workspace slot.
-//   k_panel_solve  128 rows per CTA: W21 = A21 X^T as an FP32 register-tiled
+//   k_panel_solve  128 or 64 rows per CTA: W21 = A21 X^T as an FP32 register-tiled
 //                  GEMM, L21 = W21 D^{-1}; L21 goes to the factor and, K-major,
 //                  W21 and L21 go to the staging operands of the tensor-core
 //                  updates.
@@ -868,10 +868,18 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Shared memory of k_panel_solve: two stages of (A21 chunk, X^T chunk), 32 K columns each.
-constexpr int kPanelKc = 32, kPanelLds = kSolveRows + 4;
-constexpr size_t kPanelSmemBytes = sizeof(float) * 2 * 2 * kPanelKc * kPanelLds;
-static_assert(4 * kPanelKc >= kDiagMax, "the stages hold the tile of L21 on its way to the factor");
+// Shared memory of k_panel_solve: stages of (A21 chunk, X^T chunk), 32 K columns each; two for tiles of 128 rows, all four
+// for tiles of 64.
+constexpr int kPanelKc = 32;
+template <int ROWS>
+constexpr int kPanelStages = ROWS == 64 ? 4 : 2;
+template <int ROWS>
+constexpr int kPanelStageFloats = kPanelKc * (ROWS + 4 + kDiagMax + 4);
+template <int ROWS>
+constexpr size_t panel_smem_bytes() { return sizeof(float) * kPanelStages<ROWS> * kPanelStageFloats<ROWS>; }
+static_assert(kPanelStages<128> * kPanelStageFloats<128> >= kDiagMax * 132 &&
+              kPanelStages<64> * kPanelStageFloats<64> >= kDiagMax * 68,
+              "the stages hold the tile of L21 on its way to the factor");
 
 __device__ __forceinline__ void store_op4(__nv_bfloat16* p, float a, float b, float c, float e) {
     __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, e);
@@ -896,21 +904,24 @@ __device__ __forceinline__ void store_op1(__nv_bfloat16* p, float a) { *p = __fl
 __device__ __forceinline__ void store_op1(float* p, float a) { *p = a; }
 
 // W21 = A21 X^T and L21 = W21 D^{-1} for rows [row0, row0 + rows) of the
-// front, 256 threads: thread (ty, tx) owns rows {4ty..4ty+3, 64+4ty..} and
-// columns {4tx..4tx+3, 64+4tx..} of the 128 x 128 tile (conflict-free 128-bit
+// front, 2 ROWS threads: thread (ty, tx) owns rows {4ty..4ty+3, ROWS/2+4ty..} and
+// columns {4tx..4tx+3, 64+4tx..} of the ROWS x 128 tile (conflict-free 128-bit
 // shared loads; two rows per FP32 instruction).  X^T is upper triangular, so
 // columns below 64 take no updates from K >= 64.  L21 goes to the factor through
 // shared memory, so that a column's rows are written together.  The SM's FP32 pipe
 // (6 us a tile) and the launch bound it: 11,000 rows, 25.9 us with 4-byte
 // copies and stores of 16 scattered bytes a thread, 22.5 us now (timed alone).
-template <class Op>
-__global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restrict__ tasks,
+// Launches of fewer rows take tiles of 64, half the pipe's time, with all of
+// their copies in flight at once (panel_rows in plan.cpp).
+template <class Op, int ROWS>
+__global__ void __launch_bounds__(2 * ROWS, 2) k_panel_solve(const PanelTask* __restrict__ tasks,
                                                      const SnDev* __restrict__ sn, float* __restrict__ panel,
                                                      float* __restrict__ minv, const float* __restrict__ linv,
                                                      Op* __restrict__ stage_a, Op* __restrict__ stage_b,
                                                      const StageInfo* __restrict__ stage_info) {
-    constexpr int KC = kPanelKc, LDS = kPanelLds;
-    extern __shared__ __align__(16) float psm[];   // stage s: As = psm + 2 s KC LDS, Ms = As + KC LDS
+    constexpr int KC = kPanelKc, NT = 2 * ROWS, LDS = ROWS + 4, LDM = kDiagMax + 4;
+    constexpr int NS = kPanelStages<ROWS>, SF = kPanelStageFloats<ROWS>;
+    extern __shared__ __align__(16) float psm[];   // stage s: As = psm + s SF, Ms = As + KC LDS
     const PanelTask tk = tasks[blockIdx.x];
     const SnDev d = sn[tk.s];
     const int nb = tk.nb, k0 = tk.j0, row0 = tk.row0, rows = tk.rows;
@@ -922,51 +933,53 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc2[i][0][j] = acc2[i][1][j] = 0ull;
-    // K chunks of KC columns copied asynchronously into two stages: every copy of a chunk in
-    // flight at once, and the next chunk's copies under the current chunk's products
+    // K chunks of KC columns copied asynchronously into NS stages: every copy of a chunk in
+    // flight at once, and the next NS - 1 chunks' copies under the current chunk's products
     const bool aligned = ((row0 | (int)(d.panel_off & 3)) & 3) == 0;   // rows on 16-byte boundaries
     auto issue_chunk = [&](int kc, int st) {
-        float* As = psm + 2 * st * KC * LDS;
+        float* As = psm + st * SF;
         float* Ms = As + KC * LDS;
         if (aligned) {
 #pragma unroll
-            for (int q = 0; q < (KC * kSolveRows) / 1024; ++q) {
-                const int idx = tid + 256 * q, r = (idx & 31) * 4, k = idx >> 5;
+            for (int q = 0; q < (KC * ROWS) / (4 * NT); ++q) {
+                const int idx = tid + NT * q, r = (idx % (ROWS / 4)) * 4, k = idx / (ROWS / 4);
                 const int left = kc + k < nb ? min(4, max(0, rows - r)) : 0;
                 cp_async16z(&As[k * LDS + r], left > 0 ? A + r + (long long)(kc + k) * d.ldp : A, 4 * left);
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < (KC * kSolveRows) / 256; ++q) {
-                const int idx = tid + 256 * q, r = idx & (kSolveRows - 1), k = idx >> 7;
+            for (int q = 0; q < (KC * ROWS) / NT; ++q) {
+                const int idx = tid + NT * q, r = idx % ROWS, k = idx / ROWS;
                 const bool ok = r < rows && kc + k < nb;
                 cp_async4(&As[k * LDS + r], ok ? A + r + (long long)(kc + k) * d.ldp : A, ok);
             }
         }
 #pragma unroll
-        for (int q = 0; q < (KC * kDiagMax) / 1024; ++q) {
-            const int idx = tid + 256 * q, r = (idx & 31) * 4, k = idx >> 5;
-            cp_async16z(&Ms[k * LDS + r], M + (kc + k) * kDiagMax + r, 16);
+        for (int q = 0; q < (KC * kDiagMax) / (4 * NT); ++q) {
+            const int idx = tid + NT * q, r = (idx & 31) * 4, k = idx >> 5;
+            cp_async16z(&Ms[k * LDM + r], M + (kc + k) * kDiagMax + r, 16);
         }
         cp_async_commit();
     };
-    issue_chunk(0, 0);
-    for (int kc = 0, st = 0; kc < nb; kc += KC, st ^= 1) {
-        if (kc + KC < nb) {
-            issue_chunk(kc + KC, st ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
+    const int nch = (nb + KC - 1) / KC;
+    for (int c = 0; c < min(NS - 1, nch); ++c) issue_chunk(c * KC, c);
+    for (int c = 0; c < nch; ++c) {
+        if (c + NS - 1 < nch) issue_chunk((c + NS - 1) * KC, (c + NS - 1) % NS);
+        const int later = min(NS - 1, nch - 1 - c);   // chunks in flight after this one
+        if (later >= 3) cp_async_wait<3>();
+        else if (later == 2) cp_async_wait<2>();
+        else if (later == 1) cp_async_wait<1>();
+        else cp_async_wait<0>();
         __syncthreads();
-        const float* As = psm + 2 * st * KC * LDS;
+        const int kc = c * KC;
+        const float* As = psm + (c % NS) * SF;
         const float* Ms = As + KC * LDS;
         const bool low_cols = kc < 64;   // X^T[k][j] = 0 for j < k: columns 0..63 see K < 64 only
 #pragma unroll 4
         for (int k = 0; k < KC; ++k) {
             const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[k * LDS + 4 * ty]);
-            const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[k * LDS + 64 + 4 * ty]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&Ms[k * LDS + 64 + 4 * tx]);
+            const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[k * LDS + ROWS / 2 + 4 * ty]);
+            const float4 b1 = *reinterpret_cast<const float4*>(&Ms[k * LDM + 64 + 4 * tx]);
             const float bh[4] = {b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -977,7 +990,7 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
                 acc2[1][1][4 + j] = fma2(a1.y, bb, acc2[1][1][4 + j]);
             }
             if (low_cols) {
-                const float4 b0 = *reinterpret_cast<const float4*>(&Ms[k * LDS + 4 * tx]);
+                const float4 b0 = *reinterpret_cast<const float4*>(&Ms[k * LDM + 4 * tx]);
                 const float bl[4] = {b0.x, b0.y, b0.z, b0.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -989,7 +1002,7 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
                 }
             }
         }
-        __syncthreads();   // this stage is refilled two chunks later
+        __syncthreads();   // this stage is refilled
     }
     float acc[8][8];   // [row][column]
 #pragma unroll
@@ -1010,15 +1023,16 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
             const float di = dinv[col];
 #pragma unroll
             for (int ig = 0; ig < 2; ++ig)
-                *reinterpret_cast<float4*>(&psm[(j * 32 + 16 * jg + tx) * LDS + 64 * ig + 4 * ty]) =
+                *reinterpret_cast<float4*>(&psm[(j * 32 + 16 * jg + tx) * LDS + (ROWS / 2) * ig + 4 * ty]) =
                     make_float4(acc[4 * ig + 0][4 * jg + j] * di, acc[4 * ig + 1][4 * jg + j] * di,
                                 acc[4 * ig + 2][4 * jg + j] * di, acc[4 * ig + 3][4 * jg + j] * di);
         }
     __syncthreads();
     {
-        const int warp = tid >> 5, lane = tid & 31;
+        constexpr int LPC = ROWS / 4;   // lanes of a column
+        const int lane = tid % LPC;
 #pragma unroll 4
-        for (int col = warp; col < nb; col += 8) {
+        for (int col = tid / LPC; col < nb; col += NT / LPC) {
             const float* src = &psm[((col & 3) * 32 + (col >> 2)) * LDS];
             float* dst = A + (long long)col * d.ldp;
             if (aligned && 4 * lane + 4 <= rows) {
@@ -1026,7 +1040,7 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
             } else if (aligned) {
                 for (int r = 4 * lane; r < rows; ++r) dst[r] = src[r];
             } else {
-                for (int r = lane; r < rows; r += 32) dst[r] = src[r];
+                for (int r = lane; r < rows; r += LPC) dst[r] = src[r];
             }
         }
     }
@@ -1036,7 +1050,7 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
     for (int ig = 0; ig < 2; ++ig) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int r = 64 * ig + 4 * ty + i;
+            const int r = (ROWS / 2) * ig + 4 * ty + i;
             if (r >= rows) continue;
             const long long so = g.off + (long long)(row0 + r) * g.ld + k0;
 #pragma unroll
@@ -1060,13 +1074,30 @@ __global__ void __launch_bounds__(256, 2) k_panel_solve(const PanelTask* __restr
     }
     if (tk.stage_zero_to > k0 + nb) {
         const int zc = tk.stage_zero_to - (k0 + nb);
-        for (int idx = tid; idx < rows * zc; idx += 256) {
+        for (int idx = tid; idx < rows * zc; idx += NT) {
             const int r = idx / zc, c = idx - r * zc;
             const long long o = g.off + (long long)(row0 + r) * g.ld + k0 + nb + c;
             store_op1(stage_a + o, 0.f);
             store_op1(stage_b + o, 0.f);
         }
     }
+}
+
+template <class F>
+inline void panel_for_each(F f) {   // f(kernel, shared memory) for every instantiation
+    f(k_panel_solve<float, 128>, panel_smem_bytes<128>());
+    f(k_panel_solve<float, 64>, panel_smem_bytes<64>());
+    f(k_panel_solve<__nv_bfloat16, 128>, panel_smem_bytes<128>());
+    f(k_panel_solve<__nv_bfloat16, 64>, panel_smem_bytes<64>());
+}
+
+template <class Op>
+inline void launch_panel_solve(int rows, const PanelTask* tasks, int count, const SnDev* sn, float* panel, float* minv,
+                               const float* linv, Op* stage_a, Op* stage_b, const StageInfo* info, cudaStream_t st) {
+    if (rows == 64)
+        k_panel_solve<Op, 64><<<count, 128, panel_smem_bytes<64>(), st>>>(tasks, sn, panel, minv, linv, stage_a, stage_b, info);
+    else
+        k_panel_solve<Op, 128><<<count, 256, panel_smem_bytes<128>(), st>>>(tasks, sn, panel, minv, linv, stage_a, stage_b, info);
 }
 
 }  // namespace uchol_dev

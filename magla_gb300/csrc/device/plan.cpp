@@ -102,6 +102,17 @@ int narrow_tiles(Plan& P, int jb, long long& tiles, int sms) {
     return kTcRows;
 }
 
+// Rows of the panel-solve tiles below the outer block at k0: 64 while that is at most one tile an SM.  Such a launch takes
+// as long as one tile, and half a tile is 3 us less; with more tiles than SMs the inverse, read once per tile, costs more
+// than that gains (60^3 elasticity 392.1 ms with this rule, 394.4 with two tiles an SM; 20^3 refresh 10.54 and 10.77 ms
+// without tiles of 64).
+int panel_rows(const Plan& P, const std::vector<int>& large, int k0, int NB, int sms) {
+    long long n = 0;
+    for (int s : large)
+        if (P.sn[s].w > k0) n += (P.sn[s].m - std::min(P.sn[s].w, k0 + NB) + 63) / 64;
+    return n <= sms ? 64 : 128;
+}
+
 long long job_tiles(const UpdJob& J, const SnDev& d, int T) {
     auto region = [&](int base, int lim) -> long long {
         if (lim <= base) return 0;
@@ -440,6 +451,7 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 int qb = (int)P.pivot_tasks.size();
                 int pb = (int)P.panel_tasks.size();
                 int slot = 0;
+                const int tile = panel_rows(P, large, k0, NB, cfg.sms > 0 ? cfg.sms : 152);
                 for (int s : large) {
                     const SnDev& d = P.sn[s];
                     if (d.w <= k0) continue;
@@ -447,8 +459,8 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                     const int inv = outer_inverts ? first_blk[s] + k0 / NB : -1;
                     P.pivot_tasks.push_back({s, k0, nbo, k0 + nbo, 0, -1, slot, 0, inv});
                     int zero_to = (k0 + nbo == d.w && P.stage[s].ld > d.w) ? P.stage[s].ld : 0;
-                    for (int r = k0 + nbo; r < d.m; r += kSolveRowsPlan) {
-                        int rows = std::min(kSolveRowsPlan, d.m - r);
+                    for (int r = k0 + nbo; r < d.m; r += tile) {
+                        int rows = std::min(tile, d.m - r);
                         P.panel_tasks.push_back({s, k0, nbo, r, rows, 1, slot, zero_to, inv});
                         P.panel_flops += 2.0 * rows * nbo * nbo;
                     }
@@ -456,7 +468,7 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 }
                 P.diag_slots = std::max(P.diag_slots, slot);
                 if ((int)P.pivot_tasks.size() > qb) P.launches.push_back({Launch::DiagBlock, qb, (int)P.pivot_tasks.size() - qb, 0});
-                if ((int)P.panel_tasks.size() > pb) P.launches.push_back({Launch::PanelSolve, pb, (int)P.panel_tasks.size() - pb, 0});
+                if ((int)P.panel_tasks.size() > pb) P.launches.push_back({Launch::PanelSolve, pb, (int)P.panel_tasks.size() - pb, 0, tile});
                 continue;
             }
             // FP64 path, one pivot block per step.  Plain fronts are right-looking: every step updates the whole

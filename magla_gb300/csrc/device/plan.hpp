@@ -12,7 +12,6 @@
 
 namespace uchol_dev {
 
-constexpr int kSolveRowsPlan = 128;   // rows per panel-solve task (kSolveRows of the kernel)
 constexpr int kTailRowsPlan = 1024;  // trailing rows per forward tail task, mixed path
 constexpr int kTailRowsPlan64 = 128; // and FP64 (its products hold the SM's FP64 pipe: 2 us at 64 columns)
 constexpr int kColRowsPlan = 2048;   // trailing rows per backward column-dot task (longer columns: partial sums)
@@ -79,7 +78,7 @@ struct Launch {
     int begin, count;   // task range
     long long tiles;    // update launches: total tiles (= grid size)
     int variant = 0;    // SmallFronts: lanes per front (8, 16, 32) or 0 (a CTA each); SimtUpdate: tile edge (16 or 32);
-                        // TcUpdate: rows of a tile (64, 128, 256)
+                        // TcUpdate: rows of a tile (64, 128, 256); PanelSolve: the same (64, 128)
     int stream = 0;     // 0: main stream; 1: side stream, forked from the main stream at this point;
                         // 2: main stream after joining the side stream
 };
