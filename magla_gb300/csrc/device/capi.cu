@@ -337,7 +337,7 @@ PlanConfig config_for(const uchol_options& o) {
     return c;
 }
 
-// The next smaller configuration for a memory budget that this one's plan exceeds: default choices that cost memory only
+// The next smaller configuration for a memory budget or a device that does not hold this one: default choices that cost memory only
 // for speed are given up, the wider inverse fronts and the digits of the FP64 tensor-core updates; false: none is left.
 bool relax_for_budget(PlanConfig& c, const uchol_options& o) {
     if (o.inverse_block_width == 0 && c.inv_cols > kDefaultInvCols64) c.inv_cols = kDefaultInvCols64;
@@ -777,34 +777,17 @@ void check_options(const uchol_options* o) {
                                        " front-size buckets");
 }
 
-uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_options* opts) {
-    if (!S) throw Error(UCHOL_BAD_ARG, "symbolic handle is null");
-    if (n != S->n)
-        throw Error(UCHOL_PATTERN_MISMATCH, "Matrix size " + std::to_string(n) +
-                                                " does not match the symbolic factorization built for " +
-                                                std::to_string(S->n) + " equations.");
-    if (nnz != S->nnz)
-        throw Error(UCHOL_PATTERN_MISMATCH,
-                    "The matrix sparse structure has changed since symbolic analysis (previously " +
-                        std::to_string(S->nnz) + " nonzero elements, now " + std::to_string(nnz) +
-                        "). Symbolic factorization can be reused only when the structure is unchanged. Run Analyze again.");
-    check_options(opts);
+// A factor object of one configuration: its plan and every buffer that does not depend on the right-hand sides
+// (UCHOL_OOM when the budget or the device's memory does not hold them; nothing is kept then).
+uchol_factor_s* allocate_factor(uchol_symbolic_s* S, const uchol_options& o, const PlanConfig& cfg) {
     auto F = std::make_unique<uchol_factor_s>();
     F->sym = S;
     S->refs.fetch_add(1);
-    if (opts) F->opts = *opts; else uchol_default_options(&F->opts);
-    F->precision = F->opts.precision;
+    F->opts = o;
+    F->precision = o.precision;
     F->elem = F->precision == UCHOL_PRECISION_FP64 ? 8 : 4;
-    PlanConfig cfg = config_for(F->opts);
-    CK(cudaDeviceGetAttribute(&F->sms, cudaDevAttrMultiProcessorCount, S->device));
-    cfg.sms = F->sms;
-    while (!F->dp) {
-        try {
-            F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
-        } catch (const Error& e) {
-            if (e.code != UCHOL_OOM || !relax_for_budget(cfg, F->opts)) throw;
-        }
-    }
+    F->sms = cfg.sms;
+    F->dp = S->get_plan(cfg, F->precision, o.device_memory_budget);
     const Plan& P = F->dp->plan;
     cudaStream_t st = S->stream;
     F->panel.alloc((size_t)P.factor_elems * F->elem, "factor panels");
@@ -871,6 +854,31 @@ uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_o
     F->ctl.alloc(sizeof(FactorCtl), "statistics");
     prepare_factor_kernels(F.get());
     return F.release();
+}
+
+uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_options* opts) {
+    if (!S) throw Error(UCHOL_BAD_ARG, "symbolic handle is null");
+    if (n != S->n)
+        throw Error(UCHOL_PATTERN_MISMATCH, "Matrix size " + std::to_string(n) +
+                                                " does not match the symbolic factorization built for " +
+                                                std::to_string(S->n) + " equations.");
+    if (nnz != S->nnz)
+        throw Error(UCHOL_PATTERN_MISMATCH,
+                    "The matrix sparse structure has changed since symbolic analysis (previously " +
+                        std::to_string(S->nnz) + " nonzero elements, now " + std::to_string(nnz) +
+                        "). Symbolic factorization can be reused only when the structure is unchanged. Run Analyze again.");
+    check_options(opts);
+    uchol_options o;
+    if (opts) o = *opts; else uchol_default_options(&o);
+    PlanConfig cfg = config_for(o);
+    CK(cudaDeviceGetAttribute(&cfg.sms, cudaDevAttrMultiProcessorCount, S->device));
+    for (;;) {
+        try {
+            return allocate_factor(S, o, cfg);
+        } catch (const Error& e) {
+            if (e.code != UCHOL_OOM || !relax_for_budget(cfg, o)) throw;
+        }
+    }
 }
 
 // ---- solves ----

@@ -104,7 +104,7 @@ int narrow_tiles(Plan& P, int jb, long long& tiles, int sms) {
 
 // Rows of the panel-solve tiles below the outer block at k0: 64 while that is at most one tile an SM.  Such a launch takes
 // as long as one tile, and half a tile is 3 us less; with more tiles than SMs the inverse, read once per tile, costs more
-// than that gains (60^3 elasticity 392.1 ms with this rule, 394.4 with two tiles an SM; 20^3 refresh 10.54 and 10.77 ms
+// than that gains (60 x 60 x 30 elasticity 392.1 ms with this rule, 394.4 with two tiles an SM; 20^3 refresh 10.54 and 10.77 ms
 // without tiles of 64).
 int panel_rows(const Plan& P, const std::vector<int>& large, int k0, int NB, int sms) {
     long long n = 0;

@@ -122,8 +122,8 @@ struct SolveLaunch {
 // Inverse fronts of up to kGatherRows rows read the children's and the ancestors' entries inside their kernels and the
 // last chunk of a column block adds its partial sums; a level then has four launches, not seven, which bounds chains of
 // small fronts (FP64: 20^3 elasticity 1.02 -> 0.97 ms a solve, 24^3 x 3 grid with 33 right-hand sides 7.53 -> 7.16 ms).  Every
-// block row and column of a front reads the entries again, and in larger fronts that costs more than the launches (60^3
-// elasticity, 16 right-hand sides: 401 ms with them, 423 ms without).
+// block row and column of a front reads the entries again, and in larger fronts that costs more than the launches (60 x
+// 60 x 30 elasticity, 16 right-hand sides: 401 ms with them, 423 ms without).
 constexpr int kGatherRows = 4096;
 
 struct InvLaunch {
