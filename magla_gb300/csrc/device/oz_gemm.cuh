@@ -119,6 +119,8 @@ __global__ void __launch_bounds__(256) k_oz_slice(const PanelTask* __restrict__ 
         }
 }
 
+__device__ __forceinline__ int oz_int(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }   // an integer's FP32
+
 // The value V 2^(sh) as a double (V a 64-bit integer, rounded once), zero or infinite past the range of doubles.
 __device__ __forceinline__ double oz_value(long long V, int sh) {
     const long long b = __double_as_longlong((double)V);
@@ -253,19 +255,19 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                 tmem_ld16(ta + 3 * kOzCols + 16 * h, r3);
                 tmem_ld_wait();
 #pragma unroll
-                for (int u = 0; u < 16; ++u)
-                    V[16 * h + u] = ((((long long)__float2int_rn(__uint_as_float(r0[u])) * 256 + __float2int_rn(__uint_as_float(r1[u]))) * 256 +
-                                      __float2int_rn(__uint_as_float(r2[u]))) * 256 + __float2int_rn(__uint_as_float(r3[u])));
+                for (int u = 0; u < 16; ++u) {   // |r_o| <= (o + 1) 2^21: both fit 32 bits
+                    const int t0 = oz_int(r0[u]) * 256 + oz_int(r1[u]), t1 = oz_int(r2[u]) * 256 + oz_int(r3[u]);
+                    V[16 * h + u] = ((long long)t0 << 32) + (long long)t1 * 65536;
+                }
                 tmem_ld16(ta + 4 * kOzCols + 16 * h, r0);
                 tmem_ld16(ta + 5 * kOzCols + 16 * h, r1);
                 tmem_ld16(ta + 6 * kOzCols + 16 * h, r2);
                 tmem_ld16(ta + 7 * kOzCols + 16 * h, r3);
                 tmem_ld_wait();
 #pragma unroll
-                for (int u = 0; u < 16; ++u) {
-                    const long long lo = (((long long)__float2int_rn(__uint_as_float(r0[u])) * 256 + __float2int_rn(__uint_as_float(r1[u]))) * 256 +
-                                          __float2int_rn(__uint_as_float(r2[u]))) * 256 + __float2int_rn(__uint_as_float(r3[u]));
-                    V[16 * h + u] = V[16 * h + u] * 65536 + ((lo + 32768) >> 16);   // the sum / 2^16, below 2^61
+                for (int u = 0; u < 16; ++u) {   // the sum / 2^16, rounded down after half a unit is added; below 2^61
+                    const int low = (oz_int(r2[u]) + ((oz_int(r3[u]) + 32768) >> 8)) >> 8;
+                    V[16 * h + u] += (long long)oz_int(r0[u]) * 256 + (oz_int(r1[u]) + low);
                 }
             }
             tc_fence_before();
