@@ -21,7 +21,8 @@
 // block is carried in FP64 through every elimination step inside the block
 // (d_r -= d_k L_rk^2 with the FP32 L), and the pivot test !(d > tol * scale),
 // the regularisation and D itself are FP64 (the FP32 elimination divides by D
-// rounded to FP32).  That is O(nb^2) FP64 work per block.  The FP64 residual
+// rounded to FP32).  That is O(nb^2) FP64 work per block, done beside the chain of
+// pivots, which runs on sums of two floats while every pivot is clearly decided.  The FP64 residual
 // refinement recovers full accuracy of the solution.
 #pragma once
 
