@@ -1019,7 +1019,7 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
         return la;
     };
     for (const SolveLaunch& L : P.fwd_launches) {
-        if (L.count == 0) continue;
+        if (L.count == 0 || (L.large && nrhs == 1)) continue;
         if (timer) timer->begin((int)L.kind, st);
         if (L.kind == SolveLaunch::FwdGather) {
             k_fwd_gather<Cv><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, work, fv);
@@ -1045,7 +1045,7 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
         if (timer) timer->end(st);
     }
     for (const SolveLaunch& L : P.bwd_launches) {
-        if (L.count == 0) continue;
+        if (L.count == 0 || (L.large && nrhs == 1)) continue;
         if (timer) timer->begin((int)L.kind, st);
         if (L.kind == SolveLaunch::BwdGather) {
             k_bwd_gather<Cv><<<grid(L.count, 1), 256, 0, st>>>(tasks + L.begin, A, work, fv);
@@ -1076,10 +1076,10 @@ void run_solve(uchol_factor_s* F, int nrhs, Cv* work, Cv* fv, Cv* fv2, cudaStrea
     CK(cudaGetLastError());
 }
 
-int solve_launch_count(const Plan& P) {
+int solve_launch_count(const Plan& P, int nrhs) {
     int c = 0;
-    for (const SolveLaunch& L : P.fwd_launches) c += L.count > 0;
-    for (const SolveLaunch& L : P.bwd_launches) c += L.count > 0;
+    for (const SolveLaunch& L : P.fwd_launches) c += L.count > 0 && !(L.large && nrhs == 1);
+    for (const SolveLaunch& L : P.bwd_launches) c += L.count > 0 && !(L.large && nrhs == 1);
     return c + 1;   // + the flag reset
 }
 
@@ -1175,7 +1175,7 @@ void launch_solve_graph(uchol_factor_s* F, int nrhs, Cv* work, cudaStream_t st) 
         cudaGraphDestroy(g);
         CK(e);
         F->solve_graph_nrhs = nrhs;
-        F->solve_graph_nodes = solve_launch_count(F->dp->plan);
+        F->solve_graph_nodes = solve_launch_count(F->dp->plan, nrhs);
     }
     if (phase_timing()) {
         // direct launches with one event pair each (the graph above stays for untimed calls)

@@ -6,11 +6,11 @@
 // backward:
 //   g_1 = D^-1 y_1 - L_21^T g_2        (k_bwd_inv_cols: partial sums per chunk of rows, added in
 //                                       chunk order by the last chunk of a column block or, of
-//                                       fronts of more than kGatherRows rows, by k_bwd_inv_reduce),
+//                                       large fronts, by k_bwd_inv_reduce),
 //   x_1 = Linv_11^T g_1                (k_bwd_inv_diag: one CTA per block column).
 // The algebra is the reference's supernodal substitution
 // (CAESolvers/UCHOL/UtduNumericFactorization.cs:139-207) with the triangular solve of
-// the diagonal block written as a product with its inverse (fronts of up to kGatherRows rows gather f
+// the diagonal block written as a product with its inverse (all but large fronts gather f
 // from the children and g_2 from the ancestors where they are read: two launches a level and direction, which
 // are what a chain of small fronts waits for); the result differs only
 // in rounding.  The inverse is built once per factorisation from the inverses of the
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(256, 1) k_fwd_inv_diag(const SolveBlockTask* _
         pf.fetch([&](int c, int g) {
             const int col = j * SB + c;
             if (g >= ng || col >= d.w) return Cv(0);
-            if (d.m > kGatherRows) return fv[fo + col + (long long)(rg + g) * A.fv_stride];
+            if (RG > 1 && d.m > kGatherRows) return fv[fo + col + (long long)(rg + g) * A.fv_stride];
             return add_children<Cv>(A, fo + col, rg + g, fv, work[d.first_col + col + (long long)(rg + g) * A.ldw]);
         });
     };
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_inv_tail(const SolveBlockTask* _
         for (int q = 0; q < W::FQ; ++q) {
             const int e = tid + 256 * q, g = e / SB, i = ra + e - g * SB;
             f0[q] = !(e < SB * RG && g < ng && i >= r0 && i < r1) ? Cv(0)
-                    : d.m > kGatherRows ? fv[fo + i + (long long)(rg + g) * A.fv_stride]
+                    : RG > 1 && d.m > kGatherRows ? fv[fo + i + (long long)(rg + g) * A.fv_stride]
                                               : add_children<Cv>(A, fo + i, rg + g, fv, Cv(0));
         }
         pf.commit(ybuf(0));
@@ -568,7 +568,7 @@ __device__ __forceinline__ void add_chunks(const Cv* __restrict__ slot, int nq, 
 // split) keeps an RT x GT tile of sums; column group q holds columns q + NG a.  The sums go
 // to partial slot `slot` ((slot nrhs + r) SB + c for right-hand side r, column c); the CTA
 // that completes the block's chunks (a counter, no waiting) adds them in chunk order into g,
-// k_bwd_inv_reduce those of fronts of more than kGatherRows rows.
+// k_bwd_inv_reduce those of large fronts.
 template <class T, class Cv, int SB, int RG>
 __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* __restrict__ tasks, SolveArgs A,
                                                          const CUtensorMap* __restrict__ maps, Cv* __restrict__ fv,
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* _
             pf.fetch([&](int r, int g) {
                 const int gr = tr + r;
                 if (g >= ng || gr < r0 || gr >= r1) return Cv(0);
-                return d.m > kGatherRows ? fv[fo + gr + (long long)(rg + g) * A.fv_stride]
+                return RG > 1 && d.m > kGatherRows ? fv[fo + gr + (long long)(rg + g) * A.fv_stride]
                                                : work[rows[gr] + (long long)(rg + g) * A.ldw];
             });
         };
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* _
             partial[((long long)tk.blk * A.nrhs + rg + g) * SB + c] = sum;
         }
         const int slot0 = tk.c0, nq = tk.c1;
-        if (nq == 0) {   // a wide front: k_bwd_inv_reduce adds the chunks
+        if (RG > 1 && d.m > kGatherRows) {   // k_bwd_inv_reduce adds the chunks
             __syncthreads();
             continue;
         }
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_inv_cols(const SolveBlockTask* _
     }
 }
 
-// Backward, wide fronts: g of column block kb = y / D - its nq partial sums, subtracted in chunk
+// Backward, large fronts: g of column block kb = y / D - its nq partial sums, subtracted in chunk
 // order (task {s, kb, nb, slot0, nq, -, -}: the block's chunks have slots slot0 .. slot0+nq-1),
 // one CTA per block and right-hand side (blockIdx.y), one thread per column.
 template <class Cv, int SB>

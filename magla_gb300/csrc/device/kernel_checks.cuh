@@ -369,8 +369,11 @@ int uchol_check_plan(const uchol_symbolic_desc* d, const uchol_options* opts, in
                     }
                 }
                 for (auto& kv : cols)
+                    if (reduced.count(kv.first) != (P.sn[kv.first.first].m > kGatherRows))
+                        fail("the reductions are not those of the large fronts");
+                for (auto& kv : cols)
                     for (const SolveBlockTask* t : kv.second)
-                        if (t->c0 != kv.second[0]->blk || t->c1 != (reduced.count(kv.first) ? 0 : (int)kv.second.size()))
+                        if (t->c0 != kv.second[0]->blk || t->c1 != (int)kv.second.size())
                             fail("a backward chunk does not name its block's chunks");
             }
         }

@@ -734,12 +734,16 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         // the front vectors of the level kernels' fronts and of large inverse fronts are gathered first; the others' as
         // they are read
         SolveLaunch solo = split(fronts, multi, inv);
-        std::vector<int> gathered = multi;
+        std::vector<int> large;
         for (int s : fronts)
-            if (inv_ob[s] >= 0 && P.sn[s].m > kGatherRows) gathered.push_back(s);
-        if (!gathered.empty()) {
-            auto g = gather_tasks(gathered);
+            if (inv_ob[s] >= 0 && P.sn[s].m > kGatherRows) large.push_back(s);
+        if (!multi.empty()) {
+            auto g = gather_tasks(multi);
             P.fwd_launches.push_back({SolveLaunch::FwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+        }
+        if (!large.empty()) {
+            auto g = gather_tasks(large);
+            P.fwd_launches.push_back({SolveLaunch::FwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1});
         }
         if (solo.count > 0) P.fwd_launches.push_back(solo);
         // trailing rows of the single-block fronts, in chunks from w rounded down to 4
@@ -786,12 +790,18 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
     for (int L = P.levels - 1; L >= 0; --L) {
         const auto& fronts = at_level[L];
         // the smaller inverse fronts' kernels read the ancestors' values themselves
-        std::vector<int> gathered;
-        for (int s : fronts)
-            if (inv_ob[s] < 0 || P.sn[s].m > kGatherRows) gathered.push_back(s);
+        std::vector<int> gathered, large;
+        for (int s : fronts) {
+            if (inv_ob[s] < 0) gathered.push_back(s);
+            else if (P.sn[s].m > kGatherRows) large.push_back(s);
+        }
         if (!gathered.empty()) {
             auto g = gather_tasks(gathered);
             P.bwd_launches.push_back({SolveLaunch::BwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+        }
+        if (!large.empty()) {
+            auto g = gather_tasks(large);
+            P.bwd_launches.push_back({SolveLaunch::BwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1});
         }
         // column dots against the trailing rows, 8 columns per task; columns longer than
         // kColRowsPlan rows are split into row chunks (flags = 1, blk = partial slot) whose
@@ -854,7 +864,7 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                         const int r0 = d.w + q * height;
                         SolveBlockTask ct{s, kb, nb, r0, std::min(d.m, r0 + height), 0, slots + kb * nq + q};
                         ct.c0 = slots + kb * nq;
-                        ct.c1 = wide ? 0 : nq;
+                        ct.c1 = nq;
                         P.solve_tasks.push_back(ct);
                     }
                 if (nq > 0 && wide)
@@ -876,6 +886,7 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
                 b = (int)P.solve_tasks.size();
                 P.solve_tasks.insert(P.solve_tasks.end(), reduce_tasks.begin(), reduce_tasks.end());
                 P.bwd_launches.push_back(simple(SolveLaunch::BwdInvReduce, b));
+                P.bwd_launches.back().large = 1;
             }
             P.inv_partial_slots = std::max(P.inv_partial_slots, slots);
             P.inv_diag_slots = std::max(P.inv_diag_slots, dslots);

@@ -96,6 +96,7 @@ struct SolveLaunch {
     int long_chains;                   // level launches: fronts of three or more diagonal blocks
     int ndiag;                         // level launches: bulk chunks [0, ndiag) are diagonal blocks
     long long diag_work;               // level launches: chunk updates of those
+    int large = 0;                     // gathers and reductions of large inverse fronts: not for one right-hand side
 };
 
 // Inverse fronts (cfg.inv_cols): the off-diagonal blocks (i, j), i > j, of the
@@ -112,18 +113,20 @@ struct SolveLaunch {
 //   FwdInvTail           {s, -, nb, r0, r1, -, -}: f[r0, r1) = the children's entries - L[r0:r1, 0:w] y;
 //   BwdInvCols           {s, kb, nb, r0, r1, -, slot, slot0, nq}: partial sums of L[r0:r1, block kb]^T g
 //                        into partial slot `slot` (the block's nq chunks have slots slot0 .. slot0+nq-1); the last of
-//                        them to be done writes g = y / D - their sum of the block's columns, unless the front has
-//                        more than kGatherRows rows (nq = 0 in the task);
-//   BwdInvReduce         {s, kb, nb, slot0, nq, -, -}: that sum for these fronts;
+//                        them to be done writes g = y / D - their sum of the block's columns, unless the front is
+//                        large (more than kGatherRows rows, several right-hand sides);
+//   BwdInvReduce         {s, kb, nb, slot0, nq, -, -}: that sum for large fronts;
 //   BwdInvDiag           {s, j, nb, ob_s, slot0, nc, blk, i0, i1}: the part i0 <= i <= i1 of
 //                        x_j = sum_{i >= j} Linv(i, j)^T g_i, in chunks as FwdInvDiag.
-// blk is the diagonal-inverse index of the front's block 0.  Fronts of more than kGatherRows rows have their vectors
-// gathered by launches of their own, and FwdInvTail subtracts from those.
-// Inverse fronts of up to kGatherRows rows read the children's and the ancestors' entries inside their kernels and the
-// last chunk of a column block adds its partial sums; a level then has four launches, not seven, which bounds chains of
-// small fronts (FP64: 20^3 elasticity 1.02 -> 0.97 ms a solve, 24^3 x 3 grid with 33 right-hand sides 7.53 -> 7.16 ms).  Every
-// block row and column of a front reads the entries again, and in larger fronts that costs more than the launches (60 x
-// 60 x 30 elasticity, 16 right-hand sides: 401 ms with them, 423 ms without).
+// blk is the diagonal-inverse index of the front's block 0.
+//
+// Inverse fronts read the children's and the ancestors' entries inside their kernels and the last chunk of a column
+// block adds its partial sums; a level then has four launches, not seven, which bounds chains of small fronts (FP64: 20^3
+// elasticity 1.02 -> 0.97 ms a solve, 24^3 x 3 grid with 33 right-hand sides 7.53 -> 7.16 ms).  Every block row and
+// column of a front reads the entries again, and with several right-hand sides that costs more in fronts of more than
+// kGatherRows rows than the launches (60 x 60 x 30 elasticity, 16 right-hand sides: 401 ms with them, 423 ms without);
+// their vectors are gathered and reduced by launches of their own.  One right-hand side gains there too (40^3 elasticity,
+// contrast 1e4: 53.2 -> 52.6 ms; 30^3 BF16 70.3 -> 69.8 ms), so those launches are left out of its solves.
 constexpr int kGatherRows = 4096;
 
 struct InvLaunch {
