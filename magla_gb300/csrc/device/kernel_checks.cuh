@@ -11,7 +11,8 @@ inline int round_up_int(int x, int a) { return (x + a - 1) / a * a; }
 
 // Front of m rows and w columns in the device layout (panel m x w with ldp, contribution
 // t x t with ldc), from / to a column-major m x m host array (lower triangle used).
-struct CheckFront {
+template <class T>
+struct CheckFrontOf {
     SnDev d{};
     DBuf panel, contrib, sn;
     void setup(int m, int w, cudaStream_t st) {
@@ -26,26 +27,27 @@ struct CheckFront {
         d.rows_off = 0;
         d.rel_off = 0;
         d.parent = -1;
-        panel.alloc((size_t)d.ldp * w * sizeof(float), "check front");
-        contrib.alloc((size_t)std::max(1, d.ldc * t) * sizeof(float), "check front");
+        panel.alloc((size_t)d.ldp * w * sizeof(T), "check front");
+        contrib.alloc((size_t)std::max(1, d.ldc * t) * sizeof(T), "check front");
         std::vector<SnDev> v{d};
         sn.upload(v, st, "check front");
     }
-    void upload(const float* full, cudaStream_t st) {
+    void upload(const T* full, cudaStream_t st) {
         const int m = d.m, w = d.w, t = m - w;
-        std::vector<float> p((size_t)d.ldp * w, 0.f), c((size_t)std::max(1, d.ldc * t), 0.f);
+        std::vector<T> p((size_t)d.ldp * w, T(0)), c((size_t)std::max(1, d.ldc * t), T(0));
         for (int j = 0; j < w; ++j)
             for (int i = 0; i < m; ++i) p[i + (size_t)j * d.ldp] = full[i + (size_t)j * m];
         for (int j = 0; j < t; ++j)
             for (int i = 0; i < t; ++i) c[i + (size_t)j * d.ldc] = full[(w + i) + (size_t)(w + j) * m];
-        CK(cudaMemcpyAsync(panel.p, p.data(), p.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(contrib.p, c.data(), c.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(panel.p, p.data(), p.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(contrib.p, c.data(), c.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+        CK(cudaStreamSynchronize(st));
     }
-    void download(float* full, cudaStream_t st) {
+    void download(T* full, cudaStream_t st) {
         const int m = d.m, w = d.w, t = m - w;
-        std::vector<float> p((size_t)d.ldp * w), c((size_t)std::max(1, d.ldc * t));
-        CK(cudaMemcpyAsync(p.data(), panel.p, p.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(c.data(), contrib.p, c.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
+        std::vector<T> p((size_t)d.ldp * w), c((size_t)std::max(1, d.ldc * t));
+        CK(cudaMemcpyAsync(p.data(), panel.p, p.size() * sizeof(T), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(c.data(), contrib.p, c.size() * sizeof(T), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         for (int j = 0; j < w; ++j)
             for (int i = 0; i < m; ++i) full[i + (size_t)j * m] = p[i + (size_t)j * d.ldp];
@@ -53,6 +55,8 @@ struct CheckFront {
             for (int i = 0; i < t; ++i) full[(w + i) + (size_t)(w + j) * m] = c[i + (size_t)j * d.ldc];
     }
 };
+
+using CheckFront = CheckFrontOf<float>;
 
 // Round to nearest even BF16 (the staging copies' rounding, __floats2bfloat162_rn).
 inline uint16_t to_bf16(float f) {
@@ -236,6 +240,62 @@ int uchol_check_diag_panel_rows(int tile_rows, int m, int nb, const float* front
     });
 }
 
+int uchol_check_digit_update(int m, int w, int c0, int cend, int kbeg, int kn, const double* front, const double* pivots,
+                             double* front_out) {
+    return guarded([&] {
+        if (!front || !pivots || !front_out) throw Error(UCHOL_BAD_ARG, "null argument");
+        if (m <= 0 || w <= 0 || w > m || kbeg < 0 || kbeg % kOzBlock != 0 || kn <= 0 || kbeg + kn > w ||
+            (kbeg + kn < w && kn % kOzBlock != 0))
+            throw Error(UCHOL_BAD_ARG, "the K columns must be whole outer blocks of the panel");
+        if (c0 < kbeg + kn || cend <= c0 || cend > m || (c0 < w && cend > w))
+            throw Error(UCHOL_BAD_ARG, "the columns must lie after the K columns, all in the panel or all in the contribution");
+        cudaStream_t st = nullptr;
+        CheckFrontOf<double> F;
+        F.setup(m, w, st);
+        F.upload(front, st);
+        StageInfo g{0, (w + 31) / 32 * 256, 0};
+        const long long exps = (long long)((w + kOzBlock - 1) / kOzBlock) * F.d.ldp;
+        DBuf diag, sl, sw, ex, info, tasks, jobs, maps, status;
+        diag.upload(std::vector<double>(pivots, pivots + w), st, "check");
+        sl.alloc((size_t)m * g.ld * 2, "check");
+        sw.alloc((size_t)m * g.ld * 2, "check");
+        ex.alloc((size_t)exps * 2 * sizeof(int), "check");
+        CK(cudaMemsetAsync(sl.p, 0, sl.bytes, st));
+        CK(cudaMemsetAsync(sw.p, 0, sw.bytes, st));
+        CK(cudaMemsetAsync(ex.p, 0, ex.bytes, st));
+        info.upload(std::vector<StageInfo>{g}, st, "check");
+        std::vector<PanelTask> tv;
+        for (int b = kbeg; b < kbeg + kn; b += kOzBlock) {
+            const int be = std::min(w, b + kOzBlock);
+            for (int r = be; r < m; r += 128) tv.push_back(PanelTask{0, b, be - b, r, std::min(128, m - r), 0, 0, 0});
+        }
+        tasks.upload(tv, st, "check");
+        jobs.upload(std::vector<TcJob>{TcJob{0, 0, c0, cend, kbeg, kn, 0}}, st, "check");
+        std::vector<CUtensorMap> mp(2);
+        try {
+            make_oz_maps(sl.p, sw.p, m, g.ld, mp.data());
+        } catch (const std::runtime_error& e) {
+            throw Error(UCHOL_CUDA_ERROR, e.what());
+        }
+        maps.upload(mp, st, "check");
+        status.alloc(sizeof(int), "check");
+        CK(cudaMemsetAsync(status.p, 0, sizeof(int), st));
+        CK(cudaStreamSynchronize(st));
+        CK(cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz_smem_bytes()));
+        k_oz_slice<<<(unsigned)tv.size() * kOzSplit, 256, 0, st>>>(
+            tasks.as<PanelTask>(), F.sn.as<SnDev>(), F.panel.as<double>(), diag.as<double>(), sl.as<__nv_bfloat16>(),
+            sw.as<__nv_bfloat16>(), ex.as<int>(), exps, info.as<StageInfo>());
+        k_oz_gemm<<<(unsigned)tc_job_tiles<kOzCols>(c0, cend, m), kOzThreads, oz_smem_bytes(), st>>>(
+            jobs.as<TcJob>(), 1, F.sn.as<SnDev>(), F.panel.as<double>(), F.contrib.as<double>(), maps.as<CUtensorMap>(),
+            ex.as<int>(), exps, info.as<StageInfo>(), status.as<int>());
+        counted(2);
+        CK(cudaGetLastError());
+        F.download(front_out, st);
+        int hs = 0;
+        CK(cudaMemcpy(&hs, status.p, sizeof(int), cudaMemcpyDeviceToHost));
+        if (hs != 0) throw Error(UCHOL_TIMEOUT, "a bounded device wait expired");
+    });
+}
 
 // Plan check (host only): builds the execution plan of a symbolic factorisation for the
 // given options and SM count and verifies the invariants its launches rely on; no GPU needed.

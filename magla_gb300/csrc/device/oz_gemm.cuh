@@ -10,15 +10,20 @@
 //
 // Slices.  Column k of L is scaled by 2^s and of W by 2^-s, s about log2(d_k) / 2 (exact; both are then of the size of
 // L sqrt(D), so that no column of the chunk is small in one and large in the other).  For each row i of either and chunk
-// of 128 columns (K), E_i is the largest exponent of the row's scaled entries and X = round(a 2^(62 - E_i)) a 63-bit
-// integer, written in balanced base 256: X = sum_p d_p 2^(8 (7 - p)), |d_p| <= 128.  The product of two rows over a chunk
-// is 2^(E_i + E_j - 124) sum_{p, q} 2^(8 (14 - p - q)) d_p . d_q; the orders o = p + q <= 7 are kept.  What is left out is
-// about 2^-60 of the rows' largest entries, so that a row whose other entries are 2^-7 of its largest is still summed as
-// FP64 sums it.  (Seven digits, 2^-53, cost 20% less and tripled the forward error on 20^3 elasticity, whose rows of L
-// are of that kind.)  One FP32 accumulator per order: at most 8 products of 128 terms of at most 2^14 each, so every
-// partial sum is an integer of at most 2^24 and exact.  The eight sums are combined in 64-bit integers, rounded once to
-// FP64 and added to the tile's FP64 sums, chunk by chunk; C takes one FP64 subtraction.  Every tile is one CTA's: the
-// result is deterministic.
+// of 128 columns (K), E_i is the largest exponent of the row's scaled entries and X = round(a 2^(63 - E_i)) a 64-bit
+// integer (|a| < 2^E_i), written in balanced base 256: X = sum_p d_p 2^(8 (7 - p)), |d_p| <= 128.  The product of two rows
+// over a chunk is 2^(E_i + E_j - 126) sum_{p, q} 2^(8 (14 - p - q)) d_p . d_q; the orders o = p + q <= 7 are kept.  One
+// FP32 accumulator per order: at most 8 products of 128 terms of at most 2^14 each, so every partial sum is an integer of
+// at most 2^24 and exact.  The eight sums are joined in a 64-bit integer whose unit follows the size of the result
+// (2^-60 of it), rounded to FP64 and added to the tile's FP64 sums, chunk by chunk; C takes one FP64 subtraction.
+// Every tile is one CTA's: the result is deterministic.
+//
+// What is lost.  The orders past 7 are 2^-60.7 2^(E_i + E_j) in the mean of random digits and below 2^-54 2^(E_i + E_j)
+// whatever the digits; an entry 2^-11 of its row's largest or smaller starts to lose low bits of its own.  FP64 sums lose
+// 2^-53 of sum_k |l_ik d_k l_jk|, so the digits are the more accurate where that sum is above 2^-7 of the product of the
+// rows' largest entries, and the less accurate entry by entry where two rows have their large entries in different
+// columns.  Against sqrt(c_ii c_jj), which is at least that product and in which the error of a Cholesky factorisation
+// is measured (the same under every scaling of the equations), every entry's loss is below FP64's unit roundoff.
 //
 // Layout: staging rows (front rows) of 512 bytes per 32 columns: eight slices of 32 BF16 digits, so that a 128-byte
 // swizzled box holds two slices of 32 columns.
@@ -40,13 +45,11 @@ constexpr int kOzNan = 1 << 20;      // row exponent of a chunk with an entry th
 
 inline size_t oz_smem_bytes() { return 1024 + (size_t)kOzStages * (kOzABytes + kOzBBytes) + 128; }
 
-// 16 accumulator columns of this thread's TMEM lane (no wait).
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
+// 8 accumulator columns of this thread's TMEM lane (no wait).
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -105,7 +108,7 @@ __global__ void __launch_bounds__(256) k_oz_slice(const PanelTask* __restrict__ 
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 if (q >= groups) break;
-                const int sh = e[q] - E + 9;   // X = M 2^sh, M the 53-bit significand
+                const int sh = e[q] - E + 10;   // X = M 2^sh, M the 53-bit significand
                 const unsigned long long M = ((unsigned long long)b[q] & 0xfffffffffffffull) | 0x10000000000000ull;
                 long long X = e[q] <= -50000 || sh < -54 ? 0 : (long long)(sh >= 0 ? M << sh : (M + (1ull << (-sh - 1))) >> -sh);
                 if (b[q] < 0) X = -X;
@@ -245,29 +248,37 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             }
             acc_phase ^= 1;
             tc_fence_after();
+            // T = the sum over the orders, in units of order 7: its upper half hi (orders 0 to 3, units of order 3, below
+            // 2^45.1) and its lower half lo (orders 4 to 7, below 2^47.4).  T is held as V 2^(32 - k), V a 64-bit integer:
+            // k, from 16 to 31, leaves hi all the bits of V but the sign and one
             long long V[32];
+            unsigned ks[4] = {0u, 0u, 0u, 0u};   // k - 16 of each entry, four bits
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t r0[16], r1[16], r2[16], r3[16];
-                tmem_ld16(ta + 0 * kOzCols + 16 * h, r0);
-                tmem_ld16(ta + 1 * kOzCols + 16 * h, r1);
-                tmem_ld16(ta + 2 * kOzCols + 16 * h, r2);
-                tmem_ld16(ta + 3 * kOzCols + 16 * h, r3);
+            for (int h = 0; h < 4; ++h) {
+                uint32_t r0[8], r1[8], r2[8], r3[8];
+                tmem_ld8(ta + 0 * kOzCols + 8 * h, r0);
+                tmem_ld8(ta + 1 * kOzCols + 8 * h, r1);
+                tmem_ld8(ta + 2 * kOzCols + 8 * h, r2);
+                tmem_ld8(ta + 3 * kOzCols + 8 * h, r3);
                 tmem_ld_wait();
 #pragma unroll
-                for (int u = 0; u < 16; ++u) {   // |r_o| <= (o + 1) 2^21: both fit 32 bits
+                for (int u = 0; u < 8; ++u) {   // |r_o| <= (o + 1) 2^21: both fit 32 bits
                     const int t0 = oz_int(r0[u]) * 256 + oz_int(r1[u]), t1 = oz_int(r2[u]) * 256 + oz_int(r3[u]);
-                    V[16 * h + u] = ((long long)t0 << 32) + (long long)t1 * 65536;
+                    V[8 * h + u] = (long long)t0 * 65536 + t1;
                 }
-                tmem_ld16(ta + 4 * kOzCols + 16 * h, r0);
-                tmem_ld16(ta + 5 * kOzCols + 16 * h, r1);
-                tmem_ld16(ta + 6 * kOzCols + 16 * h, r2);
-                tmem_ld16(ta + 7 * kOzCols + 16 * h, r3);
+                tmem_ld8(ta + 4 * kOzCols + 8 * h, r0);
+                tmem_ld8(ta + 5 * kOzCols + 8 * h, r1);
+                tmem_ld8(ta + 6 * kOzCols + 8 * h, r2);
+                tmem_ld8(ta + 7 * kOzCols + 8 * h, r3);
                 tmem_ld_wait();
 #pragma unroll
-                for (int u = 0; u < 16; ++u) {   // the sum / 2^16, rounded down after half a unit is added; below 2^61
-                    const int low = (oz_int(r2[u]) + ((oz_int(r3[u]) + 32768) >> 8)) >> 8;
-                    V[16 * h + u] += (long long)oz_int(r0[u]) * 256 + (oz_int(r1[u]) + low);
+                for (int u = 0; u < 8; ++u) {
+                    const long long hi = V[8 * h + u];
+                    const long long lo = ((long long)oz_int(r0[u]) * 256 + oz_int(r1[u])) * 65536 +
+                                         ((long long)oz_int(r2[u]) * 256 + oz_int(r3[u]));
+                    const int k = min(31, __clzll(hi ^ (hi >> 63)) - 2);
+                    V[8 * h + u] = (hi << k) + ((lo + (1ll << (31 - k))) >> (32 - k));
+                    ks[h] |= (unsigned)(k - 16) << (4 * u);
                 }
             }
             tc_fence_before();
@@ -275,7 +286,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 #pragma unroll
             for (int u = 0; u < 32; ++u) {
                 const int ej = __shfl_sync(0xffffffffu, ejl, u);
-                double v = oz_value(V[u], ei + ej - 2096);
+                const int k = 16 + (int)(ks[u / 8] >> (4 * (u % 8)) & 15u);
+                double v = oz_value(V[u], ei + ej - 2114 + (32 - k));   // order 7's unit: 2^(56 - 2 (1075 + 10))
                 if (ei == kOzNan || ej == kOzNan) v = __longlong_as_double(0x7ff8000000000000ll);
                 sum[u] += v;
             }
