@@ -278,6 +278,10 @@ int uchol_set_wait_limits(double solve_ms, double factor_ms);
  * usable; UCHOL_BAD_ARG when the factor has no such launch (use inverse_block_width < 0 and
  * a front wider than three solve blocks).  No counterpart in the reference. */
 int uchol_check_solve_wait(uchol_factor f, double wait_ms);
+/* Failure check of the memory fallbacks: from now on an allocation of the calling thread fails, as on a full device, when
+ * its buffers allocated from now on would then hold more than `bytes` bytes (< 0: no limit).  Returns the bytes held by
+ * those of the limit before. */
+int64_t uchol_check_allocation_limit(int64_t bytes);
 
 /* Kernel checks: one launch of a factorisation kernel of the mixed path on caller data
  * (host buffers), so that tests can compare each kernel with an FP64 computation on the

@@ -80,23 +80,32 @@ int guarded(F&& f) {
     }
 }
 
+// Allocation limit of the calling thread (uchol_check_allocation_limit): bytes it may hold in buffers allocated since the
+// limit was set (< 0: no limit), and those it holds.
+thread_local int64_t t_alloc_limit = -1, t_alloc_held = 0;
+thread_local unsigned t_alloc_epoch = 0;
+
 // Owning device allocation.
 struct DBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    unsigned epoch = 0;   // of the limit that counts the buffer in t_alloc_held (0: none)
     DBuf() = default;
     DBuf(const DBuf&) = delete;
     DBuf& operator=(const DBuf&) = delete;
     ~DBuf() { release(); }
     void release() {
         if (p) cudaFree(p);
+        if (epoch != 0 && epoch == t_alloc_epoch) t_alloc_held -= (int64_t)bytes;
         p = nullptr;
         bytes = 0;
+        epoch = 0;
     }
     void alloc(size_t b, const char* what) {
         release();
         if (b == 0) b = 16;
-        cudaError_t e = cudaMalloc(&p, b);
+        const bool over = t_alloc_limit >= 0 && t_alloc_held + (int64_t)b > t_alloc_limit;
+        cudaError_t e = over ? cudaErrorMemoryAllocation : cudaMalloc(&p, b);
         if (e != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
@@ -104,6 +113,10 @@ struct DBuf {
                                        " failed: " + cudaGetErrorString(e));
         }
         bytes = b;
+        if (t_alloc_limit >= 0) {
+            epoch = t_alloc_epoch;
+            t_alloc_held += (int64_t)b;
+        }
     }
     template <class V>
     void upload(const std::vector<V>& v, cudaStream_t s, const char* what) {
@@ -116,10 +129,45 @@ struct DBuf {
 
 struct DevPlan {
     Plan plan;
+    bool uploaded = false;
     DBuf sn, rel, asm_pos, ea_items, ea_entries, small, pivot_tasks, panel_tasks, simt_jobs, tc_jobs,
         stage;
     DBuf fvec_off, gather_ptr, gather_src, solve_tasks, inv_warp, inv_cta, inv_tasks;
     DBuf rows, child_ptr, children;   // structure of the device fronts
+
+    void upload(cudaStream_t st) {
+        const Plan& P = plan;
+        sn.upload(P.sn, st, "supernode table");
+        rel.upload(P.rel, st, "relative indices");
+        asm_pos.upload(P.assemble_pos, st, "assembly map");
+        ea_items.upload(P.ea_items, st, "plan");
+        ea_entries.upload(P.ea_entries, st, "plan");
+        small.upload(P.small_fronts, st, "plan");
+        pivot_tasks.upload(P.pivot_tasks, st, "plan");
+        panel_tasks.upload(P.panel_tasks, st, "plan");
+        simt_jobs.upload(P.simt_jobs, st, "plan");
+        tc_jobs.upload(P.tc_jobs, st, "plan");
+        stage.upload(P.stage, st, "plan");
+        fvec_off.upload(P.fvec_off, st, "plan");
+        gather_ptr.upload(P.gather_ptr, st, "plan");
+        gather_src.upload(P.gather_src, st, "plan");
+        solve_tasks.upload(P.solve_tasks, st, "plan");
+        inv_warp.upload(P.inv_warp, st, "plan");
+        inv_cta.upload(P.inv_cta, st, "plan");
+        inv_tasks.upload(P.inv_tasks, st, "plan");
+        rows.upload(P.front_rows, st, "front rows");
+        child_ptr.upload(P.child_ptr, st, "children");
+        children.upload(P.children, st, "children");
+        CK(cudaStreamSynchronize(st));
+        uploaded = true;
+    }
+    void release() {
+        for (DBuf* b : {&sn, &rel, &asm_pos, &ea_items, &ea_entries, &small, &pivot_tasks, &panel_tasks, &simt_jobs, &tc_jobs,
+                        &stage, &fvec_off, &gather_ptr, &gather_src, &solve_tasks, &inv_warp, &inv_cta, &inv_tasks, &rows,
+                        &child_ptr, &children})
+            b->release();
+        uploaded = false;
+    }
 };
 
 // Mixed path: the outer blocks' inverses are not the solves' blocks and live in the workspace slots.
@@ -174,63 +222,48 @@ struct uchol_symbolic_s {
     std::vector<int> first_col, parent, child_ptr, children, front_ptr, front_rows;
     DBuf d_perm, d_diag_idx, d_full_ptr, d_full_col, d_full_src;
     long long full_nnz = 0;
-    std::map<std::string, std::unique_ptr<DevPlan>> plans;
+    std::map<std::string, std::shared_ptr<DevPlan>> plans;
     std::mutex mu;
 
+    static std::string plan_key(const PlanConfig& c) {
+        return std::to_string(c.pivot_block) + "/" + std::to_string(c.outer_block) + "/" + std::to_string(c.small_mask) + "/" +
+               std::to_string(c.tensor_core) + "/" + std::to_string(c.solve_block) + "/" + std::to_string(c.merge_cols) + "/" +
+               std::to_string(c.merge_fill) + "/" + std::to_string(c.inv_cols) + "/" + std::to_string(c.oz_rows) + "/" +
+               std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
+    }
+
     // The plan of a configuration, built once and uploaded; `budget` > 0 rejects a plan whose
-    // factor would need more device memory (UCHOL_OOM) before anything is uploaded.
-    DevPlan* get_plan(const PlanConfig& c, int precision = UCHOL_PRECISION_FP64, int64_t budget = 0) {
-        std::string key = std::to_string(c.pivot_block) + "/" + std::to_string(c.outer_block) + "/" +
-                          std::to_string(c.small_mask) + "/" + std::to_string(c.tensor_core) + "/" +
-                          std::to_string(c.solve_block) + "/" + std::to_string(c.merge_cols) + "/" +
-                          std::to_string(c.merge_fill) + "/" + std::to_string(c.inv_cols) + "/" +
-                          std::to_string(c.oz_rows) + "/" + std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
-        auto it = plans.find(key);
-        if (it != plans.end()) {
-            check_budget(budget, planned_bytes(it->second->plan, precision, nnz, full_nnz, n));
-            return it->second.get();
+    // factor would need more device memory (UCHOL_OOM) before anything is uploaded.  A rejected
+    // plan stays on the host, so that the next attempt does not build it again.
+    std::shared_ptr<DevPlan> get_plan(const PlanConfig& c, int precision, int64_t budget) {
+        std::shared_ptr<DevPlan>& dp = plans[plan_key(c)];
+        if (!dp) {
+            auto fresh = std::make_shared<DevPlan>();
+            try {
+                fresh->plan = build_plan(n, count, first_col.data(), parent.data(), child_ptr.data(), children.data(),
+                                         front_ptr.data(), front_rows.data(), diag_idx.data(), pat_ptr.data(),
+                                         pat_rows.data(), lower_start.data(), lower_ptr.data(), lower_idx.data(), nnz, c);
+            } catch (const std::runtime_error& e) {
+                throw Error(UCHOL_BAD_ARG, std::string("inconsistent symbolic factorization: ") + e.what());
+            }
+            dp = std::move(fresh);
         }
-        auto dp = std::make_unique<DevPlan>();
-        try {
-            dp->plan = build_plan(n, count, first_col.data(), parent.data(), child_ptr.data(), children.data(),
-                                  front_ptr.data(), front_rows.data(), diag_idx.data(), pat_ptr.data(), pat_rows.data(),
-                                  lower_start.data(), lower_ptr.data(), lower_idx.data(), nnz, c);
-        } catch (const std::runtime_error& e) {
-            throw Error(UCHOL_BAD_ARG, std::string("inconsistent symbolic factorization: ") + e.what());
-        }
-        const Plan& P = dp->plan;
-        check_budget(budget, planned_bytes(P, precision, nnz, full_nnz, n));
-        dp->sn.upload(P.sn, stream, "supernode table");
-        dp->rel.upload(P.rel, stream, "relative indices");
-        dp->asm_pos.upload(P.assemble_pos, stream, "assembly map");
-        dp->ea_items.upload(P.ea_items, stream, "plan");
-        dp->ea_entries.upload(P.ea_entries, stream, "plan");
-        dp->small.upload(P.small_fronts, stream, "plan");
-        dp->pivot_tasks.upload(P.pivot_tasks, stream, "plan");
-        dp->panel_tasks.upload(P.panel_tasks, stream, "plan");
-        dp->simt_jobs.upload(P.simt_jobs, stream, "plan");
-        dp->tc_jobs.upload(P.tc_jobs, stream, "plan");
-        dp->stage.upload(P.stage, stream, "plan");
-        dp->fvec_off.upload(P.fvec_off, stream, "plan");
-        dp->gather_ptr.upload(P.gather_ptr, stream, "plan");
-        dp->gather_src.upload(P.gather_src, stream, "plan");
-        dp->solve_tasks.upload(P.solve_tasks, stream, "plan");
-        dp->inv_warp.upload(P.inv_warp, stream, "plan");
-        dp->inv_cta.upload(P.inv_cta, stream, "plan");
-        dp->inv_tasks.upload(P.inv_tasks, stream, "plan");
-        dp->rows.upload(P.front_rows, stream, "front rows");
-        dp->child_ptr.upload(P.child_ptr, stream, "children");
-        dp->children.upload(P.children, stream, "children");
-        CK(cudaStreamSynchronize(stream));
-        DevPlan* raw = dp.get();
-        plans[key] = std::move(dp);
-        return raw;
+        check_budget(budget, planned_bytes(dp->plan, precision, nnz, full_nnz, n));
+        if (!dp->uploaded) dp->upload(stream);
+        return dp;
+    }
+
+    // Takes the plan of a configuration off the device when no factor uses it: a factor that could not be
+    // allocated leaves the device as it was for the next smaller configuration.
+    void unload_plan(const PlanConfig& c) {
+        auto it = plans.find(plan_key(c));
+        if (it != plans.end() && it->second && it->second.use_count() == 1) it->second->release();
     }
 };
 
 struct uchol_factor_s {
     uchol_symbolic sym = nullptr;
-    DevPlan* dp = nullptr;
+    std::shared_ptr<DevPlan> dp;
     uchol_options opts{};
     int precision = UCHOL_PRECISION_FP64;
     size_t elem = 8;              // bytes per front element
@@ -778,7 +811,7 @@ void check_options(const uchol_options* o) {
 }
 
 // A factor object of one configuration: its plan and every buffer that does not depend on the right-hand sides
-// (UCHOL_OOM when the budget or the device's memory does not hold them; nothing is kept then).
+// (UCHOL_OOM when the budget or the device's memory does not hold them; only the plan is kept then).
 uchol_factor_s* allocate_factor(uchol_symbolic_s* S, const uchol_options& o, const PlanConfig& cfg) {
     auto F = std::make_unique<uchol_factor_s>();
     F->sym = S;
@@ -876,6 +909,7 @@ uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_o
         try {
             return allocate_factor(S, o, cfg);
         } catch (const Error& e) {
+            S->unload_plan(cfg);
             if (e.code != UCHOL_OOM || !relax_for_budget(cfg, o)) throw;
         }
     }
@@ -1430,6 +1464,14 @@ int uchol_set_wait_limits(double solve_ms, double factor_ms) {
         CK(cudaMemcpyToSymbol(g_solve_wait_ns, &s, sizeof(s)));
         CK(cudaMemcpyToSymbol(g_factor_wait_ns, &f, sizeof(f)));
     });
+}
+
+int64_t uchol_check_allocation_limit(int64_t bytes) {
+    const int64_t held = t_alloc_held;
+    t_alloc_limit = bytes;
+    t_alloc_held = 0;
+    ++t_alloc_epoch;
+    return held;
 }
 
 int uchol_check_solve_wait(uchol_factor f, double wait_ms) {
