@@ -192,6 +192,7 @@ int64_t planned_bytes(const Plan& P, int precision, long long nnz, long long ful
     else b += 2 * (P.stage_elems * 2 + P.oz_exps * 4);
     b += ((int64_t)P.inv_blocks.size() + P.inv_off_blocks) * sb * sb * elem;
     b += inv_scratch_elems(P) * elem;
+    b += ((int64_t)P.gather_ptr.size() + (int64_t)P.gather_src.size()) * 4;
     b += (nnz + full_nnz) * 8 + (int64_t)n * 8;
     return b;
 }
@@ -229,7 +230,7 @@ struct uchol_symbolic_s {
         return std::to_string(c.pivot_block) + "/" + std::to_string(c.outer_block) + "/" + std::to_string(c.small_mask) + "/" +
                std::to_string(c.tensor_core) + "/" + std::to_string(c.solve_block) + "/" + std::to_string(c.merge_cols) + "/" +
                std::to_string(c.merge_fill) + "/" + std::to_string(c.inv_cols) + "/" + std::to_string(c.oz_rows) + "/" +
-               std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
+               std::to_string(c.gather_lists) + "/" + std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
     }
 
     // The plan of a configuration, built once and uploaded; `budget` > 0 rejects a plan whose
@@ -371,9 +372,11 @@ PlanConfig config_for(const uchol_options& o) {
 }
 
 // The next smaller configuration for a memory budget or a device that does not hold this one: default choices that cost memory only
-// for speed are given up, the wider inverse fronts and the digits of the FP64 tensor-core updates; false: none is left.
+// for speed are given up, in the order of what they cost a user of the memory: the wider inverse fronts, the solves'
+// gather lists, the digits of the FP64 tensor-core updates; false: none is left.
 bool relax_for_budget(PlanConfig& c, const uchol_options& o) {
     if (o.inverse_block_width == 0 && c.inv_cols > kDefaultInvCols64) c.inv_cols = kDefaultInvCols64;
+    else if (c.gather_lists) c.gather_lists = false;
     else if (c.oz_rows > 0) c.oz_rows = 0;
     else return false;
     return true;
@@ -992,7 +995,7 @@ SolveArgs solve_args(uchol_factor_s* F, int nrhs) {
     A.child_ptr = D.child_ptr.as<int>();
     A.children = D.children.as<int>();
     A.fvec_off = D.fvec_off.as<long long>();
-    A.gather_ptr = D.gather_ptr.as<unsigned>();
+    A.gather_ptr = D.plan.gather_ptr.empty() ? nullptr : D.gather_ptr.as<unsigned>();
     A.gather_src = D.gather_src.as<unsigned>();
     A.fv_stride = D.plan.fvec_elems;
     A.n = F->sym->n;

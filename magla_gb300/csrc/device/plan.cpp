@@ -583,17 +583,17 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
         fo += round_up(P.sn[s].m, 8);
     }
     P.fvec_elems = std::max<long long>(fo, 8);
-    if (P.fvec_elems > (long long)UINT32_MAX) fail("the front vectors exceed 32-bit positions");
-    // the children's entries of every front-vector position, child by child
-    P.gather_ptr.assign(P.fvec_elems + 1, 0);
-    for (int s = 0; s < count; ++s)
-        for (int c = child_ptr[s]; c < child_ptr[s + 1]; ++c) {
-            const SnDev& cd = P.sn[children[c]];
-            for (int a = 0; a < cd.m - cd.w; ++a) ++P.gather_ptr[P.fvec_off[s] + P.rel[cd.rel_off + a] + 1];
-        }
-    for (long long q = 0; q < P.fvec_elems; ++q) P.gather_ptr[q + 1] += P.gather_ptr[q];
-    P.gather_src.assign(P.gather_ptr[P.fvec_elems], 0);
-    {
+    // the children's entries of every front-vector position, child by child (positions of 32 bits)
+    const bool lists = cfg.gather_lists && P.fvec_elems <= (long long)UINT32_MAX;
+    if (lists) {
+        P.gather_ptr.assign(P.fvec_elems + 1, 0);
+        for (int s = 0; s < count; ++s)
+            for (int c = child_ptr[s]; c < child_ptr[s + 1]; ++c) {
+                const SnDev& cd = P.sn[children[c]];
+                for (int a = 0; a < cd.m - cd.w; ++a) ++P.gather_ptr[P.fvec_off[s] + P.rel[cd.rel_off + a] + 1];
+            }
+        for (long long q = 0; q < P.fvec_elems; ++q) P.gather_ptr[q + 1] += P.gather_ptr[q];
+        P.gather_src.assign(P.gather_ptr[P.fvec_elems], 0);
         std::vector<unsigned> fill(P.gather_ptr.begin(), P.gather_ptr.end() - 1);
         for (int s = 0; s < count; ++s)
             for (int c = child_ptr[s]; c < child_ptr[s + 1]; ++c) {
@@ -732,13 +732,14 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
     for (int L = 0; L < P.levels; ++L) {
         const auto& fronts = at_level[L];
         // the front vectors of the level kernels' fronts and of large inverse fronts are gathered first; the others' as
-        // they are read
+        // they are read, given the lists of their entries
         SolveLaunch solo = split(fronts, multi, inv);
+        const std::vector<int>& gathered = lists ? multi : fronts;
         std::vector<int> large;
         for (int s : fronts)
-            if (inv_ob[s] >= 0 && P.sn[s].m > kGatherRows) large.push_back(s);
-        if (!multi.empty()) {
-            auto g = gather_tasks(multi);
+            if (lists && inv_ob[s] >= 0 && P.sn[s].m > kGatherRows) large.push_back(s);
+        if (!gathered.empty()) {
+            auto g = gather_tasks(gathered);
             P.fwd_launches.push_back({SolveLaunch::FwdGather, g.first, g.second, 0, 0, 0, 0, 0, 0, 0, 0, 0});
         }
         if (!large.empty()) {

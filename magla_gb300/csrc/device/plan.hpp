@@ -49,6 +49,7 @@ struct PlanConfig {
                                     // large fronts runs on a second stream, beside the level's outer blocks
     int oz_rows = 0;                // FP64 path, > 0: fronts of at least this many rows take their updates on the tensor
                                     // cores, from digit slices (oz_gemm.cuh)
+    bool gather_lists = true;       // forward solves read the children's entries as they go, from lists of them
     int sms = 0;                    // > 0: the device's SM count (sizes the backward inverse-front chunks)
 };
 
@@ -199,8 +200,9 @@ struct Plan {
     double simt_flops = 0.0;                   // algorithmic flops of the SIMT updates
 
     // solve tasks
-    std::vector<unsigned> gather_ptr;              // per position of the front vectors: its entries of gather_src
+    std::vector<unsigned> gather_ptr;          // per position of the front vectors: its entries of gather_src
     std::vector<unsigned> gather_src;          // front-vector positions of the children's update entries, in child order
+                                               // (both empty: every front's vector is gathered by a launch)
     std::vector<SolveBlockTask> solve_tasks;
     std::vector<SolveBlockTask> inv_blocks;    // every diagonal block, for the inversion after a factorisation
     std::vector<SolveLaunch> fwd_launches, bwd_launches;

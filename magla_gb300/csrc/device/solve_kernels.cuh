@@ -29,7 +29,7 @@ struct SolveArgs {
     const int* child_ptr;
     const int* children;
     const long long* fvec_off;
-    const unsigned* gather_ptr;  // per front-vector position: its entries of gather_src
+    const unsigned* gather_ptr;  // per front-vector position: its entries of gather_src (null: gathered by launches)
     const unsigned* gather_src;  // positions of the children's update entries, in child order
     long long fv_stride;    // elements between RHS columns in the front-vector workspace
     int n, nrhs, ldw;       // ldw: leading dimension of the work vector
@@ -75,9 +75,10 @@ __device__ __forceinline__ int warp_lower_bound(const int* __restrict__ a, int n
 }
 
 // v plus the children's update entries that land on front-vector position `pos`, added in child order: what a gather
-// launch of the front would have left there, without the launch.
+// launch of the front would have left there, without the launch; without the lists of the entries, what it has left.
 template <class Cv>
 __device__ __forceinline__ Cv add_children(const SolveArgs& A, long long pos, int r, const Cv* fv, Cv v) {
+    if (A.gather_ptr == nullptr) return fv[pos + (long long)r * A.fv_stride];
     const unsigned p1 = A.gather_ptr[pos + 1];
     for (unsigned p = A.gather_ptr[pos]; p < p1; ++p) v += fv[A.gather_src[p] + (long long)r * A.fv_stride];
     return v;
