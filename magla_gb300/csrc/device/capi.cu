@@ -230,7 +230,7 @@ struct uchol_symbolic_s {
         return std::to_string(c.pivot_block) + "/" + std::to_string(c.outer_block) + "/" + std::to_string(c.small_mask) + "/" +
                std::to_string(c.tensor_core) + "/" + std::to_string(c.solve_block) + "/" + std::to_string(c.merge_cols) + "/" +
                std::to_string(c.merge_fill) + "/" + std::to_string(c.inv_cols) + "/" + std::to_string(c.oz_rows) + "/" +
-               std::to_string(c.gather_lists) + "/" + std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
+               std::to_string(c.inv_in_place) + std::to_string(c.gather_lists) + "/" + std::to_string(c.side_extend_add) + "/" + std::to_string(c.sms);
     }
 
     // The plan of a configuration, built once and uploaded; `budget` > 0 rejects a plan whose
@@ -255,10 +255,12 @@ struct uchol_symbolic_s {
     }
 
     // Takes the plan of a configuration off the device when no factor uses it: a factor that could not be
-    // allocated leaves the device as it was for the next smaller configuration.
-    void unload_plan(const PlanConfig& c) {
+    // allocated leaves the device as it was for the next smaller configuration.  Returns the plan (null: none was built).
+    const Plan* unload_plan(const PlanConfig& c) {
         auto it = plans.find(plan_key(c));
-        if (it != plans.end() && it->second && it->second.use_count() == 1) it->second->release();
+        if (it == plans.end() || !it->second) return nullptr;
+        if (it->second.use_count() == 1) it->second->release();
+        return &it->second->plan;
     }
 };
 
@@ -372,10 +374,11 @@ PlanConfig config_for(const uchol_options& o) {
 }
 
 // The next smaller configuration for a memory budget or a device that does not hold this one: default choices that cost memory only
-// for speed are given up, in the order of what they cost a user of the memory: the wider inverse fronts, the solves'
-// gather lists, the digits of the FP64 tensor-core updates; false: none is left.
-bool relax_for_budget(PlanConfig& c, const uchol_options& o) {
+// for speed are given up, in the order of what they cost a user of the memory: the wider inverse fronts, the scratch
+// of the inversion, the solves' gather lists, the digits of the FP64 tensor-core updates; false: none is left.
+bool relax_for_budget(PlanConfig& c, const uchol_options& o, const Plan& P) {   // P: the plan of c
     if (o.inverse_block_width == 0 && c.inv_cols > kDefaultInvCols64) c.inv_cols = kDefaultInvCols64;
+    else if (inv_scratch_elems(P) > 0) c.inv_in_place = true;
     else if (c.gather_lists) c.gather_lists = false;
     else if (c.oz_rows > 0) c.oz_rows = 0;
     else return false;
@@ -621,7 +624,7 @@ void invert_diagonal_blocks(uchol_factor_s* F, cudaStream_t st) {
         k_invert_cta<T, T, SB><<<n, 256, invert_cta_smem<T, SB>(), st>>>(D.inv_cta.as<SolveBlockTask>(), sn, panel, linv);
         counted();
     }
-    T* scratch = F->inv_scratch.p ? F->inv_scratch.as<T>() : F->contrib.as<T>();
+    T* scratch = P.cfg.inv_in_place ? nullptr : F->inv_scratch.p ? F->inv_scratch.as<T>() : F->contrib.as<T>();
     for (const InvLaunch& L : P.inv_launches) {
         launch_inv_product<T, SB>(D.inv_tasks.as<SolveBlockTask>() + L.begin, L.count, L.second, F->sms, sn, panel, linv,
                                   F->linv_off.as<T>(), scratch, st);
@@ -912,8 +915,8 @@ uchol_factor_s* create_factor(uchol_symbolic_s* S, int n, int nnz, const uchol_o
         try {
             return allocate_factor(S, o, cfg);
         } catch (const Error& e) {
-            S->unload_plan(cfg);
-            if (e.code != UCHOL_OOM || !relax_for_budget(cfg, o)) throw;
+            const Plan* P = S->unload_plan(cfg);
+            if (e.code != UCHOL_OOM || !P || !relax_for_budget(cfg, o, *P)) throw;
         }
     }
 }
@@ -1622,7 +1625,7 @@ int uchol_estimate_device_bytes(const uchol_symbolic_desc* d, const uchol_option
             }
             // as create_factor
             if (o.device_memory_budget <= 0 || planned_bytes(P, o.precision, nnz, 2 * nnz - n, n) <= o.device_memory_budget ||
-                !relax_for_budget(cfg, o))
+                !relax_for_budget(cfg, o, P))
                 break;
         }
         const int64_t elem = o.precision == UCHOL_PRECISION_FP64 ? 8 : 4;

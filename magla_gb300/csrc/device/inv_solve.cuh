@@ -79,8 +79,8 @@ __global__ void __launch_bounds__(256) k_inv_product(const SolveBlockTask* __res
         const T* A = second ? inv_block<T, SB>(linv, linv_off, tk.blk, tk.r0, i, k) + o * SB
                             : P + (long long)(k * SB + o) * d.ldp;
         const long long lda = second ? SB : d.ldp;
-        const T* B = (second ? scratch + (long long)(tk.c0 - (i - k) * tk.c1) * SB * SB
-                             : inv_block<T, SB>(linv, linv_off, tk.blk, tk.r0, k, j)) + (long long)col0 * SB + o;
+        const T* B = (second && scratch ? scratch + (long long)(tk.c0 - (i - k) * tk.c1) * SB * SB
+                                        : inv_block<T, SB>(linv, linv_off, tk.blk, tk.r0, k, j)) + (long long)col0 * SB + o;
         for (int e = tid; e < KC * SB / V; e += 256) {
             const int r = e % (SB / V) * V, kk = e / (SB / V);
             const int n = second ? V : min(V, max(0, rows - r));
@@ -140,8 +140,9 @@ __global__ void __launch_bounds__(256) k_inv_product(const SolveBlockTask* __res
         }
         __syncthreads();   // this stage is refilled by the chunk after next
     }
-    T* out = second ? linv_off + ((long long)tk.r0 + (long long)i * (i - 1) / 2 + j) * SB * SB
-                    : scratch + (long long)tk.c0 * SB * SB;
+    // (in place, a CTA has read its strip of T(i, j) by now and no other CTA of the launch reads it)
+    T* out = second || !scratch ? linv_off + ((long long)tk.r0 + (long long)i * (i - 1) / 2 + j) * SB * SB
+                                : scratch + (long long)tk.c0 * SB * SB;
 #pragma unroll
     for (int q = 0; q < TC; ++q)
 #pragma unroll

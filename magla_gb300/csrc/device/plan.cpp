@@ -643,11 +643,23 @@ Plan build_from_fronts(int n, int count, const int* first_column, const int* par
             auto longer = [](const SolveBlockTask& x, const SolveBlockTask& y) { return x.flags - x.r1 > y.flags - y.r1; };
             std::stable_sort(first.begin(), first.end(), longer);
             std::stable_sort(second.begin(), second.end(), longer);
-            P.inv_scratch_blocks = std::max(P.inv_scratch_blocks, scratch);
-            P.inv_launches.push_back({(int)P.inv_tasks.size(), (int)first.size(), 0});
-            P.inv_tasks.insert(P.inv_tasks.end(), first.begin(), first.end());
-            P.inv_launches.push_back({(int)P.inv_tasks.size(), (int)second.size(), 1});
-            P.inv_tasks.insert(P.inv_tasks.end(), second.begin(), second.end());
+            auto launch = [&](const std::vector<SolveBlockTask>& tasks, int pass) {
+                if (tasks.empty()) return;
+                P.inv_launches.push_back({(int)P.inv_tasks.size(), (int)tasks.size(), pass});
+                P.inv_tasks.insert(P.inv_tasks.end(), tasks.begin(), tasks.end());
+            };
+            launch(first, 0);
+            if (!cfg.inv_in_place) {
+                P.inv_scratch_blocks = std::max(P.inv_scratch_blocks, scratch);
+                launch(second, 1);
+                continue;
+            }
+            for (int row = z; row > 0; --row) {   // sums of `row` blocks: block row `row - 1` of every group's lower half
+                std::vector<SolveBlockTask> level;
+                for (const SolveBlockTask& t : second)
+                    if (t.flags - t.r1 == row) level.push_back(t);
+                launch(level, 1);
+            }
         }
     }
     constexpr int kGatherChunk = 512;   // rows per gather CTA (one CTA per chunk and right-hand side)

@@ -49,6 +49,7 @@ struct PlanConfig {
                                     // large fronts runs on a second stream, beside the level's outer blocks
     int oz_rows = 0;                // FP64 path, > 0: fronts of at least this many rows take their updates on the tensor
                                     // cores, from digit slices (oz_gemm.cuh)
+    bool inv_in_place = false;      // the inversion's intermediate products take their results' place, not a scratch arena
     bool gather_lists = true;       // forward solves read the children's entries as they go, from lists of them
     int sms = 0;                    // > 0: the device's SM count (sizes the backward inverse-front chunks)
 };
@@ -106,7 +107,9 @@ struct SolveLaunch {
 //   inversion            {s, i, j, ob_s, k0, k1, blk, t, z}: by halves.  A group of 2 z blocks whose two halves
 //                        are inverted gets its off-diagonal half X_IJ = -X_II (L_IJ X_JJ): first
 //                        T(i, j) = sum_{k0 <= k < k1} L(i, k) X(k, j), T's block at index t of the scratch arena
-//                        (T(k, j) at t - (i - k) z), then X(i, j) = -sum_{k0 <= k < k1} X(i, k) T(k, j);
+//                        (T(k, j) at t - (i - k) z), then X(i, j) = -sum_{k0 <= k < k1} X(i, k) T(k, j).  In place
+//                        (cfg.inv_in_place), T(i, j) is where X(i, j) will be, and the second products take a launch
+//                        per block row of the halves, the last row first: row i reads T(k, j), k <= i;
 //   FwdInvDiag           {s, i, nb, ob_s, slot0, nc, blk, j0, j1}: the part j0 <= j <= j1 of
 //                        y_i = sum_{j <= i} Linv(i, j) f_j (f gathered from the children as it is read); block row i
 //                        is split in nc chunks of kInvDiagChunk blocks (partial slots slot0 .. slot0+nc-1; nc = 1: no
