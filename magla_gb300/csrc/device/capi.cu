@@ -135,38 +135,45 @@ struct DevPlan {
     DBuf fvec_off, gather_ptr, gather_src, solve_tasks, inv_warp, inv_cta, inv_tasks;
     DBuf rows, child_ptr, children;   // structure of the device fronts
 
-    void upload(cudaStream_t st) {
+    // f(buffer, host array, name) for every table
+    template <class Fn>
+    void each(Fn f) {
         const Plan& P = plan;
-        sn.upload(P.sn, st, "supernode table");
-        rel.upload(P.rel, st, "relative indices");
-        asm_pos.upload(P.assemble_pos, st, "assembly map");
-        ea_items.upload(P.ea_items, st, "plan");
-        ea_entries.upload(P.ea_entries, st, "plan");
-        small.upload(P.small_fronts, st, "plan");
-        pivot_tasks.upload(P.pivot_tasks, st, "plan");
-        panel_tasks.upload(P.panel_tasks, st, "plan");
-        simt_jobs.upload(P.simt_jobs, st, "plan");
-        tc_jobs.upload(P.tc_jobs, st, "plan");
-        stage.upload(P.stage, st, "plan");
-        fvec_off.upload(P.fvec_off, st, "plan");
-        gather_ptr.upload(P.gather_ptr, st, "plan");
-        gather_src.upload(P.gather_src, st, "plan");
-        solve_tasks.upload(P.solve_tasks, st, "plan");
-        inv_warp.upload(P.inv_warp, st, "plan");
-        inv_cta.upload(P.inv_cta, st, "plan");
-        inv_tasks.upload(P.inv_tasks, st, "plan");
-        rows.upload(P.front_rows, st, "front rows");
-        child_ptr.upload(P.child_ptr, st, "children");
-        children.upload(P.children, st, "children");
+        f(sn, P.sn, "supernode table");
+        f(rel, P.rel, "relative indices");
+        f(asm_pos, P.assemble_pos, "assembly map");
+        f(ea_items, P.ea_items, "plan");
+        f(ea_entries, P.ea_entries, "plan");
+        f(small, P.small_fronts, "plan");
+        f(pivot_tasks, P.pivot_tasks, "plan");
+        f(panel_tasks, P.panel_tasks, "plan");
+        f(simt_jobs, P.simt_jobs, "plan");
+        f(tc_jobs, P.tc_jobs, "plan");
+        f(stage, P.stage, "plan");
+        f(fvec_off, P.fvec_off, "plan");
+        f(gather_ptr, P.gather_ptr, "plan");
+        f(gather_src, P.gather_src, "plan");
+        f(solve_tasks, P.solve_tasks, "plan");
+        f(inv_warp, P.inv_warp, "plan");
+        f(inv_cta, P.inv_cta, "plan");
+        f(inv_tasks, P.inv_tasks, "plan");
+        f(rows, P.front_rows, "front rows");
+        f(child_ptr, P.child_ptr, "children");
+        f(children, P.children, "children");
+    }
+    void upload(cudaStream_t st) {
+        each([&](DBuf& b, const auto& v, const char* what) { b.upload(v, st, what); });
         CK(cudaStreamSynchronize(st));
         uploaded = true;
     }
     void release() {
-        for (DBuf* b : {&sn, &rel, &asm_pos, &ea_items, &ea_entries, &small, &pivot_tasks, &panel_tasks, &simt_jobs, &tc_jobs,
-                        &stage, &fvec_off, &gather_ptr, &gather_src, &solve_tasks, &inv_warp, &inv_cta, &inv_tasks, &rows,
-                        &child_ptr, &children})
-            b->release();
+        each([](DBuf& b, const auto&, const char*) { b.release(); });
         uploaded = false;
+    }
+    int64_t table_bytes() {
+        int64_t n = 0;
+        each([&](DBuf&, const auto& v, const char*) { n += (int64_t)(v.size() * sizeof(v[0])); });
+        return n;
     }
 };
 
@@ -178,6 +185,8 @@ long long inv_scratch_elems(const Plan& P) {
     const long long need = P.inv_scratch_blocks * P.cfg.solve_block * P.cfg.solve_block;
     return need <= P.contrib_elems ? 0 : need;
 }
+
+int64_t list_bytes(const Plan& P) { return ((int64_t)P.gather_ptr.size() + (int64_t)P.gather_src.size()) * 4; }
 
 // Device memory a factor of this plan reserves when it is created (the solve workspace,
 // which depends on the number of right-hand sides, comes on top).
@@ -192,7 +201,7 @@ int64_t planned_bytes(const Plan& P, int precision, long long nnz, long long ful
     else b += 2 * (P.stage_elems * 2 + P.oz_exps * 4);
     b += ((int64_t)P.inv_blocks.size() + P.inv_off_blocks) * sb * sb * elem;
     b += inv_scratch_elems(P) * elem;
-    b += ((int64_t)P.gather_ptr.size() + (int64_t)P.gather_src.size()) * 4;
+    b += list_bytes(P);
     b += (nnz + full_nnz) * 8 + (int64_t)n * 8;
     return b;
 }
@@ -237,6 +246,17 @@ struct uchol_symbolic_s {
     // factor would need more device memory (UCHOL_OOM) before anything is uploaded.  A rejected
     // plan stays on the host, so that the next attempt does not build it again.
     std::shared_ptr<DevPlan> get_plan(const PlanConfig& c, int precision, int64_t budget) {
+        std::shared_ptr<DevPlan> dp = host_plan(c);
+        check_budget(budget, planned_bytes(dp->plan, precision, nnz, full_nnz, n));
+        if (!dp->uploaded) try {
+            dp->upload(stream);
+        } catch (...) {
+            dp->release();
+            throw;
+        }
+        return dp;
+    }
+    std::shared_ptr<DevPlan> host_plan(const PlanConfig& c) {
         std::shared_ptr<DevPlan>& dp = plans[plan_key(c)];
         if (!dp) {
             auto fresh = std::make_shared<DevPlan>();
@@ -249,8 +269,6 @@ struct uchol_symbolic_s {
             }
             dp = std::move(fresh);
         }
-        check_budget(budget, planned_bytes(dp->plan, precision, nnz, full_nnz, n));
-        if (!dp->uploaded) dp->upload(stream);
         return dp;
     }
 
@@ -284,6 +302,7 @@ struct uchol_factor_s {
     DBuf solve_flags;                   // per diagonal block: forward and backward "solution published" flags
     DBuf solve_maps;                    // per front: tensor maps of its panel, boxes SB x SB, SB x SB/2, SB/2 x SB
     DBuf solve_status;                  // nonzero once a bounded wait of a solve expired
+    bool solve_maps_made = false;
     int coop_fwd = 0, coop_bwd = 0;     // resident CTAs of the level solve kernels (whole device)
     int ws_nrhs = 0;
     cudaStream_t capture_stream = nullptr;
@@ -301,6 +320,11 @@ struct uchol_factor_s {
     uchol_phase_times phases{};
     std::mutex mu;
 };
+
+// Refuses a factor that a full device has cost its buffers (shrink_factor).
+void require_factor(uchol_factor_s* F) {
+    if (!F->dp) throw Error(UCHOL_OOM, "the factor was lost when the device's memory ran out; factorise again");
+}
 
 // Drops one reference; the last one frees the symbolic object and its own stream.
 void symbolic_release(uchol_symbolic_s* s) {
@@ -767,7 +791,9 @@ void factorize_impl(uchol_factor_s* F, const double* values, bool on_device) {
         CK(cudaGraphUpload(F->factor_graph, st));
     }
     StreamTimer total(st);
-    if (on_device)
+    if (values == F->values.p) {
+        // factorised again from the values it holds (shrink_factor)
+    } else if (on_device)
         CK(cudaMemcpyAsync(F->values.p, values, (size_t)S->nnz * sizeof(double), cudaMemcpyDeviceToDevice, st));
     else
         CK(cudaMemcpyAsync(F->values.p, values, (size_t)S->nnz * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -816,24 +842,19 @@ void check_options(const uchol_options* o) {
                                        " front-size buckets");
 }
 
-// A factor object of one configuration: its plan and every buffer that does not depend on the right-hand sides
-// (UCHOL_OOM when the budget or the device's memory does not hold them; only the plan is kept then).
-uchol_factor_s* allocate_factor(uchol_symbolic_s* S, const uchol_options& o, const PlanConfig& cfg) {
-    auto F = std::make_unique<uchol_factor_s>();
-    F->sym = S;
-    S->refs.fetch_add(1);
-    F->opts = o;
-    F->precision = o.precision;
-    F->elem = F->precision == UCHOL_PRECISION_FP64 ? 8 : 4;
+// The plan of one configuration and every buffer of a factor that does not depend on the right-hand sides
+// (UCHOL_OOM when the budget or the device's memory does not hold them).
+void allocate_buffers(uchol_factor_s* F, const PlanConfig& cfg) {
+    uchol_symbolic_s* S = F->sym;
     F->sms = cfg.sms;
-    F->dp = S->get_plan(cfg, F->precision, o.device_memory_budget);
+    F->dp = S->get_plan(cfg, F->precision, F->opts.device_memory_budget);
     const Plan& P = F->dp->plan;
     cudaStream_t st = S->stream;
     F->panel.alloc((size_t)P.factor_elems * F->elem, "factor panels");
     F->contrib.alloc((size_t)P.contrib_elems * F->elem, "contribution blocks");
     bool side = false;
     for (const Launch& L : P.launches) side |= L.stream == 1;
-    if (side) {
+    if (side && !F->side_stream) {
         CK(cudaStreamCreateWithFlags(&F->side_stream, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&F->fork_ev, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&F->join_ev, cudaEventDisableTiming));
@@ -880,18 +901,31 @@ uchol_factor_s* allocate_factor(uchol_symbolic_s* S, const uchol_options& o, con
     }
     if (cfg.tensor_core)
         F->minv.alloc(minv_floats(std::max(1, P.diag_slots), own_inverses(cfg)) * sizeof(float), "diagonal-block inverses");
-    F->diag.alloc((size_t)std::max(1, S->n) * sizeof(double), "pivots");
     F->linv.alloc((size_t)std::max<size_t>(1, P.inv_blocks.size()) * cfg.solve_block * cfg.solve_block * F->elem,
                   "inverse diagonal blocks");
     CK(cudaMemsetAsync(F->linv.p, 0, F->linv.bytes, st));   // only lower triangles are written
     if (inv_scratch_elems(P) > 0) F->inv_scratch.alloc((size_t)inv_scratch_elems(P) * F->elem, "inversion scratch");
     F->linv_off.alloc((size_t)std::max<long long>(1, P.inv_off_blocks) * cfg.solve_block * cfg.solve_block * F->elem,
                       "inverse blocks of the inverse fronts");
-    F->values.alloc((size_t)std::max(1, S->nnz) * sizeof(double), "matrix values");
-    F->full_val.alloc((size_t)std::max<long long>(1, S->full_nnz) * sizeof(double), "matrix values");
-    F->stats.alloc(sizeof(PivotStats), "statistics");
-    F->ctl.alloc(sizeof(FactorCtl), "statistics");
-    prepare_factor_kernels(F.get());
+    if (!F->values.p) {
+        F->diag.alloc((size_t)std::max(1, S->n) * sizeof(double), "pivots");
+        F->full_val.alloc((size_t)std::max<long long>(1, S->full_nnz) * sizeof(double), "matrix values");
+        F->stats.alloc(sizeof(PivotStats), "statistics");
+        F->ctl.alloc(sizeof(FactorCtl), "statistics");
+        F->values.alloc((size_t)std::max(1, S->nnz) * sizeof(double), "matrix values");
+    }
+    prepare_factor_kernels(F);
+}
+
+// A factor object of one configuration; nothing of it is kept when its buffers cannot be allocated.
+uchol_factor_s* allocate_factor(uchol_symbolic_s* S, const uchol_options& o, const PlanConfig& cfg) {
+    auto F = std::make_unique<uchol_factor_s>();
+    F->sym = S;
+    S->refs.fetch_add(1);
+    F->opts = o;
+    F->precision = o.precision;
+    F->elem = F->precision == UCHOL_PRECISION_FP64 ? 8 : 4;
+    allocate_buffers(F.get(), cfg);
     return F.release();
 }
 
@@ -1123,6 +1157,9 @@ int solve_launch_count(const Plan& P, int nrhs) {
     return c + 1;   // + the flag reset
 }
 
+// Tile maps of the solves: three per front.
+size_t solve_map_count(const Plan& P) { return std::max<size_t>(1, 3 * P.sn.size()); }
+
 // The triangular solves of a factor for nrhs columns, captured once into a
 // CUDA graph over the factor's fixed work buffers and replayed on each call.
 template <class T, class Cv, int SB>
@@ -1162,12 +1199,12 @@ void launch_solve_graph(uchol_factor_s* F, int nrhs, Cv* work, cudaStream_t st) 
         limit(k_bwd_inv_cols<T, Cv, SB, 1>, inv_tail_smem<T, Cv, SB, 1, true>());
         limit(k_bwd_inv_cols<T, Cv, SB, RGM>, inv_tail_smem<T, Cv, SB, RGM, true>());
         if (F->coop_fwd < 2 || F->coop_bwd < 2) throw Error(UCHOL_CUDA_ERROR, "the level solve kernels do not fit");
-        if (!F->solve_maps.p) {
+        if (!F->solve_maps_made) {
             // tile copies of the solves: each front's panel (m x w), in boxes of SB x SB (level
             // kernels), SB x SB/2 and SB/2 x SB (half tiles of the inverse-front kernels)
             const Plan& P = F->dp->plan;
             const size_t nf = P.sn.size();
-            std::vector<CUtensorMap> maps(std::max<size_t>(1, 3 * nf));
+            std::vector<CUtensorMap> maps(solve_map_count(P));
             std::memset(maps.data(), 0, maps.size() * sizeof(CUtensorMap));
             const size_t es = sizeof(T);
             const cuuint32_t boxes[3][2] = {{(cuuint32_t)SB, (cuuint32_t)SB}, {(cuuint32_t)SB, (cuuint32_t)(SB / 2)},
@@ -1188,15 +1225,9 @@ void launch_solve_graph(uchol_factor_s* F, int nrhs, Cv* work, cudaStream_t st) 
                         throw Error(UCHOL_CUDA_ERROR,
                                     "cuTensorMapEncodeTiled failed for a solve tile map: " + std::to_string((int)r));
                 }
-            F->solve_maps.upload(maps, st, "solve tile maps");
+            CK(cudaMemcpyAsync(F->solve_maps.p, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, st));
             CK(cudaStreamSynchronize(st));
-        }
-        if (!F->solve_flags.p) {
-            const Plan& P = F->dp->plan;
-            F->solve_flags.alloc(sizeof(int) * (2 * std::max<size_t>(1, P.inv_blocks.size()) + P.progress_count),
-                                 "solve flags");
-            F->solve_status.alloc(sizeof(int), "solve flags");
-            CK(cudaMemsetAsync(F->solve_status.p, 0, sizeof(int), st));
+            F->solve_maps_made = true;
         }
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(F->capture_stream, cudaStreamCaptureModeThreadLocal));
@@ -1241,6 +1272,7 @@ void ensure_workspace(uchol_factor_s* F, int nrhs);
 // kernel attributes) is that of a one-column solve, made first.
 template <class T, class Cv, int SB>
 void starved_level_launch(uchol_factor_s* F, cudaStream_t st) {
+    ensure_workspace(F, 1);
     DevPlan& D = *F->dp;
     const Plan& P = D.plan;
     const SolveLaunch* Lp = nullptr;
@@ -1252,7 +1284,6 @@ void starved_level_launch(uchol_factor_s* F, cudaStream_t st) {
     if (!Lp)
         throw Error(UCHOL_BAD_ARG, "the factor has no level-solve launch with a chain of three diagonal blocks "
                                    "(use inverse_block_width < 0 and a front wider than three solve blocks)");
-    ensure_workspace(F, 1);
     CK(cudaMemsetAsync(F->work.p, 0, F->work.bytes, st));
     launch_solve_graph<T, Cv, SB>(F, 1, F->work.as<Cv>(), st);   // set-up, and a normal solve of zeros
     CK(cudaStreamSynchronize(st));
@@ -1282,28 +1313,139 @@ void starved_level_launch(uchol_factor_s* F, cudaStream_t st) {
     CK(cudaStreamSynchronize(st));
 }
 
-void ensure_workspace(uchol_factor_s* F, int nrhs) {
+// The solve workspace for nrhs right-hand sides: f(buffer, bytes) for each of its buffers.
+template <class Fn>
+void each_workspace_buffer(uchol_factor_s* F, const Plan& P, int nrhs, Fn f) {
+    const size_t cv = F->elem, n = (size_t)std::max(1, F->sym->n), k = (size_t)nrhs, sb = (size_t)P.cfg.solve_block;
+    f(F->work, n * k * cv);
+    f(F->fv, (size_t)P.fvec_elems * k * cv);
+    f(F->fv2, (size_t)P.fvec_elems * k * cv);
+    f(F->bwd_partial, (size_t)std::max(1, P.bwd_partial_slots) * 8 * k * cv);
+    f(F->inv_partial, (size_t)std::max(1, P.inv_partial_slots) * sb * k * cv);
+    f(F->inv_diag_partial, (size_t)std::max(1, P.inv_diag_slots) * sb * k * cv);
+    f(F->inv_diag_cnt, (size_t)std::max(1, P.inv_diag_slots) * k * sizeof(unsigned));
+    f(F->inv_cols_cnt, (size_t)std::max(1, P.inv_partial_slots) * k * sizeof(unsigned));
+    for (auto& v : F->vec) f(v, n * k * sizeof(double));
+    f(F->scal, (kDotBlocks * k + 16 * k) * sizeof(double));
+}
+// The same for the buffers of the solves that do not depend on nrhs.
+template <class Fn>
+void each_solve_buffer(uchol_factor_s* F, const Plan& P, Fn f) {
+    f(F->solve_maps, solve_map_count(P) * sizeof(CUtensorMap));
+    f(F->solve_flags, sizeof(int) * (2 * std::max<size_t>(1, P.inv_blocks.size()) + P.progress_count));
+    f(F->solve_status, sizeof(int));
+}
+
+void release_workspace(uchol_factor_s* F) {
+    if (F->solve_graph) cudaGraphExecDestroy(F->solve_graph);   // (it holds the buffers' addresses)
+    F->solve_graph = nullptr;
+    F->ws_nrhs = 0;
+    each_workspace_buffer(F, F->dp->plan, 1, [](DBuf& b, size_t) { b.release(); });
+}
+
+void allocate_workspace(uchol_factor_s* F, int nrhs) {
     if (F->ws_nrhs >= nrhs) return;
-    uchol_symbolic_s* S = F->sym;
-    const Plan& P = F->dp->plan;
-    size_t cv = F->precision == UCHOL_PRECISION_FP64 ? 8 : 4;
-    F->work.alloc((size_t)std::max(1, S->n) * nrhs * cv, "solve workspace");
-    F->fv.alloc((size_t)P.fvec_elems * nrhs * cv, "solve workspace");
-    F->fv2.alloc((size_t)P.fvec_elems * nrhs * cv, "solve workspace");
-    F->bwd_partial.alloc((size_t)std::max(1, P.bwd_partial_slots) * 8 * nrhs * cv, "solve workspace");
-    F->inv_partial.alloc((size_t)std::max(1, P.inv_partial_slots) * P.cfg.solve_block * nrhs * cv, "solve workspace");
-    F->inv_diag_partial.alloc((size_t)std::max(1, P.inv_diag_slots) * P.cfg.solve_block * nrhs * cv, "solve workspace");
-    F->inv_diag_cnt.alloc((size_t)std::max(1, P.inv_diag_slots) * nrhs * sizeof(unsigned), "solve workspace");
-    F->inv_cols_cnt.alloc((size_t)std::max(1, P.inv_partial_slots) * nrhs * sizeof(unsigned), "solve workspace");
-    CK(cudaMemsetAsync(F->inv_diag_cnt.p, 0, F->inv_diag_cnt.bytes, S->stream));   // the last chunk resets each
-    CK(cudaMemsetAsync(F->inv_cols_cnt.p, 0, F->inv_cols_cnt.bytes, S->stream));
-    if (F->solve_graph) {
-        CK(cudaGraphExecDestroy(F->solve_graph));
-        F->solve_graph = nullptr;
-    }
-    for (auto& v : F->vec) v.alloc((size_t)std::max(1, S->n) * nrhs * sizeof(double), "refinement vectors");
-    F->scal.alloc((size_t)(kDotBlocks * nrhs + 16 * nrhs) * sizeof(double), "refinement scalars");
+    cudaStream_t st = F->sym->stream;
+    release_workspace(F);
+    each_workspace_buffer(F, F->dp->plan, nrhs, [](DBuf& b, size_t bytes) { b.alloc(bytes, "solve workspace"); });
+    each_solve_buffer(F, F->dp->plan, [](DBuf& b, size_t bytes) {
+        if (!b.p) b.alloc(bytes, "solve workspace");
+    });
+    CK(cudaMemsetAsync(F->inv_diag_cnt.p, 0, F->inv_diag_cnt.bytes, st));   // the last chunk resets each
+    CK(cudaMemsetAsync(F->inv_cols_cnt.p, 0, F->inv_cols_cnt.bytes, st));
+    CK(cudaMemsetAsync(F->solve_status.p, 0, F->solve_status.bytes, st));
     F->ws_nrhs = nrhs;
+}
+
+// Device memory that an allocation of this thread can take.
+int64_t free_device_bytes() {
+    size_t avail = 0, total = 0;
+    CK(cudaMemGetInfo(&avail, &total));
+    return t_alloc_limit < 0 ? (int64_t)avail : std::min((int64_t)avail, t_alloc_limit - t_alloc_held);
+}
+
+// Gives up memory that a factor holds for speed, for `extra` bytes and the workspace of nrhs right-hand sides: the next
+// smaller configuration that leaves room for them takes the factor's place, factorised again from the values it holds.
+// False, with the factor as it was but for its workspace, when there is none.
+bool shrink_factor(uchol_factor_s* F, int nrhs, int64_t extra) {
+    uchol_symbolic_s* S = F->sym;
+    std::lock_guard<std::mutex> lk(S->mu);
+    const PlanConfig old = F->dp->plan.cfg;
+    auto planned = [&](DevPlan& D, bool tables) {   // with the tensor maps and, if asked for, all of the plan's tables
+        const Plan& P = D.plan;
+        return planned_bytes(P, F->precision, S->nnz, S->full_nnz, S->n) - list_bytes(P) +
+               (P.stage_elems > 0 ? (int64_t)(2 * P.map_front.size() * sizeof(CUtensorMap)) : 0) + (tables ? D.table_bytes() : 0);
+    };
+    release_workspace(F);
+    each_solve_buffer(F, F->dp->plan, [](DBuf& b, size_t) { b.release(); });
+    F->solve_maps_made = false;
+    // (two owners: this factor and the analysis, so that the tables leave with it; a page for small buffers)
+    const int64_t room = free_device_bytes() + planned(*F->dp, F->dp.use_count() == 2) + 4096;
+    PlanConfig cfg = old;
+    auto next = [&] {   // the next smaller configuration with room for the solve
+        while (relax_for_budget(cfg, F->opts, S->host_plan(cfg)->plan)) {
+            DevPlan& D = *S->host_plan(cfg);
+            const Plan& P = D.plan;
+            int64_t need = planned(D, !D.uploaded) + extra;
+            auto add = [&](DBuf&, size_t bytes) { need += (int64_t)bytes; };
+            each_workspace_buffer(F, P, nrhs, add);
+            each_solve_buffer(F, P, add);
+            if (need <= room) return true;
+        }
+        return false;
+    };
+    if (!next()) return false;
+    const bool had_failed = F->last.failed_pivot >= 0;
+    CK(cudaStreamSynchronize(S->stream));
+    for (bool restored = false;;) {
+        if (F->factor_graph) cudaGraphExecDestroy(F->factor_graph);
+        F->factor_graph = nullptr;
+        for (DBuf* b : {&F->panel, &F->contrib, &F->stage_a, &F->stage_b, &F->oz_exps, &F->maps, &F->tc_ws, &F->tc_counters,
+                        &F->minv, &F->linv, &F->linv_off, &F->inv_scratch})
+            b->release();
+        if (F->dp) {
+            const PlanConfig left = F->dp->plan.cfg;
+            F->dp.reset();
+            S->unload_plan(left);
+        }
+        try {
+            allocate_buffers(F, cfg);
+            break;
+        } catch (const Error& e) {
+            if (e.code != UCHOL_OOM || restored) {
+                F->dp.reset();   // lost: require_factor refuses every later call
+                throw;
+            }
+            if (next()) continue;
+            cfg = old;   // what the factor had
+            restored = true;
+        }
+    }
+    try {
+        factorize_impl(F, F->values.as<double>(), true);
+    } catch (const Error& e) {
+        if (e.code != UCHOL_NOT_SPD || !had_failed) throw;
+    }
+    return true;
+}
+
+// Runs `allocate` (the workspace of nrhs right-hand sides and `extra` bytes more, of which it keeps nothing when it fails); on
+// a full device once more after each step by which the factor can be made smaller.
+template <class Fn>
+void with_room(uchol_factor_s* F, int nrhs, int64_t extra, Fn allocate) {
+    require_factor(F);
+    for (;;) {
+        try {
+            return allocate();
+        } catch (const Error& e) {
+            if (e.code != UCHOL_OOM) throw;
+            if (!shrink_factor(F, nrhs, extra)) throw;
+        }
+    }
+}
+
+void ensure_workspace(uchol_factor_s* F, int nrhs) {
+    with_room(F, nrhs, 0, [&] { allocate_workspace(F, nrhs); });
 }
 
 // x = A^-1 b through the factor only (device buffers, original order).
@@ -1485,6 +1627,7 @@ int uchol_check_solve_wait(uchol_factor f, double wait_ms) {
         if (!f) throw Error(UCHOL_BAD_ARG, "factor handle is null");
         if (!(wait_ms > 0.0)) throw Error(UCHOL_BAD_ARG, "the wait limit must be positive");
         std::lock_guard<std::mutex> lk(f->mu);
+        require_factor(f);
         cudaStream_t st = f->sym->stream;
         unsigned long long old = kDefaultSolveWaitNs;
         CK(cudaMemcpyFromSymbol(&old, g_solve_wait_ns, sizeof(old)));
@@ -1692,6 +1835,7 @@ int uchol_refactorize(uchol_factor f, const double* values, int on_device, uchol
     return guarded([&] {
         if (!f || (!values && f->sym->nnz > 0)) throw Error(UCHOL_BAD_ARG, "null argument");
         std::lock_guard<std::mutex> lk(f->mu);
+        require_factor(f);
         factorize_impl(f, values, on_device != 0);
         if (stats) *stats = f->last;
     });
@@ -1865,10 +2009,17 @@ int uchol_solve_refined(uchol_factor f, int n, int nrhs, const double* b, int ld
         if (n == 0 || nrhs == 0) return;
         std::lock_guard<std::mutex> lk(f->mu);
         cudaStream_t st = f->sym->stream;
-        ensure_workspace(f, nrhs);
         DBuf db, dx;
-        db.alloc((size_t)n * nrhs * 8, "right-hand sides");
-        dx.alloc((size_t)n * nrhs * 8, "solutions");
+        with_room(f, nrhs, (int64_t)2 * n * nrhs * 8, [&] {
+            allocate_workspace(f, nrhs);
+            try {
+                db.alloc((size_t)n * nrhs * 8, "right-hand sides");
+                dx.alloc((size_t)n * nrhs * 8, "solutions");
+            } catch (...) {
+                db.release();
+                throw;
+            }
+        });
         CK(cudaMemcpy2DAsync(db.p, (size_t)n * 8, b, (size_t)ldb * 8, (size_t)n * 8, nrhs, cudaMemcpyHostToDevice, st));
         int code = UCHOL_OK;
         std::string msg;
