@@ -314,6 +314,8 @@ int uchol_check_diag_panel(int m, int nb, const float* front, double threshold, 
 int uchol_check_diag_panel_rows(int tile_rows, int m, int nb, const float* front, double threshold, double regularization,
                            int allow_regularization, float* l_out, double* d_out, float* w_stage_out,
                            int* counts_out);
+/* uchol_check_reciprocal: out[i] = the FP64 pivots' reciprocal of p[i]. */
+int uchol_check_reciprocal(int n, const double* p, double* out);
 /* uchol_check_digit_update: the FP64 update from 8-bit digits (k_oz_slice + k_oz_gemm), C[i, j] -= sum over the panel
  * columns k in [kbeg, kbeg + kn) of L[i, k] d_k L[j, k], on the columns [c0, cend) of an m-row, w-column front
  * (column-major m x m; unit L in the panel's K columns, pivots d_0 .. d_{w-1}).  kbeg: a multiple of 128; kn: whole

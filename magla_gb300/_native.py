@@ -177,6 +177,7 @@ GPU_SYMBOLS = {
                                          C.c_void_p, C.c_void_p, c_int_p]),
     "uchol_check_diag_panel_rows": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_double, C.c_double, C.c_int, C.c_void_p,
                                          C.c_void_p, C.c_void_p, c_int_p]),
+    "uchol_check_reciprocal": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p]),
     "uchol_check_digit_update": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
                                            C.c_void_p]),
     "uchol_check_plan": (C.c_int, [C.POINTER(SymbolicDesc), C.POINTER(Options), C.c_int, c_int_p]),

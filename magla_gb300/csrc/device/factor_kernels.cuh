@@ -54,8 +54,9 @@ __global__ void k_finish_scale(PivotStats* st, FactorCtl* ctl, double pivot_tole
 }
 
 // 1 / p for p > 0 without a division's FP64 instructions (64 cycles each): the FP32 reciprocal of p's leading bits as
-// x0, then one third-order Newton step, x = x0 + x0 (e + e^2) with e = 1 - p x0.  |e| < 2^-21, so the step's own error
-// is below 2^-63 and x is 1 / p rounded once (0.5003 ulp at most).  p outside 2^+-120 is divided.
+// x0, then one third-order Newton step, x = x0 + x0 (e + e^2) with e = 1 - p x0.  |e| < 2^-22 (2^-23 for the FP32
+// reciprocal's ulp, 2^-23 for the bits of p that it does not see), so the step leaves |e|^3 < 2^-66 and the roundings of e and
+// e + e^2 (each below 2^-74): less than 2^-12 ulp before x is rounded, 0.5003 ulp in all.  p outside 2^+-120 is divided.
 __device__ __forceinline__ double reciprocal(double p) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(p);
     const unsigned e = (unsigned)(b >> 52);

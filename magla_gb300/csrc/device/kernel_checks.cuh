@@ -58,6 +58,11 @@ struct CheckFrontOf {
 
 using CheckFront = CheckFrontOf<float>;
 
+__global__ void k_check_reciprocal(const double* p, double* out, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = reciprocal(p[i]);
+}
+
 // Round to nearest even BF16 (the staging copies' rounding, __floats2bfloat162_rn).
 inline uint16_t to_bf16(float f) {
     uint32_t u;
@@ -237,6 +242,19 @@ int uchol_check_diag_panel_rows(int tile_rows, int m, int nb, const float* front
             counts_out[1] = hs.negative;
             counts_out[2] = hs.failed == INT_MAX ? -1 : hs.failed;
         }
+    });
+}
+
+int uchol_check_reciprocal(int n, const double* p, double* out) {
+    return guarded([&] {
+        if (n <= 0 || !p || !out) throw Error(UCHOL_BAD_ARG, "null argument");
+        DBuf a, b;
+        a.upload(std::vector<double>(p, p + n), nullptr, "check");
+        b.alloc((size_t)n * sizeof(double), "check");
+        k_check_reciprocal<<<(n + 255) / 256, 256>>>(a.as<double>(), b.as<double>(), n);
+        counted();
+        CK(cudaGetLastError());
+        CK(cudaMemcpy(out, b.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost));
     });
 }
 
