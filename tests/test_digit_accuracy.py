@@ -73,3 +73,28 @@ def test_entries_of_graded_rows(gpu_lib, m, w, c0, cend, kbeg, kn, g):
         rms = [float(np.sqrt(np.mean((e[lower] / (size[lower] + 1e-300)) ** 2))) for e in (err, fp64)]
         if lower.sum() > 1000:   # (a mean of enough entries)
             assert rms[0] <= rms[1], rms
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("where", ["row", "column", "pivot"])
+def test_not_finite_entries_reach_their_rows_and_columns_only(gpu_lib, value, where):
+    """A staged entry that is not finite makes its row's and its column's entries of C NaN, a pivot every one; all others are
+    those of the finite front."""
+    m, w, c0, cend, kbeg, kn = 420, 300, 300, 420, 0, 300
+    front, pivots, _ = graded_front(m, w, 0, 8)
+    clean = digit_update(front, pivots, w, c0, cend, kbeg, kn)
+    i, k = (330, 200) if where == "row" else (419, 17)   # in the middle of a tile; the last row, the first chunk
+    if where == "pivot":
+        pivots[k] = value
+    else:
+        front[i, k] = value
+    out = digit_update(front, pivots, w, c0, cend, kbeg, kn)
+    rows, cols = np.tril_indices(m)
+    hit = np.zeros((m, m), bool)
+    updated = (cols >= c0) & (cols < cend)
+    reached = updated & ((rows == i) | (cols == i) | (where == "pivot"))
+    hit[rows[reached], cols[reached]] = True
+    low = np.tril(np.ones((m, m), bool))
+    low[:, :w] = False
+    assert np.all(np.isnan(out[hit])) and hit.sum() > 0
+    assert np.array_equal(out[low & ~hit], clean[low & ~hit])
