@@ -42,6 +42,9 @@ constexpr int kOzStages = 2;
 constexpr int kOzABytes = kOzSlices / 2 * kOzRows * 128, kOzBBytes = kOzSlices / 2 * kOzCols * 128;
 constexpr int kOzThreads = 64 + 256;   // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int kOzNan = 1 << 20;      // row exponent of a chunk with an entry that is not finite
+constexpr int kOzZeroRow = 1023;     // and of one without digits (any value)
+// Two row exponents from kOzLow to kOzHigh put every nonzero integer of the epilogue into the range of normal doubles.
+constexpr int kOzLow = 600, kOzHigh = 1500;
 
 inline size_t oz_smem_bytes() { return 1024 + (size_t)kOzStages * (kOzABytes + kOzBBytes) + 128; }
 
@@ -87,7 +90,7 @@ __global__ void __launch_bounds__(256) k_oz_slice(const PanelTask* __restrict__ 
 #pragma unroll
         for (int side = 0; side < 2; ++side) {   // L, W
             long long b[4];
-            int e[4], E = 0;
+            int e[4], E = -100000, least = 1;
             bool finite = true;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -95,14 +98,30 @@ __global__ void __launch_bounds__(256) k_oz_slice(const PanelTask* __restrict__ 
                 b[q] = __double_as_longlong(side ? l * dk[q] : l);
                 const int raw = (int)((b[q] >> 52) & 0x7ff);
                 finite = finite && raw != 0x7ff;
-                e[q] = raw == 0 ? -100000 : raw + (side ? -scale[q] : scale[q]);
-                E = q == 0 ? e[q] : max(E, e[q]);
+                least = min(least, raw);
+                e[q] = raw + (side ? -scale[q] : scale[q]);
             }
+            if (__any_sync(0xffffffffu, least == 0)) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const long long frac = b[q] & 0xfffffffffffffll;
+                    if (((b[q] >> 52) & 0x7ff) != 0) continue;
+                    if (frac == 0) {
+                        e[q] = -100000;
+                    } else {   // subnormal: its leading bit to 52
+                        const int z = __clzll(frac) - 11;
+                        b[q] = (b[q] & (1ll << 63)) | (frac << z);
+                        e[q] += 1 - z;
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) E = max(E, e[q]);
             for (int o = 16; o > 0; o >>= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
             const bool all_finite = __all_sync(0xffffffffu, finite);
             if (lane == 0)
                 exps[(side ? w_exps : 0) + g.eoff + (long long)(tk.j0 / kOzChunk) * d.ldp + row0 + r] =
-                    !all_finite ? kOzNan : E <= -50000 ? 0 : E;
+                    !all_finite ? kOzNan : E <= -50000 ? kOzZeroRow : E;
             __nv_bfloat16* out = (side ? stage_w : stage_l) + g.off + (long long)(row0 + r) * g.ld +
                                  (long long)(tk.j0 / kOzGroup) * kOzGroupElems + lane;
 #pragma unroll
@@ -124,11 +143,13 @@ __global__ void __launch_bounds__(256) k_oz_slice(const PanelTask* __restrict__ 
 
 __device__ __forceinline__ int oz_int(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }   // an integer's FP32
 
-// The value V 2^(sh) as a double (V a 64-bit integer, rounded once), zero or infinite past the range of doubles.
+// The value V 2^(sh) as a double (V a 64-bit integer, rounded once, and once more if the result is subnormal), zero or
+// infinite past the range of doubles.
 __device__ __forceinline__ double oz_value(long long V, int sh) {
     const long long b = __double_as_longlong((double)V);
     const int e = (int)((b >> 52) & 0x7ff) + sh;
-    if (V == 0 || e <= 0) return 0.0;
+    if (V == 0 || e < -63) return 0.0;
+    if (e <= 0) return __longlong_as_double(b + ((long long)(sh + 64) << 52)) * 0x1p-64;
     return e >= 0x7ff ? __longlong_as_double((b & (1ll << 63)) | 0x7ff0000000000000ll) : __longlong_as_double(b + ((long long)sh << 52));
 }
 
@@ -240,7 +261,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
         bool ok = true;
         for (int c = g0; c < g1 && ok; c += kPerChunk) {
             const long long eo = (long long)(c / kPerChunk) * d.ldp;
-            const int ei = i < d.m ? ex[eo + i] : 0, ejl = jb + lane < d.m ? ex[w_exps + eo + jb + lane] : 0;
+            const int ei = i < d.m ? ex[eo + i] : kOzZeroRow, ejl = jb + lane < d.m ? ex[w_exps + eo + jb + lane] : kOzZeroRow;
+            const bool normal = __all_sync(0xffffffffu, min(ei, ejl) >= kOzLow && max(ei, ejl) <= kOzHigh);
             ok = __all_sync(0xffffffffu, mbar_wait(acc_full, acc_phase));
             if (!ok) {
                 fail();
@@ -249,8 +271,10 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             acc_phase ^= 1;
             tc_fence_after();
             // T = the sum over the orders, in units of order 7: its upper half hi (orders 0 to 3, units of order 3, below
-            // 2^45.1) and its lower half lo (orders 4 to 7, below 2^47.4).  T is held as V 2^(32 - k), V a 64-bit integer:
-            // k, from 16 to 31, leaves hi all the bits of V but the sign and one
+            // 2^45.1) and its lower half lo (orders 4 to 7, below 2^47.4), which carries into hi.  T is held as V 2^(32 - k), V
+            // its leading 64 bits: k, from 17 to 31, shifts out hi's copies of the sign.  This stands between the products
+            // of one chunk and the next, so its instructions count: 64-bit shifts and a rounding here were 2 ms of the
+            // 30^3 elasticity step
             long long V[32];
             unsigned ks[4] = {0u, 0u, 0u, 0u};   // k - 16 of each entry, four bits
 #pragma unroll
@@ -273,23 +297,41 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                 tmem_ld_wait();
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const long long hi = V[8 * h + u];
-                    const long long lo = ((long long)oz_int(r0[u]) * 256 + oz_int(r1[u])) * 65536 +
-                                         ((long long)oz_int(r2[u]) * 256 + oz_int(r3[u]));
-                    const int k = min(31, __clzll(hi ^ (hi >> 63)) - 2);
-                    V[8 * h + u] = (hi << k) + ((lo + (1ll << (31 - k))) >> (32 - k));
-                    ks[h] |= (unsigned)(k - 16) << (4 * u);
+                    const long long lo = (long long)oz_int(r0[u]) * (1 << 24) +
+                                         ((long long)oz_int(r1[u]) * 65536 + ((long long)oz_int(r2[u]) * 256 + oz_int(r3[u])));
+                    const long long hi = V[8 * h + u] + (lo >> 32);
+                    const unsigned w0 = (unsigned)lo, w1 = (unsigned)hi, w2 = (unsigned)(hi >> 32);
+                    unsigned k;   // copies of the sign in w2, less one; 30 if it is nothing else
+                    asm("bfind.shiftamt.s32 %0, %1;" : "=r"(k) : "r"(w2));
+                    k = (k - 1u) & 31u;
+                    V[8 * h + u] = (long long)((unsigned long long)__funnelshift_l(w1, w2, k) << 32 | __funnelshift_l(w0, w1, k));
+                    ks[h] |= (k & 15u) << (4 * u);
                 }
             }
             tc_fence_before();
             mbar_arrive(acc_empty);
+            // V 2^(32 - k) in order 7's unit, 2^(56 - 2 (1075 + 10)) times the rows' powers
+            if (normal) {
 #pragma unroll
-            for (int u = 0; u < 32; ++u) {
-                const int ej = __shfl_sync(0xffffffffu, ejl, u);
-                const int k = 16 + (int)(ks[u / 8] >> (4 * (u % 8)) & 15u);
-                double v = oz_value(V[u], ei + ej - 2114 + (32 - k));   // order 7's unit: 2^(56 - 2 (1075 + 10))
-                if (ei == kOzNan || ej == kOzNan) v = __longlong_as_double(0x7ff8000000000000ll);
-                sum[u] += v;
+                for (int u = 0; u < 32; ++u) {
+                    const int sh = ei + __shfl_sync(0xffffffffu, ejl, u) - 2098 - (int)(ks[u / 8] >> (4 * (u % 8)) & 15u);
+                    const double v = __longlong_as_double(__double_as_longlong((double)V[u]) + ((long long)sh << 52));
+                    sum[u] += V[u] == 0 ? 0.0 : v;
+                }
+            } else {   // a loop over copies: unrolled, this rare form cost the other 0.8 ms of the 30^3 elasticity step
+                long long Vc[32];
+                double vc[32];
+#pragma unroll
+                for (int u = 0; u < 32; ++u) Vc[u] = V[u];
+#pragma unroll 1
+                for (int u = 0; u < 32; ++u) {
+                    const int ej = __shfl_sync(0xffffffffu, ejl, u);
+                    const unsigned kw = u < 8 ? ks[0] : u < 16 ? ks[1] : u < 24 ? ks[2] : ks[3];
+                    vc[u] = ei == kOzNan || ej == kOzNan ? __longlong_as_double(0x7ff8000000000000ll)
+                                                         : oz_value(Vc[u], ei + ej - 2098 - (int)(kw >> (4 * (u % 8)) & 15u));
+                }
+#pragma unroll
+                for (int u = 0; u < 32; ++u) sum[u] += vc[u];
             }
         }
         if (ok && i < d.m) {

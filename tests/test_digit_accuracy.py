@@ -98,3 +98,25 @@ def test_not_finite_entries_reach_their_rows_and_columns_only(gpu_lib, value, wh
     low[:, :w] = False
     assert np.all(np.isnan(out[hit])) and hit.sum() > 0
     assert np.array_equal(out[low & ~hit], clean[low & ~hit])
+
+
+@pytest.mark.parametrize("exponent", [-1000, -1021, -1030])
+def test_subnormal_products(gpu_lib, exponent):
+    """Pivots at the lower end of the range: products l d, and entries of C, that are subnormal count like any others."""
+    m, w, c0, cend, kbeg, kn = 300, 200, 200, 300, 0, 200
+    rng = np.random.default_rng(-exponent)
+    front = np.tril(rng.uniform(-1.0, 1.0, (m, m)) * 2.0 ** exponent)
+    front[:, :w] = np.tril(rng.uniform(0.5, 1.0, (m, w)) * 2.0 ** -rng.integers(0, 30, (m, w)))
+    pivots = rng.uniform(1.0, 2.0, w) * 2.0 ** exponent
+    out = digit_update(front, pivots, w, c0, cend, kbeg, kn)
+    ext = np.longdouble
+    L = front[:, :kn]
+    ref = front.astype(ext) - (L.astype(ext) * pivots) @ L.astype(ext).T
+    size = np.abs(L) @ np.abs(L * pivots).T
+    # the digits' loss (test_entries_of_graded_rows) against rows whose largest entry is at most 1, sqrt(d) being in both, and
+    # roundings to the smallest subnormal: each product l d, each chunk's sum (twice) and addition, the subtraction
+    tiny = 2.0 ** -1074
+    bound = 2 * 2.0 ** (exponent + 1 - 56) + U * (4 * size + np.abs(front) + np.abs(ref).astype(float)) + (kn + 8) * tiny
+    lower = np.tril(np.ones((m, m), bool))
+    lower[:, :c0] = False
+    assert np.all(np.abs((out - ref).astype(float))[lower] <= bound[lower])
