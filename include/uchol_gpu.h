@@ -104,11 +104,18 @@ typedef struct {
                                            FP64) and at most this many columns keep the inverse of their
                                            diagonal block's unit-lower triangle (built after each
                                            factorisation), so that their triangular solves are products
-                                           instead of a chain of block solves.  0 = 8192 on the mixed paths and 2048 in FP64, < 0 = off. */
+                                           instead of a chain of block solves.  0 = 8192 on the mixed
+                                           paths (for refined solves; 2048 is better for fewer than about five
+                                           applications of a factor) and 2048 in FP64, < 0 = off. */
     int64_t device_memory_budget;       /* > 0: a factorisation whose factor, contribution arena, staging,
-                                           inverses and value copies (uchol_estimate_device_bytes) exceed
-                                           this many bytes fails with UCHOL_OOM before any of it is
-                                           allocated; 0 = no budget.  The reference's counterpart is its
+                                           inverses, gather lists and value copies
+                                           (uchol_estimate_device_bytes) exceed this many bytes gives up
+                                           defaults that hold memory for speed (inverses past 2048 columns,
+                                           the inversion's scratch, the gather lists, the FP64 updates'
+                                           digits) and, when that is not enough, fails with UCHOL_OOM before
+                                           any of it is allocated; 0 = no budget (the same steps are taken
+                                           on a full device, also when a solve finds no room for its
+                                           workspace).  The reference's counterpart is its
                                            EstimatePeakBytes (UtduSymbolicFactorization.cs:203-219). */
     int split_min_kblocks;              /* mixed paths: a tensor-core update launch with fewer tiles than SMs is
                                            split in K (stream-K) only when its tiles have at least this many

@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(128) k_trsm(const PanelTask* __restrict__ task
 }
 
 // Update C[i, j] -= sum_k L[i,k] d_k L[j,k] of one TS x TS tile (lower triangle, i >= j), TS = 16 or 32: 2 or 8 us of
-// the SM's FP64 pipe at 32 columns (Launch::tile: 32 once that still makes two CTAs per SM).  Consecutive threads
+// the SM's FP64 pipe at 32 columns (Launch::variant: 32 once that still makes two CTAs per SM).  Consecutive threads
 // hold consecutive rows of C.
 template <int TS>
 __host__ __device__ constexpr int simt_threads() { return 128; }   // a warp per scheduler

@@ -6,7 +6,7 @@
 // Why: the FP64 pipe does two multiply-adds a clock and SM (1.25 TFLOP/s on the GPU); the update is a contraction, and
 // 36 exact digit products at 1.9 PFLOP/s are worth 40 times that.  What bounds it: an SM's shared-memory path (a
 // 128 x 64 tile reads 6 KB per 16-deep product) and the accumulators' read-out.  30^3 elasticity, 5.4e11 operations:
-// 500 ms on the FP64 pipe (1.07 TFLOP/s), 33 ms here.
+// 500 ms on the FP64 pipe (1.07 TFLOP/s), 32.6 ms here.
 //
 // Slices.  Column k of L is scaled by 2^s and of W by 2^-s, s about log2(d_k) / 2 (exact; both are then of the size of
 // L sqrt(D), so that no column of the chunk is small in one and large in the other).  For each row i of either and chunk

@@ -2,12 +2,15 @@
 // every large front of a level, once the block has received the updates of
 // all earlier columns of its supernode:
 //
-//   k_diag_block   one CTA per front: A11 = L11 D L11^T in FP32 shared memory
-//                  (32-column sub-blocks: a register-resident warp LDL^T
-//                  that also yields the sub-block's inverse, the rows below
-//                  by a small product with that inverse, a rank-32 trailing
-//                  update), then X = L11^{-1}.  Writes L11
-//                  and D to the factor, X^T, D and D^{-1} to a workspace slot.
+//   k_diag_block   one CTA per front: A11 = L11 D L11^T in FP32 shared memory, a
+//                  role per warp over 32-column sub-blocks (the chain of pivots,
+//                  the elimination of the rows below and of the identity, which
+//                  becomes X^T = L11^{-T}, the FP64 pivots, the updates).  Writes
+//                  L11 and D to the factor, D and D^{-1} to a workspace slot, and
+//                  X^T to the solves' inverse of the block (PanelTask::inv) or,
+//                  where the solves' blocks are others, to the slot.  A block with
+//                  a pivot that the chain does not decide is done again by
+//                  diag_block_exact, pivot by pivot in FP64.
 //   k_panel_solve  128 or 64 rows per CTA: W21 = A21 X^T as an FP32 register-tiled
 //                  GEMM, L21 = W21 D^{-1}; L21 goes to the factor and, K-major,
 //                  W21 and L21 go to the staging operands of the tensor-core

@@ -76,7 +76,6 @@ double job_flops(const UpdJob& J, const SnDev& d) {
     return 2.0 * J.kn * entries;
 }
 
-// Tile count of an update job (must match decode_tile).
 // Rows of the tiles of the tensor-core launch of jobs jb and after, whose tiles of kTcRows rows are counted in `tiles`:
 // the fewest that keep the launch within one tile an SM (its tiles are counted anew then).  A small tile's time is its
 // operands' way to the SM and its epilogue, both nearly proportional to its rows: an outer block's own update takes
@@ -113,6 +112,7 @@ int panel_rows(const Plan& P, const std::vector<int>& large, int k0, int NB, int
     return n <= sms ? 64 : 128;
 }
 
+// Tile count of an update job (must match decode_tile).
 long long job_tiles(const UpdJob& J, const SnDev& d, int T) {
     auto region = [&](int base, int lim) -> long long {
         if (lim <= base) return 0;

@@ -19,8 +19,13 @@ constexpr int kColRowsPlan64 = 1024; // and FP64
 constexpr int kInvColRowsPlan = 1024;   // trailing rows per backward partial-sum task of an inverse front
 // Widest front whose diagonal block is kept inverted for the solves.  The inverse costs w^3 / 3 operations per
 // factorisation and saves a chain of w / SB block solves (about 9 us each in the mixed path) per solve and direction.
-// FP32 at 8192 columns: 3.4 ms against 1.1 ms per application of the factor, of which a refined solve makes two at least
-// (40^3 contrast, eight steps: 62.5 -> 58.0 ms; 30^3 BF16 78.1 -> 76.2).  FP64, where the pipe does 1.2 TFLOP/s and one
+// FP32, factorisation / one application of the factor to 1, 4 and 16 right-hand sides in ms, by the widest inverse:
+//   40^3 elasticity, contrast 1e4   2048: 27.6 / 3.22 7.47 10.5   4096: 28.6 / 2.87 6.26 8.99   8192: 33.6 / 2.02 3.72 6.08
+//   30^3 elasticity, BF16           2048: 38.4 / 4.16 9.67 12.6   4096: 39.2 / 3.93 9.00 11.8   8192: 40.4 / 3.65 8.09 10.7
+//                                   16384: 66.3 / 2.28 4.01 6.23
+// 8192 pays from five applications a factorisation on with one right-hand side and from two with several; refined solves
+// make five to ten (40^3 contrast 62.5 -> 58.0 ms a step, 30^3 BF16 78.1 -> 76.2).  16384 would take nineteen.  A caller of
+// fewer applications sets the option to 2048 (40^3, one: 30.8 ms against 35.6).  FP64, where the pipe does 1.2 TFLOP/s and one
 // application is usual: 4096 columns cost 20 ms more on 30^3 elasticity (84 -> 105 ms).
 constexpr int kDefaultInvCols = 8192;     // mixed path
 constexpr int kDefaultInvCols64 = 2048;   // FP64
@@ -125,12 +130,19 @@ struct SolveLaunch {
 // blk is the diagonal-inverse index of the front's block 0.
 //
 // Inverse fronts read the children's and the ancestors' entries inside their kernels and the last chunk of a column
-// block adds its partial sums; a level then has four launches, not seven, which bounds chains of small fronts (FP64: 20^3
-// elasticity 1.02 -> 0.97 ms a solve, 24^3 x 3 grid with 33 right-hand sides 7.53 -> 7.16 ms).  Every block row and
-// column of a front reads the entries again, and with several right-hand sides that costs more in fronts of more than
-// kGatherRows rows than the launches (60 x 60 x 30 elasticity, 16 right-hand sides: 401 ms with them, 423 ms without);
-// their vectors are gathered and reduced by launches of their own.  One right-hand side gains there too (40^3 elasticity,
-// contrast 1e4: 53.2 -> 52.6 ms; 30^3 BF16 70.3 -> 69.8 ms), so those launches are left out of its solves.
+// block adds its partial sums; a level then has four launches, not seven, which bounds chains of small fronts (24^3 x 3
+// grid, FP64, 33 right-hand sides: 7.53 -> 7.16 ms; 20^3 elasticity with one is the same within its noise, 1.02 ms).  Every
+// block row and column of a front reads the entries again, which costs more the wider the front is and the more right-hand
+// sides there are; fronts of more than kGatherRows rows are gathered and reduced by launches of their own.  One application
+// in ms with those launches for every front / as here / for none, by right-hand sides:
+//   60 x 60 x 30 elasticity, natural order   2: 27.2 / 27.2 / 25.4   4: 28.6 / 28.6 / 27.9   8: 29.8 / 29.9 / 32.2   16: 32.7 / 32.9 / 37.4
+//   40 x 40 x 20 elasticity, natural order   2: 12.7 / 12.7 / 11.4   8: 14.0 / 14.1 / 16.2   16: 14.9 / 15.0 / 18.7
+//   30^3 elasticity, AMD                     2: 2.03 / 1.99 / 1.91   4: 2.25 / 2.24 / 2.19   8: 2.56 / 2.64 / 2.64   16: 3.17 / 3.33 / 3.38
+// (2048 rows: as the first on the natural orders, as here on 30^3; 8192: as the last, but 27.1, 28.6, 30.1 and 33.2 on the
+// first mesh.)  So 4096 is within 5% of the better side from 8 right-hand sides on and gives up 4 to 11% at 2: the number of
+// right-hand sides matters more than the rows.
+// One right-hand side gains without them (40^3 elasticity, contrast 1e4: 53.2 -> 52.6 ms; 30^3 BF16 70.3 -> 69.8 ms), so
+// its solves leave those launches out.
 constexpr int kGatherRows = 4096;
 
 struct InvLaunch {

@@ -62,7 +62,8 @@ class UtduSolverOptions:
         self.SmallFrontBuckets = 0   # bit b: fronts of 32b < m <= 32(b+1) rows are factorised whole (0 = 0x7)
         self.ChainMergeWidth = 0     # widest device front grouped from a chain of supernodes (0 = 2048, < 0 = off)
         self.InverseBlockWidth = 0   # widest front whose diagonal block is kept inverted for the solves (0 = 8192, 2048 in FP64; < 0 = off)
-        self.DeviceMemoryBudget = 0  # bytes; > 0: factorisations needing more fail with OOM before allocating
+        # bytes; > 0: factorisations needing more give up defaults that hold memory for speed, then fail with OOM
+        self.DeviceMemoryBudget = 0
         # reduced precision breaks down (a pivot regularised or not finite): factorise again in the
         # next higher precision, BF16 -> TF32 -> FP64
         self.PrecisionFallback = True
