@@ -321,11 +321,6 @@ struct uchol_factor_s {
     std::mutex mu;
 };
 
-// Refuses a factor that a full device has cost its buffers (shrink_factor).
-void require_factor(uchol_factor_s* F) {
-    if (!F->dp) throw Error(UCHOL_OOM, "the factor was lost when the device's memory ran out; factorise again");
-}
-
 // Drops one reference; the last one frees the symbolic object and its own stream.
 void symbolic_release(uchol_symbolic_s* s) {
     if (s->refs.fetch_sub(1) != 1) return;
@@ -1364,6 +1359,29 @@ int64_t free_device_bytes() {
     return t_alloc_limit < 0 ? (int64_t)avail : std::min((int64_t)avail, t_alloc_limit - t_alloc_held);
 }
 
+// Every buffer that allocate_buffers makes but the values' and the results', the graph of them, and the plan's hold.
+void release_buffers(uchol_factor_s* F) {
+    if (F->factor_graph) cudaGraphExecDestroy(F->factor_graph);
+    F->factor_graph = nullptr;
+    for (DBuf* b : {&F->panel, &F->contrib, &F->stage_a, &F->stage_b, &F->oz_exps, &F->maps, &F->tc_ws, &F->tc_counters,
+                    &F->minv, &F->linv, &F->linv_off, &F->inv_scratch})
+        b->release();
+    if (!F->dp) return;
+    const PlanConfig left = F->dp->plan.cfg;
+    F->dp.reset();
+    F->sym->unload_plan(left);
+}
+
+// Factorises from the values that the factor holds.
+void factorize_again(uchol_factor_s* F) {
+    const bool had_failed = F->last.failed_pivot >= 0;
+    try {
+        factorize_impl(F, F->values.as<double>(), true);
+    } catch (const Error& e) {
+        if (e.code != UCHOL_NOT_SPD || !had_failed) throw;
+    }
+}
+
 // Gives up memory that a factor holds for speed, for `extra` bytes and the workspace of nrhs right-hand sides: the next
 // smaller configuration that leaves room for them takes the factor's place, factorised again from the values it holds.
 // False, with the factor as it was but for its workspace, when there is none.
@@ -1395,25 +1413,15 @@ bool shrink_factor(uchol_factor_s* F, int nrhs, int64_t extra) {
         return false;
     };
     if (!next()) return false;
-    const bool had_failed = F->last.failed_pivot >= 0;
     CK(cudaStreamSynchronize(S->stream));
     for (bool restored = false;;) {
-        if (F->factor_graph) cudaGraphExecDestroy(F->factor_graph);
-        F->factor_graph = nullptr;
-        for (DBuf* b : {&F->panel, &F->contrib, &F->stage_a, &F->stage_b, &F->oz_exps, &F->maps, &F->tc_ws, &F->tc_counters,
-                        &F->minv, &F->linv, &F->linv_off, &F->inv_scratch})
-            b->release();
-        if (F->dp) {
-            const PlanConfig left = F->dp->plan.cfg;
-            F->dp.reset();
-            S->unload_plan(left);
-        }
+        release_buffers(F);
         try {
             allocate_buffers(F, cfg);
             break;
         } catch (const Error& e) {
             if (e.code != UCHOL_OOM || restored) {
-                F->dp.reset();   // lost: require_factor refuses every later call
+                release_buffers(F);   // restore_factor tries again at the next call
                 throw;
             }
             if (next()) continue;
@@ -1421,19 +1429,35 @@ bool shrink_factor(uchol_factor_s* F, int nrhs, int64_t extra) {
             restored = true;
         }
     }
-    try {
-        factorize_impl(F, F->values.as<double>(), true);
-    } catch (const Error& e) {
-        if (e.code != UCHOL_NOT_SPD || !had_failed) throw;
-    }
+    factorize_again(F);
     return true;
+}
+
+// A factor that a full device has left without buffers (shrink_factor, when others took what it gave up) is made again from
+// the values it holds, or refused while there is no room for it.
+void restore_factor(uchol_factor_s* F) {
+    if (F->dp) return;
+    uchol_symbolic_s* S = F->sym;
+    std::lock_guard<std::mutex> lk(S->mu);
+    PlanConfig cfg = config_for(F->opts);
+    cfg.sms = F->sms;
+    for (;;) {
+        try {
+            allocate_buffers(F, cfg);
+            break;
+        } catch (const Error& e) {
+            release_buffers(F);
+            if (e.code != UCHOL_OOM || !relax_for_budget(cfg, F->opts, S->host_plan(cfg)->plan)) throw;
+        }
+    }
+    factorize_again(F);
 }
 
 // Runs `allocate` (the workspace of nrhs right-hand sides and `extra` bytes more, of which it keeps nothing when it fails); on
 // a full device once more after each step by which the factor can be made smaller.
 template <class Fn>
 void with_room(uchol_factor_s* F, int nrhs, int64_t extra, Fn allocate) {
-    require_factor(F);
+    restore_factor(F);
     for (;;) {
         try {
             return allocate();
@@ -1627,7 +1651,7 @@ int uchol_check_solve_wait(uchol_factor f, double wait_ms) {
         if (!f) throw Error(UCHOL_BAD_ARG, "factor handle is null");
         if (!(wait_ms > 0.0)) throw Error(UCHOL_BAD_ARG, "the wait limit must be positive");
         std::lock_guard<std::mutex> lk(f->mu);
-        require_factor(f);
+        restore_factor(f);
         cudaStream_t st = f->sym->stream;
         unsigned long long old = kDefaultSolveWaitNs;
         CK(cudaMemcpyFromSymbol(&old, g_solve_wait_ns, sizeof(old)));
@@ -1835,7 +1859,7 @@ int uchol_refactorize(uchol_factor f, const double* values, int on_device, uchol
     return guarded([&] {
         if (!f || (!values && f->sym->nnz > 0)) throw Error(UCHOL_BAD_ARG, "null argument");
         std::lock_guard<std::mutex> lk(f->mu);
-        require_factor(f);
+        restore_factor(f);
         factorize_impl(f, values, on_device != 0);
         if (stats) *stats = f->last;
     });

@@ -889,7 +889,7 @@ int uchol_refactorize_dmatrix(uchol_factor f, uchol_dmatrix m, uchol_factor_stat
         if (m->n != S->n || m->nnz != S->nnz)
             throw Error(UCHOL_PATTERN_MISMATCH, "the matrix does not have the structure of the symbolic factorization");
         std::lock_guard<std::mutex> lk(f->mu);
-        require_factor(f);
+        restore_factor(f);
         std::lock_guard<std::mutex> lm(m->mu);
         if (m->checked_symbolic != (const void*)S) {
             if (m->row_ptr != S->row_ptr || m->col != S->col)

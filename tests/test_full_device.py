@@ -146,3 +146,26 @@ def test_a_solve_that_does_not_fit_leaves_the_factor(limit, kw):
             assert np.array_equal(x, y)
     limit(-1)
     assert np.array_equal(y, s.Factorize(m, sym)._apply(b[:, :17]))
+
+
+def test_a_factor_that_cannot_be_put_back_waits_for_room(limit):
+    """The memory that the factor gives up goes to others (here: was not counted), so that neither a smaller factor nor the
+    one before can be allocated: calls are refused while there is no room, and answered once there is."""
+    m = dense(1300)
+    s = solver()
+    b = np.asfortranarray(np.random.default_rng(5).uniform(-1.0, 1.0, (1300, 50)))
+    sym = s.Analyze(m)
+    f, g, h = (s.Factorize(m, sym) for _ in range(3))
+    x = g._apply(b)
+    d = f.Diagonal.copy()
+    limit(1 << 20)
+    for call in (lambda: f._apply(b), lambda: f._apply(b[:, 0]), lambda: f.SolveRefined(b), lambda: f.DeviceResidualNorms(b, b),
+                 lambda: f.Refactorize(m), lambda: h._apply(b)):
+        with pytest.raises(DeviceOutOfMemoryError):
+            call()
+    assert np.array_equal(f.Diagonal, d)
+    limit(-1)
+    assert np.array_equal(f._apply(b), x)
+    h.Refactorize(m)
+    assert np.array_equal(h._apply(b), x)
+    assert np.array_equal(g._apply(b), x)
